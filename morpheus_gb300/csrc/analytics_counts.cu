@@ -63,7 +63,7 @@ __global__ void csr_diag_counts(const int32_t* __restrict__ ro, const int32_t* _
   for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nrows; r += warps) {
     for (int32_t j = ro[r] + lane; j < ro[r + 1]; j += 32) {
       const int64_t c = ci[j];
-      if (c >= 0 && c < ncols) prim::hist_add(h, out, (unsigned long long)(c - r + nrows - 1));
+      if (c >= 0 && c < ncols) prim::hist_add(h, out, (uint64_t)(c - r + nrows - 1));
     }
   }
   __syncthreads();
@@ -78,7 +78,7 @@ __global__ void coo_diag_counts(const int32_t* __restrict__ ri, const int32_t* _
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nnz; k += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = ri[k], c = ci[k];
     if (r >= 0 && r < nrows && c >= 0 && c < ncols)
-      prim::hist_add(h, out, (unsigned long long)(c - r + nrows - 1));
+      prim::hist_add(h, out, (uint64_t)(c - r + nrows - 1));
   }
   __syncthreads();
   prim::hist_flush(h, out);
@@ -171,7 +171,7 @@ __global__ void ell_diag_counts(const int32_t* __restrict__ ci, const T* __restr
     for (int64_t n = 0; n < k; n++) {
       const int64_t c = __ldg(ci + r + pitch * n);
       if (c != MGB_INVALID_INDEX && __ldg(v + r + pitch * n) != T(0) && c >= 0 && c < ncols)
-        prim::hist_add(h, out, (unsigned long long)(c - r + nrows - 1));
+        prim::hist_add(h, out, (uint64_t)(c - r + nrows - 1));
     }
   }
   __syncthreads();

@@ -123,7 +123,7 @@ __global__ void histogram_kernel(const int32_t* __restrict__ keys, int64_t n, in
   __syncthreads();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int32_t k = keys[i];
-    if (k >= 0 && k < nbins) hist_add(h, counts, (unsigned long long)k);
+    if (k >= 0 && k < nbins) hist_add<true>(h, counts, (uint64_t)k);
   }
   __syncthreads();
   hist_flush(h, counts);
