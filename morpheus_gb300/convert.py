@@ -23,7 +23,7 @@ from . import _lib
 from .algorithms import _stream_handle, _suffix
 from .containers import (COO_FORMAT, CSR_FORMAT, DIA_FORMAT, ELL_FORMAT, HDC_FORMAT, HYB_FORMAT, NFORMATS,
                          CooMatrix, CsrMatrix, DiaMatrix, DynamicMatrix, EllMatrix, HdcMatrix, HybMatrix,
-                         _Matrix, conversion_error_e, formats_e)
+                         _Matrix, conversion_error_e, formats_e, get_pad_size)
 from .exceptions import MorpheusException, NotImplementedException
 
 _NAME = {COO_FORMAT: "coo", CSR_FORMAT: "csr", DIA_FORMAT: "dia", ELL_FORMAT: "ell", HYB_FORMAT: "hyb",
@@ -37,6 +37,10 @@ def _dev_check(A: _Matrix) -> None:
 
 def _call(name, *args):
     _lib.call(name, *args)
+
+
+def _empty(n, dtype, device) -> torch.Tensor:
+    return torch.empty(int(n), dtype=dtype, device=device)
 
 
 def _i64():
@@ -73,7 +77,9 @@ def from_coo(coo: CooMatrix, fmt: int, hyb_width: int = 0, stream=None) -> _Matr
     elif fmt == DIA_FORMAT:
         nd = _i64()
         _call("mgb_convert_coo_to_dia_plan", C.byref(sd), C.byref(nd), sh)
-        out = DiaMatrix(n, m, z, nd.value, dtype=dt, device=dev)
+        # the conversion writes every offset and slab value: nothing to clear
+        out = DiaMatrix(n, m, z, nd.value, diagonal_offsets=_empty(nd.value, torch.int32, dev),
+                        values=_empty(get_pad_size(n, 32) * nd.value, dt, dev), dtype=dt, device=dev)
     elif fmt == ELL_FORMAT:
         w = _i64()
         _call("mgb_convert_coo_to_ell_plan", C.byref(sd), C.byref(w), sh)
@@ -157,4 +163,3 @@ def is_sorted(A: CooMatrix, stream=None) -> bool:
 
 
 __all__ = ["convert", "convert_inplace", "to_coo", "from_coo", "sort_by_row_and_column", "is_sorted"]
-_ = torch

@@ -13,6 +13,7 @@
 // reference's fill-tolerance test (impl/Morpheus_Utils.hpp:91-105, in FP32).
 #include <algorithm>
 #include <climits>
+#include <cstdint>
 #include <vector>
 
 #include "primitives.cuh"
@@ -48,52 +49,16 @@ int fill(T* p, T v, int64_t n, cudaStream_t s) {
   return MGB_SUCCESS;
 }
 
-// min index whose row is out of [0, nrows) (or n), via atomicMin
-__global__ void first_bad_row(const int32_t* __restrict__ r, int64_t n, int64_t nrows, unsigned long long* out) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    if (r[i] < 0 || r[i] >= nrows) atomicMin(out, (unsigned long long)i);
-}
-__global__ void first_bad_col(const int32_t* __restrict__ c, int64_t n, int64_t ncols, unsigned long long* out) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    if (c[i] < 0 || c[i] >= ncols) atomicMin(out, (unsigned long long)i);
-}
+using prim::Words;
+using prim::words_alloc;
+using prim::words_read;
 
-// Device words an entry point reads back with one copy and one stream
-// synchronisation: the validation result, the plan's sizes and the
-// sortedness flags, computed by kernels queued one after another.
-struct Words {
-  unsigned long long bad_row, bad_col;  // first index out of range (~0: none)
-  int64_t total, total2;                // plan sizes
-  int32_t sorted, dup, maxv, pad;
-};
-
-int words_alloc(Scratch& sc, Words** d, cudaStream_t s) {
-  MGB_SCRATCH(sc, *d, 1);
-  MGB_CUDA_CHECK(cudaMemsetAsync(*d, 0xff, 2 * sizeof(unsigned long long), s));
-  MGB_CUDA_CHECK(cudaMemsetAsync(&(*d)->total, 0, sizeof(Words) - 2 * sizeof(unsigned long long), s));
-  return MGB_SUCCESS;
-}
-
-int words_read(const Words* d, Words* h, cudaStream_t s) {
-  MGB_CUDA_CHECK(cudaMemcpyAsync(h, d, sizeof(Words), cudaMemcpyDeviceToHost, s));
-  MGB_CUDA_CHECK(cudaStreamSynchronize(s));
-  return MGB_SUCCESS;
-}
-
-// MGB_ERR_INVALID_INPUT (read by the caller with its other words) if any row
-// is outside [0, nrows) or column outside [0, ncols): the reference has no
-// check and indexes out of bounds there.  Queued without a synchronisation.
-int validate_async(const int32_t* rows, const int32_t* cols, int64_t n, int64_t nrows, int64_t ncols, Words* d,
-                   cudaStream_t s) {
-  if (n <= 0) return MGB_SUCCESS;
-  first_bad_row<<<grid_for(n), 256, 0, s>>>(rows, n, nrows, &d->bad_row);
-  MGB_LAUNCH_CHECK();
-  first_bad_col<<<grid_for(n), 256, 0, s>>>(cols, n, ncols, &d->bad_col);
-  MGB_LAUNCH_CHECK();
-  return MGB_SUCCESS;
-}
-
-inline bool words_valid(const Words& h) { return h.bad_row == ~0ull && h.bad_col == ~0ull; }
+// MGB_ERR_INVALID_INPUT if any row is outside [0, nrows) or column outside
+// [0, ncols): the reference has no check and indexes out of bounds there.
+inline bool words_valid(const Words& h) { return (h.seen & prim::COO_BAD_INDEX) == 0; }
+inline bool words_rows_sorted(const Words& h) { return (h.seen & prim::COO_ROWS_UNSORTED) == 0; }
+// sorted by (row, column) without equal pairs: no two entries share a place
+inline bool words_distinct(const Words& h) { return (h.seen & (prim::COO_UNSORTED | prim::COO_DUPLICATE)) == 0; }
 
 int sorted_and_dup(const int32_t* r, const int32_t* c, int64_t n, bool* sorted, bool* dup, cudaStream_t s) {
   Scratch sc(s);
@@ -199,12 +164,8 @@ int coo_to_csr(const mgb_coo* src, mgb_csr* dst, cudaStream_t s) {
   Words* dw;
   int st = words_alloc(sc, &dw, s);
   if (st) return st;
-  st = validate_async(src->row_indices, src->column_indices, n, N, src->ncols, dw, s);
+  st = prim::coo_pass(src->row_indices, src->column_indices, n, N, src->ncols, dw, nullptr, nullptr, s);
   if (st) return st;
-  if (n > 0) {
-    st = prim::rows_sorted_flag(src->row_indices, n, &dw->sorted, s);
-    if (st) return st;
-  }
   Words hw;
   st = words_read(dw, &hw, s);
   if (st) return st;
@@ -216,7 +177,7 @@ int coo_to_csr(const mgb_coo* src, mgb_csr* dst, cudaStream_t s) {
   MGB_CUDA_CHECK(cudaMemsetAsync(counts + N, 0, sizeof(int32_t), s));
   st = prim::exclusive_scan<int32_t, int32_t>(counts, dst->row_offsets, N + 1, s);
   if (st || n == 0) return st;
-  if (hw.sorted) {
+  if (words_rows_sorted(hw)) {
     MGB_CUDA_CHECK(cudaMemcpyAsync(dst->column_indices, src->column_indices, sizeof(int32_t) * n,
                                    cudaMemcpyDeviceToDevice, s));
     MGB_CUDA_CHECK(cudaMemcpyAsync(dst->values, src->values, sizeof(T) * n, cudaMemcpyDeviceToDevice, s));
@@ -314,44 +275,161 @@ int dia_to_coo(const mgb_dia* src, mgb_coo* dst, cudaStream_t s) {
 
 // ---------------------------------------------------------------- COO -> DIA
 // impl/Dia/Serial/Morpheus_Convert_Impl.hpp:120-169
-__global__ void diag_bins(const int32_t* __restrict__ r, const int32_t* __restrict__ c, int64_t n, int64_t nrows,
-                          int32_t* bins) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    bins[i] = (int32_t)((int64_t)c[i] - r[i] + nrows - 1);
-}
-__global__ void nonzero_flags(const int32_t* __restrict__ a, int64_t n, uint8_t* f) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    f[i] = a[i] != 0;
-}
-__global__ void bins_to_offsets(const uint8_t* __restrict__ f, const int32_t* __restrict__ slot, int64_t nb,
-                                int64_t nrows, int32_t* offs) {
-  for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += (int64_t)gridDim.x * blockDim.x)
-    if (f[b]) offs[slot[b]] = (int32_t)(b - nrows + 1);
-}
 
 // place values(row, slot) = v; owner != nullptr resolves collisions to the
 // highest COO position (the reference's loop order: last write wins)
 template <typename T>
-__global__ void dia_place(const int32_t* __restrict__ r, const int32_t* __restrict__ bins, const T* __restrict__ v,
-                          int64_t n, const int32_t* __restrict__ slot, int64_t pitch, T* vals, int32_t* owner,
-                          int pass) {
+__global__ void dia_place(const int32_t* __restrict__ r, const int32_t* __restrict__ c, const T* __restrict__ v,
+                          int64_t n, int64_t nrows, const int32_t* __restrict__ slot, int64_t pitch, T* vals,
+                          int32_t* owner, int pass) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t at = r[i] + pitch * (int64_t)slot[bins[i]];
+    const int64_t at = r[i] + pitch * (int64_t)slot[(int64_t)c[i] - r[i] + nrows - 1];
     if (owner == nullptr) vals[at] = v[i];
     else if (pass == 0) atomicMax(owner + at, (int32_t)i);
     else if (owner[at] == (int32_t)i) vals[at] = v[i];
   }
 }
 
-int diag_histogram(const mgb_coo* src, int32_t** bins, int32_t** counts, Scratch& sc, cudaStream_t s) {
-  const int64_t nb = src->nrows + src->ncols - 1;
-  MGB_SCRATCH(sc, *bins, src->nnz);
-  MGB_SCRATCH(sc, *counts, nb > 0 ? nb : 1);
-  if (src->nnz) {
-    diag_bins<<<grid_for(src->nnz), 256, 0, s>>>(src->row_indices, src->column_indices, src->nnz, src->nrows, *bins);
-    MGB_LAUNCH_CHECK();
+// ---- slabs from row-sorted entries, tile by tile
+//
+// A CTA owns R consecutive rows of D diagonals at a time: the rows' entries
+// (one contiguous range) go through shared memory to their (diagonal, row)
+// place, and the tile is written column by column, padding included, in
+// consecutive rows.  So every value of the slab is written once, in full
+// sectors, and nothing is cleared before.  Placing each entry with its own
+// 8-byte store into a cleared slab took 2,012 us on the 27-point stencil at
+// 160^3 (HBM 35 %; the entries, the slab and the row starts once are 400 us
+// at the copy rate).  The tile's rows are padded to an odd stride: the
+// entries of a row go to different banks.  Diagonals are looked up in a table
+// in shared memory while they are few (DIA_HASH_DIAGS), else in the bin ->
+// slot array.
+constexpr int DIA_TILE_THREADS = 256;
+constexpr int DIA_TILE_BYTES = 32 * 1024;
+constexpr int DIA_HASH_DIAGS = 256;  // at most a quarter of the table's slots
+constexpr int DIA_HASH_SLOTS = 1024;
+constexpr int32_t DIA_HASH_FREE = INT32_MIN;  // no offset: |offset| < 2^31 - 1
+
+struct DiaTable {
+  int32_t *key, *slot;  // diagonal offset (DIA_HASH_FREE: none) and its slot
+};
+__device__ __forceinline__ unsigned dia_hash(int32_t d) {
+  return (((uint32_t)d * 0x9E3779B1u) >> 16) & (DIA_HASH_SLOTS - 1);
+}
+
+// every thread; the caller synchronises.  Equal offsets keep the lowest slot.
+__device__ __forceinline__ void dia_table_clear(DiaTable t) {
+  for (int i = threadIdx.x; i < DIA_HASH_SLOTS; i += blockDim.x) {
+    t.key[i] = DIA_HASH_FREE;
+    t.slot[i] = INT32_MAX;
   }
-  return prim::histogram(*bins, src->nnz, *counts, nb, s);
+}
+__device__ __forceinline__ void dia_table_fill(DiaTable t, const int32_t* __restrict__ offs, int nd) {
+  for (int k = threadIdx.x; k < nd; k += blockDim.x) {
+    const int32_t d = offs[k];
+    unsigned h = dia_hash(d);
+    for (int p = 0; p < DIA_HASH_SLOTS; p++) {
+      const int32_t was = atomicCAS(t.key + h, DIA_HASH_FREE, d);
+      if (was == DIA_HASH_FREE || was == d) break;
+      h = (h + 1) & (DIA_HASH_SLOTS - 1);
+    }
+    atomicMin(t.slot + h, k);
+  }
+}
+__device__ __forceinline__ int dia_table_find(DiaTable t, int32_t d) {
+  unsigned h = dia_hash(d);
+  int32_t k;
+  while ((k = t.key[h]) != d) {
+    if (k == DIA_HASH_FREE) return -1;
+    h = (h + 1) & (DIA_HASH_SLOTS - 1);
+  }
+  return t.slot[h];
+}
+
+template <typename T>
+__global__ void __launch_bounds__(DIA_TILE_THREADS)
+dia_fill_tiles(const int32_t* __restrict__ r, const int32_t* __restrict__ c, const T* __restrict__ v,
+               const int32_t* __restrict__ start, int64_t nrows, int64_t pitch, int nd,
+               const int32_t* __restrict__ offs, const int32_t* __restrict__ bin_slot, T* __restrict__ out, int R,
+               int D) {
+  extern __shared__ __align__(16) unsigned char dia_smem[];
+  T* tile = reinterpret_cast<T*>(dia_smem);
+  __shared__ int32_t h_key[DIA_HASH_SLOTS], h_slot[DIA_HASH_SLOTS];
+  const DiaTable table{h_key, h_slot};
+  const bool hashed = nd <= DIA_HASH_DIAGS;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, S = R + 1;
+  if (hashed) dia_table_clear(table);
+  for (int i = threadIdx.x; i < D * S; i += DIA_TILE_THREADS) tile[i] = T(0);
+  __syncthreads();
+  if (hashed) dia_table_fill(table, offs, nd);
+  __syncthreads();
+  const int64_t ntiles = (pitch + R - 1) / R;
+  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const int64_t r0 = t * R;
+    const int32_t e0 = start[min(r0, nrows)], e1 = start[min(r0 + R, nrows)];
+    for (int d0 = 0; d0 < nd; d0 += D) {
+      const int dn = min(D, nd - d0);
+      for (int64_t e = (int64_t)e0 + threadIdx.x; e < e1; e += 4 * DIA_TILE_THREADS) {
+        int32_t row[4], col[4];
+        T val[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const int64_t i = e + k * DIA_TILE_THREADS;
+          if (i < e1) {
+            row[k] = __ldcs(r + i);
+            col[k] = __ldcs(c + i);
+            val[k] = __ldcs(v + i);
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          if (e + k * DIA_TILE_THREADS < e1) {
+            const int32_t d = col[k] - row[k];
+            const int s = (hashed ? dia_table_find(table, d) : bin_slot[(int64_t)d + nrows - 1]) - d0;
+            if (s >= 0 && s < dn) tile[s * S + (int)(row[k] - r0)] = val[k];
+          }
+      }
+      __syncthreads();
+      for (int d = w; d < dn; d += DIA_TILE_THREADS / 32)
+        for (int q = lane; q < R; q += 32) {
+          if (r0 + q < pitch) __stcs(out + r0 + q + pitch * (int64_t)(d0 + d), tile[d * S + q]);
+          tile[d * S + q] = T(0);
+        }
+      __syncthreads();
+    }
+  }
+}
+
+// Tile shape for nd diagonals: the most rows (32..512) whose tile of all
+// diagonals fits DIA_TILE_BYTES, else 32 rows of as many diagonals as fit
+// (the rows' entries are then read once per group of diagonals).
+template <typename T>
+void dia_tile_shape(int64_t nd, int* R, int* D) {
+  *R = 512;
+  while (*R > 32 && nd * (*R + 1) * (int64_t)sizeof(T) > DIA_TILE_BYTES) *R >>= 1;
+  *D = (int)std::min<int64_t>(nd, DIA_TILE_BYTES / ((*R + 1) * (int64_t)sizeof(T)));
+}
+// More groups than this (thousands of diagonals) and the entries are placed
+// one by one instead.
+constexpr int64_t DIA_TILE_GROUPS = 16;
+
+template <typename T>
+int launch_dia_fill(const mgb_coo* src, const int32_t* start, int64_t pitch, int64_t nd, const int32_t* offs,
+                    const int32_t* bin_slot, T* out, cudaStream_t s) {
+  int R, D;
+  dia_tile_shape<T>(nd, &R, &D);
+  const size_t smem = sizeof(T) * (size_t)D * (R + 1);
+  const unsigned grid = blocks_for((pitch + R - 1) / R, 1, (int64_t)num_sms() * 8);
+  dia_fill_tiles<T><<<grid, DIA_TILE_THREADS, smem, s>>>(src->row_indices, src->column_indices,
+                                                         static_cast<const T*>(src->values), start, src->nrows, pitch,
+                                                         (int)nd, offs, bin_slot, out, R, D);
+  MGB_LAUNCH_CHECK();
+  return MGB_SUCCESS;
+}
+template <typename T>
+bool dia_tiled(int64_t nd) {
+  int R, D;
+  dia_tile_shape<T>(nd, &R, &D);
+  return (nd + D - 1) / D <= DIA_TILE_GROUPS;
 }
 
 // Argument checks of a COO source (the index range checks are queued with
@@ -364,36 +442,30 @@ int check_coo_args(const mgb_coo* src) {
   return MGB_SUCCESS;
 }
 
-// COO -> DIA sizes: the diagonal histogram, its occupied bins and their
-// exclusive scan (slot of every occupied diagonal), queued with the
-// validation and, when `flags`, the sortedness flags; one host read.
+// COO -> DIA sizes: one pass over the indices counts the diagonals, checks
+// the ranges and the order and (starts) finds the row starts; the occupied
+// bins are counted; one host read.
 struct DiaPlan {
-  int32_t *bins = nullptr, *counts = nullptr, *slot = nullptr;
-  uint8_t* f = nullptr;
+  int32_t *counts = nullptr, *start = nullptr;
+  int64_t* sums = nullptr;
   Words h{};
 };
-int dia_plan(const mgb_coo* src, bool flags, DiaPlan* p, Scratch& sc, cudaStream_t s) {
+int dia_plan(const mgb_coo* src, bool starts, DiaPlan* p, Scratch& sc, cudaStream_t s) {
   int st = check_coo_args(src);
   if (st) return st;
   Words* dw;
   st = words_alloc(sc, &dw, s);
   if (st) return st;
-  st = validate_async(src->row_indices, src->column_indices, src->nnz, src->nrows, src->ncols, dw, s);
+  const int64_t nb = src->nrows + src->ncols - 1;
+  MGB_SCRATCH(sc, p->counts, nb > 0 ? nb : 1);
+  if (starts) MGB_SCRATCH(sc, p->start, src->nrows + 1);
+  st = prim::coo_pass(src->row_indices, src->column_indices, src->nnz, src->nrows, src->ncols, dw, p->counts,
+                      p->start, s);
   if (st) return st;
-  if (src->nnz > 0) {
-    const int64_t nb = src->nrows + src->ncols - 1;
-    st = diag_histogram(src, &p->bins, &p->counts, sc, s);
+  if (src->nnz > 0 && nb > 0) {
+    MGB_SCRATCH(sc, p->sums, prim::bin_tiles(nb));
+    st = prim::select_bins(p->counts, nb, 1, p->sums, &dw->total, nullptr, s);
     if (st) return st;
-    MGB_SCRATCH(sc, p->f, nb);
-    MGB_SCRATCH(sc, p->slot, nb);
-    nonzero_flags<<<grid_for(nb), 256, 0, s>>>(p->counts, nb, p->f);
-    MGB_LAUNCH_CHECK();
-    st = prim::exclusive_scan<uint8_t, int32_t>(p->f, p->slot, nb, s, &dw->total);
-    if (st) return st;
-    if (flags) {
-      st = prim::coo_sorted_flags(src->row_indices, src->column_indices, src->nnz, &dw->sorted, &dw->dup, s);
-      if (st) return st;
-    }
   }
   st = words_read(dw, &p->h, s);
   if (st) return st;
@@ -426,15 +498,18 @@ int coo_to_dia(const mgb_coo* src, mgb_dia* dst, cudaStream_t s) {
   if (nd == 0) return MGB_SUCCESS;
   MGB_REQUIRE(dst->diagonal_offsets && dst->values, MGB_ERR_BAD_ARGUMENT);
   const int64_t n = src->nnz, nb = src->nrows + src->ncols - 1;
-  int32_t *bins = p.bins, *slot = p.slot;
-  bins_to_offsets<<<grid_for(nb), 256, 0, s>>>(p.f, slot, nb, src->nrows, dst->diagonal_offsets);
-  MGB_LAUNCH_CHECK();
-  MGB_CUDA_CHECK(cudaMemsetAsync(dst->values, 0, sizeof(T) * dst->pitch * nd, s));
-  const bool sorted = p.h.sorted != 0, dup = p.h.dup != 0;
+  st = prim::select_bins_apply(p.counts, nb, 1, p.sums, src->nrows, -1, dst->diagonal_offsets, s);
+  if (st) return st;
+  const int32_t* slot = p.counts;  // bin -> slot now
   const T* v = static_cast<const T*>(src->values);
   T* out = static_cast<T*>(dst->values);
-  if (sorted && !dup) {
-    dia_place<T><<<grid_for(n), 256, 0, s>>>(src->row_indices, bins, v, n, slot, dst->pitch, out, nullptr, 0);
+  const bool distinct = words_distinct(p.h);
+  if (distinct && dia_tiled<T>(nd))
+    return launch_dia_fill<T>(src, p.start, dst->pitch, nd, dst->diagonal_offsets, slot, out, s);
+  MGB_CUDA_CHECK(cudaMemsetAsync(dst->values, 0, sizeof(T) * dst->pitch * nd, s));
+  if (distinct) {
+    dia_place<T><<<grid_for(n), 256, 0, s>>>(src->row_indices, src->column_indices, v, n, src->nrows, slot,
+                                             dst->pitch, out, nullptr, 0);
     MGB_LAUNCH_CHECK();
   } else {
     int32_t* owner;
@@ -442,7 +517,8 @@ int coo_to_dia(const mgb_coo* src, mgb_dia* dst, cudaStream_t s) {
     st = fill<int32_t>(owner, -1, dst->pitch * nd, s);
     if (st) return st;
     for (int pass = 0; pass < 2; pass++) {
-      dia_place<T><<<grid_for(n), 256, 0, s>>>(src->row_indices, bins, v, n, slot, dst->pitch, out, owner, pass);
+      dia_place<T><<<grid_for(n), 256, 0, s>>>(src->row_indices, src->column_indices, v, n, src->nrows, slot,
+                                               dst->pitch, out, owner, pass);
       MGB_LAUNCH_CHECK();
     }
   }
@@ -777,7 +853,7 @@ int coo_to_ell(const mgb_coo* src, mgb_ell* dst, cudaStream_t s) {
   int32_t* slot;
   MGB_SCRATCH(sc, slot, src->nnz);
   bool coll = false;
-  st = compute_slots(src, p.h.sorted != 0, p.counts, slot, &coll, sc, s);
+  st = compute_slots(src, words_rows_sorted(p.h), p.counts, slot, &coll, sc, s);
   if (st) return st;
   return place_ell<T>(src, dst, W, slot, coll, nullptr, sc, s);
 }
@@ -798,7 +874,7 @@ int row_plan(const mgb_coo* src, int64_t width, RowPlan* p, Scratch& sc, cudaStr
   Words* dw;
   int st = words_alloc(sc, &dw, s);
   if (st) return st;
-  st = validate_async(src->row_indices, src->column_indices, src->nnz, N, src->ncols, dw, s);
+  st = prim::coo_pass(src->row_indices, src->column_indices, src->nnz, N, src->ncols, dw, nullptr, nullptr, s);
   if (st) return st;
   MGB_SCRATCH(sc, p->counts, N + 1);
   st = prim::histogram(src->row_indices, src->nnz, p->counts, N, s);
@@ -811,8 +887,6 @@ int row_plan(const mgb_coo* src, int64_t width, RowPlan* p, Scratch& sc, cudaStr
     st = prim::reduce_max_i32(p->counts, N, &dw->maxv, s);
     if (st) return st;
   }
-  st = prim::rows_sorted_flag(src->row_indices, src->nnz, &dw->sorted, s);
-  if (st) return st;
   st = words_read(dw, &p->h, s);
   if (st) return st;
   return words_valid(p->h) ? MGB_SUCCESS : MGB_ERR_INVALID_INPUT;
@@ -867,7 +941,7 @@ int coo_to_hyb(const mgb_coo* src, mgb_hyb* dst, cudaStream_t s) {
   MGB_SCRATCH(sc, slot, n);
   MGB_SCRATCH(sc, to_coo, n);
   bool coll = false;
-  st = compute_slots(src, p.h.sorted != 0, p.counts, slot, &coll, sc, s);
+  st = compute_slots(src, words_rows_sorted(p.h), p.counts, slot, &coll, sc, s);
   if (st) return st;
   st = place_ell<T>(src, e, W, slot, coll, to_coo, sc, s);
   if (st || n == 0) return st;
@@ -914,22 +988,6 @@ int hdc_to_coo(const mgb_hdc* src, mgb_coo* dst, cudaStream_t s) {
 
 // ---------------------------------------------------------------- COO -> HDC
 // impl/Hdc/Serial/Morpheus_Convert_Impl.hpp:132-226
-__global__ void true_diag_flags(const int32_t* __restrict__ counts, int64_t nb, int32_t min_elem, uint8_t* f,
-                                int32_t* dia_counts) {
-  for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += (int64_t)gridDim.x * blockDim.x) {
-    const bool t = counts[b] >= min_elem;
-    f[b] = t;
-    dia_counts[b] = t ? counts[b] : 0;
-  }
-}
-// midpoint bin recorded as offset 0 (exact only for square matrices)
-__global__ void hdc_offsets(const uint8_t* __restrict__ f, const int32_t* __restrict__ slot, int64_t nb,
-                            int64_t nrows, int32_t* offs) {
-  const int64_t mid = nb / 2;
-  for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += (int64_t)gridDim.x * blockDim.x)
-    if (f[b]) offs[slot[b]] = (b == mid) ? 0 : (int32_t)(b - nrows + 1);
-}
-
 // first matching stored offset (the reference's break on the first match)
 __global__ void hdc_classify(const int32_t* __restrict__ r, const int32_t* __restrict__ c, int64_t n,
                              const int32_t* __restrict__ offs, int64_t nd, int32_t* dslot, uint8_t* is_csr) {
@@ -958,41 +1016,30 @@ __global__ void hdc_dia_place(const int32_t* __restrict__ r, const T* __restrict
   }
 }
 
-// COO -> HDC sizes: the diagonal histogram, the true diagonals (>= floor(0.2
-// N) entries), their slots and entry count, queued with the validation and
-// (when `flags`) the sortedness flags; one host read.
+// COO -> HDC sizes: one pass over the indices as for DIA, then the true
+// diagonals (>= floor(0.2 N) entries) and their entry count; one host read.
 struct HdcPlan {
-  int32_t *bins = nullptr, *counts = nullptr, *slot = nullptr;
-  uint8_t* f = nullptr;
+  int32_t* counts = nullptr;
+  int64_t* sums = nullptr;
+  int32_t min_elem = 0;
   Words h{};
 };
-int hdc_plan(const mgb_coo* src, bool flags, HdcPlan* p, Scratch& sc, cudaStream_t s) {
+int hdc_plan(const mgb_coo* src, HdcPlan* p, Scratch& sc, cudaStream_t s) {
   int st = check_coo_args(src);
   if (st) return st;
   MGB_REQUIRE(src->nrows > 0 && src->ncols > 0, MGB_ERR_INVALID_INPUT);
   const int64_t nb = src->nrows + src->ncols - 1;
-  const int32_t min_elem = (int32_t)((double)src->nrows * 0.2);  // HdcMatrix::true_diagonal_ratio
+  p->min_elem = (int32_t)((double)src->nrows * 0.2);  // HdcMatrix::true_diagonal_ratio
   Words* dw;
   st = words_alloc(sc, &dw, s);
   if (st) return st;
-  st = validate_async(src->row_indices, src->column_indices, src->nnz, src->nrows, src->ncols, dw, s);
+  MGB_SCRATCH(sc, p->counts, nb);
+  MGB_SCRATCH(sc, p->sums, prim::bin_tiles(nb));
+  st = prim::coo_pass(src->row_indices, src->column_indices, src->nnz, src->nrows, src->ncols, dw, p->counts, nullptr,
+                      s);
   if (st) return st;
-  st = diag_histogram(src, &p->bins, &p->counts, sc, s);
+  st = prim::select_bins(p->counts, nb, p->min_elem, p->sums, &dw->total, &dw->total2, s);
   if (st) return st;
-  int32_t* dcounts;
-  MGB_SCRATCH(sc, p->f, nb);
-  MGB_SCRATCH(sc, dcounts, nb);
-  MGB_SCRATCH(sc, p->slot, nb);
-  true_diag_flags<<<grid_for(nb), 256, 0, s>>>(p->counts, nb, min_elem, p->f, dcounts);
-  MGB_LAUNCH_CHECK();
-  st = prim::exclusive_scan<uint8_t, int32_t>(p->f, p->slot, nb, s, &dw->total);
-  if (st) return st;
-  st = prim::reduce_sum_i32(dcounts, nb, &dw->total2, s);
-  if (st) return st;
-  if (flags && src->nnz > 0) {
-    st = prim::coo_sorted_flags(src->row_indices, src->column_indices, src->nnz, &dw->sorted, &dw->dup, s);
-    if (st) return st;
-  }
   st = words_read(dw, &p->h, s);
   if (st) return st;
   if (!words_valid(p->h)) return MGB_ERR_INVALID_INPUT;
@@ -1004,7 +1051,7 @@ int coo_to_hdc_plan(const mgb_coo* src, int64_t* ndiags, int64_t* dia_nnz, int64
   MGB_REQUIRE(ndiags && dia_nnz && csr_nnz, MGB_ERR_BAD_ARGUMENT);
   Scratch sc(s);
   HdcPlan p;
-  const int st = hdc_plan(src, false, &p, sc, s);
+  const int st = hdc_plan(src, &p, sc, s);
   if (st == MGB_SUCCESS || st == MGB_ERR_FORMAT_CONVERSION) {
     *ndiags = p.h.total;
     *dia_nnz = p.h.total2;
@@ -1018,7 +1065,7 @@ int coo_to_hdc(const mgb_coo* src, mgb_hdc* dst, cudaStream_t s) {
   MGB_REQUIRE(dst != nullptr, MGB_ERR_BAD_ARGUMENT);
   Scratch sc(s);
   HdcPlan p;
-  int st = hdc_plan(src, true, &p, sc, s);
+  int st = hdc_plan(src, &p, sc, s);
   if (st) return st;
   const int64_t nd = p.h.total, dn = p.h.total2, cn = src->nnz - p.h.total2;
   mgb_dia* D = &dst->dia;
@@ -1030,11 +1077,10 @@ int coo_to_hdc(const mgb_coo* src, mgb_hdc* dst, cudaStream_t s) {
   MGB_REQUIRE(C->row_offsets && (nd == 0 || (D->diagonal_offsets && D->values)), MGB_ERR_BAD_ARGUMENT);
   MGB_REQUIRE(cn == 0 || (C->column_indices && C->values), MGB_ERR_BAD_ARGUMENT);
   const int64_t n = src->nnz, N = src->nrows, nb = src->nrows + src->ncols - 1;
-  uint8_t* f = p.f;
-  int32_t* slot = p.slot;
   if (nd > 0) {
-    hdc_offsets<<<grid_for(nb), 256, 0, s>>>(f, slot, nb, N, D->diagonal_offsets);
-    MGB_LAUNCH_CHECK();
+    // the midpoint bin is recorded as offset 0 (exact only for square matrices)
+    st = prim::select_bins_apply(p.counts, nb, p.min_elem, p.sums, N, nb / 2, D->diagonal_offsets, s);
+    if (st) return st;
     // std::sort of the stored offsets (impl/Hdc/Serial/Morpheus_Convert_Impl.hpp:193-195)
     std::vector<int32_t> h((size_t)nd);
     MGB_CUDA_CHECK(cudaMemcpyAsync(h.data(), D->diagonal_offsets, sizeof(int32_t) * nd, cudaMemcpyDeviceToHost, s));
@@ -1063,9 +1109,8 @@ int coo_to_hdc(const mgb_coo* src, mgb_hdc* dst, cudaStream_t s) {
   // entries to CSR than were counted (the reference writes out of bounds):
   // the scatter below stops at cn, and the count is checked at the end
   const T* v = static_cast<const T*>(src->values);
-  const bool sorted = p.h.sorted != 0, dup = p.h.dup != 0;
   if (nd > 0) {
-    if (sorted && !dup) {
+    if (words_distinct(p.h)) {
       hdc_dia_place<T><<<grid_for(n), 256, 0, s>>>(src->row_indices, v, dslot, n, D->pitch, static_cast<T*>(D->values),
                                                     nullptr, 0);
       MGB_LAUNCH_CHECK();
@@ -1123,7 +1168,7 @@ int coo_sort(mgb_coo* A, cudaStream_t s) {
   st = prim::reduce_max_i32(A->row_indices, A->nnz, &dw->maxv, s);
   if (st) return st;
   // rows and columns must be >= 0 (the counting sort indexes by them)
-  st = validate_async(A->row_indices, A->column_indices, A->nnz, INT32_MAX, INT32_MAX, dw, s);
+  st = prim::coo_pass(A->row_indices, A->column_indices, A->nnz, INT32_MAX, INT32_MAX, dw, nullptr, nullptr, s);
   if (st) return st;
   Words hw;
   st = words_read(dw, &hw, s);

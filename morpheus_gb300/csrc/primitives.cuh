@@ -54,8 +54,6 @@ int histogram(const int32_t* keys, int64_t n, int32_t* counts, int64_t nbins, cu
 // duplicate (row, col) exists (only meaningful when sorted).
 int coo_sorted_flags(const int32_t* rows, const int32_t* cols, int64_t n, int32_t* d_flag,
                      int32_t* d_dup, cudaStream_t s);
-// 1 if rows are non-decreasing.
-int rows_sorted_flag(const int32_t* rows, int64_t n, int32_t* d_flag, cudaStream_t s);
 
 // Sort the keys of each segment [seg[i], seg[i+1]) ascending (keys unique
 // within a segment, so any sort is stable).  nseg segments, seg has nseg+1
@@ -68,6 +66,42 @@ int segmented_sort_u64(uint64_t* keys, const int32_t* seg, int64_t nseg, int64_t
 // reference's two stable counting sorts (by column, then by row).
 int stable_sort_rows_cols(const int32_t* rows, const int32_t* cols, int64_t n, int64_t nrows,
                           int32_t* out_rows, int32_t* out_cols, int32_t* perm, cudaStream_t s);
+
+// ---- one pass over COO indices ------------------------------------------------
+// Device words an entry point reads back with one copy and one stream
+// synchronisation: what the index pass saw, and the plan's sizes, computed by
+// kernels queued one after another.
+constexpr int32_t COO_BAD_INDEX = 1;      // a row outside [0, nrows) or a column outside [0, ncols)
+constexpr int32_t COO_ROWS_UNSORTED = 2;  // a row smaller than the one before it
+constexpr int32_t COO_UNSORTED = 4;       // a (row, column) smaller than the one before it
+constexpr int32_t COO_DUPLICATE = 8;      // a (row, column) equal to the one before it
+struct Words {
+  int64_t total, total2;  // plan sizes
+  int32_t seen;           // COO_* bits
+  int32_t maxv, pad[2];
+};
+int words_alloc(Scratch& sc, Words** d, cudaStream_t s);          // zeroed
+int words_read(const Words* d, Words* h, cudaStream_t s);         // synchronises
+
+// Reads every (row, column) once, queued without a synchronisation:
+// d->seen |= the COO_* bits; diag != nullptr (nrows + ncols - 1 counters,
+// zeroed here): the entries on each diagonal, bin column - row + nrows - 1;
+// start != nullptr (nrows + 1 entries): the first entry of every row, valid
+// when the rows are in range and non-decreasing.  Entries out of range are
+// reported and not counted.
+int coo_pass(const int32_t* rows, const int32_t* cols, int64_t n, int64_t nrows, int64_t ncols, Words* d,
+             int32_t* diag, int32_t* start, cudaStream_t s);
+
+// The bins with counts[b] >= threshold, in order: how many to *d_total, their
+// counts' sum to *d_sum (if not null), and tile prefixes in sums
+// (bin_tiles(nb) entries) for select_bins_apply, which replaces counts[b] by
+// the bin's slot (-1: not selected) and writes offsets[slot] = b - nrows + 1
+// (zero_bin: the bin recorded as offset 0, -1 for none).
+int64_t bin_tiles(int64_t nb);
+int select_bins(const int32_t* counts, int64_t nb, int32_t threshold, int64_t* sums, int64_t* d_total, int64_t* d_sum,
+                cudaStream_t s);
+int select_bins_apply(int32_t* counts, int64_t nb, int32_t threshold, const int64_t* sums, int64_t nrows,
+                      int64_t zero_bin, int32_t* offsets, cudaStream_t s);
 
 // Copy a device scalar to the host (synchronises the stream).
 template <typename T>

@@ -1,0 +1,68 @@
+"""GPU conversions at the edges of their tiles: every result bit-identical to the oracle's Serial convert."""
+import numpy as np
+import pytest
+
+from morpheus_gb300 import generators as gen
+from test_convert_gpu import check_all_targets, both
+from helpers import assert_same_matrix
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def diagonals(N, M, nd, seed, dtype, keep=0.7):
+    """Sorted COO with entries on nd random diagonals (each slot present with probability `keep`)."""
+    rng = np.random.default_rng(seed)
+    offs = np.sort(rng.choice(np.arange(-(N - 1), M), nd, replace=False))
+    r = np.arange(N)[:, None]
+    c = r + offs[None, :]
+    m = (c >= 0) & (c < M) & (rng.random((N, nd)) < keep)
+    rows, cols = np.broadcast_to(r, c.shape)[m], c[m]
+    return {"format": 0, "nrows": N, "ncols": M, "nnz": rows.size, "row_indices": rows.astype(np.int32),
+            "column_indices": cols.astype(np.int32), "values": rng.standard_normal(rows.size).astype(dtype)}
+
+
+# one diagonal; 512-row tiles; the last size whose diagonals fit one tile and the first that needs 32 rows or
+# several groups of diagonals; the lookup table's limit (256); more groups than the tiles take
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("N,nd", [(1, 1), (33, 3), (1025, 7), (513, 8), (700, 63), (640, 124), (611, 125), (500, 256),
+                                  (501, 257), (900, 700), (1500, 2100), (2301, 4200)])
+def test_dia_tiles(cuda, N, nd, dtype):
+    hm = diagonals(N, N, min(nd, 2 * N - 1), seed=N + nd, dtype=dtype, keep=0.7 if nd < 1000 else 0.1)
+    got, ref = both(hm, O.DIA)
+    assert_same_matrix(got, ref)
+
+
+@pytest.mark.parametrize("N,M", [(97, 400), (400, 97)])
+def test_dia_tiles_nonsquare(cuda, N, M):
+    got, ref = both(diagonals(N, M, 40, seed=N, dtype=np.float64), O.DIA)
+    assert_same_matrix(got, ref)
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("gap", [1, 255, 256, 257, 3000])
+def test_row_starts_over_gaps(cuda, gap, shift):
+    """Empty rows before, between (around the gap that a CTA fills together) and after the entries; entries from
+    an offset in their arrays that 16-byte loads do not allow."""
+    rng = np.random.default_rng(gap)
+    rows = np.repeat(np.arange(7, 7 + 40 * (gap + 1), gap + 1), rng.integers(1, 9, 40))
+    n = rows.size
+    N = int(rows[-1]) + 1 + 2 * gap
+    cols = np.concatenate([np.sort(rng.choice(N, int((rows == r).sum()), replace=False)) for r in np.unique(rows)])
+    hm = {"format": 0, "nrows": N, "ncols": N, "nnz": n, "row_indices": rows.astype(np.int32),
+          "column_indices": cols.astype(np.int32), "values": rng.standard_normal(n)}
+    if not shift:
+        check_all_targets(hm)
+        return
+    import torch
+
+    import morpheus_gb300 as mgb
+    A = mgb.CooMatrix(N, N, n, *(torch.from_numpy(np.concatenate([a[:1], a])).cuda()[1:] for a in (
+        hm["row_indices"], hm["column_indices"], hm["values"])))
+    for fmt in (1, 2, 3, 4, 5):
+        want = O.OracleMatrix.from_host(hm).convert(fmt).to_host()
+        assert_same_matrix(mgb.matrix_to_host(mgb.from_coo(A, fmt)), want)
+
+
+def test_stencil_tiles(cuda):
+    check_all_targets(gen.stencil_27pt(23, seed=5))
