@@ -392,7 +392,8 @@ int mgb_spmv_batched_csr_autotune_f32(const mgb_csr_batch_item* d_items, int64_t
  * with MGB_ERR_INVALID_INPUT (the reference indexes out of bounds there).
  * Conversions synchronise the stream (they read sizes back to the host). */
 
-/* impl/Csr/Serial/Morpheus_Convert_Impl.hpp:70-97; dst: nnz entries */
+/* impl/Csr/Serial/Morpheus_Convert_Impl.hpp:70-97; dst: nnz entries.  dst may
+ * share src's column and value arrays: only the rows are then written. */
 int mgb_convert_csr_to_coo_f64(const mgb_csr* src, mgb_coo* dst, void* stream);
 int mgb_convert_csr_to_coo_f32(const mgb_csr* src, mgb_coo* dst, void* stream);
 /* impl/Csr/Serial/Morpheus_Convert_Impl.hpp:99-151; dst: nrows+1 offsets, nnz entries */

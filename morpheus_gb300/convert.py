@@ -52,14 +52,32 @@ def to_coo(A: _Matrix, stream=None) -> CooMatrix:
     if isinstance(A, DynamicMatrix):
         A = A.active()
     _dev_check(A)
-    sfx = _suffix(A.dtype)
+    _suffix(A.dtype)
     if A.FORMAT == COO_FORMAT:
         return CooMatrix(A.nrows(), A.ncols(), A.nnnz(), A.row_indices().clone(), A.column_indices().clone(),
                          A.values().clone(), A.dtype, A.device)
-    out = CooMatrix(A.nrows(), A.ncols(), A.nnnz(), dtype=A.dtype, device=A.device)
+    z = A.nnnz()  # the conversions write every entry: nothing to clear
+    return _fill_coo(A, _empty(z, torch.int32, A.device), _empty(z, A.dtype, A.device), stream)
+
+
+def _fill_coo(A: _Matrix, cols: torch.Tensor, vals: torch.Tensor, stream) -> CooMatrix:
+    out = CooMatrix(A.nrows(), A.ncols(), A.nnnz(), _empty(A.nnnz(), torch.int32, A.device), cols, vals, A.dtype,
+                    A.device)
     sd, dd = A._desc(), out._desc()
-    _call(f"mgb_convert_{_NAME[A.FORMAT]}_to_coo_{sfx}", C.byref(sd), C.byref(dd), _stream_handle(stream))
+    _call(f"mgb_convert_{_NAME[A.FORMAT]}_to_coo_{_suffix(A.dtype)}", C.byref(sd), C.byref(dd),
+          _stream_handle(stream))
     return out
+
+
+def _as_coo(A: _Matrix, stream=None) -> CooMatrix:
+    """A's entries as a COO that is only read: a CSR matrix's columns and
+    values are shared with it, and only its rows are expanded."""
+    if A.FORMAT == COO_FORMAT:
+        return A
+    if A.FORMAT != CSR_FORMAT:
+        return to_coo(A, stream)
+    _dev_check(A)
+    return _fill_coo(A, A.column_indices(), A.values(), stream)
 
 
 def from_coo(coo: CooMatrix, fmt: int, hyb_width: int = 0, stream=None) -> _Matrix:
@@ -110,9 +128,10 @@ def convert(src, dst, stream=None, hyb_width: int = 0):
     target = dst.active_index() if isinstance(dst, DynamicMatrix) else dst.FORMAT
     if src.FORMAT == target:
         out = from_coo(to_coo(src), target, hyb_width=hyb_width) if target == COO_FORMAT else _deep_copy(src)
+    elif target == COO_FORMAT:
+        out = to_coo(src, stream)
     else:
-        tmp = src if src.FORMAT == COO_FORMAT else to_coo(src, stream)
-        out = from_coo(tmp, target, hyb_width=hyb_width, stream=stream)
+        out = from_coo(_as_coo(src, stream), target, hyb_width=hyb_width, stream=stream)
     if isinstance(dst, DynamicMatrix):
         dst.assign(out)
     else:
@@ -137,11 +156,11 @@ def convert_inplace(dyn: DynamicMatrix, fmt, stream=None, hyb_width: int = 0) ->
     if dyn.active_index() == fmt:
         return conversion_error_e.CONV_SUCCESS
     try:
-        temp = to_coo(dyn.active(), stream)
+        temp = to_coo(dyn.active(), stream) if fmt == COO_FORMAT else _as_coo(dyn.active(), stream)
     except MorpheusException:
         return conversion_error_e.DYNAMIC_TO_PROXY
     try:
-        out = from_coo(temp, fmt, hyb_width=hyb_width, stream=stream)
+        out = temp if fmt == COO_FORMAT else from_coo(temp, fmt, hyb_width=hyb_width, stream=stream)
     except MorpheusException:
         return conversion_error_e.PROXY_TO_DYNAMIC
     dyn.assign(out)

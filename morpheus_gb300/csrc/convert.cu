@@ -131,12 +131,34 @@ int zero_coo(mgb_coo* d, cudaStream_t s) {
 
 // ---------------------------------------------------------------- CSR <-> COO
 // impl/Csr/Serial/Morpheus_Convert_Impl.hpp:70-97
-__global__ void expand_rows(const int32_t* __restrict__ ro, int64_t nrows, int64_t nnz, int32_t* rows,
-                            int64_t shift) {
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t a = max((int64_t)ro[r], (int64_t)0), b = min((int64_t)ro[r + 1], nnz);
-    for (int64_t j = a; j < b; j++) rows[j + shift] = (int32_t)r;
+// rows[j + shift] = the row of CSR entry j, one warp per 32 rows, in 16-byte
+// stores (a thread per row wrote 4 bytes at a time: 608 us for the 437 MB of
+// the 27-point stencil at 160^3).  Entries before the first offset or past
+// the last one (offsets that do not span the entries) get row 0.
+__global__ void __launch_bounds__(256) expand_rows(const int32_t* __restrict__ ro, int64_t nrows, int64_t nnz,
+                                                   int32_t* __restrict__ rows, int64_t shift) {
+  __shared__ int32_t s_ro[8][33];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int32_t* out = rows + shift;
+  const bool vec = reinterpret_cast<uintptr_t>(out) % 16 == 0;
+  for (int64_t r0 = ((int64_t)blockIdx.x * 8 + w) * 32; r0 < nrows; r0 += (int64_t)gridDim.x * 256) {
+    int32_t v[4];
+    prim::warp_row_quads(
+        ro, r0, nrows, s_ro[w], lane, [](int32_t, int, int) {}, [&](int k, int64_t r) { v[k] = (int32_t)r; },
+        [&](int32_t e0, int lo, int hi) {
+          if (vec && lo == 0 && hi == 4 && e0 >= 0 && (int64_t)e0 + 4 <= nnz) {
+            __stcs(reinterpret_cast<int4*>(out + e0), make_int4(v[0], v[1], v[2], v[3]));
+          } else {
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+              if (k >= lo && k < hi && e0 + k >= 0 && (int64_t)e0 + k < nnz) out[e0 + k] = v[k];
+          }
+        });
   }
+  const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x, nt = (int64_t)gridDim.x * 256;
+  const int64_t first = min((int64_t)ro[0], nnz), last = max((int64_t)ro[nrows], (int64_t)0);
+  for (int64_t j = t; j < first; j += nt) out[j] = 0;
+  for (int64_t j = last + t; j < nnz; j += nt) out[j] = 0;
 }
 
 template <typename T>
@@ -147,9 +169,11 @@ int csr_to_coo(const mgb_csr* src, mgb_coo* dst, cudaStream_t s) {
   if (src->nnz == 0) return MGB_SUCCESS;
   expand_rows<<<grid_for(src->nrows), 256, 0, s>>>(src->row_offsets, src->nrows, src->nnz, dst->row_indices, 0);
   MGB_LAUNCH_CHECK();
-  MGB_CUDA_CHECK(cudaMemcpyAsync(dst->column_indices, src->column_indices, sizeof(int32_t) * src->nnz,
-                                 cudaMemcpyDeviceToDevice, s));
-  MGB_CUDA_CHECK(cudaMemcpyAsync(dst->values, src->values, sizeof(T) * src->nnz, cudaMemcpyDeviceToDevice, s));
+  if (dst->column_indices != src->column_indices)
+    MGB_CUDA_CHECK(cudaMemcpyAsync(dst->column_indices, src->column_indices, sizeof(int32_t) * src->nnz,
+                                   cudaMemcpyDeviceToDevice, s));
+  if (dst->values != src->values)
+    MGB_CUDA_CHECK(cudaMemcpyAsync(dst->values, src->values, sizeof(T) * src->nnz, cudaMemcpyDeviceToDevice, s));
   return MGB_SUCCESS;
 }
 

@@ -123,7 +123,7 @@ __global__ void histogram_kernel(const int32_t* __restrict__ keys, int64_t n, in
   __syncthreads();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int32_t k = keys[i];
-    if (k >= 0 && k < nbins) hist_add<true>(h, counts, (uint64_t)k);
+    if (k >= 0 && k < nbins) hist_add32<true>(h, counts, (uint32_t)k);
   }
   __syncthreads();
   hist_flush(h, counts);
@@ -152,7 +152,7 @@ __global__ void sorted_flags_kernel(const int32_t* __restrict__ r, const int32_t
 // Row starts: the entry where the row changes from p to q is the start of
 // the rows p + 1..q; gaps longer than PASS_GAP are left to the whole CTA at
 // the end, and the rows before the first and after the last entry to the grid.
-constexpr int PASS_GAP = 256;
+constexpr uint32_t PASS_GAP = 256;
 constexpr int PASS_GAPS = 256;
 
 template <bool DIAG, bool STARTS>
@@ -173,11 +173,15 @@ __global__ void __launch_bounds__(256) coo_pass_kernel(const int32_t* __restrict
   }
   __syncthreads();
   const int lane = threadIdx.x & 31;
-  int32_t bits = 0;
+  // valid indices are below 2^31: unsigned comparisons (order flags that
+  // negative indices upset do not matter, such a matrix is refused)
+  const uint32_t nr = (uint32_t)min(nrows, (int64_t)1 << 31), nc = (uint32_t)min(ncols, (int64_t)1 << 31);
+  const uint32_t mid = (uint32_t)(nrows - 1);
+  bool bad = false, rows_down = false, down = false, equal = false;
   for (int64_t base = (int64_t)blockIdx.x * 1024; base < n; base += (int64_t)gridDim.x * 1024) {
     const int64_t i0 = base + (int64_t)threadIdx.x * 4;
     const int m = (int)min((int64_t)4, n - i0);  // this thread's entries (<= 0: none)
-    int32_t rr[4] = {0, 0, 0, 0}, cc[4] = {0, 0, 0, 0};
+    uint32_t rr[4] = {0, 0, 0, 0}, cc[4] = {0, 0, 0, 0};
     if (vec && m == 4) {
       const int4 a = __ldg(reinterpret_cast<const int4*>(r + i0)), b = __ldg(reinterpret_cast<const int4*>(c + i0));
       rr[0] = a.x; rr[1] = a.y; rr[2] = a.z; rr[3] = a.w;
@@ -187,35 +191,43 @@ __global__ void __launch_bounds__(256) coo_pass_kernel(const int32_t* __restrict
       for (int k = 0; k < 4; k++)
         if (k < m) { rr[k] = r[i0 + k]; cc[k] = c[i0 + k]; }
     }
-    int32_t pr = __shfl_up_sync(0xffffffffu, rr[3], 1), pc = __shfl_up_sync(0xffffffffu, cc[3], 1);
+    uint32_t pr = __shfl_up_sync(0xffffffffu, rr[3], 1), pc = __shfl_up_sync(0xffffffffu, cc[3], 1);
     if (lane == 0 && m > 0 && i0 > 0) { pr = r[i0 - 1]; pc = c[i0 - 1]; }
+    if (i0 == 0) { pr = rr[0]; pc = 0; }  // the first entry: nothing before it
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       if (k >= m) break;
-      const bool ok = rr[k] >= 0 && rr[k] < nrows && cc[k] >= 0 && cc[k] < ncols;
-      if (!ok) bits |= COO_BAD_INDEX;
-      if (i0 + k > 0) {
-        if (rr[k] < pr) bits |= COO_ROWS_UNSORTED | COO_UNSORTED;
-        if (rr[k] == pr && cc[k] < pc) bits |= COO_UNSORTED;
-        if (rr[k] == pr && cc[k] == pc) bits |= COO_DUPLICATE;
-        if (STARTS && rr[k] > pr && pr >= 0 && rr[k] < nrows) {
-          const int32_t at = (int32_t)(i0 + k);
-          int g = PASS_GAPS;
-          if (rr[k] - pr > PASS_GAP) g = atomicAdd(&ngaps, 1);
-          if (g < PASS_GAPS) {
-            gap_from[g] = pr + 1;
-            gap_to[g] = rr[k];
-            gap_at[g] = at;
-          } else {
-            for (int32_t q = pr + 1; q <= rr[k]; q++) start[q] = at;
+      const bool ok = rr[k] < nr && cc[k] < nc;
+      bad |= !ok;
+      if (rr[k] == pr) {
+        down |= cc[k] < pc;
+        equal |= cc[k] == pc && (k > 0 || i0 > 0);
+      } else {
+        rows_down |= rr[k] < pr;
+        if constexpr (STARTS) {
+          if (rr[k] == pr + 1) {
+            if (rr[k] < nr) start[rr[k]] = (int32_t)(i0 + k);
+          } else if (rr[k] > pr && rr[k] < nr) {
+            const int32_t at = (int32_t)(i0 + k);
+            int g = PASS_GAPS;
+            if (rr[k] - pr > PASS_GAP) g = atomicAdd(&ngaps, 1);
+            if (g < PASS_GAPS) {
+              gap_from[g] = (int32_t)(pr + 1);
+              gap_to[g] = (int32_t)rr[k];
+              gap_at[g] = at;
+            } else {
+              for (uint32_t q = pr + 1; q <= rr[k]; q++) start[q] = at;
+            }
           }
         }
       }
-      if (DIAG && ok) hist_add(h, diag, (uint64_t)((int64_t)cc[k] - rr[k] + nrows - 1));
+      if (DIAG && ok) hist_add32(h, diag, cc[k] - rr[k] + mid);
       pr = rr[k];
       pc = cc[k];
     }
   }
+  const int bits = (bad ? COO_BAD_INDEX : 0) | (rows_down ? COO_ROWS_UNSORTED | COO_UNSORTED : 0) |
+                   (down ? COO_UNSORTED : 0) | (equal ? COO_DUPLICATE : 0);
   if (bits) atomicOr(&s_bits, bits);
   __syncthreads();
   if (threadIdx.x == 0 && s_bits) atomicOr(seen, s_bits);

@@ -150,16 +150,11 @@ __device__ __forceinline__ void hist_init(CtaHist h) {
 
 __device__ __forceinline__ unsigned hist_home(uint32_t key) { return (key * 0x9E3779B1u) >> (32 - HIST_SLOTS_LOG2); }
 
-// counts one occurrence of key (global[key] += 1, in the end).  MERGE: lanes
+// counts one occurrence of key < HIST_EMPTY (global[key] += 1, in the end).  MERGE: lanes
 // that go to the global counter with the same key add once (runs of equal
 // keys: the rows of row-sorted entries).
 template <bool MERGE = false>
-__device__ __forceinline__ void hist_add(CtaHist h, int32_t* global, uint64_t key64) {
-  if (key64 >= HIST_EMPTY) {
-    atomicAdd(global + key64, 1);
-    return;
-  }
-  const uint32_t key = (uint32_t)key64;
+__device__ __forceinline__ void hist_add32(CtaHist h, int32_t* global, uint32_t key) {
   unsigned slot = hist_home(key);
   volatile uint32_t* keys = h.keys;
   uint32_t k = keys[slot];
@@ -186,6 +181,12 @@ __device__ __forceinline__ void hist_add(CtaHist h, int32_t* global, uint64_t ke
   }
 }
 
+// the same for keys that may not fit the table's 32 bits
+__device__ __forceinline__ void hist_add(CtaHist h, int32_t* global, uint64_t key) {
+  if (key < HIST_EMPTY) hist_add32(h, global, (uint32_t)key);
+  else atomicAdd(global + key, 1);
+}
+
 // every thread of the CTA, after a __syncthreads() that follows the last hist_add
 __device__ __forceinline__ void hist_flush(CtaHist h, int32_t* global) {
   for (int i = threadIdx.x; i < HIST_SLOTS; i += blockDim.x) {
@@ -195,34 +196,38 @@ __device__ __forceinline__ void hist_flush(CtaHist h, int32_t* global) {
 }
 
 // ---- entries of CSR rows, one warp per 32 rows ------------------------------
-// Calls f(r, e) for every entry e of the rows [r0, min(r0 + 32, nrows)), 32
-// consecutive entries at a time (coalesced, however long the rows are): the
-// offsets of the 32 rows lie in shared memory (s_ro, 33 per warp) and every
-// lane moves along them as its entry moves.  PRE(e) is called for four steps
-// ahead of their f, so that the loads it makes are in flight together; its
-// result is f's third argument.
-template <typename PRE, typename F>
-__device__ __forceinline__ void warp_row_entries(const int32_t* __restrict__ ro, int64_t r0, int64_t nrows,
-                                                 int32_t* s_ro, int lane, PRE pre, F f) {
+// Visits every entry of the rows [r0, min(r0 + 32, nrows)), 128 consecutive
+// entries at a time and four per lane, however long the rows are: the offsets
+// of the 32 rows lie in shared memory (s_ro, 33 per warp), a lane finds the
+// row of its first entry by a 5-step search and moves on from there.  For each
+// group of four, e0 a multiple of 4: load(e0, lo, hi), then f(k, r) for every k in
+// [lo, hi) (entry e0 + k, row r), then store(e0, lo, hi); entries outside
+// [lo, hi) belong to other warps.
+template <typename LOAD, typename F, typename STORE>
+__device__ __forceinline__ void warp_row_quads(const int32_t* __restrict__ ro, int64_t r0, int64_t nrows,
+                                               int32_t* s_ro, int lane, LOAD load, F f, STORE store) {
   __syncwarp();
   s_ro[lane] = ro[min(r0 + lane, nrows)];
   if (lane == 0) s_ro[32] = ro[min(r0 + 32, nrows)];
   __syncwarp();
-  const int64_t end = s_ro[32];
-  int q = 0;
-  for (int64_t e0 = (int64_t)s_ro[0] + lane; e0 < end; e0 += 128) {
-    decltype(pre(e0)) v[4];
+  const int32_t b = s_ro[0], t = s_ro[32];
+  for (int64_t at = (int64_t)(b & ~3) + 4 * lane; at < t; at += 128) {
+    const int32_t e0 = (int32_t)at;
+    const int lo = max(b - e0, 0), hi = min(t - e0, 4);
+    if (lo >= hi) continue;
+    load(e0, lo, hi);
+    int q = 0;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1)
+      if (s_ro[q + d] <= e0 + lo) q += d;
+    int32_t next = s_ro[q + 1];
 #pragma unroll
     for (int k = 0; k < 4; k++)
-      if (e0 + 32 * k < end) v[k] = pre(e0 + 32 * k);
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const int64_t e = e0 + 32 * k;
-      if (e < end) {
-        while (q < 31 && e >= s_ro[q + 1]) q++;
-        f(r0 + q, e, v[k]);
+      if (k >= lo && k < hi) {
+        while (q < 31 && e0 + k >= next) next = s_ro[++q + 1];
+        f(k, r0 + q);
       }
-    }
+    store(e0, lo, hi);
   }
 }
 
