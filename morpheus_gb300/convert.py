@@ -80,6 +80,28 @@ def _as_coo(A: _Matrix, stream=None) -> CooMatrix:
     return _fill_coo(A, A.column_indices(), A.values(), stream)
 
 
+# Containers that a conversion fills: it writes every index, offset and value
+# (padding included), so their arrays are not cleared first.
+
+def _new_csr(n, m, z, dt, dev) -> CsrMatrix:
+    return CsrMatrix(n, m, z, _empty(n + 1, torch.int32, dev), _empty(z, torch.int32, dev), _empty(z, dt, dev), dt, dev)
+
+
+def _new_coo(n, m, z, dt, dev) -> CooMatrix:
+    return CooMatrix(n, m, z, _empty(z, torch.int32, dev), _empty(z, torch.int32, dev), _empty(z, dt, dev), dt, dev)
+
+
+def _new_dia(n, m, z, nd, dt, dev) -> DiaMatrix:
+    return DiaMatrix(n, m, z, nd, diagonal_offsets=_empty(nd, torch.int32, dev),
+                     values=_empty(get_pad_size(n, 32) * nd, dt, dev), dtype=dt, device=dev)
+
+
+def _new_ell(n, m, z, w, dt, dev) -> EllMatrix:
+    slab = n * get_pad_size(w, 32)
+    return EllMatrix(n, m, z, w, column_indices=_empty(slab, torch.int32, dev), values=_empty(slab, dt, dev), dtype=dt,
+                     device=dev)
+
+
 def from_coo(coo: CooMatrix, fmt: int, hyb_width: int = 0, stream=None) -> _Matrix:
     """COO -> a new container of format `fmt` (the reference's COO -> Y)."""
     _dev_check(coo)
@@ -91,27 +113,23 @@ def from_coo(coo: CooMatrix, fmt: int, hyb_width: int = 0, stream=None) -> _Matr
     if fmt == COO_FORMAT:
         return to_coo(coo)
     if fmt == CSR_FORMAT:
-        out = CsrMatrix(n, m, z, dtype=dt, device=dev)
+        out = _new_csr(n, m, z, dt, dev)
     elif fmt == DIA_FORMAT:
         nd = _i64()
         _call("mgb_convert_coo_to_dia_plan", C.byref(sd), C.byref(nd), sh)
-        # the conversion writes every offset and slab value: nothing to clear
-        out = DiaMatrix(n, m, z, nd.value, diagonal_offsets=_empty(nd.value, torch.int32, dev),
-                        values=_empty(get_pad_size(n, 32) * nd.value, dt, dev), dtype=dt, device=dev)
+        out = _new_dia(n, m, z, nd.value, dt, dev)
     elif fmt == ELL_FORMAT:
         w = _i64()
         _call("mgb_convert_coo_to_ell_plan", C.byref(sd), C.byref(w), sh)
-        out = EllMatrix(n, m, z, w.value, dtype=dt, device=dev)
+        out = _new_ell(n, m, z, w.value, dt, dev)
     elif fmt == HYB_FORMAT:
         w, en, cn = _i64(), _i64(), _i64()
         _call("mgb_convert_coo_to_hyb_plan", C.byref(sd), int(hyb_width), C.byref(w), C.byref(en), C.byref(cn), sh)
-        out = HybMatrix(EllMatrix(n, m, en.value, w.value, dtype=dt, device=dev),
-                        CooMatrix(n, m, cn.value, dtype=dt, device=dev), dt, dev)
+        out = HybMatrix(_new_ell(n, m, en.value, w.value, dt, dev), _new_coo(n, m, cn.value, dt, dev), dt, dev)
     elif fmt == HDC_FORMAT:
         nd, dn, cn = _i64(), _i64(), _i64()
         _call("mgb_convert_coo_to_hdc_plan", C.byref(sd), C.byref(nd), C.byref(dn), C.byref(cn), sh)
-        out = HdcMatrix(DiaMatrix(n, m, dn.value, nd.value, dtype=dt, device=dev),
-                        CsrMatrix(n, m, cn.value, dtype=dt, device=dev), dt, dev)
+        out = HdcMatrix(_new_dia(n, m, dn.value, nd.value, dt, dev), _new_csr(n, m, cn.value, dt, dev), dt, dev)
     else:
         raise NotImplementedException(f"format {fmt}")
     dd = out._desc()

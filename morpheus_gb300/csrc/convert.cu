@@ -720,32 +720,11 @@ __global__ void run_slots(const uint8_t* __restrict__ f, const int32_t* __restri
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     slot[i] = (int32_t)(i - starts[excl[i] + f[i] - 1]);
 }
-__global__ void sorted_slots(const int32_t* __restrict__ r, const int32_t* __restrict__ row_start, int64_t n,
-                             int32_t* slot) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    slot[i] = (int32_t)(i - row_start[r[i]]);
-}
-
-// Slot of every entry in its row (the reference's placement counter, which
-// restarts whenever the row changes).  rows_sorted: the rows are
-// non-decreasing (read by the caller); counts: the row histogram (N + 1
-// entries, the last one zero).
-int compute_slots(const mgb_coo* src, bool rows_sorted_flag, int32_t* counts, int32_t* slot, bool* collisions,
-                  Scratch& sc, cudaStream_t s) {
-  const int64_t n = src->nnz, N = src->nrows;
-  *collisions = false;
+// Slot of every entry in its run (the reference's placement counter, which
+// restarts whenever the row changes), for rows in any order.
+int compute_slots(const mgb_coo* src, int32_t* slot, Scratch& sc, cudaStream_t s) {
+  const int64_t n = src->nnz;
   if (n == 0) return MGB_SUCCESS;
-  int st = MGB_SUCCESS;
-  if (rows_sorted_flag) {
-    int32_t* start;
-    MGB_SCRATCH(sc, start, N + 1);
-    st = prim::exclusive_scan<int32_t, int32_t>(counts, start, N + 1, s);
-    if (st) return st;
-    sorted_slots<<<grid_for(n), 256, 0, s>>>(src->row_indices, start, n, slot);
-    MGB_LAUNCH_CHECK();
-    return MGB_SUCCESS;
-  }
-  *collisions = true;
   uint8_t* f;
   int32_t *excl, *starts;
   MGB_SCRATCH(sc, f, n);
@@ -753,8 +732,7 @@ int compute_slots(const mgb_coo* src, bool rows_sorted_flag, int32_t* counts, in
   MGB_SCRATCH(sc, starts, n);
   run_flags<<<grid_for(n), 256, 0, s>>>(src->row_indices, n, f);
   MGB_LAUNCH_CHECK();
-  st = prim::exclusive_scan<uint8_t, int32_t>(f, excl, n, s);
-  if (st) return st;
+  if (int st = prim::exclusive_scan<uint8_t, int32_t>(f, excl, n, s)) return st;
   run_starts<<<grid_for(n), 256, 0, s>>>(f, excl, n, starts);
   MGB_LAUNCH_CHECK();
   run_slots<<<grid_for(n), 256, 0, s>>>(f, excl, starts, n, slot);
@@ -776,10 +754,7 @@ __global__ void ell_place(const int32_t* __restrict__ r, const int32_t* __restri
     }
     if (to_coo && pass == 0) to_coo[i] = 0;
     const int64_t at = r[i] + pitch * k;
-    if (owner == nullptr) {
-      eci[at] = c[i];
-      ev[at] = v[i];
-    } else if (pass == 0) {
+    if (pass == 0) {
       atomicMax(owner + at, (int32_t)i);
     } else if (owner[at] == (int32_t)i) {
       eci[at] = c[i];
@@ -801,44 +776,203 @@ __global__ void coo_part_scatter(const int32_t* __restrict__ r, const int32_t* _
     }
 }
 
+// ELL slab of a COO whose rows are in any order.
 template <typename T>
-int place_ell(const mgb_coo* src, mgb_ell* e, int64_t W, const int32_t* slot, bool collisions, uint8_t* to_coo,
-              Scratch& sc, cudaStream_t s) {
+int place_ell(const mgb_coo* src, mgb_ell* e, int64_t W, const int32_t* slot, uint8_t* to_coo, Scratch& sc,
+              cudaStream_t s) {
   const int64_t n = src->nnz;
   const int64_t slab = e->pitch * e->width;
   int st = fill<int32_t>(e->column_indices, MGB_INVALID_INDEX, slab, s);
   if (st) return st;
   if (slab) MGB_CUDA_CHECK(cudaMemsetAsync(e->values, 0, sizeof(T) * slab, s));
   if (n == 0) return MGB_SUCCESS;
-  const T* v = static_cast<const T*>(src->values);
-  T* ev = static_cast<T*>(e->values);
-  if (!collisions) {
-    ell_place<T><<<grid_for(n), 256, 0, s>>>(src->row_indices, src->column_indices, v, slot, n, W, e->pitch,
-                                             e->column_indices, ev, nullptr, 0, to_coo);
-    MGB_LAUNCH_CHECK();
-    return MGB_SUCCESS;
-  }
   int32_t* owner;
   MGB_SCRATCH(sc, owner, slab > 0 ? slab : 1);
   st = fill<int32_t>(owner, -1, slab, s);
   if (st) return st;
   for (int pass = 0; pass < 2; pass++) {
-    ell_place<T><<<grid_for(n), 256, 0, s>>>(src->row_indices, src->column_indices, v, slot, n, W, e->pitch,
-                                             e->column_indices, ev, owner, pass, to_coo);
+    ell_place<T><<<grid_for(n), 256, 0, s>>>(src->row_indices, src->column_indices,
+                                             static_cast<const T*>(src->values), slot, n, W, e->pitch,
+                                             e->column_indices, static_cast<T*>(e->values), owner, pass, to_coo);
     MGB_LAUNCH_CHECK();
   }
   return MGB_SUCCESS;
 }
 
-// The row histogram of a COO source (N + 1 entries, the last one zero),
-// queued with the validation, the rows-sorted flag and (width > 0) the
-// number of entries a width-W ELL part holds, or (width == 0) the longest
-// row; one host read.
+// ELL slab of row-sorted entries: a CTA takes R rows, brings their entries
+// (one contiguous range) through shared memory and writes every slot column
+// of the rows, padding included, in consecutive rows: the slab is written once
+// in full sectors and not cleared before.  Rows whose entries do not fit
+// ELL_TILE are read where they lie.  A pad after every 32 staged entries
+// spreads rows of even length over the banks.  Placing each entry alone into
+// a cleared slab: see the figures at launch_ell_fill.
+constexpr int ELL_TILE = 2048;
+constexpr int ELL_TILE_ROWS = 256;
+__device__ __forceinline__ int ell_pad(int i) { return i + (i >> 5); }
+
+template <typename T>
+__global__ void __launch_bounds__(256)
+ell_fill_tiles(const int32_t* __restrict__ c, const T* __restrict__ v, const int32_t* __restrict__ start,
+               int64_t nrows, int64_t pitch, int64_t width, int64_t W, int32_t* __restrict__ eci, T* __restrict__ ev,
+               int R) {
+  __shared__ T s_v[ELL_TILE + ELL_TILE / 32];
+  __shared__ int32_t s_c[ELL_TILE + ELL_TILE / 32];
+  __shared__ int32_t s_start[ELL_TILE_ROWS + 1];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t ntiles = (pitch + R - 1) / R;
+  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const int64_t r0 = t * R;
+    for (int q = threadIdx.x; q <= R; q += 256) s_start[q] = start[min(r0 + q, nrows)];
+    __syncthreads();
+    const int32_t e0 = s_start[0], n = s_start[R] - e0;
+    const bool staged = n <= ELL_TILE;
+    if (staged)
+      for (int i = threadIdx.x; i < n; i += 256) {
+        s_c[ell_pad(i)] = __ldcs(c + e0 + i);
+        s_v[ell_pad(i)] = __ldcs(v + e0 + i);
+      }
+    __syncthreads();
+    for (int q = lane; q < R; q += 32) {
+      const int64_t row = r0 + q;
+      if (row >= pitch) break;
+      const int32_t b = s_start[q];
+      const int64_t len = min((int64_t)(s_start[q + 1] - b), W);
+      for (int64_t k = w; k < width; k += 8) {
+        int32_t col = MGB_INVALID_INDEX;
+        T val = T(0);
+        if (k < len) {
+          const int i = b - e0 + (int)k;
+          col = staged ? s_c[ell_pad(i)] : __ldg(c + e0 + i);
+          val = staged ? s_v[ell_pad(i)] : __ldg(v + e0 + i);
+        }
+        __stcs(eci + row + pitch * k, col);
+        __stcs(ev + row + pitch * k, val);
+      }
+    }
+    __syncthreads();
+  }
+}
+
+template <typename T>
+int launch_ell_fill(const mgb_coo* src, const int32_t* start, mgb_ell* e, int64_t W, cudaStream_t s) {
+  if (e->pitch * e->width == 0) return MGB_SUCCESS;
+  // as many rows as keep the mean tile at 5/8 of the staging (rows of unequal length: most tiles fit)
+  const int64_t mean = src->nnz / std::max<int64_t>(1, src->nrows) + 1;
+  int R = ELL_TILE_ROWS;
+  while (R > 32 && R * mean > ELL_TILE * 5 / 8) R >>= 1;
+  ell_fill_tiles<T><<<blocks_for((e->pitch + R - 1) / R, 1, (int64_t)num_sms() * 8), 256, 0, s>>>(
+      src->column_indices, static_cast<const T*>(src->values), start, src->nrows, e->pitch, e->width, W,
+      e->column_indices, static_cast<T*>(e->values), R);
+  MGB_LAUNCH_CHECK();
+  return MGB_SUCCESS;
+}
+
+// HYB's COO part of row-sorted entries: excess[r] = the row's entries past
+// the ELL width; with their exclusive scan, one warp per 32 rows copies the
+// rows that have some.
+__global__ void row_excess(const int32_t* __restrict__ start, int64_t nrows, int64_t W, int32_t* excess) {
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += (int64_t)gridDim.x * blockDim.x)
+    excess[r] = (int32_t)max((int64_t)(start[r + 1] - start[r]) - W, (int64_t)0);
+}
+template <typename T>
+__global__ void __launch_bounds__(256)
+copy_excess(const int32_t* __restrict__ c, const T* __restrict__ v, const int32_t* __restrict__ start,
+            const int32_t* __restrict__ base, int64_t nrows, int64_t W, int32_t* __restrict__ orow,
+            int32_t* __restrict__ ocol, T* __restrict__ oval) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = (int64_t)gridDim.x * 8;
+  for (int64_t r0 = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * 32; r0 < nrows; r0 += warps * 32) {
+    const int64_t r = r0 + lane;
+    int32_t from = 0, n = 0, to = 0;
+    if (r < nrows) {
+      from = (int32_t)min((int64_t)start[r] + W, (int64_t)INT32_MAX);
+      n = max(start[r + 1] - from, 0);
+      to = base[r];
+    }
+    for (unsigned m = __ballot_sync(0xffffffffu, n > 0); m; m &= m - 1) {
+      const int j = __ffs(m) - 1;
+      const int32_t f = __shfl_sync(0xffffffffu, from, j), k = __shfl_sync(0xffffffffu, n, j);
+      const int32_t o = __shfl_sync(0xffffffffu, to, j);
+      for (int32_t i = lane; i < k; i += 32) {
+        orow[o + i] = (int32_t)(r0 + j);
+        ocol[o + i] = c[f + i];
+        oval[o + i] = v[f + i];
+      }
+    }
+  }
+}
+
+// The longest row and, for width > 0, the entries that a width-W ELL part
+// holds (sum of min(length, width)), over row starts or a row histogram.
+struct RowsFromStart {
+  const int32_t* p;
+  __device__ int operator()(int64_t r) const { return p[r + 1] - p[r]; }
+};
+struct RowsFromCounts {
+  const int32_t* p;
+  __device__ int operator()(int64_t r) const { return p[r]; }
+};
+template <typename LEN>
+__global__ void __launch_bounds__(256) row_sizes(LEN len, int64_t nrows, int64_t width, Words* d) {
+  __shared__ int64_t s_sum[8];
+  __shared__ int32_t s_max[8];
+  int64_t sum = 0;
+  int32_t mx = 0;
+  for (int64_t r = (int64_t)blockIdx.x * 256 + threadIdx.x; r < nrows; r += (int64_t)gridDim.x * 256) {
+    const int32_t n = len(r);
+    mx = max(mx, n);
+    sum += min((int64_t)n, width);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if ((threadIdx.x & 31) == 0) {
+    s_sum[threadIdx.x >> 5] = sum;
+    s_max[threadIdx.x >> 5] = mx;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < 8; i++) {
+      sum += s_sum[i];
+      mx = max(mx, s_max[i]);
+    }
+    atomicAdd(reinterpret_cast<unsigned long long*>(&d->total), (unsigned long long)sum);
+    atomicMax(&d->maxv, mx);
+  }
+}
+
+// COO -> ELL / HYB sizes: one pass over the indices (ranges, order, row
+// starts) and one over the rows; one host read.  A COO whose rows are not
+// sorted has no row starts: its row histogram and a second read follow.
 struct RowPlan {
-  int32_t* counts = nullptr;
+  int32_t* start = nullptr;
   Words h{};
 };
-int row_plan(const mgb_coo* src, int64_t width, RowPlan* p, Scratch& sc, cudaStream_t s);
+int row_plan(const mgb_coo* src, int64_t width, RowPlan* p, Scratch& sc, cudaStream_t s) {
+  const int64_t N = src->nrows;
+  Words* dw;
+  int st = words_alloc(sc, &dw, s);
+  if (st) return st;
+  MGB_SCRATCH(sc, p->start, N + 1);
+  st = prim::coo_pass(src->row_indices, src->column_indices, src->nnz, N, src->ncols, dw, nullptr, p->start, s);
+  if (st) return st;
+  const unsigned grid = blocks_for(N, 256, (int64_t)num_sms() * 8);
+  row_sizes<<<grid, 256, 0, s>>>(RowsFromStart{p->start}, N, width, dw);
+  MGB_LAUNCH_CHECK();
+  st = words_read(dw, &p->h, s);
+  if (st) return st;
+  if (!words_valid(p->h)) return MGB_ERR_INVALID_INPUT;
+  if (words_rows_sorted(p->h)) return MGB_SUCCESS;
+  const int32_t seen = p->h.seen;
+  MGB_CUDA_CHECK(cudaMemsetAsync(dw, 0, sizeof(Words), s));
+  st = prim::histogram(src->row_indices, src->nnz, p->start, N, s);
+  if (st) return st;
+  row_sizes<<<grid, 256, 0, s>>>(RowsFromCounts{p->start}, N, width, dw);
+  MGB_LAUNCH_CHECK();
+  st = words_read(dw, &p->h, s);
+  p->h.seen = seen;
+  return st;
+}
 
 int coo_to_ell_plan(const mgb_coo* src, int64_t* epr, cudaStream_t s) {
   MGB_REQUIRE(epr != nullptr, MGB_ERR_BAD_ARGUMENT);
@@ -874,48 +1008,17 @@ int coo_to_ell(const mgb_coo* src, mgb_ell* dst, cudaStream_t s) {
                   dst->entries_per_row == W && dst->width >= W && dst->pitch >= src->nrows,
               MGB_ERR_INVALID_INPUT);
   MGB_REQUIRE(dst->width * dst->pitch == 0 || (dst->column_indices && dst->values), MGB_ERR_BAD_ARGUMENT);
+  if (src->nrows == 0) return MGB_SUCCESS;
+  if (words_rows_sorted(p.h)) return launch_ell_fill<T>(src, p.start, dst, W, s);
   int32_t* slot;
   MGB_SCRATCH(sc, slot, src->nnz);
-  bool coll = false;
-  st = compute_slots(src, words_rows_sorted(p.h), p.counts, slot, &coll, sc, s);
+  st = compute_slots(src, slot, sc, s);
   if (st) return st;
-  return place_ell<T>(src, dst, W, slot, coll, nullptr, sc, s);
-}
-
-__global__ void sum_min_kernel(const int32_t* __restrict__ counts, int64_t n, int64_t W, unsigned long long* out) {
-  int64_t acc = 0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    acc += min((int64_t)counts[i], W);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(out, (unsigned long long)acc);
+  return place_ell<T>(src, dst, W, slot, nullptr, sc, s);
 }
 
 // impl/Hyb/Serial/Morpheus_Convert_Impl.hpp:110-151 (width = max(1, nnz/nrows)
 // unless the caller passes one)
-int row_plan(const mgb_coo* src, int64_t width, RowPlan* p, Scratch& sc, cudaStream_t s) {
-  const int64_t N = src->nrows;
-  Words* dw;
-  int st = words_alloc(sc, &dw, s);
-  if (st) return st;
-  st = prim::coo_pass(src->row_indices, src->column_indices, src->nnz, N, src->ncols, dw, nullptr, nullptr, s);
-  if (st) return st;
-  MGB_SCRATCH(sc, p->counts, N + 1);
-  st = prim::histogram(src->row_indices, src->nnz, p->counts, N, s);
-  if (st) return st;
-  MGB_CUDA_CHECK(cudaMemsetAsync(p->counts + N, 0, sizeof(int32_t), s));
-  if (width > 0) {
-    sum_min_kernel<<<grid_for(N), 256, 0, s>>>(p->counts, N, width, reinterpret_cast<unsigned long long*>(&dw->total));
-    MGB_LAUNCH_CHECK();
-  } else {
-    st = prim::reduce_max_i32(p->counts, N, &dw->maxv, s);
-    if (st) return st;
-  }
-  st = words_read(dw, &p->h, s);
-  if (st) return st;
-  return words_valid(p->h) ? MGB_SUCCESS : MGB_ERR_INVALID_INPUT;
-}
-
 int coo_to_hyb_plan(const mgb_coo* src, int64_t width, int64_t* epr, int64_t* ell_nnz, int64_t* coo_nnz,
                     cudaStream_t s) {
   MGB_REQUIRE(epr && ell_nnz && coo_nnz && width >= 0, MGB_ERR_BAD_ARGUMENT);
@@ -958,16 +1061,31 @@ int coo_to_hyb(const mgb_coo* src, mgb_hyb* dst, cudaStream_t s) {
   MGB_REQUIRE(e->width * e->pitch == 0 || (e->column_indices && e->values), MGB_ERR_BAD_ARGUMENT);
   MGB_REQUIRE(cn == 0 || (c->row_indices && c->column_indices && c->values), MGB_ERR_BAD_ARGUMENT);
   const int64_t n = src->nnz;
+  if (words_rows_sorted(p.h)) {
+    st = launch_ell_fill<T>(src, p.start, e, W, s);
+    if (st || cn == 0) return st;
+    int32_t *excess, *base;
+    MGB_SCRATCH(sc, excess, src->nrows);
+    MGB_SCRATCH(sc, base, src->nrows);
+    row_excess<<<grid_for(src->nrows), 256, 0, s>>>(p.start, src->nrows, W, excess);
+    MGB_LAUNCH_CHECK();
+    st = prim::exclusive_scan<int32_t, int32_t>(excess, base, src->nrows, s);
+    if (st) return st;
+    copy_excess<T><<<grid_for(src->nrows), 256, 0, s>>>(
+        src->column_indices, static_cast<const T*>(src->values), p.start, base, src->nrows, W, c->row_indices,
+        c->column_indices, static_cast<T*>(c->values));
+    MGB_LAUNCH_CHECK();
+    return MGB_SUCCESS;
+  }
   st = zero_coo<T>(c, s);
   if (st) return st;
   int32_t* slot;
   uint8_t* to_coo;
   MGB_SCRATCH(sc, slot, n);
   MGB_SCRATCH(sc, to_coo, n);
-  bool coll = false;
-  st = compute_slots(src, words_rows_sorted(p.h), p.counts, slot, &coll, sc, s);
+  st = compute_slots(src, slot, sc, s);
   if (st) return st;
-  st = place_ell<T>(src, e, W, slot, coll, to_coo, sc, s);
+  st = place_ell<T>(src, e, W, slot, to_coo, sc, s);
   if (st || n == 0) return st;
   int64_t* pos;
   MGB_SCRATCH(sc, pos, n);

@@ -66,3 +66,15 @@ def test_row_starts_over_gaps(cuda, gap, shift):
 
 def test_stencil_tiles(cuda):
     check_all_targets(gen.stencil_27pt(23, seed=5))
+
+
+# rows of a staged tile's limits (32 x 64 entries), even lengths, a row beyond the staging, a slab wider than the rows
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("N,lens,width", [(1, [3], 0), (257, [5], 4), (300, [16, 32], 0), (65, [64], 40),
+                                          (100, [63, 65], 33), (70, [0, 2500, 1, 0], 7), (511, [0, 1, 2], 1)])
+def test_ell_and_hyb_tiles(cuda, N, lens, width, dtype):
+    A = gen.random_lengths_csr(N, 4000, np.resize(np.asarray(lens), N), seed=N, dtype=dtype)
+    coo = gen.csr_to_coo_host(A)
+    for fmt, w in ((O.ELL, 0), (O.HYB, 0), (O.HYB, width)):
+        got, ref = both(coo, fmt, hyb_width=w)
+        assert_same_matrix(got, ref, f"{fmt} width {w}:")
