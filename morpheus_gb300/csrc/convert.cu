@@ -188,25 +188,28 @@ int coo_to_csr(const mgb_coo* src, mgb_csr* dst, cudaStream_t s) {
   Words* dw;
   int st = words_alloc(sc, &dw, s);
   if (st) return st;
-  st = prim::coo_pass(src->row_indices, src->column_indices, n, N, src->ncols, dw, nullptr, nullptr, s);
+  // sorted rows: the row starts are the offsets (a histogram and its scan before)
+  int32_t* start;
+  MGB_SCRATCH(sc, start, N + 1);
+  st = prim::coo_pass(src->row_indices, src->column_indices, n, N, src->ncols, dw, nullptr, start, s);
   if (st) return st;
   Words hw;
   st = words_read(dw, &hw, s);
   if (st) return st;
   if (!words_valid(hw)) return MGB_ERR_INVALID_INPUT;
-  int32_t* counts;
-  MGB_SCRATCH(sc, counts, N + 1);
-  st = prim::histogram(src->row_indices, n, counts, N, s);
-  if (st) return st;
-  MGB_CUDA_CHECK(cudaMemsetAsync(counts + N, 0, sizeof(int32_t), s));
-  st = prim::exclusive_scan<int32_t, int32_t>(counts, dst->row_offsets, N + 1, s);
-  if (st || n == 0) return st;
   if (words_rows_sorted(hw)) {
+    MGB_CUDA_CHECK(cudaMemcpyAsync(dst->row_offsets, start, sizeof(int32_t) * (N + 1), cudaMemcpyDeviceToDevice, s));
+    if (n == 0) return MGB_SUCCESS;
     MGB_CUDA_CHECK(cudaMemcpyAsync(dst->column_indices, src->column_indices, sizeof(int32_t) * n,
                                    cudaMemcpyDeviceToDevice, s));
     MGB_CUDA_CHECK(cudaMemcpyAsync(dst->values, src->values, sizeof(T) * n, cudaMemcpyDeviceToDevice, s));
     return MGB_SUCCESS;
   }
+  st = prim::histogram(src->row_indices, n, start, N, s);
+  if (st) return st;
+  MGB_CUDA_CHECK(cudaMemsetAsync(start + N, 0, sizeof(int32_t), s));
+  st = prim::exclusive_scan<int32_t, int32_t>(start, dst->row_offsets, N + 1, s);
+  if (st) return st;
   // unsorted rows: stable partition by row (keys = COO position only)
   int32_t *zeros, *r2, *c2, *perm;
   MGB_SCRATCH(sc, zeros, n);
@@ -329,6 +332,7 @@ __global__ void dia_place(const int32_t* __restrict__ r, const int32_t* __restri
 // slot array.
 constexpr int DIA_TILE_THREADS = 256;
 constexpr int DIA_TILE_BYTES = 32 * 1024;
+constexpr int DIA_TILE_ROWS = 512;  // at most
 constexpr int DIA_HASH_DIAGS = 256;  // at most a quarter of the table's slots
 constexpr int DIA_HASH_SLOTS = 1024;
 constexpr int32_t DIA_HASH_FREE = INT32_MIN;  // no offset: |offset| < 2^31 - 1
@@ -369,18 +373,22 @@ __device__ __forceinline__ int dia_table_find(DiaTable t, int32_t d) {
   return t.slot[h];
 }
 
-template <typename T>
+// REM (HDC): also rem[row] = the row's entries on no stored diagonal.
+template <typename T, bool REM>
 __global__ void __launch_bounds__(DIA_TILE_THREADS)
 dia_fill_tiles(const int32_t* __restrict__ r, const int32_t* __restrict__ c, const T* __restrict__ v,
                const int32_t* __restrict__ start, int64_t nrows, int64_t pitch, int nd,
-               const int32_t* __restrict__ offs, const int32_t* __restrict__ bin_slot, T* __restrict__ out, int R,
-               int D) {
+               const int32_t* __restrict__ offs, const int32_t* __restrict__ bin_slot, T* __restrict__ out,
+               int32_t* __restrict__ rem, int R, int D) {
   extern __shared__ __align__(16) unsigned char dia_smem[];
   T* tile = reinterpret_cast<T*>(dia_smem);
   __shared__ int32_t h_key[DIA_HASH_SLOTS], h_slot[DIA_HASH_SLOTS];
+  __shared__ int32_t s_rem[REM ? DIA_TILE_ROWS : 1];
   const DiaTable table{h_key, h_slot};
   const bool hashed = nd <= DIA_HASH_DIAGS;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, S = R + 1;
+  if constexpr (REM)
+    for (int i = threadIdx.x; i < R; i += DIA_TILE_THREADS) s_rem[i] = 0;
   if (hashed) dia_table_clear(table);
   for (int i = threadIdx.x; i < D * S; i += DIA_TILE_THREADS) tile[i] = T(0);
   __syncthreads();
@@ -408,11 +416,18 @@ dia_fill_tiles(const int32_t* __restrict__ r, const int32_t* __restrict__ c, con
         for (int k = 0; k < 4; k++)
           if (e + k * DIA_TILE_THREADS < e1) {
             const int32_t d = col[k] - row[k];
-            const int s = (hashed ? dia_table_find(table, d) : bin_slot[(int64_t)d + nrows - 1]) - d0;
+            const int found = hashed ? dia_table_find(table, d) : bin_slot[(int64_t)d + nrows - 1];
+            const int s = found - d0;
             if (s >= 0 && s < dn) tile[s * S + (int)(row[k] - r0)] = val[k];
+            if (REM && found < 0 && d0 == 0) atomicAdd(s_rem + (int)(row[k] - r0), 1);
           }
       }
       __syncthreads();
+      if (REM && d0 == 0)
+        for (int q = threadIdx.x; q < R; q += DIA_TILE_THREADS) {
+          if (r0 + q < nrows) rem[r0 + q] = s_rem[q];
+          s_rem[q] = 0;
+        }
       for (int d = w; d < dn; d += DIA_TILE_THREADS / 32)
         for (int q = lane; q < R; q += 32) {
           if (r0 + q < pitch) __stcs(out + r0 + q + pitch * (int64_t)(d0 + d), tile[d * S + q]);
@@ -428,7 +443,7 @@ dia_fill_tiles(const int32_t* __restrict__ r, const int32_t* __restrict__ c, con
 // (the rows' entries are then read once per group of diagonals).
 template <typename T>
 void dia_tile_shape(int64_t nd, int* R, int* D) {
-  *R = 512;
+  *R = DIA_TILE_ROWS;
   while (*R > 32 && nd * (*R + 1) * (int64_t)sizeof(T) > DIA_TILE_BYTES) *R >>= 1;
   *D = (int)std::min<int64_t>(nd, DIA_TILE_BYTES / ((*R + 1) * (int64_t)sizeof(T)));
 }
@@ -438,19 +453,26 @@ constexpr int64_t DIA_TILE_GROUPS = 16;
 
 template <typename T>
 int launch_dia_fill(const mgb_coo* src, const int32_t* start, int64_t pitch, int64_t nd, const int32_t* offs,
-                    const int32_t* bin_slot, T* out, cudaStream_t s) {
+                    const int32_t* bin_slot, T* out, int32_t* rem, cudaStream_t s) {
   int R, D;
   dia_tile_shape<T>(nd, &R, &D);
   const size_t smem = sizeof(T) * (size_t)D * (R + 1);
   const unsigned grid = blocks_for((pitch + R - 1) / R, 1, (int64_t)num_sms() * 8);
-  dia_fill_tiles<T><<<grid, DIA_TILE_THREADS, smem, s>>>(src->row_indices, src->column_indices,
-                                                         static_cast<const T*>(src->values), start, src->nrows, pitch,
-                                                         (int)nd, offs, bin_slot, out, R, D);
+  const T* v = static_cast<const T*>(src->values);
+  if (rem != nullptr)
+    dia_fill_tiles<T, true><<<grid, DIA_TILE_THREADS, smem, s>>>(src->row_indices, src->column_indices, v, start,
+                                                                 src->nrows, pitch, (int)nd, offs, bin_slot, out, rem,
+                                                                 R, D);
+  else
+    dia_fill_tiles<T, false><<<grid, DIA_TILE_THREADS, smem, s>>>(src->row_indices, src->column_indices, v, start,
+                                                                  src->nrows, pitch, (int)nd, offs, bin_slot, out,
+                                                                  nullptr, R, D);
   MGB_LAUNCH_CHECK();
   return MGB_SUCCESS;
 }
 template <typename T>
 bool dia_tiled(int64_t nd) {
+  if (nd == 0) return false;
   int R, D;
   dia_tile_shape<T>(nd, &R, &D);
   return (nd + D - 1) / D <= DIA_TILE_GROUPS;
@@ -529,7 +551,7 @@ int coo_to_dia(const mgb_coo* src, mgb_dia* dst, cudaStream_t s) {
   T* out = static_cast<T*>(dst->values);
   const bool distinct = words_distinct(p.h);
   if (distinct && dia_tiled<T>(nd))
-    return launch_dia_fill<T>(src, p.start, dst->pitch, nd, dst->diagonal_offsets, slot, out, s);
+    return launch_dia_fill<T>(src, p.start, dst->pitch, nd, dst->diagonal_offsets, slot, out, nullptr, s);
   MGB_CUDA_CHECK(cudaMemsetAsync(dst->values, 0, sizeof(T) * dst->pitch * nd, s));
   if (distinct) {
     dia_place<T><<<grid_for(n), 256, 0, s>>>(src->row_indices, src->column_indices, v, n, src->nrows, slot,
@@ -1158,15 +1180,64 @@ __global__ void hdc_dia_place(const int32_t* __restrict__ r, const T* __restrict
   }
 }
 
+// CSR remainder of row-sorted entries: base = the exclusive scan of the rows'
+// remainders.  Entries are row-sorted, so those of 32 rows that lie on no
+// stored diagonal go, in order, to the consecutive places from base[first
+// row] on: one warp per 32 rows, ranks by ballot.
+template <typename T>
+__global__ void __launch_bounds__(256)
+hdc_remainder(const int32_t* __restrict__ r, const int32_t* __restrict__ c, const T* __restrict__ v,
+              const int32_t* __restrict__ start, const int32_t* __restrict__ base, int64_t nrows, int nd,
+              const int32_t* __restrict__ offs, const int32_t* __restrict__ bin_slot, int64_t limit,
+              int32_t* __restrict__ ocol, T* __restrict__ oval) {
+  __shared__ int32_t h_key[DIA_HASH_SLOTS], h_slot[DIA_HASH_SLOTS];
+  const DiaTable table{h_key, h_slot};
+  const bool hashed = nd <= DIA_HASH_DIAGS;
+  if (hashed) dia_table_clear(table);
+  __syncthreads();
+  if (hashed) dia_table_fill(table, offs, nd);
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = (int64_t)gridDim.x * 8;
+  for (int64_t r0 = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * 32; r0 < nrows; r0 += warps * 32) {
+    const int64_t r1 = min(r0 + 32, nrows);
+    const int64_t e1 = start[r1];
+    int64_t to = base[r0];
+    if (to == base[r1]) continue;  // every entry on a stored diagonal
+    for (int64_t e0 = start[r0]; e0 < e1; e0 += 128) {
+      int32_t row[4], col[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const int64_t e = e0 + 32 * k + lane;
+        row[k] = e < e1 ? __ldcs(r + e) : 0;
+        col[k] = e < e1 ? __ldcs(c + e) : 0;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const int64_t e = e0 + 32 * k + lane;
+        const int32_t d = col[k] - row[k];
+        const bool miss = e < e1 && (hashed ? dia_table_find(table, d) : bin_slot[(int64_t)d + nrows - 1]) < 0;
+        const unsigned m = __ballot_sync(0xffffffffu, miss);
+        const int64_t p = to + __popc(m & ((1u << lane) - 1));
+        if (miss && p < limit) {
+          ocol[p] = col[k];
+          oval[p] = v[e];
+        }
+        to += __popc(m);
+      }
+    }
+  }
+}
+
 // COO -> HDC sizes: one pass over the indices as for DIA, then the true
 // diagonals (>= floor(0.2 N) entries) and their entry count; one host read.
 struct HdcPlan {
-  int32_t* counts = nullptr;
+  int32_t *counts = nullptr, *start = nullptr;
   int64_t* sums = nullptr;
   int32_t min_elem = 0;
   Words h{};
 };
-int hdc_plan(const mgb_coo* src, HdcPlan* p, Scratch& sc, cudaStream_t s) {
+int hdc_plan(const mgb_coo* src, bool starts, HdcPlan* p, Scratch& sc, cudaStream_t s) {
   int st = check_coo_args(src);
   if (st) return st;
   MGB_REQUIRE(src->nrows > 0 && src->ncols > 0, MGB_ERR_INVALID_INPUT);
@@ -1177,8 +1248,9 @@ int hdc_plan(const mgb_coo* src, HdcPlan* p, Scratch& sc, cudaStream_t s) {
   if (st) return st;
   MGB_SCRATCH(sc, p->counts, nb);
   MGB_SCRATCH(sc, p->sums, prim::bin_tiles(nb));
-  st = prim::coo_pass(src->row_indices, src->column_indices, src->nnz, src->nrows, src->ncols, dw, p->counts, nullptr,
-                      s);
+  if (starts) MGB_SCRATCH(sc, p->start, src->nrows + 1);
+  st = prim::coo_pass(src->row_indices, src->column_indices, src->nnz, src->nrows, src->ncols, dw, p->counts,
+                      p->start, s);
   if (st) return st;
   st = prim::select_bins(p->counts, nb, p->min_elem, p->sums, &dw->total, &dw->total2, s);
   if (st) return st;
@@ -1193,7 +1265,7 @@ int coo_to_hdc_plan(const mgb_coo* src, int64_t* ndiags, int64_t* dia_nnz, int64
   MGB_REQUIRE(ndiags && dia_nnz && csr_nnz, MGB_ERR_BAD_ARGUMENT);
   Scratch sc(s);
   HdcPlan p;
-  const int st = hdc_plan(src, &p, sc, s);
+  const int st = hdc_plan(src, false, &p, sc, s);
   if (st == MGB_SUCCESS || st == MGB_ERR_FORMAT_CONVERSION) {
     *ndiags = p.h.total;
     *dia_nnz = p.h.total2;
@@ -1207,7 +1279,7 @@ int coo_to_hdc(const mgb_coo* src, mgb_hdc* dst, cudaStream_t s) {
   MGB_REQUIRE(dst != nullptr, MGB_ERR_BAD_ARGUMENT);
   Scratch sc(s);
   HdcPlan p;
-  int st = hdc_plan(src, &p, sc, s);
+  int st = hdc_plan(src, true, &p, sc, s);
   if (st) return st;
   const int64_t nd = p.h.total, dn = p.h.total2, cn = src->nnz - p.h.total2;
   mgb_dia* D = &dst->dia;
@@ -1223,18 +1295,51 @@ int coo_to_hdc(const mgb_coo* src, mgb_hdc* dst, cudaStream_t s) {
     // the midpoint bin is recorded as offset 0 (exact only for square matrices)
     st = prim::select_bins_apply(p.counts, nb, p.min_elem, p.sums, N, nb / 2, D->diagonal_offsets, s);
     if (st) return st;
-    // std::sort of the stored offsets (impl/Hdc/Serial/Morpheus_Convert_Impl.hpp:193-195)
-    std::vector<int32_t> h((size_t)nd);
-    MGB_CUDA_CHECK(cudaMemcpyAsync(h.data(), D->diagonal_offsets, sizeof(int32_t) * nd, cudaMemcpyDeviceToHost, s));
-    MGB_CUDA_CHECK(cudaStreamSynchronize(s));
-    std::sort(h.begin(), h.end());
-    MGB_CUDA_CHECK(cudaMemcpyAsync(D->diagonal_offsets, h.data(), sizeof(int32_t) * nd, cudaMemcpyHostToDevice, s));
-    MGB_CUDA_CHECK(cudaMemsetAsync(D->values, 0, sizeof(T) * D->pitch * nd, s));
+    // std::sort of the stored offsets (impl/Hdc/Serial/Morpheus_Convert_Impl.hpp:193-195):
+    // they are in order already unless the midpoint bin is not offset 0
+    if (src->nrows != src->ncols) {
+      std::vector<int32_t> h((size_t)nd);
+      MGB_CUDA_CHECK(cudaMemcpyAsync(h.data(), D->diagonal_offsets, sizeof(int32_t) * nd, cudaMemcpyDeviceToHost, s));
+      MGB_CUDA_CHECK(cudaStreamSynchronize(s));
+      std::sort(h.begin(), h.end());
+      MGB_CUDA_CHECK(cudaMemcpyAsync(D->diagonal_offsets, h.data(), sizeof(int32_t) * nd, cudaMemcpyHostToDevice, s));
+      MGB_CUDA_CHECK(cudaStreamSynchronize(s));  // h lives on this stack frame
+    }
   }
   if (n == 0) {
+    if (nd > 0) MGB_CUDA_CHECK(cudaMemsetAsync(D->values, 0, sizeof(T) * D->pitch * nd, s));
     MGB_CUDA_CHECK(cudaMemsetAsync(C->row_offsets, 0, sizeof(int32_t) * (N + 1), s));
     return MGB_SUCCESS;
   }
+  const T* v = static_cast<const T*>(src->values);
+  // A square matrix's bins are its offsets, so the entries off the true
+  // diagonals are exactly the cn counted ones; the midpoint bin of another
+  // shape is not (below).
+  if (src->nrows == src->ncols && words_distinct(p.h)) {
+    if (nd == 0) {
+      MGB_CUDA_CHECK(cudaMemcpyAsync(C->row_offsets, p.start, sizeof(int32_t) * (N + 1), cudaMemcpyDeviceToDevice, s));
+      MGB_CUDA_CHECK(cudaMemcpyAsync(C->column_indices, src->column_indices, sizeof(int32_t) * n,
+                                     cudaMemcpyDeviceToDevice, s));
+      MGB_CUDA_CHECK(cudaMemcpyAsync(C->values, v, sizeof(T) * n, cudaMemcpyDeviceToDevice, s));
+      return MGB_SUCCESS;
+    }
+    if (dia_tiled<T>(nd)) {
+      int32_t* rem;
+      MGB_SCRATCH(sc, rem, N + 1);
+      MGB_CUDA_CHECK(cudaMemsetAsync(rem + N, 0, sizeof(int32_t), s));
+      st = launch_dia_fill<T>(src, p.start, D->pitch, nd, D->diagonal_offsets, p.counts, static_cast<T*>(D->values),
+                              rem, s);
+      if (st) return st;
+      st = prim::exclusive_scan<int32_t, int32_t>(rem, C->row_offsets, N + 1, s);
+      if (st || cn == 0) return st;
+      hdc_remainder<T><<<blocks_for(N, 256, (int64_t)num_sms() * 8), 256, 0, s>>>(
+          src->row_indices, src->column_indices, v, p.start, C->row_offsets, N, (int)nd, D->diagonal_offsets, p.counts,
+          cn, C->column_indices, static_cast<T*>(C->values));
+      MGB_LAUNCH_CHECK();
+      return MGB_SUCCESS;
+    }
+  }
+  if (nd > 0) MGB_CUDA_CHECK(cudaMemsetAsync(D->values, 0, sizeof(T) * D->pitch * nd, s));
   int32_t* dslot;
   uint8_t* is_csr;
   int64_t *cpos, *d_csr;
@@ -1250,7 +1355,6 @@ int coo_to_hdc(const mgb_coo* src, mgb_hdc* dst, cudaStream_t s) {
   // a non-square matrix with a true diagonal in the midpoint bin sends more
   // entries to CSR than were counted (the reference writes out of bounds):
   // the scatter below stops at cn, and the count is checked at the end
-  const T* v = static_cast<const T*>(src->values);
   if (nd > 0) {
     if (words_distinct(p.h)) {
       hdc_dia_place<T><<<grid_for(n), 256, 0, s>>>(src->row_indices, v, dslot, n, D->pitch, static_cast<T*>(D->values),

@@ -78,3 +78,12 @@ def test_ell_and_hyb_tiles(cuda, N, lens, width, dtype):
     for fmt, w in ((O.ELL, 0), (O.HYB, 0), (O.HYB, width)):
         got, ref = both(coo, fmt, hyb_width=w)
         assert_same_matrix(got, ref, f"{fmt} width {w}:")
+
+
+# all, some or none of the entries on true diagonals; more true diagonals than the lookup table takes
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("N,nd,keep", [(3, 3, 1.0), (64, 5, 0.9), (513, 40, 0.6), (700, 500, 0.5), (1200, 1500, 0.4),
+                                       (400, 300, 0.1)])
+def test_hdc_tiles(cuda, N, nd, keep, dtype):
+    got, ref = both(diagonals(N, N, nd, seed=nd, dtype=dtype, keep=keep), O.HDC)
+    assert_same_matrix(got, ref)
