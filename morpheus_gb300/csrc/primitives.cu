@@ -152,24 +152,30 @@ __global__ void sorted_flags_kernel(const int32_t* __restrict__ r, const int32_t
 // Row starts: the entry where the row changes from p to q is the start of
 // the rows p + 1..q; gaps longer than PASS_GAP are left to the whole CTA at
 // the end, and the rows before the first and after the last entry to the grid.
+// Rows that go down make the starts useless, and entries in random order have
+// gaps of a third of the matrix each: the first such row that a CTA sees stops
+// the writing of starts in that CTA at once and in the others at their next
+// tile.
 constexpr uint32_t PASS_GAP = 256;
 constexpr int PASS_GAPS = 256;
 
 template <bool DIAG, bool STARTS>
 __global__ void __launch_bounds__(256) coo_pass_kernel(const int32_t* __restrict__ r, const int32_t* __restrict__ c,
                                                        int64_t n, int64_t nrows, int64_t ncols, bool vec,
-                                                       int32_t* __restrict__ seen, int32_t* __restrict__ diag,
+                                                       int32_t* seen, int32_t* __restrict__ diag,
                                                        int32_t* __restrict__ start) {
   __shared__ uint32_t h_keys[DIAG ? HIST_SLOTS : 1];
   __shared__ int32_t h_counts[DIAG ? HIST_SLOTS : 1];
   __shared__ int h_full;
   __shared__ int32_t gap_from[STARTS ? PASS_GAPS : 1], gap_to[STARTS ? PASS_GAPS : 1], gap_at[STARTS ? PASS_GAPS : 1];
-  __shared__ int ngaps, s_bits;
+  __shared__ int ngaps, s_bits, s_stop;
+  volatile int* stop = &s_stop;
   const CtaHist h{h_keys, h_counts, &h_full};
   if constexpr (DIAG) hist_init(h);
   if (threadIdx.x == 0) {
     ngaps = 0;
     s_bits = 0;
+    s_stop = 0;
   }
   __syncthreads();
   const int lane = threadIdx.x & 31;
@@ -181,6 +187,7 @@ __global__ void __launch_bounds__(256) coo_pass_kernel(const int32_t* __restrict
   for (int64_t base = (int64_t)blockIdx.x * 1024; base < n; base += (int64_t)gridDim.x * 1024) {
     const int64_t i0 = base + (int64_t)threadIdx.x * 4;
     const int m = (int)min((int64_t)4, n - i0);  // this thread's entries (<= 0: none)
+    if (STARTS && (*reinterpret_cast<volatile int32_t*>(seen) & COO_ROWS_UNSORTED)) *stop = 1;
     uint32_t rr[4] = {0, 0, 0, 0}, cc[4] = {0, 0, 0, 0};
     if (vec && m == 4) {
       const int4 a = __ldg(reinterpret_cast<const int4*>(r + i0)), b = __ldg(reinterpret_cast<const int4*>(c + i0));
@@ -203,11 +210,17 @@ __global__ void __launch_bounds__(256) coo_pass_kernel(const int32_t* __restrict
         down |= cc[k] < pc;
         equal |= cc[k] == pc && (k > 0 || i0 > 0);
       } else {
-        rows_down |= rr[k] < pr;
+        if (rr[k] < pr) {
+          rows_down = true;
+          if (STARTS && !*stop) {
+            *stop = 1;
+            atomicOr(seen, COO_ROWS_UNSORTED);
+          }
+        }
         if constexpr (STARTS) {
           if (rr[k] == pr + 1) {
             if (rr[k] < nr) start[rr[k]] = (int32_t)(i0 + k);
-          } else if (rr[k] > pr && rr[k] < nr) {
+          } else if (rr[k] > pr && rr[k] < nr && !*stop) {
             const int32_t at = (int32_t)(i0 + k);
             int g = PASS_GAPS;
             if (rr[k] - pr > PASS_GAP) g = atomicAdd(&ngaps, 1);
@@ -233,7 +246,7 @@ __global__ void __launch_bounds__(256) coo_pass_kernel(const int32_t* __restrict
   if (threadIdx.x == 0 && s_bits) atomicOr(seen, s_bits);
   if constexpr (DIAG) hist_flush(h, diag);
   if constexpr (STARTS) {
-    for (int g = 0; g < min(ngaps, PASS_GAPS); g++)
+    for (int g = 0; g < (s_stop ? 0 : min(ngaps, PASS_GAPS)); g++)
       for (int64_t q = (int64_t)gap_from[g] + threadIdx.x; q <= gap_to[g]; q += 256) start[q] = gap_at[g];
     const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x, nt = (int64_t)gridDim.x * 256;
     const int64_t first = n > 0 ? min((int64_t)r[0], nrows) : nrows;
