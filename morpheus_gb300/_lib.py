@@ -56,6 +56,10 @@ class Hdc(C.Structure):
     _fields_ = [("dia", Dia), ("csr", Csr)]
 
 
+class CooPlan(C.Structure):
+    _fields_ = [("sizes", i64 * 3), ("format", C.c_int32), ("seen", C.c_int32), ("parts", vp * 3)]
+
+
 # name -> (restype, argtypes)
 _SIGS: dict[str, tuple] = {
     "mgb_status_string": (C.c_char_p, [C.c_int]),
@@ -127,6 +131,9 @@ _SIGS["mgb_convert_coo_to_hyb_plan"] = (C.c_int, [_P(Coo), i64, _P(i64), _P(i64)
 _SIGS["mgb_convert_coo_to_hdc_plan"] = (C.c_int, [_P(Coo), _P(i64), _P(i64), _P(i64), vp])
 for _dt in ("f64", "f32"):
     _SIGS[f"mgb_coo_sort_by_row_and_column_{_dt}"] = (C.c_int, [_P(Coo), vp])
+    _SIGS[f"mgb_convert_coo_planned_{_dt}"] = (C.c_int, [_P(Coo), _P(CooPlan), vp, vp])
+_SIGS["mgb_convert_coo_workspace_bytes"] = (C.c_int, [_P(Coo), C.c_int, _P(i64)])
+_SIGS["mgb_convert_coo_plan"] = (C.c_int, [_P(Coo), C.c_int, i64, vp, i64, _P(CooPlan), vp])
 _SIGS["mgb_coo_is_sorted"] = (C.c_int, [_P(Coo), _P(C.c_int), vp])
 _SIGS["mgb_peak_dfma_f64"] = (C.c_int, [i64, i64, vp, vp])
 _SIGS["mgb_peak_gather_f64"] = (C.c_int, [vp, i64, i64, i64, vp, vp])

@@ -43,10 +43,6 @@ def _empty(n, dtype, device) -> torch.Tensor:
     return torch.empty(int(n), dtype=dtype, device=device)
 
 
-def _i64():
-    return C.c_int64()
-
-
 def to_coo(A: _Matrix, stream=None) -> CooMatrix:
     """Any container -> a new COO container (the reference's X -> COO)."""
     if isinstance(A, DynamicMatrix):
@@ -114,26 +110,29 @@ def from_coo(coo: CooMatrix, fmt: int, hyb_width: int = 0, stream=None) -> _Matr
         return to_coo(coo)
     if fmt == CSR_FORMAT:
         out = _new_csr(n, m, z, dt, dev)
-    elif fmt == DIA_FORMAT:
-        nd = _i64()
-        _call("mgb_convert_coo_to_dia_plan", C.byref(sd), C.byref(nd), sh)
-        out = _new_dia(n, m, z, nd.value, dt, dev)
-    elif fmt == ELL_FORMAT:
-        w = _i64()
-        _call("mgb_convert_coo_to_ell_plan", C.byref(sd), C.byref(w), sh)
-        out = _new_ell(n, m, z, w.value, dt, dev)
-    elif fmt == HYB_FORMAT:
-        w, en, cn = _i64(), _i64(), _i64()
-        _call("mgb_convert_coo_to_hyb_plan", C.byref(sd), int(hyb_width), C.byref(w), C.byref(en), C.byref(cn), sh)
-        out = HybMatrix(_new_ell(n, m, en.value, w.value, dt, dev), _new_coo(n, m, cn.value, dt, dev), dt, dev)
-    elif fmt == HDC_FORMAT:
-        nd, dn, cn = _i64(), _i64(), _i64()
-        _call("mgb_convert_coo_to_hdc_plan", C.byref(sd), C.byref(nd), C.byref(dn), C.byref(cn), sh)
-        out = HdcMatrix(_new_dia(n, m, dn.value, nd.value, dt, dev), _new_csr(n, m, cn.value, dt, dev), dt, dev)
-    else:
+        dd = out._desc()
+        _call(f"mgb_convert_coo_to_csr_{sfx}", C.byref(sd), C.byref(dd), sh)
+        return out
+    if fmt not in _NAME:
         raise NotImplementedException(f"format {fmt}")
+    nb, plan = C.c_int64(), _lib.CooPlan()
+    _call("mgb_convert_coo_workspace_bytes", C.byref(sd), fmt, C.byref(nb))
+    ws = _empty(nb.value, torch.uint8, dev)
+    if stream is not None:  # the block goes back to the current stream's pool, the kernels run on this one
+        ws.record_stream(stream if isinstance(stream, torch.cuda.Stream) else torch.cuda.ExternalStream(int(stream)))
+    _call("mgb_convert_coo_plan", C.byref(sd), fmt, int(hyb_width), C.c_void_p(ws.data_ptr()), nb.value,
+          C.byref(plan), sh)
+    s0, s1, s2 = plan.sizes
+    if fmt == DIA_FORMAT:
+        out = _new_dia(n, m, z, s0, dt, dev)
+    elif fmt == ELL_FORMAT:
+        out = _new_ell(n, m, z, s0, dt, dev)
+    elif fmt == HYB_FORMAT:
+        out = HybMatrix(_new_ell(n, m, s1, s0, dt, dev), _new_coo(n, m, s2, dt, dev), dt, dev)
+    else:
+        out = HdcMatrix(_new_dia(n, m, s1, s0, dt, dev), _new_csr(n, m, s2, dt, dev), dt, dev)
     dd = out._desc()
-    _call(f"mgb_convert_coo_to_{_NAME[fmt]}_{sfx}", C.byref(sd), C.byref(dd), sh)
+    _call(f"mgb_convert_coo_planned_{sfx}", C.byref(sd), C.byref(plan), C.byref(dd), sh)
     return out
 
 

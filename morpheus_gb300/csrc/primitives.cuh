@@ -9,15 +9,28 @@ namespace mgb {
 namespace prim {
 
 // RAII stream-ordered scratch; freed with cudaFreeAsync on the same stream.
+// A caller's workspace, where there is one, is used up first (256-byte
+// pieces, in the order asked for; never freed here).
 class Scratch {
  public:
-  explicit Scratch(cudaStream_t s) : s_(s) {}
+  explicit Scratch(cudaStream_t s, void* workspace = nullptr, size_t bytes = 0)
+      : s_(s), ws_(static_cast<char*>(workspace)), left_(workspace ? bytes : 0) {}
   ~Scratch() {
     for (int i = 0; i < n_; i++) cudaFreeAsync(p_[i], s_);
   }
+  Scratch(const Scratch&) = delete;
+  Scratch& operator=(const Scratch&) = delete;
+  static size_t padded(size_t bytes) { return (bytes + 255) / 256 * 256; }
   template <typename T>
   cudaError_t get(T** out, size_t count) {
     *out = nullptr;
+    const size_t need = padded(count ? count * sizeof(T) : 16);
+    if (need <= left_) {
+      *out = reinterpret_cast<T*>(ws_);
+      ws_ += need;
+      left_ -= need;
+      return cudaSuccess;
+    }
     if (n_ >= 32) return cudaErrorMemoryAllocation;
     void* p = nullptr;
     cudaError_t e = cudaMallocAsync(&p, count ? count * sizeof(T) : 16, s_);
@@ -30,6 +43,8 @@ class Scratch {
 
  private:
   cudaStream_t s_;
+  char* ws_;
+  size_t left_;
   void* p_[32];
   int n_ = 0;
 };

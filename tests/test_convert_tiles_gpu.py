@@ -87,3 +87,44 @@ def test_ell_and_hyb_tiles(cuda, N, lens, width, dtype):
 def test_hdc_tiles(cuda, N, nd, keep, dtype):
     got, ref = both(diagonals(N, N, nd, seed=nd, dtype=dtype, keep=keep), O.HDC)
     assert_same_matrix(got, ref)
+
+
+def _two_call(A, fmt, like):
+    """The conversion through its own *_plan and fill entry points, into a container of `like`'s sizes."""
+    import ctypes as C
+
+    import morpheus_gb300 as mgb
+    from morpheus_gb300 import _lib
+    from morpheus_gb300.convert import _new_coo, _new_csr, _new_dia, _new_ell
+    name = {2: "dia", 3: "ell", 4: "hyb", 5: "hdc"}[fmt]
+    sd, sizes = A._desc(), [C.c_int64() for _ in range(1 if fmt < 4 else 3)]
+    more = [0] if fmt == 4 else []
+    _lib.call(f"mgb_convert_coo_to_{name}_plan", C.byref(sd), *more, *[C.byref(z) for z in sizes], None)
+    n, m, z, dt, dev = A.nrows(), A.ncols(), A.nnnz(), A.dtype, A.device
+    s = [v.value for v in sizes]
+    out = {2: lambda: _new_dia(n, m, z, s[0], dt, dev), 3: lambda: _new_ell(n, m, z, s[0], dt, dev),
+           4: lambda: mgb.HybMatrix(_new_ell(n, m, s[1], s[0], dt, dev), _new_coo(n, m, s[2], dt, dev), dt, dev),
+           5: lambda: mgb.HdcMatrix(_new_dia(n, m, s[1], s[0], dt, dev), _new_csr(n, m, s[2], dt, dev), dt, dev)}[fmt]()
+    dd = out._desc()
+    _lib.call(f"mgb_convert_coo_to_{name}_f64", C.byref(sd), C.byref(dd), None)
+    return mgb.matrix_to_host(out)
+
+
+@pytest.mark.parametrize("fmt", [2, 3, 4, 5])
+@pytest.mark.parametrize("shuffled", [False, True])
+def test_planned_conversion_equals_separate_calls(cuda, fmt, shuffled):
+    import torch
+
+    import morpheus_gb300 as mgb
+    hm = diagonals(301, 301, 60, seed=fmt, dtype=np.float64)
+    if shuffled:
+        p = np.random.default_rng(1).permutation(hm["nnz"])
+        hm = dict(hm, row_indices=hm["row_indices"][p], column_indices=hm["column_indices"][p], values=hm["values"][p])
+    A = mgb.matrix_from_host(hm)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    planned = mgb.from_coo(A, fmt, stream=side)
+    side.synchronize()
+    got = mgb.matrix_to_host(planned)
+    assert_same_matrix(got, _two_call(A, fmt, planned))
+    assert_same_matrix(got, O.OracleMatrix.from_host(hm).convert(fmt).to_host())
