@@ -112,6 +112,9 @@ int mgb_version(void);
 
 /* Text of the last CUDA error seen by this thread (static storage). */
 const char* mgb_last_cuda_error_string(void);
+/* Gives back the device memory that the library's scratch pool of the current
+ * device keeps between calls (at most 32 MiB).  Synchronises the device. */
+int mgb_scratch_release(void);
 
 /* ---- SpMV: y = A*x (init != 0) or y += A*x (init == 0) ------------------
  * Morpheus::multiply<ExecSpace>(A, x, y[, init])
@@ -173,7 +176,7 @@ int mgb_spmv_coo_f32(const mgb_coo* A, const float* x, float* y, int init, void*
  * reference.  For callers that may not allocate device memory while they run
  * (real-time loops that forbid allocation once running, hosts that reserve all
  * device memory up front, plugins whose host owns the allocator): the carry
- * buffer is a fixed 4 MiB file-scope device array instead of cudaMallocAsync,
+ * buffer is a fixed 4 MiB file-scope device array instead of pool scratch,
  * and no allocating call is made.  Limits: A->nnz <= 357,892,096, otherwise
  * MGB_ERR_INVALID_INPUT before any work is queued; every GPU that loads the
  * library holds the 4 MiB until exit; the first call on a device looks up the

@@ -65,6 +65,7 @@ _SIGS: dict[str, tuple] = {
     "mgb_status_string": (C.c_char_p, [C.c_int]),
     "mgb_version": (C.c_int, []),
     "mgb_last_cuda_error_string": (C.c_char_p, []),
+    "mgb_scratch_release": (C.c_int, []),
 }
 for _fmt, _st in (("csr", Csr), ("coo", Coo), ("dia", Dia), ("ell", Ell), ("hyb", Hyb), ("hdc", Hdc)):
     for _dt in ("f64", "f32"):

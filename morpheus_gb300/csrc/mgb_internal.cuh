@@ -22,6 +22,12 @@ int num_sms();
 // MGB_ERR_CUDA once after a failed num_sms() query on this thread, else MGB_SUCCESS.
 int take_device_query_error();
 
+// Unique ID of the current CUDA context (0: unknown).
+unsigned long long current_ctx_id();
+
+// Stream-ordered scratch from the library's pool (freed with cudaFreeAsync).
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
+
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 }  // namespace mgb

@@ -1,6 +1,6 @@
 // primitives.cuh -- device-wide building blocks for the GPU conversions:
 // exclusive scan, reductions, stable (row, col) sort of COO entries and
-// per-row segmented sort.  All scratch is stream-ordered (cudaMallocAsync).
+// per-row segmented sort.  All scratch is stream-ordered.
 #pragma once
 
 #include "mgb_internal.cuh"
@@ -33,7 +33,7 @@ class Scratch {
     }
     if (n_ >= 32) return cudaErrorMemoryAllocation;
     void* p = nullptr;
-    cudaError_t e = cudaMallocAsync(&p, count ? count * sizeof(T) : 16, s_);
+    cudaError_t e = scratch_alloc(&p, count ? count * sizeof(T) : 16, s_);
     if (e == cudaSuccess) {
       p_[n_++] = p;
       *out = static_cast<T*>(p);

@@ -238,7 +238,7 @@ int grad(const float* params, const float* mu, const float* sigma, const float* 
   }
   const int64_t nblocks = (n + G_SAMPLES - 1) / G_SAMPLES;
   float* scratch = nullptr;
-  MGB_CUDA_CHECK(cudaMallocAsync((void**)&scratch, sizeof(float) * nblocks * (NPARAMS + 1), s));
+  MGB_CUDA_CHECK(scratch_alloc((void**)&scratch, sizeof(float) * nblocks * (NPARAMS + 1), s));
   float* partial = scratch;
   float* lpart = scratch + nblocks * NPARAMS;
   mlp_grad_kernel<<<(unsigned)nblocks, G_WARPS * 32, grad_smem(), s>>>(params, mu, sigma, X, labels, mask, n,

@@ -197,7 +197,7 @@ int launch_coo(const mgb_coo* A, const T* x, T* y, int init, cudaStream_t s) {
   const int64_t ncarry = 2 * nchunks;
   void* scratch = nullptr;
   const size_t rows_bytes = ((sizeof(int32_t) * ncarry + 255) / 256) * 256;
-  MGB_CUDA_CHECK(cudaMallocAsync(&scratch, rows_bytes + sizeof(T) * ncarry, s));
+  MGB_CUDA_CHECK(scratch_alloc(&scratch, rows_bytes + sizeof(T) * ncarry, s));
   int32_t* cr = static_cast<int32_t*>(scratch);
   T* cv = reinterpret_cast<T*>(static_cast<char*>(scratch) + rows_bytes);
   const int64_t blocks = (nchunks + COO_WARPS - 1) / COO_WARPS;
@@ -244,7 +244,7 @@ int mgb_spmv_coo_f32(const mgb_coo* A, const float* x, float* y, int init, void*
 // loops of a host application that forbids allocation once it is running,
 // embedded hosts that reserve all device memory up front, and plugins whose
 // host process owns the allocator.  mgb_spmv_coo_f64 takes
-// its carry buffer from cudaMallocAsync; this variant takes it from a fixed
+// its carry buffer from the library's scratch pool; this variant takes it from a fixed
 // file-scope device array instead, so it never calls cudaMalloc, cudaFree or
 // any allocating routine.
 //
@@ -267,8 +267,6 @@ int mgb_spmv_coo_f32(const mgb_coo* A, const float* x, float* y, int init, void*
 //    carry slot it reads.  Calls that overlap on the GPU (other streams, other
 //    host threads) race on the array; serialise them.
 // ---------------------------------------------------------------------------
-#include <cuda.h>  // CUcontext / CUresult types only: the driver calls are resolved at run time
-
 #include <mutex>
 
 namespace mgb {
@@ -288,35 +286,6 @@ struct NoallocSlot {
 };
 std::mutex g_noalloc_mutex;
 NoallocSlot g_noalloc[128] = {};
-
-// cuCtxGetCurrent / cuCtxGetId through the runtime's driver entry points (no
-// link against the driver library).  Context IDs are unique for the life of
-// the process, unlike context handles, which a new context may reuse.
-using CtxGetCurrentFn = CUresult (*)(CUcontext*);
-using CtxGetIdFn = CUresult (*)(CUcontext, unsigned long long*);
-
-unsigned long long current_ctx_id() {
-  static CtxGetCurrentFn get_current = nullptr;
-  static CtxGetIdFn get_id = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      get_current = reinterpret_cast<CtxGetCurrentFn>(f);
-    f = nullptr;
-    if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      get_id = reinterpret_cast<CtxGetIdFn>(f);
-  });
-  CUcontext c = nullptr;
-  unsigned long long id = 0;
-  if (get_current == nullptr || get_id == nullptr || get_current(&c) != CUDA_SUCCESS || c == nullptr ||
-      get_id(c, &id) != CUDA_SUCCESS)
-    return 0;
-  return id;
-}
 
 // Device address of the scratch array in the current context: looked up on
 // the first call per device and again whenever the current context changed.

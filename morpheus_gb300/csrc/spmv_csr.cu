@@ -165,7 +165,7 @@ int launch_split(const mgb_csr* A, const T* x, T* y, int init, cudaStream_t s, T
     const int64_t ncarry = 2 * nchunks;
     void* scratch = nullptr;
     const size_t rows_bytes = ((sizeof(int32_t) * (size_t)ncarry + 255) / 256) * 256;
-    MGB_CUDA_CHECK(cudaMallocAsync(&scratch, rows_bytes + sizeof(T) * (size_t)ncarry, s));
+    MGB_CUDA_CHECK(scratch_alloc(&scratch, rows_bytes + sizeof(T) * (size_t)ncarry, s));
     int32_t* cr = static_cast<int32_t*>(scratch);
     T* cv = reinterpret_cast<T*>(static_cast<char*>(scratch) + rows_bytes);
     int64_t blocks = (nchunks + CSR_WARPS - 1) / CSR_WARPS;

@@ -314,7 +314,7 @@ int choose(const mgb_csr* A, int* variant, cudaStream_t s) {
   if (A->nrows == 0 || A->nnz == 0) return MGB_SUCCESS;
   MGB_REQUIRE(A->row_offsets != nullptr && A->column_indices != nullptr, MGB_ERR_BAD_ARGUMENT);
   unsigned long long* d = nullptr;
-  MGB_CUDA_CHECK(cudaMallocAsync((void**)&d, 3 * sizeof(unsigned long long), s));
+  MGB_CUDA_CHECK(scratch_alloc((void**)&d, 3 * sizeof(unsigned long long), s));
   cudaError_t e = cudaMemsetAsync(d, 0, 3 * sizeof(unsigned long long), s);
   if (e == cudaSuccess) {
     int64_t blocks = (A->nrows + 255) / 256;

@@ -15,7 +15,7 @@
 // Reductions: a grid of at most 4 CTAs per SM accumulates with one FMA (dot)
 // or add (reduce) per element and 16-byte loads, reduces in-CTA with
 // shuffles, and a one-CTA kernel sums the per-CTA partials.  The partials live
-// in stream-ordered scratch (cudaMallocAsync), so no global state is shared
+// in stream-ordered scratch, so no global state is shared
 // between calls or streams.
 #include "mgb_internal.cuh"
 
@@ -197,7 +197,7 @@ int launch_reduce(int64_t n, const T* x, const T* y, T* d_result, cudaStream_t s
   const int64_t cap = (int64_t)num_sms() * 4;
   if (blocks > cap) blocks = cap;
   T* partial = nullptr;
-  MGB_CUDA_CHECK(cudaMallocAsync((void**)&partial, sizeof(T) * blocks, s));
+  MGB_CUDA_CHECK(scratch_alloc((void**)&partial, sizeof(T) * blocks, s));
   reduce_partial<T, MODE><<<(unsigned)blocks, RED_THREADS, 0, s>>>(n, x, y, partial);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) {
@@ -214,7 +214,7 @@ template <typename T, int MODE>
 int reduce_to_host(int64_t n, const T* x, const T* y, T* result, cudaStream_t s) {
   MGB_REQUIRE(result != nullptr, MGB_ERR_BAD_ARGUMENT);
   T* d = nullptr;
-  MGB_CUDA_CHECK(cudaMallocAsync((void**)&d, sizeof(T), s));
+  MGB_CUDA_CHECK(scratch_alloc((void**)&d, sizeof(T), s));
   int st = launch_reduce<T, MODE>(n, x, y, d, s);
   if (st == MGB_SUCCESS) {
     cudaError_t e = cudaMemcpyAsync(result, d, sizeof(T), cudaMemcpyDeviceToHost, s);
