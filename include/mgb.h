@@ -436,17 +436,20 @@ int mgb_convert_coo_to_hdc_plan(const mgb_coo* src, int64_t* ndiags, int64_t* di
 int mgb_convert_coo_to_hdc_f64(const mgb_coo* src, mgb_hdc* dst, void* stream);
 int mgb_convert_coo_to_hdc_f32(const mgb_coo* src, mgb_hdc* dst, void* stream);
 
-/* COO -> DIA / ELL / HYB / HDC (format: formats_e 2..5) in two calls that read
- * the indices for the sizes once: the plan call has the semantics of the
+/* COO -> CSR / DIA / ELL / HYB / HDC (format: formats_e 1..5) in two calls that
+ * read the indices for the sizes once: the plan call has the semantics of the
  * *_plan calls above and keeps what it found in the caller's workspace (device
  * memory, 256-byte aligned, workspace_bytes of it), the planned call fills
- * dst (an mgb_dia / mgb_ell / mgb_hyb / mgb_hdc by plan->format) like the
- * conversions above.  sizes: DIA {ndiags}; ELL {entries_per_row}; HYB
- * {entries_per_row, ELL nnz, COO nnz}; HDC {ndiags, DIA nnz, CSR nnz}.  A plan is
- * good for one fill of the same source, on a stream ordered after the plan
- * call's; the workspace may be freed once that fill has run. */
+ * dst (an mgb_csr / mgb_dia / mgb_ell / mgb_hyb / mgb_hdc by plan->format) like
+ * the conversions above.  sizes: DIA {ndiags}; ELL {entries_per_row}; HYB
+ * {entries_per_row, ELL nnz, COO nnz}; HDC {ndiags, DIA nnz, CSR nnz}.  The planned
+ * call takes fill_bytes of a second workspace (same alignment; null: it
+ * allocates).  A plan is good for one fill of the same source, on a stream
+ * ordered after the plan call's; the workspaces may be freed once that fill has
+ * run. */
 typedef struct {
   int64_t sizes[3];
+  int64_t fill_bytes;
   int32_t format;
   int32_t seen;   /* internal */
   void* parts[3]; /* internal: pointers into the workspace */
@@ -454,12 +457,19 @@ typedef struct {
 int mgb_convert_coo_workspace_bytes(const mgb_coo* src, int format, int64_t* bytes);
 int mgb_convert_coo_plan(const mgb_coo* src, int format, int64_t hyb_width, void* workspace, int64_t bytes,
                          mgb_coo_plan* plan, void* stream);
-int mgb_convert_coo_planned_f64(const mgb_coo* src, const mgb_coo_plan* plan, void* dst, void* stream);
-int mgb_convert_coo_planned_f32(const mgb_coo* src, const mgb_coo_plan* plan, void* dst, void* stream);
+int mgb_convert_coo_planned_f64(const mgb_coo* src, const mgb_coo_plan* plan, void* dst, void* workspace,
+                                int64_t bytes, void* stream);
+int mgb_convert_coo_planned_f32(const mgb_coo* src, const mgb_coo_plan* plan, void* dst, void* workspace,
+                                int64_t bytes, void* stream);
 
 /* In-place stable sort by (row, column): impl/Coo/Serial/Morpheus_Sort_Impl.hpp:109-164 */
 int mgb_coo_sort_by_row_and_column_f64(mgb_coo* A, void* stream);
 int mgb_coo_sort_by_row_and_column_f32(mgb_coo* A, void* stream);
+/* The same with its scratch in the caller's workspace (device memory, 256-byte
+ * aligned; what does not fit is allocated). */
+int mgb_coo_sort_workspace_bytes(const mgb_coo* A, int64_t* bytes);
+int mgb_coo_sort_by_row_and_column_ws_f64(mgb_coo* A, void* workspace, int64_t bytes, void* stream);
+int mgb_coo_sort_by_row_and_column_ws_f32(mgb_coo* A, void* workspace, int64_t bytes, void* stream);
 /* impl/Coo/Serial/Morpheus_Sort_Impl.hpp:166-186; *sorted = 1 or 0 */
 int mgb_coo_is_sorted(const mgb_coo* A, int* sorted, void* stream);
 

@@ -23,7 +23,7 @@ from . import _lib
 from .algorithms import _stream_handle, _suffix
 from .containers import (COO_FORMAT, CSR_FORMAT, DIA_FORMAT, ELL_FORMAT, HDC_FORMAT, HYB_FORMAT, NFORMATS,
                          CooMatrix, CsrMatrix, DiaMatrix, DynamicMatrix, EllMatrix, HdcMatrix, HybMatrix,
-                         _Matrix, conversion_error_e, formats_e, get_pad_size)
+                         _Matrix, _ptr, conversion_error_e, formats_e, get_pad_size)
 from .exceptions import MorpheusException, NotImplementedException
 
 _NAME = {COO_FORMAT: "coo", CSR_FORMAT: "csr", DIA_FORMAT: "dia", ELL_FORMAT: "ell", HYB_FORMAT: "hyb",
@@ -41,6 +41,15 @@ def _call(name, *args):
 
 def _empty(n, dtype, device) -> torch.Tensor:
     return torch.empty(int(n), dtype=dtype, device=device)
+
+
+def _workspace(nbytes: int, device, stream) -> torch.Tensor:
+    """Scratch of a call on `stream`, from torch's pool of the current stream
+    (given back to it once the call's kernels have run)."""
+    ws = _empty(nbytes, torch.uint8, device)
+    if stream is not None and nbytes:
+        ws.record_stream(stream if isinstance(stream, torch.cuda.Stream) else torch.cuda.ExternalStream(int(stream)))
+    return ws
 
 
 def to_coo(A: _Matrix, stream=None) -> CooMatrix:
@@ -108,20 +117,14 @@ def from_coo(coo: CooMatrix, fmt: int, hyb_width: int = 0, stream=None) -> _Matr
     fmt = int(fmt)
     if fmt == COO_FORMAT:
         return to_coo(coo)
-    if fmt == CSR_FORMAT:
-        out = _new_csr(n, m, z, dt, dev)
-        dd = out._desc()
-        _call(f"mgb_convert_coo_to_csr_{sfx}", C.byref(sd), C.byref(dd), sh)
-        return out
     if fmt not in _NAME:
         raise NotImplementedException(f"format {fmt}")
     nb, plan = C.c_int64(), _lib.CooPlan()
     _call("mgb_convert_coo_workspace_bytes", C.byref(sd), fmt, C.byref(nb))
-    ws = _empty(nb.value, torch.uint8, dev)
-    if stream is not None:  # the block goes back to the current stream's pool, the kernels run on this one
-        ws.record_stream(stream if isinstance(stream, torch.cuda.Stream) else torch.cuda.ExternalStream(int(stream)))
-    _call("mgb_convert_coo_plan", C.byref(sd), fmt, int(hyb_width), C.c_void_p(ws.data_ptr()), nb.value,
-          C.byref(plan), sh)
+    ws = _workspace(nb.value, dev, stream)
+    # sizes known before the plan: allocate while the GPU still has work queued
+    out = _new_csr(n, m, z, dt, dev) if fmt == CSR_FORMAT else None
+    _call("mgb_convert_coo_plan", C.byref(sd), fmt, int(hyb_width), _ptr(ws), nb.value, C.byref(plan), sh)
     s0, s1, s2 = plan.sizes
     if fmt == DIA_FORMAT:
         out = _new_dia(n, m, z, s0, dt, dev)
@@ -129,10 +132,11 @@ def from_coo(coo: CooMatrix, fmt: int, hyb_width: int = 0, stream=None) -> _Matr
         out = _new_ell(n, m, z, s0, dt, dev)
     elif fmt == HYB_FORMAT:
         out = HybMatrix(_new_ell(n, m, s1, s0, dt, dev), _new_coo(n, m, s2, dt, dev), dt, dev)
-    else:
+    elif fmt == HDC_FORMAT:
         out = HdcMatrix(_new_dia(n, m, s1, s0, dt, dev), _new_csr(n, m, s2, dt, dev), dt, dev)
     dd = out._desc()
-    _call(f"mgb_convert_coo_planned_{sfx}", C.byref(sd), C.byref(plan), C.byref(dd), sh)
+    fill = _workspace(plan.fill_bytes, dev, stream) if plan.fill_bytes else None
+    _call(f"mgb_convert_coo_planned_{sfx}", C.byref(sd), C.byref(plan), C.byref(dd), _ptr(fill), plan.fill_bytes, sh)
     return out
 
 
@@ -186,8 +190,11 @@ def convert_inplace(dyn: DynamicMatrix, fmt, stream=None, hyb_width: int = 0) ->
 
 def sort_by_row_and_column(A: CooMatrix, stream=None) -> None:
     _dev_check(A)
-    d = A._desc()
-    _call(f"mgb_coo_sort_by_row_and_column_{_suffix(A.dtype)}", C.byref(d), _stream_handle(stream))
+    d, nb = A._desc(), C.c_int64()
+    _call("mgb_coo_sort_workspace_bytes", C.byref(d), C.byref(nb))
+    ws = _workspace(nb.value, A.device, stream)
+    _call(f"mgb_coo_sort_by_row_and_column_ws_{_suffix(A.dtype)}", C.byref(d), _ptr(ws), nb.value,
+          _stream_handle(stream))
 
 
 def is_sorted(A: CooMatrix, stream=None) -> bool:

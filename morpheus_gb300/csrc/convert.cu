@@ -74,31 +74,11 @@ int sorted_and_dup(const int32_t* r, const int32_t* c, int64_t n, bool* sorted, 
   return MGB_SUCCESS;
 }
 
-template <typename T>
-__global__ void gather_values(const T* __restrict__ src, const int32_t* __restrict__ perm, T* dst, int64_t n) {
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
-    dst[k] = src[perm[k]];
-}
-
 // In-place stable (row, col) sort of a COO array with rows in [0, nbins).
 template <typename T>
-int sort_coo_inplace(int32_t* rows, int32_t* cols, T* vals, int64_t n, int64_t nbins, cudaStream_t s) {
+int sort_coo_inplace(int32_t* rows, int32_t* cols, T* vals, int64_t n, int64_t nbins, Scratch& sc, cudaStream_t s) {
   if (n <= 1) return MGB_SUCCESS;
-  Scratch sc(s);
-  int32_t *r2, *c2, *perm;
-  T* v2;
-  MGB_SCRATCH(sc, r2, n);
-  MGB_SCRATCH(sc, c2, n);
-  MGB_SCRATCH(sc, perm, n);
-  MGB_SCRATCH(sc, v2, n);
-  int st = prim::stable_sort_rows_cols(rows, cols, n, nbins, r2, c2, perm, s);
-  if (st) return st;
-  gather_values<T><<<grid_for(n), 256, 0, s>>>(vals, perm, v2, n);
-  MGB_LAUNCH_CHECK();
-  MGB_CUDA_CHECK(cudaMemcpyAsync(rows, r2, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, s));
-  MGB_CUDA_CHECK(cudaMemcpyAsync(cols, c2, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, s));
-  MGB_CUDA_CHECK(cudaMemcpyAsync(vals, v2, sizeof(T) * n, cudaMemcpyDeviceToDevice, s));
-  return MGB_SUCCESS;
+  return prim::row_sort<T, true>(rows, cols, vals, n, nbins, nullptr, rows, cols, vals, sc, s);
 }
 
 // The reference's "if (!is_sorted(dst)) sort_by_row_and_column(dst)" on a
@@ -109,8 +89,9 @@ int sort_if_unsorted(mgb_coo* dst, cudaStream_t s) {
   bool sorted = false;
   int st = sorted_and_dup(dst->row_indices, dst->column_indices, dst->nnz, &sorted, nullptr, s);
   if (st || sorted) return st;
+  Scratch sc(s);
   return sort_coo_inplace<T>(dst->row_indices, dst->column_indices, static_cast<T*>(dst->values), dst->nnz,
-                             dst->nrows, s);
+                             dst->nrows, sc, s);
 }
 
 int check_coo_dst(const mgb_coo* d, int64_t nrows, int64_t ncols, int64_t nnz) {
@@ -178,53 +159,49 @@ int csr_to_coo(const mgb_csr* src, mgb_coo* dst, cudaStream_t s) {
 }
 
 // impl/Csr/Serial/Morpheus_Convert_Impl.hpp:99-151: counting scatter, COO order within a row
+struct CsrPlan {
+  int32_t* start = nullptr;  // of sorted rows: the row offsets
+  Words h{};
+};
+int csr_plan(const mgb_coo* src, CsrPlan* p, Scratch& sc, cudaStream_t s) {
+  Words* dw;
+  int st = words_alloc(sc, &dw, s);
+  if (st) return st;
+  MGB_SCRATCH(sc, p->start, src->nrows + 1);
+  st = prim::coo_pass(src->row_indices, src->column_indices, src->nnz, src->nrows, src->ncols, dw, nullptr, p->start,
+                      s);
+  if (st) return st;
+  st = words_read(dw, &p->h, s);
+  if (st) return st;
+  return words_valid(p->h) ? MGB_SUCCESS : MGB_ERR_INVALID_INPUT;
+}
+
+template <typename T>
+int csr_fill(const mgb_coo* src, const CsrPlan& p, mgb_csr* dst, Scratch& sc, cudaStream_t s) {
+  const int64_t n = src->nnz, N = src->nrows;
+  MGB_REQUIRE(dst->nrows == N && dst->ncols == src->ncols && dst->nnz == n, MGB_ERR_INVALID_INPUT);
+  MGB_REQUIRE(dst->row_offsets != nullptr, MGB_ERR_BAD_ARGUMENT);
+  if (!words_rows_sorted(p.h))
+    return prim::row_sort<T, false>(src->row_indices, src->column_indices, static_cast<const T*>(src->values), n, N,
+                                    dst->row_offsets, nullptr, dst->column_indices, static_cast<T*>(dst->values), sc,
+                                    s);
+  MGB_CUDA_CHECK(cudaMemcpyAsync(dst->row_offsets, p.start, sizeof(int32_t) * (N + 1), cudaMemcpyDeviceToDevice, s));
+  if (n == 0) return MGB_SUCCESS;
+  MGB_CUDA_CHECK(cudaMemcpyAsync(dst->column_indices, src->column_indices, sizeof(int32_t) * n,
+                                 cudaMemcpyDeviceToDevice, s));
+  MGB_CUDA_CHECK(cudaMemcpyAsync(dst->values, src->values, sizeof(T) * n, cudaMemcpyDeviceToDevice, s));
+  return MGB_SUCCESS;
+}
+
 template <typename T>
 int coo_to_csr(const mgb_coo* src, mgb_csr* dst, cudaStream_t s) {
   MGB_REQUIRE(src != nullptr && dst != nullptr, MGB_ERR_BAD_ARGUMENT);
   MGB_REQUIRE(dst->nrows == src->nrows && dst->ncols == src->ncols && dst->nnz == src->nnz, MGB_ERR_INVALID_INPUT);
   MGB_REQUIRE(dst->row_offsets != nullptr, MGB_ERR_BAD_ARGUMENT);
-  const int64_t n = src->nnz, N = src->nrows;
   Scratch sc(s);
-  Words* dw;
-  int st = words_alloc(sc, &dw, s);
-  if (st) return st;
-  // sorted rows: the row starts are the offsets (a histogram and its scan before)
-  int32_t* start;
-  MGB_SCRATCH(sc, start, N + 1);
-  st = prim::coo_pass(src->row_indices, src->column_indices, n, N, src->ncols, dw, nullptr, start, s);
-  if (st) return st;
-  Words hw;
-  st = words_read(dw, &hw, s);
-  if (st) return st;
-  if (!words_valid(hw)) return MGB_ERR_INVALID_INPUT;
-  if (words_rows_sorted(hw)) {
-    MGB_CUDA_CHECK(cudaMemcpyAsync(dst->row_offsets, start, sizeof(int32_t) * (N + 1), cudaMemcpyDeviceToDevice, s));
-    if (n == 0) return MGB_SUCCESS;
-    MGB_CUDA_CHECK(cudaMemcpyAsync(dst->column_indices, src->column_indices, sizeof(int32_t) * n,
-                                   cudaMemcpyDeviceToDevice, s));
-    MGB_CUDA_CHECK(cudaMemcpyAsync(dst->values, src->values, sizeof(T) * n, cudaMemcpyDeviceToDevice, s));
-    return MGB_SUCCESS;
-  }
-  st = prim::histogram(src->row_indices, n, start, N, s);
-  if (st) return st;
-  MGB_CUDA_CHECK(cudaMemsetAsync(start + N, 0, sizeof(int32_t), s));
-  st = prim::exclusive_scan<int32_t, int32_t>(start, dst->row_offsets, N + 1, s);
-  if (st) return st;
-  // unsorted rows: stable partition by row (keys = COO position only)
-  int32_t *zeros, *r2, *c2, *perm;
-  MGB_SCRATCH(sc, zeros, n);
-  MGB_SCRATCH(sc, r2, n);
-  MGB_SCRATCH(sc, c2, n);
-  MGB_SCRATCH(sc, perm, n);
-  MGB_CUDA_CHECK(cudaMemsetAsync(zeros, 0, sizeof(int32_t) * n, s));
-  st = prim::stable_sort_rows_cols(src->row_indices, zeros, n, N, r2, c2, perm, s);
-  if (st) return st;
-  gather_values<int32_t><<<grid_for(n), 256, 0, s>>>(src->column_indices, perm, dst->column_indices, n);
-  MGB_LAUNCH_CHECK();
-  gather_values<T><<<grid_for(n), 256, 0, s>>>(static_cast<const T*>(src->values), perm,
-                                                static_cast<T*>(dst->values), n);
-  MGB_LAUNCH_CHECK();
-  return MGB_SUCCESS;
+  CsrPlan p;
+  const int st = csr_plan(src, &p, sc, s);
+  return st ? st : csr_fill<T>(src, p, dst, sc, s);
 }
 
 // ---------------------------------------------------------------- DIA -> COO
@@ -480,11 +457,11 @@ bool dia_tiled(int64_t nd) {
 
 // Argument checks of a COO source (the index range checks are queued with
 // validate_async and read with the caller's other words).
-int check_coo_args(const mgb_coo* src) {
+int check_coo_args(const mgb_coo* src, bool diagonals = true) {
   MGB_REQUIRE(src != nullptr, MGB_ERR_BAD_ARGUMENT);
   MGB_REQUIRE(src->nrows >= 0 && src->ncols >= 0 && src->nnz >= 0, MGB_ERR_BAD_ARGUMENT);
   MGB_REQUIRE(src->nnz == 0 || (src->row_indices && src->column_indices && src->values), MGB_ERR_BAD_ARGUMENT);
-  MGB_REQUIRE(src->nrows + src->ncols < INT32_MAX, MGB_ERR_INVALID_INPUT);
+  MGB_REQUIRE(!diagonals || src->nrows + src->ncols < INT32_MAX, MGB_ERR_INVALID_INPUT);
   return MGB_SUCCESS;
 }
 
@@ -1437,7 +1414,7 @@ int coo_to_hdc(const mgb_coo* src, mgb_hdc* dst, cudaStream_t s) {
 // read for the sizes once, where a *_plan call and its conversion each read
 // them (260 us of 2,342 for the selector's switch of the 160^3 stencil), and
 // nothing that size is allocated.
-enum { PLAN_DIA = 2, PLAN_ELL = 3, PLAN_HYB = 4, PLAN_HDC = 5 };  // formats_e
+enum { PLAN_CSR = 1, PLAN_DIA = 2, PLAN_ELL = 3, PLAN_HYB = 4, PLAN_HDC = 5 };  // formats_e
 
 size_t plan_bytes(const mgb_coo* src, int format) {
   size_t b = Scratch::padded(sizeof(Words)) + Scratch::padded(sizeof(int32_t) * (size_t)(src->nrows + 1));
@@ -1448,8 +1425,8 @@ size_t plan_bytes(const mgb_coo* src, int format) {
 }
 
 int coo_plan_bytes(const mgb_coo* src, int format, int64_t* bytes) {
-  MGB_REQUIRE(bytes != nullptr && format >= PLAN_DIA && format <= PLAN_HDC, MGB_ERR_BAD_ARGUMENT);
-  int st = check_coo_args(src);
+  MGB_REQUIRE(bytes != nullptr && format >= PLAN_CSR && format <= PLAN_HDC, MGB_ERR_BAD_ARGUMENT);
+  int st = check_coo_args(src, format != PLAN_CSR);
   if (st) return st;
   *bytes = (int64_t)plan_bytes(src, format);
   return MGB_SUCCESS;
@@ -1457,8 +1434,8 @@ int coo_plan_bytes(const mgb_coo* src, int format, int64_t* bytes) {
 
 int coo_plan(const mgb_coo* src, int format, int64_t hyb_width, void* ws, int64_t bytes, mgb_coo_plan* plan,
              cudaStream_t s) {
-  MGB_REQUIRE(plan != nullptr && format >= PLAN_DIA && format <= PLAN_HDC, MGB_ERR_BAD_ARGUMENT);
-  int st = check_coo_args(src);
+  MGB_REQUIRE(plan != nullptr && format >= PLAN_CSR && format <= PLAN_HDC, MGB_ERR_BAD_ARGUMENT);
+  int st = check_coo_args(src, format != PLAN_CSR);
   if (st) return st;
   MGB_REQUIRE(ws != nullptr && reinterpret_cast<uintptr_t>(ws) % 256 == 0 &&
                   bytes >= (int64_t)plan_bytes(src, format),
@@ -1466,7 +1443,13 @@ int coo_plan(const mgb_coo* src, int format, int64_t hyb_width, void* ws, int64_
   *plan = mgb_coo_plan{};
   plan->format = format;
   Scratch sc(s, ws, (size_t)bytes);
-  if (format == PLAN_DIA) {
+  if (format == PLAN_CSR) {
+    CsrPlan p;
+    st = csr_plan(src, &p, sc, s);
+    plan->seen = p.h.seen;
+    plan->parts[1] = p.start;
+    if (!words_rows_sorted(p.h)) plan->fill_bytes = prim::row_sort_bytes(src->nnz, src->nrows);
+  } else if (format == PLAN_DIA) {
     DiaPlan p;
     st = dia_plan(src, true, &p, sc, s);
     plan->sizes[0] = p.h.total;
@@ -1499,9 +1482,9 @@ int coo_plan(const mgb_coo* src, int format, int64_t hyb_width, void* ws, int64_
 }
 
 template <typename T>
-int coo_planned(const mgb_coo* src, const mgb_coo_plan* plan, void* dst, cudaStream_t s) {
+int coo_planned(const mgb_coo* src, const mgb_coo_plan* plan, void* dst, void* ws, int64_t bytes, cudaStream_t s) {
   MGB_REQUIRE(plan != nullptr && dst != nullptr, MGB_ERR_BAD_ARGUMENT);
-  int st = check_coo_args(src);
+  int st = check_coo_args(src, plan->format != PLAN_CSR);
   if (st) return st;
   auto* counts = static_cast<int32_t*>(plan->parts[0]);
   auto* start = static_cast<int32_t*>(plan->parts[1]);
@@ -1509,6 +1492,13 @@ int coo_planned(const mgb_coo* src, const mgb_coo_plan* plan, void* dst, cudaStr
   Words h{};
   h.seen = plan->seen;
   h.total = plan->sizes[0];
+  if (plan->format == PLAN_CSR) {
+    MGB_REQUIRE(ws == nullptr || reinterpret_cast<uintptr_t>(ws) % 256 == 0, MGB_ERR_BAD_ARGUMENT);
+    Scratch sc(s, ws, (size_t)std::max<int64_t>(bytes, 0));
+    CsrPlan p;
+    p.start = start, p.h = h;
+    return csr_fill<T>(src, p, static_cast<mgb_csr*>(dst), sc, s);
+  }
   if (plan->format == PLAN_DIA) {
     DiaPlan p;
     p.counts = counts, p.start = start, p.sums = sums, p.h = h;
@@ -1534,11 +1524,12 @@ int coo_planned(const mgb_coo* src, const mgb_coo_plan* plan, void* dst, cudaStr
 
 // ---------------------------------------------------------------- sort API
 template <typename T>
-int coo_sort(mgb_coo* A, cudaStream_t s) {
+int coo_sort(mgb_coo* A, void* ws, int64_t bytes, cudaStream_t s) {
   MGB_REQUIRE(A != nullptr && A->nnz >= 0, MGB_ERR_BAD_ARGUMENT);
   if (A->nnz <= 1) return MGB_SUCCESS;
   MGB_REQUIRE(A->row_indices && A->column_indices && A->values, MGB_ERR_BAD_ARGUMENT);
-  Scratch sc(s);
+  MGB_REQUIRE(ws == nullptr || reinterpret_cast<uintptr_t>(ws) % 256 == 0, MGB_ERR_BAD_ARGUMENT);
+  Scratch sc(s, ws, (size_t)std::max<int64_t>(bytes, 0));
   Words* dw;
   int st = words_alloc(sc, &dw, s);
   if (st) return st;
@@ -1552,7 +1543,7 @@ int coo_sort(mgb_coo* A, cudaStream_t s) {
   if (st) return st;
   if (!words_valid(hw)) return MGB_ERR_INVALID_INPUT;
   return sort_coo_inplace<T>(A->row_indices, A->column_indices, static_cast<T*>(A->values), A->nnz,
-                             (int64_t)hw.maxv + 1, s);
+                             (int64_t)hw.maxv + 1, sc, s);
 }
 
 int coo_is_sorted(const mgb_coo* A, int* out, cudaStream_t s) {
@@ -1611,17 +1602,30 @@ int mgb_convert_coo_plan(const mgb_coo* src, int format, int64_t hyb_width, void
                          mgb_coo_plan* plan, void* stream) {
   return mgb::coo_plan(src, format, hyb_width, workspace, bytes, plan, mgb::as_stream(stream));
 }
-int mgb_convert_coo_planned_f64(const mgb_coo* src, const mgb_coo_plan* plan, void* dst, void* stream) {
-  return mgb::coo_planned<double>(src, plan, dst, mgb::as_stream(stream));
+int mgb_convert_coo_planned_f64(const mgb_coo* src, const mgb_coo_plan* plan, void* dst, void* workspace,
+                                int64_t bytes, void* stream) {
+  return mgb::coo_planned<double>(src, plan, dst, workspace, bytes, mgb::as_stream(stream));
 }
-int mgb_convert_coo_planned_f32(const mgb_coo* src, const mgb_coo_plan* plan, void* dst, void* stream) {
-  return mgb::coo_planned<float>(src, plan, dst, mgb::as_stream(stream));
+int mgb_convert_coo_planned_f32(const mgb_coo* src, const mgb_coo_plan* plan, void* dst, void* workspace,
+                                int64_t bytes, void* stream) {
+  return mgb::coo_planned<float>(src, plan, dst, workspace, bytes, mgb::as_stream(stream));
 }
 int mgb_coo_sort_by_row_and_column_f64(mgb_coo* A, void* stream) {
-  return mgb::coo_sort<double>(A, mgb::as_stream(stream));
+  return mgb::coo_sort<double>(A, nullptr, 0, mgb::as_stream(stream));
 }
 int mgb_coo_sort_by_row_and_column_f32(mgb_coo* A, void* stream) {
-  return mgb::coo_sort<float>(A, mgb::as_stream(stream));
+  return mgb::coo_sort<float>(A, nullptr, 0, mgb::as_stream(stream));
+}
+int mgb_coo_sort_workspace_bytes(const mgb_coo* A, int64_t* bytes) {
+  MGB_REQUIRE(A != nullptr && bytes != nullptr && A->nnz >= 0 && A->nrows >= 0, MGB_ERR_BAD_ARGUMENT);
+  *bytes = (int64_t)mgb::Scratch::padded(sizeof(mgb::Words)) + mgb::prim::row_sort_bytes(A->nnz, A->nrows);
+  return MGB_SUCCESS;
+}
+int mgb_coo_sort_by_row_and_column_ws_f64(mgb_coo* A, void* workspace, int64_t bytes, void* stream) {
+  return mgb::coo_sort<double>(A, workspace, bytes, mgb::as_stream(stream));
+}
+int mgb_coo_sort_by_row_and_column_ws_f32(mgb_coo* A, void* workspace, int64_t bytes, void* stream) {
+  return mgb::coo_sort<float>(A, workspace, bytes, mgb::as_stream(stream));
 }
 int mgb_coo_is_sorted(const mgb_coo* A, int* sorted, void* stream) {
   return mgb::coo_is_sorted(A, sorted, mgb::as_stream(stream));

@@ -1,5 +1,6 @@
 // primitives.cu -- scan, reductions, histograms and sorts used by convert.cu.
 #include <climits>
+#include <type_traits>
 
 #include "primitives.cuh"
 
@@ -436,22 +437,348 @@ __global__ void __launch_bounds__(SEG_MED_THREADS) sort_large_segments(uint64_t*
   }
 }
 
-__global__ void scatter_row_keys(const int32_t* __restrict__ rows, const int32_t* __restrict__ cols, int64_t n,
-                                 int32_t* cursor, uint64_t* keys) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t slot = atomicAdd(cursor + rows[i], 1);
-    keys[slot] = ((uint64_t)(uint32_t)cols[i] << 32) | (uint64_t)(uint32_t)i;
+// ---- sort by row ---------------------------------------------------------
+// An entry on its way to its row: position in the source, column, value bits
+// (16 bytes, so that one aligned store brings it there).
+struct __align__(16) RowRecord {
+  uint32_t i;
+  int32_t col;
+  uint64_t val;
+};
+__device__ __forceinline__ RowRecord load_record(const RowRecord* p) {
+  const uint4 u = __ldg(reinterpret_cast<const uint4*>(p));
+  return RowRecord{u.x, (int32_t)u.y, (uint64_t)u.z | ((uint64_t)u.w << 32)};
+}
+__device__ __forceinline__ uint64_t bits_of(double v) { return (uint64_t)__double_as_longlong(v); }
+__device__ __forceinline__ uint64_t bits_of(float v) { return (uint64_t)__float_as_uint(v); }
+template <typename T> __device__ __forceinline__ T value_of(uint64_t b);
+template <> __device__ __forceinline__ double value_of<double>(uint64_t b) { return __longlong_as_double((long long)b); }
+template <> __device__ __forceinline__ float value_of<float>(uint64_t b) { return __uint_as_float((unsigned)b); }
+
+// The order within a row: by source position (COLS false: a stable partition
+// by row), or by column and then position.
+template <bool COLS>
+__device__ __forceinline__ uint64_t record_key(const RowRecord& r) {
+  return COLS ? ((uint64_t)(uint32_t)r.col << 32) | r.i : r.i;
+}
+
+// rank[i] = how many entries of the row came to its counter before (any
+// order).  Lanes of a warp with the same row add once; the search for them is
+// left out where no neighbouring lanes share a row.
+__global__ void __launch_bounds__(256) row_ranks(const int32_t* __restrict__ rows, int64_t n, int32_t* counts,
+                                                 int32_t* __restrict__ rank) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;; i += (int64_t)gridDim.x * 256) {
+    const bool in = i < n;
+    const unsigned active = __ballot_sync(0xffffffffu, in);
+    if (!active) break;
+    const int32_t r = in ? __ldcs(rows + i) : -1;
+    const int32_t up = __shfl_up_sync(0xffffffffu, r, 1);
+    if (!__any_sync(0xffffffffu, in && lane > 0 && up == r)) {
+      if (in) rank[i] = atomicAdd(counts + r, 1);
+      continue;
+    }
+    const unsigned same = __match_any_sync(0xffffffffu, r);
+    const int leader = __ffs(same) - 1;
+    int32_t base = 0;
+    if (in && lane == leader) base = atomicAdd(counts + r, __popc(same));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    if (in) rank[i] = base + __popc(same & ((1u << lane) - 1));
   }
 }
 
-__global__ void gather_sorted(const uint64_t* __restrict__ keys, const int32_t* __restrict__ rows, int64_t n,
-                              int32_t* out_rows, int32_t* out_cols, int32_t* perm) {
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t key = keys[k];
-    const int32_t p = (int32_t)(uint32_t)(key & 0xffffffffull);
-    perm[k] = p;
-    out_cols[k] = (int32_t)(uint32_t)(key >> 32);
-    out_rows[k] = rows[p];
+template <typename T>
+__global__ void __launch_bounds__(256) row_scatter(const int32_t* __restrict__ rows, const int32_t* __restrict__ cols,
+                                                   const T* __restrict__ vals, const int32_t* __restrict__ start,
+                                                   const int32_t* __restrict__ rank, int64_t n, RowRecord* rec) {
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
+    const int64_t at = (int64_t)__ldg(start + __ldcs(rows + i)) + __ldcs(rank + i);
+    const uint64_t v = bits_of(__ldcs(vals + i));
+    reinterpret_cast<uint4*>(rec)[at] =
+        make_uint4((unsigned)i, (unsigned)__ldcs(cols + i), (unsigned)v, (unsigned)(v >> 32));
+  }
+}
+
+// Rows of at most SORT_SHORT entries are sorted in tiles: CTA t takes the rows
+// that start in [t, t + 1) * SORT_WINDOW.  Longer ones are listed (lists: medium
+// ones first, then those beyond SORT_MED).
+constexpr int SORT_WINDOW = 1024;
+constexpr int SORT_SHORT = 512;
+constexpr int SORT_MED = 4096;
+constexpr int SORT_CAP = SORT_WINDOW + SORT_SHORT;  // entries of a tile, a long last row left out
+constexpr int SORT_PER = SORT_CAP / 256;
+
+__global__ void sort_plan(const int32_t* __restrict__ start, int64_t nrows, int64_t ntiles, int32_t* tile_row,
+                          int32_t* medium, int32_t* large, int32_t* counters) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t r0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); r0 <= nrows;
+       r0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t r = r0 + lane;
+    int len = 0;
+    if (r <= nrows) {
+      const int64_t s = start[r];
+      const int64_t k_lo = r == 0 ? 0 : (int64_t)start[r - 1] / SORT_WINDOW + 1;
+      const int64_t k_hi = r == nrows ? ntiles : s / SORT_WINDOW;
+      for (int64_t k = k_lo; k <= k_hi; k++) tile_row[k] = (int32_t)r;
+      if (r < nrows) len = start[r + 1] - (int32_t)s;
+    }
+#pragma unroll
+    for (int cls = 0; cls < 2; cls++) {
+      const bool mine = cls == 0 ? len > SORT_SHORT && len <= SORT_MED : len > SORT_MED;
+      const unsigned m = __ballot_sync(0xffffffffu, mine);
+      if (!m) continue;
+      int32_t base = 0;
+      if (lane == __ffs(m) - 1) base = atomicAdd(counters + cls, __popc(m));
+      base = __shfl_sync(0xffffffffu, base, __ffs(m) - 1);
+      if (mine) (cls == 0 ? medium : large)[base + __popc(m & ((1u << lane) - 1))] = (int32_t)r;
+    }
+  }
+}
+
+// One thread per entry: its place is its row's start plus the number of
+// smaller keys in the row, counted over the row's keys in shared memory (the
+// lanes of a row read the same word).  Sorting each row with a warp's or a
+// CTA's bitonic network spent 1,100 us on the 1e6 lognormal rows (15 M entries)
+// that this kernel sorts with the gather of columns and values in: rows of
+// 15 entries leave most of a network's lanes idle, and its barriers bound it.
+template <typename T, bool COLS>
+__global__ void __launch_bounds__(256)
+sort_tiles(const RowRecord* __restrict__ rec, const int32_t* __restrict__ start, const int32_t* __restrict__ tile_row,
+           int32_t* __restrict__ orow, int32_t* __restrict__ ocol, T* __restrict__ oval) {
+  using Key = typename std::conditional<COLS, uint64_t, uint32_t>::type;
+  __shared__ Key s_key[SORT_CAP];
+  __shared__ uint16_t s_head[SORT_CAP], s_end[SORT_CAP];  // an entry's row start; at a row start, the row's end
+  __shared__ int32_t s_row[SORT_CAP];                     // at a row start, the row
+  __shared__ int s_warp[8];
+  const int64_t r0 = tile_row[blockIdx.x], r1 = tile_row[blockIdx.x + 1];
+  if (r0 >= r1) return;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int32_t base = start[r0];
+  int32_t end = start[r1];
+  if (end - start[r1 - 1] > SORT_SHORT) end = start[r1 - 1];  // a long last row
+  const int m = end - base;
+  for (int e = threadIdx.x; e < SORT_CAP; e += 256) s_head[e] = 0;
+  RowRecord mine[SORT_PER];
+#pragma unroll
+  for (int k = 0; k < SORT_PER; k++) {
+    const int e = k * 256 + threadIdx.x;
+    if (e < m) {
+      mine[k] = load_record(rec + base + e);
+      s_key[e] = (Key)record_key<COLS>(mine[k]);
+    }
+  }
+  __syncthreads();
+  for (int64_t r = r0 + threadIdx.x; r < r1; r += 256) {
+    const int b = start[r] - base, t = start[r + 1] - base;
+    if (b < t && b < m) {
+      s_head[b] = (uint16_t)b;
+      s_end[b] = (uint16_t)(t - b > SORT_SHORT ? b : t);  // a long row inside the tile: nothing to do here
+      s_row[b] = (int32_t)r;
+    }
+  }
+  __syncthreads();
+  // every entry's row start: the largest marked position up to it
+  int run[SORT_PER];
+  int top = 0;
+#pragma unroll
+  for (int k = 0; k < SORT_PER; k++) run[k] = top = max(top, (int)s_head[threadIdx.x * SORT_PER + k]);
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int o = __shfl_up_sync(0xffffffffu, top, d);
+    if (lane >= d) top = max(top, o);
+  }
+  if (lane == 31) s_warp[w] = top;
+  int before = __shfl_up_sync(0xffffffffu, top, 1);
+  if (lane == 0) before = 0;
+  __syncthreads();
+  for (int i = 0; i < w; i++) before = max(before, s_warp[i]);
+#pragma unroll
+  for (int k = 0; k < SORT_PER; k++) s_head[threadIdx.x * SORT_PER + k] = (uint16_t)max(run[k], before);
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < SORT_PER; k++) {
+    const int e = k * 256 + threadIdx.x;
+    if (e >= m) break;
+    const int h = s_head[e], t = s_end[h];
+    if (t == h) continue;
+    const Key key = s_key[e];
+    int at = h;
+#pragma unroll 4
+    for (int j = h; j < t; j++) at += s_key[j] < key ? 1 : 0;
+    if (orow != nullptr) orow[base + at] = s_row[h];
+    ocol[base + at] = mine[k].col;
+    oval[base + at] = value_of<T>(mine[k].val);
+  }
+}
+
+// bitonic sort of m (power of two) records in shared memory
+template <bool COLS>
+__device__ void bitonic_records(RowRecord* sk, int m) {
+  for (int k = 2; k <= m; k <<= 1) {
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      for (int i = threadIdx.x; i < m; i += blockDim.x) {
+        const int p = i ^ j;
+        if (p > i) {
+          const RowRecord a = sk[i], b = sk[p];
+          const bool up = ((i & k) == 0);
+          if ((record_key<COLS>(a) > record_key<COLS>(b)) == up) { sk[i] = b; sk[p] = a; }
+        }
+      }
+      __syncthreads();
+    }
+  }
+}
+// past the last record (no entry has this column and position)
+__device__ __forceinline__ RowRecord record_max() { return RowRecord{~0u, -1, 0}; }
+
+template <typename T>
+__device__ __forceinline__ void write_records(const RowRecord* src, int64_t b, int64_t n, int32_t row, int32_t* orow,
+                                              int32_t* ocol, T* oval) {
+  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
+    if (orow != nullptr) orow[b + i] = row;
+    ocol[b + i] = src[i].col;
+    oval[b + i] = value_of<T>(src[i].val);
+  }
+}
+
+constexpr int SORT_LONG_THREADS = 512;
+constexpr int SORT_RUN = 128;
+
+// One CTA per row of SORT_SHORT < length <= SORT_MED.  Every thread keeps its
+// records in registers and only moves keys: the place in a run of SORT_RUN by
+// counting, then doubled runs by one binary search of the neighbouring run
+// per level.  (A bitonic network over 16-byte records: 129 us where a few rows
+// of thousands of entries are all there is.)
+template <typename T, bool COLS>
+__global__ void __launch_bounds__(SORT_LONG_THREADS)
+sort_medium_rows(const RowRecord* __restrict__ rec, const int32_t* __restrict__ start,
+                 const int32_t* __restrict__ list, const int32_t* __restrict__ count, int32_t* __restrict__ orow,
+                 int32_t* __restrict__ ocol, T* __restrict__ oval) {
+  using Key = typename std::conditional<COLS, uint64_t, uint32_t>::type;
+  constexpr int PER = SORT_MED / SORT_LONG_THREADS;
+  extern __shared__ __align__(16) unsigned char sort_smem[];
+  Key* from = reinterpret_cast<Key*>(sort_smem);
+  Key* to = from + SORT_MED;
+  for (int64_t w = blockIdx.x; w < *count; w += gridDim.x) {
+    const int32_t r = list[w];
+    const int32_t b = start[r], len = start[r + 1] - b;
+    RowRecord mine[PER];
+    int pos[PER];
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+      const int e = k * SORT_LONG_THREADS + threadIdx.x;
+      if (e < len) {
+        mine[k] = load_record(rec + b + e);
+        from[e] = (Key)record_key<COLS>(mine[k]);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+      const int e = k * SORT_LONG_THREADS + threadIdx.x;
+      if (e < len) {
+        const int c0 = e & ~(SORT_RUN - 1), c1 = min(c0 + SORT_RUN, len);
+        const Key key = (Key)record_key<COLS>(mine[k]);
+        int at = c0;
+#pragma unroll 8
+        for (int j = c0; j < c1; j++) at += from[j] < key ? 1 : 0;
+        pos[k] = at;
+        to[at] = key;
+      }
+    }
+    __syncthreads();
+    for (int width = SORT_RUN; width < len; width <<= 1) {
+      Key* t = from;
+      from = to;
+      to = t;
+#pragma unroll
+      for (int k = 0; k < PER; k++) {
+        const int e = k * SORT_LONG_THREADS + threadIdx.x;
+        if (e < len) {
+          const Key key = (Key)record_key<COLS>(mine[k]);
+          const int own = pos[k] & ~(width - 1), other = own ^ width;
+          int lo = min(other, len), hi = min(other + width, len);
+          const int first = lo;
+          while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (from[mid] < key) lo = mid + 1; else hi = mid;
+          }
+          pos[k] = min(own, other) + (pos[k] - own) + (lo - first);
+          to[pos[k]] = key;
+        }
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+      const int e = k * SORT_LONG_THREADS + threadIdx.x;
+      if (e < len) {
+        if (orow != nullptr) orow[b + pos[k]] = r;
+        ocol[b + pos[k]] = mine[k].col;
+        oval[b + pos[k]] = value_of<T>(mine[k].val);
+      }
+    }
+    __syncthreads();  // the next row's keys
+  }
+}
+
+// large rows: sort chunks of SORT_MED in shared memory, then merge runs pairwise
+// (merge path: each thread emits a contiguous slice of the output)
+template <bool COLS>
+__device__ int64_t merge_corank(const RowRecord* a, int64_t na, const RowRecord* b, int64_t nb, int64_t k) {
+  // number of elements taken from a among the first k outputs
+  int64_t lo = k > nb ? k - nb : 0, hi = k < na ? k : na;
+  while (lo < hi) {
+    const int64_t mid = (lo + hi) >> 1;
+    if (record_key<COLS>(a[mid]) <= record_key<COLS>(b[k - mid - 1])) lo = mid + 1; else hi = mid;
+  }
+  return lo;
+}
+
+template <typename T, bool COLS>
+__global__ void __launch_bounds__(SORT_LONG_THREADS)
+sort_large_rows(RowRecord* rec, RowRecord* tmp, const int32_t* __restrict__ start, const int32_t* __restrict__ list,
+                const int32_t* __restrict__ count, int32_t* __restrict__ orow, int32_t* __restrict__ ocol,
+                T* __restrict__ oval) {
+  extern __shared__ RowRecord sk[];
+  for (int64_t w = blockIdx.x; w < *count; w += gridDim.x) {
+    const int32_t r = list[w];
+    const int64_t b = start[r], len = start[r + 1] - b;
+    RowRecord* src = rec + b;
+    RowRecord* dst = tmp + b;
+    for (int64_t c0 = 0; c0 < len; c0 += SORT_MED) {
+      const int cl = (int)min((int64_t)SORT_MED, len - c0);
+      __syncthreads();
+      for (int i = threadIdx.x; i < SORT_MED; i += blockDim.x) sk[i] = i < cl ? src[c0 + i] : record_max();
+      __syncthreads();
+      bitonic_records<COLS>(sk, SORT_MED);
+      for (int i = threadIdx.x; i < cl; i += blockDim.x) src[c0 + i] = sk[i];
+    }
+    __syncthreads();
+    bool in_src = true;
+    for (int64_t width = SORT_MED; width < len; width <<= 1) {
+      const RowRecord* from = in_src ? src : dst;
+      RowRecord* to = in_src ? dst : src;
+      for (int64_t a0 = 0; a0 < len; a0 += 2 * width) {
+        const int64_t na = min(width, len - a0);
+        const int64_t nb = max((int64_t)0, min(width, len - a0 - width));
+        const int64_t tot = na + nb;
+        const int64_t per = (tot + blockDim.x - 1) / blockDim.x;
+        const int64_t k0 = min(tot, (int64_t)threadIdx.x * per), k1 = min(tot, k0 + per);
+        const RowRecord* A = from + a0;
+        const RowRecord* B = from + a0 + na;
+        int64_t ia = merge_corank<COLS>(A, na, B, nb, k0);
+        int64_t ib = k0 - ia;
+        for (int64_t k = k0; k < k1; k++) {
+          if (ib >= nb || (ia < na && record_key<COLS>(A[ia]) <= record_key<COLS>(B[ib]))) to[a0 + k] = A[ia++];
+          else to[a0 + k] = B[ib++];
+        }
+      }
+      __syncthreads();
+      in_src = !in_src;
+    }
+    write_records<T>(in_src ? src : dst, b, len, r, orow, ocol, oval);
+    __syncthreads();
   }
 }
 
@@ -597,30 +924,72 @@ int segmented_sort_u64(uint64_t* keys, const int32_t* seg, int64_t nseg, int64_t
   return MGB_SUCCESS;
 }
 
-int stable_sort_rows_cols(const int32_t* rows, const int32_t* cols, int64_t n, int64_t nrows, int32_t* out_rows,
-                          int32_t* out_cols, int32_t* perm, cudaStream_t s) {
-  if (n <= 0) return MGB_SUCCESS;
-  Scratch sc(s);
-  int32_t *counts, *starts, *cursor;
-  uint64_t* keys;
+int64_t row_sort_bytes(int64_t n, int64_t nrows) {
+  return (int64_t)(Scratch::padded(sizeof(RowRecord) * (size_t)n) + Scratch::padded(sizeof(int32_t) * (size_t)n) +
+                   2 * Scratch::padded(sizeof(int32_t) * (size_t)(nrows + 1)) +
+                   Scratch::padded(sizeof(int32_t) * (size_t)(n / SORT_WINDOW + 2)) +
+                   Scratch::padded(sizeof(int32_t) * (size_t)(n / SORT_SHORT + 1)) +
+                   Scratch::padded(sizeof(int32_t) * (size_t)(n / SORT_MED + 1)) + 256);
+}
+
+template <typename T, bool COLS>
+int row_sort(const int32_t* rows, const int32_t* cols, const T* vals, int64_t n, int64_t nrows, int32_t* start,
+             int32_t* orow, int32_t* ocol, T* oval, Scratch& sc, cudaStream_t s) {
+  RowRecord* rec;
+  int32_t *counts, *rank, *tile_row, *medium, *large, *counters;
+  MGB_SCRATCH(sc, rec, n);
+  MGB_SCRATCH(sc, rank, n);
   MGB_SCRATCH(sc, counts, nrows + 1);
-  MGB_SCRATCH(sc, starts, nrows + 1);
-  MGB_SCRATCH(sc, cursor, nrows + 1);
-  MGB_SCRATCH(sc, keys, n);
-  int st = histogram(rows, n, counts, nrows, s);
-  if (st) return st;
-  MGB_CUDA_CHECK(cudaMemsetAsync(counts + nrows, 0, sizeof(int32_t), s));
-  st = exclusive_scan<int32_t, int32_t>(counts, starts, nrows + 1, s);
-  if (st) return st;
-  MGB_CUDA_CHECK(cudaMemcpyAsync(cursor, starts, sizeof(int32_t) * (nrows + 1), cudaMemcpyDeviceToDevice, s));
-  scatter_row_keys<<<blocks_for(n, 256, (int64_t)num_sms() * 16), 256, 0, s>>>(rows, cols, n, cursor, keys);
+  if (start == nullptr) MGB_SCRATCH(sc, start, nrows + 1);
+  const int64_t ntiles = n / SORT_WINDOW + 1;
+  MGB_SCRATCH(sc, tile_row, ntiles + 1);
+  MGB_SCRATCH(sc, medium, n / SORT_SHORT + 1);
+  MGB_SCRATCH(sc, large, n / SORT_MED + 1);
+  MGB_SCRATCH(sc, counters, 2);
+  MGB_CUDA_CHECK(cudaMemsetAsync(counts, 0, sizeof(int32_t) * (nrows + 1), s));
+  MGB_CUDA_CHECK(cudaMemsetAsync(counters, 0, 2 * sizeof(int32_t), s));
+  const unsigned grid = blocks_for(n, 256, (int64_t)num_sms() * 8);
+  row_ranks<<<grid, 256, 0, s>>>(rows, n, counts, rank);
   MGB_LAUNCH_CHECK();
-  st = segmented_sort_u64(keys, starts, nrows, n, s);
+  int st = exclusive_scan<int32_t, int32_t>(counts, start, nrows + 1, s);
   if (st) return st;
-  gather_sorted<<<blocks_for(n, 256, (int64_t)num_sms() * 16), 256, 0, s>>>(keys, rows, n, out_rows, out_cols, perm);
+  row_scatter<T><<<grid, 256, 0, s>>>(rows, cols, vals, start, rank, n, rec);
   MGB_LAUNCH_CHECK();
+  sort_plan<<<blocks_for(nrows + 1, 256, (int64_t)num_sms() * 8), 256, 0, s>>>(start, nrows, ntiles, tile_row, medium,
+                                                                                large, counters);
+  MGB_LAUNCH_CHECK();
+  int32_t h[2] = {0, 0};
+  if (n > SORT_SHORT) {
+    MGB_CUDA_CHECK(cudaMemcpyAsync(h, counters, sizeof(h), cudaMemcpyDeviceToHost, s));
+    MGB_CUDA_CHECK(cudaStreamSynchronize(s));
+  }
+  sort_tiles<T, COLS><<<(unsigned)ntiles, 256, 0, s>>>(rec, start, tile_row, orow, ocol, oval);
+  MGB_LAUNCH_CHECK();
+  constexpr int smem = SORT_MED * (int)sizeof(RowRecord);
+  if (h[0] > 0) {
+    constexpr int keys = 2 * SORT_MED * (COLS ? 8 : 4);
+    MGB_CUDA_CHECK(cudaFuncSetAttribute(sort_medium_rows<T, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, keys));
+    sort_medium_rows<T, COLS><<<(unsigned)min((int64_t)h[0], (int64_t)num_sms() * 3), SORT_LONG_THREADS, keys, s>>>(
+        rec, start, medium, counters, orow, ocol, oval);
+    MGB_LAUNCH_CHECK();
+  }
+  if (h[1] > 0) {
+    RowRecord* tmp;
+    MGB_SCRATCH(sc, tmp, n);
+    MGB_CUDA_CHECK(cudaFuncSetAttribute(sort_large_rows<T, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    sort_large_rows<T, COLS><<<(unsigned)min((int64_t)h[1], (int64_t)num_sms() * 3), SORT_LONG_THREADS, smem, s>>>(
+        rec, tmp, start, large, counters + 1, orow, ocol, oval);
+    MGB_LAUNCH_CHECK();
+  }
   return MGB_SUCCESS;
 }
+#define MGB_ROW_SORT(T, COLS)                                                                                        \
+  template int row_sort<T, COLS>(const int32_t*, const int32_t*, const T*, int64_t, int64_t, int32_t*, int32_t*,     \
+                                 int32_t*, T*, Scratch&, cudaStream_t);
+MGB_ROW_SORT(double, false)
+MGB_ROW_SORT(double, true)
+MGB_ROW_SORT(float, false)
+MGB_ROW_SORT(float, true)
 
 }  // namespace prim
 }  // namespace mgb

@@ -1,6 +1,7 @@
 // primitives.cuh -- device-wide building blocks for the GPU conversions:
-// exclusive scan, reductions, stable (row, col) sort of COO entries and
-// per-row segmented sort.  All scratch is stream-ordered.
+// exclusive scan, reductions, the pass over COO indices and the stable (row,
+// col) sort of COO entries.  All scratch is stream-ordered or
+// the caller's.
 #pragma once
 
 #include "mgb_internal.cuh"
@@ -75,12 +76,17 @@ int coo_sorted_flags(const int32_t* rows, const int32_t* cols, int64_t n, int32_
 // entries (int32 offsets into keys).
 int segmented_sort_u64(uint64_t* keys, const int32_t* seg, int64_t nseg, int64_t nkeys, cudaStream_t s);
 
-// Stable sort of COO entries by (row, col): writes the permutation (source
-// index per output slot) to perm[n] and the sorted rows/cols to
-// out_rows/out_cols.  Rows must lie in [0, nrows).  Equivalent to the
-// reference's two stable counting sorts (by column, then by row).
-int stable_sort_rows_cols(const int32_t* rows, const int32_t* cols, int64_t n, int64_t nrows,
-                          int32_t* out_rows, int32_t* out_cols, int32_t* perm, cudaStream_t s);
+// COO entries brought into row order: start (nrows + 1 entries; null: kept in
+// scratch) = the first entry of every row, ocol / oval (and orow unless null)
+// = the entries by row and, within a row, in source order (COLS false) or by
+// column and then source order (COLS true: the reference's two stable counting
+// sorts, by column and then by row).  Rows must lie in [0, nrows).  The outputs
+// may be the inputs.  Synchronises the stream for n > 512.  Scratch: up to
+// row_sort_bytes (rows beyond 4,096 entries: 16 n more).
+template <typename T, bool COLS>
+int row_sort(const int32_t* rows, const int32_t* cols, const T* vals, int64_t n, int64_t nrows, int32_t* start,
+             int32_t* orow, int32_t* ocol, T* oval, Scratch& sc, cudaStream_t s);
+int64_t row_sort_bytes(int64_t n, int64_t nrows);
 
 // ---- one pass over COO indices ------------------------------------------------
 // Device words an entry point reads back with one copy and one stream

@@ -128,3 +128,31 @@ def test_planned_conversion_equals_separate_calls(cuda, fmt, shuffled):
     got = mgb.matrix_to_host(planned)
     assert_same_matrix(got, _two_call(A, fmt, planned))
     assert_same_matrix(got, O.OracleMatrix.from_host(hm).convert(fmt).to_host())
+
+
+# rows at the limits of the sorted tiles (512), of a tile's window (1024), of the shared-memory sort (4096) and of its
+# merge passes; many empty rows; a few rows that hold everything
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("N,lens", [(1, [1]), (5, [0, 7, 0]), (900, [1, 2, 31, 32, 33]), (40, [511, 512, 513, 3]),
+                                    (12, [1023, 1, 1024, 600, 600]), (5, [4096, 4097, 0, 2]), (3, [20000, 5]),
+                                    (60000, [1] + [0] * 99)])
+def test_row_sort_tiles(cuda, N, lens, dtype):
+    import torch
+
+    import morpheus_gb300 as mgb
+    rng = np.random.default_rng(N)
+    rows = np.repeat(np.arange(N), np.resize(np.asarray(lens), N))
+    cols = rng.integers(0, 3000, rows.size)  # duplicates among them
+    p = rng.permutation(rows.size)
+    hm = {"format": 0, "nrows": N, "ncols": 3000, "nnz": rows.size, "row_indices": rows[p].astype(np.int32),
+          "column_indices": cols.astype(np.int32), "values": rng.standard_normal(rows.size).astype(dtype)}
+    got, ref = both(hm, O.CSR)
+    assert_same_matrix(got, ref)
+    om = O.OracleMatrix.from_host(hm)
+    om.sort_by_row_and_column()
+    A = mgb.matrix_from_host(hm)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    mgb.sort_by_row_and_column(A, stream=side)
+    side.synchronize()
+    assert_same_matrix(mgb.matrix_to_host(A), om.to_host())
