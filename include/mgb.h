@@ -462,6 +462,19 @@ int mgb_convert_coo_planned_f64(const mgb_coo* src, const mgb_coo_plan* plan, vo
 int mgb_convert_coo_planned_f32(const mgb_coo* src, const mgb_coo_plan* plan, void* dst, void* workspace,
                                 int64_t bytes, void* stream);
 
+/* The same for the entries of a CSR matrix, DIA / ELL / HYB / HDC (formats_e 2..5):
+ * what a conversion through its COO form gives, without its row indices.  A plan
+ * whose format comes back as 0 was not made (offsets that do not rise from 0 to
+ * nnz, columns out of order or repeated in a row for DIA and HDC, thousands of
+ * diagonals, no rows): convert through COO. */
+int mgb_convert_csr_workspace_bytes(const mgb_csr* src, int format, int64_t* bytes);
+int mgb_convert_csr_plan_f64(const mgb_csr* src, int format, int64_t hyb_width, void* workspace, int64_t bytes,
+                             mgb_coo_plan* plan, void* stream);
+int mgb_convert_csr_plan_f32(const mgb_csr* src, int format, int64_t hyb_width, void* workspace, int64_t bytes,
+                             mgb_coo_plan* plan, void* stream);
+int mgb_convert_csr_planned_f64(const mgb_csr* src, const mgb_coo_plan* plan, void* dst, void* stream);
+int mgb_convert_csr_planned_f32(const mgb_csr* src, const mgb_coo_plan* plan, void* dst, void* stream);
+
 /* In-place stable sort by (row, column): impl/Coo/Serial/Morpheus_Sort_Impl.hpp:109-164 */
 int mgb_coo_sort_by_row_and_column_f64(mgb_coo* A, void* stream);
 int mgb_coo_sort_by_row_and_column_f32(mgb_coo* A, void* stream);

@@ -134,7 +134,10 @@ for _dt in ("f64", "f32"):
     _SIGS[f"mgb_coo_sort_by_row_and_column_{_dt}"] = (C.c_int, [_P(Coo), vp])
     _SIGS[f"mgb_convert_coo_planned_{_dt}"] = (C.c_int, [_P(Coo), _P(CooPlan), vp, vp, i64, vp])
     _SIGS[f"mgb_coo_sort_by_row_and_column_ws_{_dt}"] = (C.c_int, [_P(Coo), vp, i64, vp])
+    _SIGS[f"mgb_convert_csr_plan_{_dt}"] = (C.c_int, [_P(Csr), C.c_int, i64, vp, i64, _P(CooPlan), vp])
+    _SIGS[f"mgb_convert_csr_planned_{_dt}"] = (C.c_int, [_P(Csr), _P(CooPlan), vp, vp])
 _SIGS["mgb_coo_sort_workspace_bytes"] = (C.c_int, [_P(Coo), _P(i64)])
+_SIGS["mgb_convert_csr_workspace_bytes"] = (C.c_int, [_P(Csr), C.c_int, _P(i64)])
 _SIGS["mgb_convert_coo_workspace_bytes"] = (C.c_int, [_P(Coo), C.c_int, _P(i64)])
 _SIGS["mgb_convert_coo_plan"] = (C.c_int, [_P(Coo), C.c_int, i64, vp, i64, _P(CooPlan), vp])
 _SIGS["mgb_coo_is_sorted"] = (C.c_int, [_P(Coo), _P(C.c_int), vp])

@@ -74,17 +74,6 @@ def _fill_coo(A: _Matrix, cols: torch.Tensor, vals: torch.Tensor, stream) -> Coo
     return out
 
 
-def _as_coo(A: _Matrix, stream=None) -> CooMatrix:
-    """A's entries as a COO that is only read: a CSR matrix's columns and
-    values are shared with it, and only its rows are expanded."""
-    if A.FORMAT == COO_FORMAT:
-        return A
-    if A.FORMAT != CSR_FORMAT:
-        return to_coo(A, stream)
-    _dev_check(A)
-    return _fill_coo(A, A.column_indices(), A.values(), stream)
-
-
 # Containers that a conversion fills: it writes every index, offset and value
 # (padding included), so their arrays are not cleared first.
 
@@ -125,19 +114,50 @@ def from_coo(coo: CooMatrix, fmt: int, hyb_width: int = 0, stream=None) -> _Matr
     # sizes known before the plan: allocate while the GPU still has work queued
     out = _new_csr(n, m, z, dt, dev) if fmt == CSR_FORMAT else None
     _call("mgb_convert_coo_plan", C.byref(sd), fmt, int(hyb_width), _ptr(ws), nb.value, C.byref(plan), sh)
-    s0, s1, s2 = plan.sizes
-    if fmt == DIA_FORMAT:
-        out = _new_dia(n, m, z, s0, dt, dev)
-    elif fmt == ELL_FORMAT:
-        out = _new_ell(n, m, z, s0, dt, dev)
-    elif fmt == HYB_FORMAT:
-        out = HybMatrix(_new_ell(n, m, s1, s0, dt, dev), _new_coo(n, m, s2, dt, dev), dt, dev)
-    elif fmt == HDC_FORMAT:
-        out = HdcMatrix(_new_dia(n, m, s1, s0, dt, dev), _new_csr(n, m, s2, dt, dev), dt, dev)
+    out = out or _planned_container(coo, fmt, plan)
     dd = out._desc()
     fill = _workspace(plan.fill_bytes, dev, stream) if plan.fill_bytes else None
     _call(f"mgb_convert_coo_planned_{sfx}", C.byref(sd), C.byref(plan), C.byref(dd), _ptr(fill), plan.fill_bytes, sh)
     return out
+
+
+def _planned_container(src: _Matrix, fmt: int, plan) -> _Matrix:
+    n, m, z, dt, dev = src.nrows(), src.ncols(), src.nnnz(), src.dtype, src.device
+    s0, s1, s2 = plan.sizes
+    if fmt == DIA_FORMAT:
+        return _new_dia(n, m, z, s0, dt, dev)
+    if fmt == ELL_FORMAT:
+        return _new_ell(n, m, z, s0, dt, dev)
+    if fmt == HYB_FORMAT:
+        return HybMatrix(_new_ell(n, m, s1, s0, dt, dev), _new_coo(n, m, s2, dt, dev), dt, dev)
+    return HdcMatrix(_new_dia(n, m, s1, s0, dt, dev), _new_csr(n, m, s2, dt, dev), dt, dev)
+
+
+def _from_csr(A: CsrMatrix, fmt: int, hyb_width: int = 0, stream=None) -> _Matrix:
+    """CSR -> a new DIA / ELL / HYB / HDC container, as through COO but without
+    its row indices (which are made where the library has no such path)."""
+    _dev_check(A)
+    sfx, sh, sd = _suffix(A.dtype), _stream_handle(stream), A._desc()
+    if fmt in (DIA_FORMAT, ELL_FORMAT, HYB_FORMAT, HDC_FORMAT):
+        nb, plan = C.c_int64(), _lib.CooPlan()
+        _call("mgb_convert_csr_workspace_bytes", C.byref(sd), fmt, C.byref(nb))
+        ws = _workspace(nb.value, A.device, stream)
+        _call(f"mgb_convert_csr_plan_{sfx}", C.byref(sd), fmt, int(hyb_width), _ptr(ws), nb.value, C.byref(plan), sh)
+        if plan.format:
+            out = _planned_container(A, fmt, plan)
+            dd = out._desc()
+            _call(f"mgb_convert_csr_planned_{sfx}", C.byref(sd), C.byref(plan), C.byref(dd), sh)
+            return out
+    return from_coo(_fill_coo(A, A.column_indices(), A.values(), stream), fmt, hyb_width=hyb_width, stream=stream)
+
+
+def _convert_to(A: _Matrix, fmt: int, hyb_width: int, stream) -> _Matrix:
+    """A in another format, through COO as the reference does."""
+    if fmt == COO_FORMAT:
+        return to_coo(A, stream)
+    if A.FORMAT == CSR_FORMAT:
+        return _from_csr(A, fmt, hyb_width, stream)
+    return from_coo(A if A.FORMAT == COO_FORMAT else to_coo(A, stream), fmt, hyb_width=hyb_width, stream=stream)
 
 
 def convert(src, dst, stream=None, hyb_width: int = 0):
@@ -149,10 +169,8 @@ def convert(src, dst, stream=None, hyb_width: int = 0):
     target = dst.active_index() if isinstance(dst, DynamicMatrix) else dst.FORMAT
     if src.FORMAT == target:
         out = from_coo(to_coo(src), target, hyb_width=hyb_width) if target == COO_FORMAT else _deep_copy(src)
-    elif target == COO_FORMAT:
-        out = to_coo(src, stream)
     else:
-        out = from_coo(_as_coo(src, stream), target, hyb_width=hyb_width, stream=stream)
+        out = _convert_to(src, target, hyb_width, stream)
     if isinstance(dst, DynamicMatrix):
         dst.assign(out)
     else:
@@ -176,12 +194,16 @@ def convert_inplace(dyn: DynamicMatrix, fmt, stream=None, hyb_width: int = 0) ->
         return conversion_error_e.PROXY_TO_DYNAMIC
     if dyn.active_index() == fmt:
         return conversion_error_e.CONV_SUCCESS
+    src = dyn.active()
     try:
-        temp = to_coo(dyn.active(), stream) if fmt == COO_FORMAT else _as_coo(dyn.active(), stream)
+        _dev_check(src)
+        _suffix(src.dtype)
+        if fmt == COO_FORMAT or src.FORMAT not in (COO_FORMAT, CSR_FORMAT):
+            src = to_coo(src, stream)
     except MorpheusException:
         return conversion_error_e.DYNAMIC_TO_PROXY
     try:
-        out = temp if fmt == COO_FORMAT else from_coo(temp, fmt, hyb_width=hyb_width, stream=stream)
+        out = src if fmt == COO_FORMAT else _convert_to(src, fmt, hyb_width, stream)
     except MorpheusException:
         return conversion_error_e.PROXY_TO_DYNAMIC
     dyn.assign(out)

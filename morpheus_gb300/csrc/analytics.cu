@@ -98,42 +98,29 @@ __global__ void row_stats_kernel(LEN lens, int64_t nrows, int64_t hyb_w,
 
 // Diagonal bin (c - r + nrows - 1) of every entry, and (lens != nullptr) its
 // row's length increased by the row's entries inside the matrix: one warp per
-// 32 rows, four entries per lane.  Bound by the issue slots of the counting
-// beside the column indices (HBM).  A thread per row read its columns
-// uncoalesced: 606 us on the 27-point stencil at 160^3.
+// 32 rows, a lane per entry.  Bound by the issue slots of the counting beside
+// the column indices (HBM).  A thread per row read its columns uncoalesced:
+// 606 us on the 27-point stencil at 160^3.
 __global__ void __launch_bounds__(256) csr_diag_kernel(const int32_t* __restrict__ ro, const int32_t* __restrict__ ci,
                                                        int64_t nrows, int64_t ncols, int32_t* lens,
                                                        int32_t* counts) {
   MGB_CTA_HIST(h);
-  __shared__ int32_t s_ro[8][33];
+  __shared__ prim::WarpRows s_rows[8];
   prim::hist_init(h);
   __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const bool vec = reinterpret_cast<uintptr_t>(ci) % 16 == 0;
   const bool wide = nrows + ncols > (int64_t)INT_MAX;  // bins past 32 bits
   const uint32_t nc = (uint32_t)min(ncols, (int64_t)1 << 31);
-  for (int64_t r0 = ((int64_t)blockIdx.x * 8 + w) * 32; r0 < nrows; r0 += (int64_t)gridDim.x * 256) {
-    int32_t c[4];
-    prim::warp_row_quads(
-        ro, r0, nrows, s_ro[w], lane,
-        [&](int32_t e0, int lo, int hi) {
-          if (vec && lo == 0 && hi == 4) {
-            const int4 v = __ldcs(reinterpret_cast<const int4*>(ci + e0));
-            c[0] = v.x; c[1] = v.y; c[2] = v.z; c[3] = v.w;
-          } else {
-#pragma unroll
-            for (int k = 0; k < 4; k++)
-              if (k >= lo && k < hi) c[k] = ci[e0 + k];
-          }
-        },
-        [&](int k, int64_t r) {
-          if ((uint32_t)c[k] >= nc) return;
+  for (int64_t r0 = ((int64_t)blockIdx.x * 8 + w) * 32; r0 < nrows; r0 += (int64_t)gridDim.x * 256)
+    prim::warp_row_walk(
+        ro, r0, nrows, s_rows[w], lane, 0, 1, [&](int64_t e) { return (uint32_t)__ldcs(ci + e); },
+        [&](bool in, int q, int64_t, uint32_t c) {
+          if (!in || c >= nc) return;
+          const int64_t r = r0 + q;
           if (lens != nullptr) prim::warp_merged_add(lens, r);
-          if (wide) prim::hist_add(h, counts, (uint64_t)(c[k] - r + nrows - 1));
-          else prim::hist_add32(h, counts, (uint32_t)c[k] - (uint32_t)r + (uint32_t)(nrows - 1));
-        },
-        [](int32_t, int, int) {});
-  }
+          if (wide) prim::hist_add(h, counts, (uint64_t)(c - r + nrows - 1));
+          else prim::hist_add32(h, counts, c - (uint32_t)r + (uint32_t)(nrows - 1));
+        });
   __syncthreads();
   prim::hist_flush(h, counts);
 }

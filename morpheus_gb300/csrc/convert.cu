@@ -112,30 +112,20 @@ int zero_coo(mgb_coo* d, cudaStream_t s) {
 
 // ---------------------------------------------------------------- CSR <-> COO
 // impl/Csr/Serial/Morpheus_Convert_Impl.hpp:70-97
-// rows[j + shift] = the row of CSR entry j, one warp per 32 rows, in 16-byte
-// stores (a thread per row wrote 4 bytes at a time: 608 us for the 437 MB of
+// rows[j + shift] = the row of CSR entry j, one warp per 32 rows, 32 entries
+// per store (a thread per row wrote 4 bytes at a time: 608 us for the 437 MB of
 // the 27-point stencil at 160^3).  Entries before the first offset or past
 // the last one (offsets that do not span the entries) get row 0.
 __global__ void __launch_bounds__(256) expand_rows(const int32_t* __restrict__ ro, int64_t nrows, int64_t nnz,
                                                    int32_t* __restrict__ rows, int64_t shift) {
-  __shared__ int32_t s_ro[8][33];
+  __shared__ prim::WarpRows s_rows[8];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int32_t* out = rows + shift;
-  const bool vec = reinterpret_cast<uintptr_t>(out) % 16 == 0;
-  for (int64_t r0 = ((int64_t)blockIdx.x * 8 + w) * 32; r0 < nrows; r0 += (int64_t)gridDim.x * 256) {
-    int32_t v[4];
-    prim::warp_row_quads(
-        ro, r0, nrows, s_ro[w], lane, [](int32_t, int, int) {}, [&](int k, int64_t r) { v[k] = (int32_t)r; },
-        [&](int32_t e0, int lo, int hi) {
-          if (vec && lo == 0 && hi == 4 && e0 >= 0 && (int64_t)e0 + 4 <= nnz) {
-            __stcs(reinterpret_cast<int4*>(out + e0), make_int4(v[0], v[1], v[2], v[3]));
-          } else {
-#pragma unroll
-            for (int k = 0; k < 4; k++)
-              if (k >= lo && k < hi && e0 + k >= 0 && (int64_t)e0 + k < nnz) out[e0 + k] = v[k];
-          }
-        });
-  }
+  for (int64_t r0 = ((int64_t)blockIdx.x * 8 + w) * 32; r0 < nrows; r0 += (int64_t)gridDim.x * 256)
+    prim::warp_row_walk(ro, r0, nrows, s_rows[w], lane, 0, 1, [](int64_t) { return 0; },
+                        [&](bool in, int q, int64_t e, int) {
+                          if (in && e >= 0 && e < nnz) __stcs(out + e, (int32_t)(r0 + q));
+                        });
   const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x, nt = (int64_t)gridDim.x * 256;
   const int64_t first = min((int64_t)ro[0], nnz), last = max((int64_t)ro[nrows], (int64_t)0);
   for (int64_t j = t; j < first; j += nt) out[j] = 0;
@@ -297,8 +287,8 @@ __global__ void dia_place(const int32_t* __restrict__ r, const int32_t* __restri
 // ---- slabs from row-sorted entries, tile by tile
 //
 // A CTA owns R consecutive rows of D diagonals at a time: the rows' entries
-// (one contiguous range) go through shared memory to their (diagonal, row)
-// place, and the tile is written column by column, padding included, in
+// (one contiguous range, found and told apart by the row starts: the row
+// indices are not read) go through shared memory to their (diagonal, row) place, and the tile is written column by column, padding included, in
 // consecutive rows.  So every value of the slab is written once, in full
 // sectors, and nothing is cleared before.  Placing each entry with its own
 // 8-byte store into a cleared slab took 2,012 us on the 27-point stencil at
@@ -307,7 +297,7 @@ __global__ void dia_place(const int32_t* __restrict__ r, const int32_t* __restri
 // entries of a row go to different banks.  Diagonals are looked up in a table
 // in shared memory while they are few (DIA_HASH_DIAGS), else in the bin ->
 // slot array.
-constexpr int DIA_TILE_THREADS = 256;
+constexpr int DIA_TILE_THREADS = 128;
 constexpr int DIA_TILE_BYTES = 32 * 1024;
 constexpr int DIA_TILE_ROWS = 512;  // at most
 constexpr int DIA_HASH_DIAGS = 256;  // at most a quarter of the table's slots
@@ -353,17 +343,20 @@ __device__ __forceinline__ int dia_table_find(DiaTable t, int32_t d) {
 // REM (HDC): also rem[row] = the row's entries on no stored diagonal.
 template <typename T, bool REM>
 __global__ void __launch_bounds__(DIA_TILE_THREADS)
-dia_fill_tiles(const int32_t* __restrict__ r, const int32_t* __restrict__ c, const T* __restrict__ v,
-               const int32_t* __restrict__ start, int64_t nrows, int64_t pitch, int nd,
-               const int32_t* __restrict__ offs, const int32_t* __restrict__ bin_slot, T* __restrict__ out,
-               int32_t* __restrict__ rem, int R, int D) {
+dia_fill_tiles(const int32_t* __restrict__ c, const T* __restrict__ v, const int32_t* __restrict__ start,
+               int64_t nrows, int64_t pitch, int nd, const int32_t* __restrict__ offs,
+               const int32_t* __restrict__ bin_slot, T* __restrict__ out, int32_t* __restrict__ rem, int R, int D) {
+  constexpr int WARPS = DIA_TILE_THREADS / 32;
   extern __shared__ __align__(16) unsigned char dia_smem[];
   T* tile = reinterpret_cast<T*>(dia_smem);
   __shared__ int32_t h_key[DIA_HASH_SLOTS], h_slot[DIA_HASH_SLOTS];
   __shared__ int32_t s_rem[REM ? DIA_TILE_ROWS : 1];
+  __shared__ prim::WarpRows s_rows[WARPS];
   const DiaTable table{h_key, h_slot};
   const bool hashed = nd <= DIA_HASH_DIAGS;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, S = R + 1;
+  const int groups = R / 32;                              // of 32 rows
+  const int share = groups < WARPS ? WARPS / groups : 1;  // warps that share a group's entries
   if constexpr (REM)
     for (int i = threadIdx.x; i < R; i += DIA_TILE_THREADS) s_rem[i] = 0;
   if (hashed) dia_table_clear(table);
@@ -372,32 +365,28 @@ dia_fill_tiles(const int32_t* __restrict__ r, const int32_t* __restrict__ c, con
   if (hashed) dia_table_fill(table, offs, nd);
   __syncthreads();
   const int64_t ntiles = (pitch + R - 1) / R;
+  struct Entry {
+    int32_t col;
+    T val;
+  };
   for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int64_t r0 = t * R;
-    const int32_t e0 = start[min(r0, nrows)], e1 = start[min(r0 + R, nrows)];
     for (int d0 = 0; d0 < nd; d0 += D) {
       const int dn = min(D, nd - d0);
-      for (int64_t e = (int64_t)e0 + threadIdx.x; e < e1; e += 4 * DIA_TILE_THREADS) {
-        int32_t row[4], col[4];
-        T val[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          const int64_t i = e + k * DIA_TILE_THREADS;
-          if (i < e1) {
-            row[k] = __ldcs(r + i);
-            col[k] = __ldcs(c + i);
-            val[k] = __ldcs(v + i);
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-          if (e + k * DIA_TILE_THREADS < e1) {
-            const int32_t d = col[k] - row[k];
-            const int found = hashed ? dia_table_find(table, d) : bin_slot[(int64_t)d + nrows - 1];
-            const int s = found - d0;
-            if (s >= 0 && s < dn) tile[s * S + (int)(row[k] - r0)] = val[k];
-            if (REM && found < 0 && d0 == 0) atomicAdd(s_rem + (int)(row[k] - r0), 1);
-          }
+      for (int g = w / share; g < groups; g += WARPS / share) {
+        const int64_t g0 = r0 + 32 * g;
+        if (g0 >= nrows) break;
+        prim::warp_row_walk(
+            start, g0, nrows, s_rows[w], lane, w % share, share,
+            [&](int64_t e) { return Entry{__ldcs(c + e), __ldcs(v + e)}; },
+            [&](bool in, int q, int64_t, Entry x) {
+              if (!in) return;
+              const int32_t d = x.col - (int32_t)(g0 + q);
+              const int found = hashed ? dia_table_find(table, d) : bin_slot[(int64_t)d + nrows - 1];
+              const int s = found - d0;
+              if (s >= 0 && s < dn) tile[s * S + 32 * g + q] = x.val;
+              if (REM && found < 0 && d0 == 0) atomicAdd(s_rem + 32 * g + q, 1);
+            });
       }
       __syncthreads();
       if (REM && d0 == 0)
@@ -405,7 +394,7 @@ dia_fill_tiles(const int32_t* __restrict__ r, const int32_t* __restrict__ c, con
           if (r0 + q < nrows) rem[r0 + q] = s_rem[q];
           s_rem[q] = 0;
         }
-      for (int d = w; d < dn; d += DIA_TILE_THREADS / 32)
+      for (int d = w; d < dn; d += WARPS)
         for (int q = lane; q < R; q += 32) {
           if (r0 + q < pitch) __stcs(out + r0 + q + pitch * (int64_t)(d0 + d), tile[d * S + q]);
           tile[d * S + q] = T(0);
@@ -434,16 +423,14 @@ int launch_dia_fill(const mgb_coo* src, const int32_t* start, int64_t pitch, int
   int R, D;
   dia_tile_shape<T>(nd, &R, &D);
   const size_t smem = sizeof(T) * (size_t)D * (R + 1);
-  const unsigned grid = blocks_for((pitch + R - 1) / R, 1, (int64_t)num_sms() * 8);
+  const unsigned grid = blocks_for((pitch + R - 1) / R, 1, (int64_t)num_sms() * 16);
   const T* v = static_cast<const T*>(src->values);
   if (rem != nullptr)
-    dia_fill_tiles<T, true><<<grid, DIA_TILE_THREADS, smem, s>>>(src->row_indices, src->column_indices, v, start,
-                                                                 src->nrows, pitch, (int)nd, offs, bin_slot, out, rem,
-                                                                 R, D);
+    dia_fill_tiles<T, true><<<grid, DIA_TILE_THREADS, smem, s>>>(src->column_indices, v, start, src->nrows, pitch,
+                                                                 (int)nd, offs, bin_slot, out, rem, R, D);
   else
-    dia_fill_tiles<T, false><<<grid, DIA_TILE_THREADS, smem, s>>>(src->row_indices, src->column_indices, v, start,
-                                                                  src->nrows, pitch, (int)nd, offs, bin_slot, out,
-                                                                  nullptr, R, D);
+    dia_fill_tiles<T, false><<<grid, DIA_TILE_THREADS, smem, s>>>(src->column_indices, v, start, src->nrows, pitch,
+                                                                  (int)nd, offs, bin_slot, out, nullptr, R, D);
   MGB_LAUNCH_CHECK();
   return MGB_SUCCESS;
 }
@@ -465,25 +452,41 @@ int check_coo_args(const mgb_coo* src, bool diagonals = true) {
   return MGB_SUCCESS;
 }
 
+// One pass over the entries' indices into *dw (and the diagonal counts unless
+// null); *start: a CSR matrix's offsets, else, if asked for, row starts in
+// scratch.
+int index_pass(const mgb_coo* src, const int32_t* ro, bool starts, Words* dw, int32_t* diag, const int32_t** start,
+               Scratch& sc, cudaStream_t s) {
+  if (ro != nullptr) {
+    *start = ro;
+    return prim::csr_pass(ro, src->column_indices, src->nnz, src->nrows, src->ncols, dw, diag, s);
+  }
+  int32_t* own = nullptr;
+  if (starts) MGB_SCRATCH(sc, own, src->nrows + 1);
+  *start = own;
+  return prim::coo_pass(src->row_indices, src->column_indices, src->nnz, src->nrows, src->ncols, dw, diag, own, s);
+}
+
 // COO -> DIA sizes: one pass over the indices counts the diagonals, checks
 // the ranges and the order and (starts) finds the row starts; the occupied
 // bins are counted; one host read.
+// ro: the offsets of a CSR matrix, whose entries src then holds without row
+// indices (here and in the plans below).
 struct DiaPlan {
-  int32_t *counts = nullptr, *start = nullptr;
+  int32_t* counts = nullptr;
+  const int32_t* start = nullptr;
   int64_t* sums = nullptr;
   Words h{};
 };
-int dia_plan(const mgb_coo* src, bool starts, DiaPlan* p, Scratch& sc, cudaStream_t s) {
-  int st = check_coo_args(src);
+int dia_plan(const mgb_coo* src, const int32_t* ro, bool starts, DiaPlan* p, Scratch& sc, cudaStream_t s) {
+  int st = ro ? MGB_SUCCESS : check_coo_args(src);
   if (st) return st;
   Words* dw;
   st = words_alloc(sc, &dw, s);
   if (st) return st;
   const int64_t nb = src->nrows + src->ncols - 1;
   MGB_SCRATCH(sc, p->counts, nb > 0 ? nb : 1);
-  if (starts) MGB_SCRATCH(sc, p->start, src->nrows + 1);
-  st = prim::coo_pass(src->row_indices, src->column_indices, src->nnz, src->nrows, src->ncols, dw, p->counts,
-                      p->start, s);
+  st = index_pass(src, ro, starts, dw, p->counts, &p->start, sc, s);
   if (st) return st;
   if (src->nnz > 0 && nb > 0) {
     MGB_SCRATCH(sc, p->sums, prim::bin_tiles(nb));
@@ -502,7 +505,7 @@ int coo_to_dia_plan(const mgb_coo* src, int64_t* ndiags, cudaStream_t s) {
   *ndiags = 0;
   Scratch sc(s);
   DiaPlan p;
-  const int st = dia_plan(src, false, &p, sc, s);
+  const int st = dia_plan(src, nullptr, false, &p, sc, s);
   if (st == MGB_SUCCESS || st == MGB_ERR_FORMAT_CONVERSION) *ndiags = p.h.total;
   return st;
 }
@@ -550,7 +553,7 @@ template <typename T>
 int coo_to_dia(const mgb_coo* src, mgb_dia* dst, cudaStream_t s) {
   Scratch sc(s);
   DiaPlan p;
-  const int st = dia_plan(src, true, &p, sc, s);
+  const int st = dia_plan(src, nullptr, true, &p, sc, s);
   return st ? st : dia_fill<T>(src, p, dst, s);
 }
 
@@ -950,16 +953,15 @@ __global__ void __launch_bounds__(256) row_sizes(LEN len, int64_t nrows, int64_t
 // starts) and one over the rows; one host read.  A COO whose rows are not
 // sorted has no row starts: its row histogram and a second read follow.
 struct RowPlan {
-  int32_t* start = nullptr;
+  const int32_t* start = nullptr;
   Words h{};
 };
-int row_plan(const mgb_coo* src, int64_t width, RowPlan* p, Scratch& sc, cudaStream_t s) {
+int row_plan(const mgb_coo* src, const int32_t* ro, int64_t width, RowPlan* p, Scratch& sc, cudaStream_t s) {
   const int64_t N = src->nrows;
   Words* dw;
   int st = words_alloc(sc, &dw, s);
   if (st) return st;
-  MGB_SCRATCH(sc, p->start, N + 1);
-  st = prim::coo_pass(src->row_indices, src->column_indices, src->nnz, N, src->ncols, dw, nullptr, p->start, s);
+  st = index_pass(src, ro, true, dw, nullptr, &p->start, sc, s);
   if (st) return st;
   const unsigned grid = blocks_for(N, 256, (int64_t)num_sms() * 8);
   row_sizes<<<grid, 256, 0, s>>>(RowsFromStart{p->start}, N, width, dw);
@@ -970,9 +972,11 @@ int row_plan(const mgb_coo* src, int64_t width, RowPlan* p, Scratch& sc, cudaStr
   if (words_rows_sorted(p->h)) return MGB_SUCCESS;
   const int32_t seen = p->h.seen;
   MGB_CUDA_CHECK(cudaMemsetAsync(dw, 0, sizeof(Words), s));
-  st = prim::histogram(src->row_indices, src->nnz, p->start, N, s);
+  int32_t* counts;
+  MGB_SCRATCH(sc, counts, N);
+  st = prim::histogram(src->row_indices, src->nnz, counts, N, s);
   if (st) return st;
-  row_sizes<<<grid, 256, 0, s>>>(RowsFromCounts{p->start}, N, width, dw);
+  row_sizes<<<grid, 256, 0, s>>>(RowsFromCounts{counts}, N, width, dw);
   MGB_LAUNCH_CHECK();
   st = words_read(dw, &p->h, s);
   p->h.seen = seen;
@@ -980,11 +984,11 @@ int row_plan(const mgb_coo* src, int64_t width, RowPlan* p, Scratch& sc, cudaStr
 }
 
 // Sizes of a COO's ELL form; h.maxv is the ELL width.
-int ell_plan(const mgb_coo* src, RowPlan* p, Scratch& sc, cudaStream_t s) {
-  int st = check_coo_args(src);
+int ell_plan(const mgb_coo* src, const int32_t* ro, RowPlan* p, Scratch& sc, cudaStream_t s) {
+  int st = ro ? MGB_SUCCESS : check_coo_args(src);
   if (st) return st;
   if (src->nrows == 0) return src->nnz > 0 ? MGB_ERR_INVALID_INPUT : MGB_SUCCESS;  // every row out of range
-  st = row_plan(src, 0, p, sc, s);
+  st = row_plan(src, ro, 0, p, sc, s);
   if (st) return st;
   p->h.maxv = std::max(p->h.maxv, 0);
   if (exceeds_tolerance(src->nrows, src->nnz, p->h.maxv)) return MGB_ERR_FORMAT_CONVERSION;
@@ -996,7 +1000,7 @@ int coo_to_ell_plan(const mgb_coo* src, int64_t* epr, cudaStream_t s) {
   *epr = 0;
   Scratch sc(s);
   RowPlan p;
-  const int st = ell_plan(src, &p, sc, s);
+  const int st = ell_plan(src, nullptr, &p, sc, s);
   if (st == MGB_SUCCESS || st == MGB_ERR_FORMAT_CONVERSION) *epr = p.h.maxv;
   return st;
 }
@@ -1022,19 +1026,20 @@ template <typename T>
 int coo_to_ell(const mgb_coo* src, mgb_ell* dst, cudaStream_t s) {
   Scratch sc(s);
   RowPlan p;
-  const int st = ell_plan(src, &p, sc, s);
+  const int st = ell_plan(src, nullptr, &p, sc, s);
   return st ? st : ell_fill<T>(src, p, dst, s);
 }
 
 // impl/Hyb/Serial/Morpheus_Convert_Impl.hpp:110-151 (width = max(1, nnz/nrows)
 // unless the caller passes one)
-int hyb_plan(const mgb_coo* src, int64_t width, int64_t* W, RowPlan* p, Scratch& sc, cudaStream_t s) {
+int hyb_plan(const mgb_coo* src, const int32_t* ro, int64_t width, int64_t* W, RowPlan* p, Scratch& sc,
+             cudaStream_t s) {
   MGB_REQUIRE(width >= 0, MGB_ERR_BAD_ARGUMENT);
-  int st = check_coo_args(src);
+  int st = ro ? MGB_SUCCESS : check_coo_args(src);
   if (st) return st;
   MGB_REQUIRE(src->nrows > 0, MGB_ERR_INVALID_INPUT);  // the reference divides by nrows
   *W = width > 0 ? width : std::max<int64_t>(1, src->nnz / src->nrows);
-  st = row_plan(src, *W, p, sc, s);
+  st = row_plan(src, ro, *W, p, sc, s);
   if (st) return st;
   if (exceeds_tolerance(src->nrows, p->h.total, *W)) return MGB_ERR_FORMAT_CONVERSION;
   return MGB_SUCCESS;
@@ -1046,7 +1051,7 @@ int coo_to_hyb_plan(const mgb_coo* src, int64_t width, int64_t* epr, int64_t* el
   Scratch sc(s);
   RowPlan p;
   int64_t W = 0;
-  const int st = hyb_plan(src, width, &W, &p, sc, s);
+  const int st = hyb_plan(src, nullptr, width, &W, &p, sc, s);
   if (st == MGB_SUCCESS || st == MGB_ERR_FORMAT_CONVERSION) {
     *epr = W;
     *ell_nnz = p.h.total;
@@ -1113,7 +1118,7 @@ int coo_to_hyb(const mgb_coo* src, mgb_hyb* dst, cudaStream_t s) {
   Scratch sc(s);
   RowPlan p;
   int64_t W = 0;
-  const int st = hyb_plan(src, dst->ell.entries_per_row, &W, &p, sc, s);
+  const int st = hyb_plan(src, nullptr, dst->ell.entries_per_row, &W, &p, sc, s);
   return st ? st : hyb_fill<T>(src, p, W, dst, s);
 }
 
@@ -1183,53 +1188,43 @@ __global__ void hdc_dia_place(const int32_t* __restrict__ r, const T* __restrict
 // row] on: one warp per 32 rows, ranks by ballot.
 template <typename T>
 __global__ void __launch_bounds__(256)
-hdc_remainder(const int32_t* __restrict__ r, const int32_t* __restrict__ c, const T* __restrict__ v,
-              const int32_t* __restrict__ start, const int32_t* __restrict__ base, int64_t nrows, int nd,
-              const int32_t* __restrict__ offs, const int32_t* __restrict__ bin_slot, int64_t limit,
-              int32_t* __restrict__ ocol, T* __restrict__ oval) {
+hdc_remainder(const int32_t* __restrict__ c, const T* __restrict__ v, const int32_t* __restrict__ start,
+              const int32_t* __restrict__ base, int64_t nrows, int nd, const int32_t* __restrict__ offs,
+              const int32_t* __restrict__ bin_slot, int64_t limit, int32_t* __restrict__ ocol,
+              T* __restrict__ oval) {
   __shared__ int32_t h_key[DIA_HASH_SLOTS], h_slot[DIA_HASH_SLOTS];
+  __shared__ prim::WarpRows s_rows[8];
   const DiaTable table{h_key, h_slot};
   const bool hashed = nd <= DIA_HASH_DIAGS;
   if (hashed) dia_table_clear(table);
   __syncthreads();
   if (hashed) dia_table_fill(table, offs, nd);
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * 8;
-  for (int64_t r0 = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * 32; r0 < nrows; r0 += warps * 32) {
-    const int64_t r1 = min(r0 + 32, nrows);
-    const int64_t e1 = start[r1];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int64_t r0 = ((int64_t)blockIdx.x * 8 + w) * 32; r0 < nrows; r0 += (int64_t)gridDim.x * 256) {
     int64_t to = base[r0];
-    if (to == base[r1]) continue;  // every entry on a stored diagonal
-    for (int64_t e0 = start[r0]; e0 < e1; e0 += 128) {
-      int32_t row[4], col[4];
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        const int64_t e = e0 + 32 * k + lane;
-        row[k] = e < e1 ? __ldcs(r + e) : 0;
-        col[k] = e < e1 ? __ldcs(c + e) : 0;
-      }
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        const int64_t e = e0 + 32 * k + lane;
-        const int32_t d = col[k] - row[k];
-        const bool miss = e < e1 && (hashed ? dia_table_find(table, d) : bin_slot[(int64_t)d + nrows - 1]) < 0;
-        const unsigned m = __ballot_sync(0xffffffffu, miss);
-        const int64_t p = to + __popc(m & ((1u << lane) - 1));
-        if (miss && p < limit) {
-          ocol[p] = col[k];
-          oval[p] = v[e];
-        }
-        to += __popc(m);
-      }
-    }
+    if (to == base[min(r0 + 32, nrows)]) continue;  // every entry on a stored diagonal
+    prim::warp_row_walk(
+        start, r0, nrows, s_rows[w], lane, 0, 1, [&](int64_t e) { return __ldcs(c + e); },
+        [&](bool in, int q, int64_t e, int32_t col) {
+          const int32_t d = col - (int32_t)(r0 + q);
+          const bool miss = in && (hashed ? dia_table_find(table, d) : bin_slot[(int64_t)d + nrows - 1]) < 0;
+          const unsigned m = __ballot_sync(0xffffffffu, miss);
+          const int64_t p = to + __popc(m & ((1u << lane) - 1));
+          if (miss && p < limit) {
+            ocol[p] = col;
+            oval[p] = v[e];
+          }
+          to += __popc(m);
+        });
   }
 }
 
 // COO -> HDC sizes: one pass over the indices as for DIA, then the true
 // diagonals (>= floor(0.2 N) entries) and their entry count; one host read.
 struct HdcPlan {
-  int32_t *counts = nullptr, *start = nullptr;
+  int32_t* counts = nullptr;
+  const int32_t* start = nullptr;
   int64_t* sums = nullptr;
   int32_t min_elem = 0;
   Words h{};
@@ -1237,8 +1232,8 @@ struct HdcPlan {
 int32_t hdc_min_elem(const mgb_coo* src) {
   return (int32_t)((double)src->nrows * 0.2);  // HdcMatrix::true_diagonal_ratio
 }
-int hdc_plan(const mgb_coo* src, bool starts, HdcPlan* p, Scratch& sc, cudaStream_t s) {
-  int st = check_coo_args(src);
+int hdc_plan(const mgb_coo* src, const int32_t* ro, bool starts, HdcPlan* p, Scratch& sc, cudaStream_t s) {
+  int st = ro ? MGB_SUCCESS : check_coo_args(src);
   if (st) return st;
   MGB_REQUIRE(src->nrows > 0 && src->ncols > 0, MGB_ERR_INVALID_INPUT);
   const int64_t nb = src->nrows + src->ncols - 1;
@@ -1248,9 +1243,7 @@ int hdc_plan(const mgb_coo* src, bool starts, HdcPlan* p, Scratch& sc, cudaStrea
   if (st) return st;
   MGB_SCRATCH(sc, p->counts, nb);
   MGB_SCRATCH(sc, p->sums, prim::bin_tiles(nb));
-  if (starts) MGB_SCRATCH(sc, p->start, src->nrows + 1);
-  st = prim::coo_pass(src->row_indices, src->column_indices, src->nnz, src->nrows, src->ncols, dw, p->counts,
-                      p->start, s);
+  st = index_pass(src, ro, starts, dw, p->counts, &p->start, sc, s);
   if (st) return st;
   st = prim::select_bins(p->counts, nb, p->min_elem, p->sums, &dw->total, &dw->total2, s);
   if (st) return st;
@@ -1265,7 +1258,7 @@ int coo_to_hdc_plan(const mgb_coo* src, int64_t* ndiags, int64_t* dia_nnz, int64
   MGB_REQUIRE(ndiags && dia_nnz && csr_nnz, MGB_ERR_BAD_ARGUMENT);
   Scratch sc(s);
   HdcPlan p;
-  const int st = hdc_plan(src, false, &p, sc, s);
+  const int st = hdc_plan(src, nullptr, false, &p, sc, s);
   if (st == MGB_SUCCESS || st == MGB_ERR_FORMAT_CONVERSION) {
     *ndiags = p.h.total;
     *dia_nnz = p.h.total2;
@@ -1331,8 +1324,8 @@ int hdc_fill(const mgb_coo* src, const HdcPlan& p, mgb_hdc* dst, cudaStream_t s)
       st = prim::exclusive_scan<int32_t, int32_t>(rem, C->row_offsets, N + 1, s);
       if (st || cn == 0) return st;
       hdc_remainder<T><<<blocks_for(N, 256, (int64_t)num_sms() * 8), 256, 0, s>>>(
-          src->row_indices, src->column_indices, v, p.start, C->row_offsets, N, (int)nd, D->diagonal_offsets, p.counts,
-          cn, C->column_indices, static_cast<T*>(C->values));
+          src->column_indices, v, p.start, C->row_offsets, N, (int)nd, D->diagonal_offsets, p.counts, cn,
+          C->column_indices, static_cast<T*>(C->values));
       MGB_LAUNCH_CHECK();
       return MGB_SUCCESS;
     }
@@ -1404,7 +1397,7 @@ int coo_to_hdc(const mgb_coo* src, mgb_hdc* dst, cudaStream_t s) {
   MGB_REQUIRE(dst != nullptr, MGB_ERR_BAD_ARGUMENT);
   Scratch sc(s);
   HdcPlan p;
-  const int st = hdc_plan(src, true, &p, sc, s);
+  const int st = hdc_plan(src, nullptr, true, &p, sc, s);
   return st ? st : hdc_fill<T>(src, p, dst, s);
 }
 
@@ -1413,12 +1406,14 @@ int coo_to_hdc(const mgb_coo* src, mgb_hdc* dst, cudaStream_t s) {
 // workspace, and mgb_convert_coo_planned_* fills from there: the indices are
 // read for the sizes once, where a *_plan call and its conversion each read
 // them (260 us of 2,342 for the selector's switch of the 160^3 stencil), and
-// nothing that size is allocated.
+// nothing that size is allocated.  mgb_convert_csr_plan does the same for the
+// entries of a CSR matrix, whose offsets take the place of the row starts: its
+// row indices are neither made nor read.
 enum { PLAN_CSR = 1, PLAN_DIA = 2, PLAN_ELL = 3, PLAN_HYB = 4, PLAN_HDC = 5 };  // formats_e
 
-size_t plan_bytes(const mgb_coo* src, int format) {
-  size_t b = Scratch::padded(sizeof(Words)) + Scratch::padded(sizeof(int32_t) * (size_t)(src->nrows + 1));
-  const int64_t nb = std::max<int64_t>(1, src->nrows + src->ncols - 1);
+size_t plan_bytes(int64_t nrows, int64_t ncols, int format) {
+  size_t b = Scratch::padded(sizeof(Words)) + Scratch::padded(sizeof(int32_t) * (size_t)(nrows + 1));
+  const int64_t nb = std::max<int64_t>(1, nrows + ncols - 1);
   if (format == PLAN_DIA || format == PLAN_HDC)
     b += Scratch::padded(sizeof(int32_t) * (size_t)nb) + Scratch::padded(sizeof(int64_t) * (size_t)prim::bin_tiles(nb));
   return b;
@@ -1428,21 +1423,21 @@ int coo_plan_bytes(const mgb_coo* src, int format, int64_t* bytes) {
   MGB_REQUIRE(bytes != nullptr && format >= PLAN_CSR && format <= PLAN_HDC, MGB_ERR_BAD_ARGUMENT);
   int st = check_coo_args(src, format != PLAN_CSR);
   if (st) return st;
-  *bytes = (int64_t)plan_bytes(src, format);
+  *bytes = (int64_t)plan_bytes(src->nrows, src->ncols, format);
   return MGB_SUCCESS;
 }
 
-int coo_plan(const mgb_coo* src, int format, int64_t hyb_width, void* ws, int64_t bytes, mgb_coo_plan* plan,
-             cudaStream_t s) {
-  MGB_REQUIRE(plan != nullptr && format >= PLAN_CSR && format <= PLAN_HDC, MGB_ERR_BAD_ARGUMENT);
-  int st = check_coo_args(src, format != PLAN_CSR);
-  if (st) return st;
-  MGB_REQUIRE(ws != nullptr && reinterpret_cast<uintptr_t>(ws) % 256 == 0 &&
-                  bytes >= (int64_t)plan_bytes(src, format),
+inline bool bad_workspace(const void* ws) { return reinterpret_cast<uintptr_t>(ws) % 256 != 0; }
+
+// The common part: src's entries with, for a CSR matrix, its offsets.
+int plan_any(const mgb_coo* src, const int32_t* ro, int format, int64_t hyb_width, void* ws, int64_t bytes,
+             mgb_coo_plan* plan, cudaStream_t s) {
+  MGB_REQUIRE(ws != nullptr && !bad_workspace(ws) && bytes >= (int64_t)plan_bytes(src->nrows, src->ncols, format),
               MGB_ERR_BAD_ARGUMENT);
   *plan = mgb_coo_plan{};
   plan->format = format;
   Scratch sc(s, ws, (size_t)bytes);
+  int st;
   if (format == PLAN_CSR) {
     CsrPlan p;
     st = csr_plan(src, &p, sc, s);
@@ -1451,41 +1446,47 @@ int coo_plan(const mgb_coo* src, int format, int64_t hyb_width, void* ws, int64_
     if (!words_rows_sorted(p.h)) plan->fill_bytes = prim::row_sort_bytes(src->nnz, src->nrows);
   } else if (format == PLAN_DIA) {
     DiaPlan p;
-    st = dia_plan(src, true, &p, sc, s);
+    st = dia_plan(src, ro, true, &p, sc, s);
     plan->sizes[0] = p.h.total;
     plan->seen = p.h.seen;
-    plan->parts[0] = p.counts, plan->parts[1] = p.start, plan->parts[2] = p.sums;
+    plan->parts[0] = p.counts, plan->parts[1] = const_cast<int32_t*>(p.start), plan->parts[2] = p.sums;
   } else if (format == PLAN_HDC) {
     HdcPlan p;
-    st = hdc_plan(src, true, &p, sc, s);
+    st = hdc_plan(src, ro, true, &p, sc, s);
     plan->sizes[0] = p.h.total;
     plan->sizes[1] = p.h.total2;
     plan->sizes[2] = src->nnz - p.h.total2;
     plan->seen = p.h.seen;
-    plan->parts[0] = p.counts, plan->parts[1] = p.start, plan->parts[2] = p.sums;
+    plan->parts[0] = p.counts, plan->parts[1] = const_cast<int32_t*>(p.start), plan->parts[2] = p.sums;
   } else {
     RowPlan p;
     int64_t W = 0;
     if (format == PLAN_ELL) {
-      st = ell_plan(src, &p, sc, s);
+      st = ell_plan(src, ro, &p, sc, s);
       plan->sizes[0] = p.h.maxv;
     } else {
-      st = hyb_plan(src, hyb_width, &W, &p, sc, s);
+      st = hyb_plan(src, ro, hyb_width, &W, &p, sc, s);
       plan->sizes[0] = W;
       plan->sizes[1] = p.h.total;
       plan->sizes[2] = src->nnz - p.h.total;
     }
     plan->seen = p.h.seen;
-    plan->parts[1] = p.start;
+    plan->parts[1] = const_cast<int32_t*>(p.start);
   }
   return st;
 }
 
+int coo_plan(const mgb_coo* src, int format, int64_t hyb_width, void* ws, int64_t bytes, mgb_coo_plan* plan,
+             cudaStream_t s) {
+  MGB_REQUIRE(plan != nullptr && format >= PLAN_CSR && format <= PLAN_HDC, MGB_ERR_BAD_ARGUMENT);
+  int st = check_coo_args(src, format != PLAN_CSR);
+  if (st) return st;
+  return plan_any(src, nullptr, format, hyb_width, ws, bytes, plan, s);
+}
+
 template <typename T>
 int coo_planned(const mgb_coo* src, const mgb_coo_plan* plan, void* dst, void* ws, int64_t bytes, cudaStream_t s) {
-  MGB_REQUIRE(plan != nullptr && dst != nullptr, MGB_ERR_BAD_ARGUMENT);
-  int st = check_coo_args(src, plan->format != PLAN_CSR);
-  if (st) return st;
+  MGB_REQUIRE(plan != nullptr && dst != nullptr && src != nullptr, MGB_ERR_BAD_ARGUMENT);
   auto* counts = static_cast<int32_t*>(plan->parts[0]);
   auto* start = static_cast<int32_t*>(plan->parts[1]);
   auto* sums = static_cast<int64_t*>(plan->parts[2]);
@@ -1493,7 +1494,7 @@ int coo_planned(const mgb_coo* src, const mgb_coo_plan* plan, void* dst, void* w
   h.seen = plan->seen;
   h.total = plan->sizes[0];
   if (plan->format == PLAN_CSR) {
-    MGB_REQUIRE(ws == nullptr || reinterpret_cast<uintptr_t>(ws) % 256 == 0, MGB_ERR_BAD_ARGUMENT);
+    MGB_REQUIRE(!bad_workspace(ws), MGB_ERR_BAD_ARGUMENT);
     Scratch sc(s, ws, (size_t)std::max<int64_t>(bytes, 0));
     CsrPlan p;
     p.start = start, p.h = h;
@@ -1520,6 +1521,59 @@ int coo_planned(const mgb_coo* src, const mgb_coo_plan* plan, void* dst, void* w
   MGB_REQUIRE(plan->format == PLAN_HYB, MGB_ERR_BAD_ARGUMENT);
   p.h.total = plan->sizes[1];
   return hyb_fill<T>(src, p, plan->sizes[0], static_cast<mgb_hyb*>(dst), s);
+}
+
+// The entries of a CSR matrix without row indices: every routine that fills
+// from row starts takes them.
+mgb_coo csr_entries(const mgb_csr* A) {
+  return mgb_coo{A->nrows, A->ncols, A->nnz, nullptr, A->column_indices, A->values};
+}
+
+int csr_source_bytes(const mgb_csr* src, int format, int64_t* bytes) {
+  MGB_REQUIRE(src != nullptr && bytes != nullptr && format >= PLAN_DIA && format <= PLAN_HDC, MGB_ERR_BAD_ARGUMENT);
+  MGB_REQUIRE(!bad_sizes(src->nrows, src->ncols, src->nnz), MGB_ERR_BAD_ARGUMENT);
+  MGB_REQUIRE(src->nrows + src->ncols < INT32_MAX, MGB_ERR_INVALID_INPUT);
+  *bytes = (int64_t)plan_bytes(src->nrows, src->ncols, format);
+  return MGB_SUCCESS;
+}
+
+// format 0 in the plan: not a case for the fills from row starts (offsets that
+// do not span the entries, columns out of order or repeated in a row, more
+// diagonals than the tiles take, a HDC that is not square): the matrix goes
+// through its COO form.
+template <typename T>
+bool csr_fillable(const mgb_csr* src, int format, const mgb_coo_plan& p) {
+  if (p.seen & prim::COO_BAD_OFFSETS) return false;
+  if (format == PLAN_ELL || format == PLAN_HYB) return true;
+  Words h{};
+  h.seen = p.seen;
+  if (!words_distinct(h) || (format == PLAN_HDC && src->nrows != src->ncols)) return false;
+  return p.sizes[0] == 0 || dia_tiled<T>(p.sizes[0]);
+}
+
+template <typename T>
+int csr_source_plan(const mgb_csr* src, int format, int64_t hyb_width, void* ws, int64_t bytes, mgb_coo_plan* plan,
+                    cudaStream_t s) {
+  int64_t need = 0;
+  MGB_REQUIRE(plan != nullptr, MGB_ERR_BAD_ARGUMENT);
+  int st = csr_source_bytes(src, format, &need);
+  if (st) return st;
+  *plan = mgb_coo_plan{};
+  MGB_REQUIRE(src->row_offsets != nullptr && (src->nnz == 0 || (src->column_indices && src->values)),
+              MGB_ERR_BAD_ARGUMENT);
+  if (src->nrows == 0) return MGB_SUCCESS;  // format 0
+  const mgb_coo e = csr_entries(src);
+  st = plan_any(&e, src->row_offsets, format, hyb_width, ws, bytes, plan, s);
+  if (plan->seen & prim::COO_BAD_OFFSETS) st = MGB_SUCCESS;
+  if (st == MGB_SUCCESS && !csr_fillable<T>(src, format, *plan)) *plan = mgb_coo_plan{};
+  return st;
+}
+
+template <typename T>
+int csr_source_planned(const mgb_csr* src, const mgb_coo_plan* plan, void* dst, cudaStream_t s) {
+  MGB_REQUIRE(src != nullptr && plan != nullptr && plan->format >= PLAN_DIA, MGB_ERR_BAD_ARGUMENT);
+  const mgb_coo e = csr_entries(src);
+  return coo_planned<T>(&e, plan, dst, nullptr, 0, s);
 }
 
 // ---------------------------------------------------------------- sort API
@@ -1609,6 +1663,23 @@ int mgb_convert_coo_planned_f64(const mgb_coo* src, const mgb_coo_plan* plan, vo
 int mgb_convert_coo_planned_f32(const mgb_coo* src, const mgb_coo_plan* plan, void* dst, void* workspace,
                                 int64_t bytes, void* stream) {
   return mgb::coo_planned<float>(src, plan, dst, workspace, bytes, mgb::as_stream(stream));
+}
+int mgb_convert_csr_workspace_bytes(const mgb_csr* src, int format, int64_t* bytes) {
+  return mgb::csr_source_bytes(src, format, bytes);
+}
+int mgb_convert_csr_plan_f64(const mgb_csr* src, int format, int64_t hyb_width, void* workspace, int64_t bytes,
+                             mgb_coo_plan* plan, void* stream) {
+  return mgb::csr_source_plan<double>(src, format, hyb_width, workspace, bytes, plan, mgb::as_stream(stream));
+}
+int mgb_convert_csr_plan_f32(const mgb_csr* src, int format, int64_t hyb_width, void* workspace, int64_t bytes,
+                             mgb_coo_plan* plan, void* stream) {
+  return mgb::csr_source_plan<float>(src, format, hyb_width, workspace, bytes, plan, mgb::as_stream(stream));
+}
+int mgb_convert_csr_planned_f64(const mgb_csr* src, const mgb_coo_plan* plan, void* dst, void* stream) {
+  return mgb::csr_source_planned<double>(src, plan, dst, mgb::as_stream(stream));
+}
+int mgb_convert_csr_planned_f32(const mgb_csr* src, const mgb_coo_plan* plan, void* dst, void* stream) {
+  return mgb::csr_source_planned<float>(src, plan, dst, mgb::as_stream(stream));
 }
 int mgb_coo_sort_by_row_and_column_f64(mgb_coo* A, void* stream) {
   return mgb::coo_sort<double>(A, nullptr, 0, mgb::as_stream(stream));

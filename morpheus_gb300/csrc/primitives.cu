@@ -257,6 +257,58 @@ __global__ void __launch_bounds__(256) coo_pass_kernel(const int32_t* __restrict
   }
 }
 
+template <bool DIAG>
+__global__ void __launch_bounds__(256) csr_pass_kernel(const int32_t* __restrict__ ro, const int32_t* __restrict__ c,
+                                                       int64_t n, int64_t nrows, int64_t ncols, int32_t* seen,
+                                                       int32_t* __restrict__ diag) {
+  __shared__ uint32_t h_keys[DIAG ? HIST_SLOTS : 1];
+  __shared__ int32_t h_counts[DIAG ? HIST_SLOTS : 1];
+  __shared__ int h_full, s_bits;
+  __shared__ WarpRows s_rows[8];
+  const CtaHist h{h_keys, h_counts, &h_full};
+  if constexpr (DIAG) hist_init(h);
+  if (threadIdx.x == 0) s_bits = 0;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t nc = (uint32_t)min(ncols, (int64_t)1 << 31);
+  bool bad = false, offsets = false, down = false, equal = false;
+  for (int64_t r0 = ((int64_t)blockIdx.x * 8 + w) * 32; r0 < nrows; r0 += (int64_t)gridDim.x * 256) {
+    const int64_t r = r0 + lane;
+    if (r < nrows) {
+      const int32_t a = ro[r], z = ro[r + 1];
+      offsets |= a > z || a < 0 || z > n || (r == 0 && a != 0) || (r == nrows - 1 && z != n);
+    }
+    if (__any_sync(0xffffffffu, offsets)) break;  // nothing of such rows is read
+    int32_t prev_q = -1;
+    uint32_t prev_c = 0;  // of the group before
+    prim::warp_row_walk(
+        ro, r0, nrows, s_rows[w], lane, 0, 1, [&](int64_t e) { return (uint32_t)__ldcs(c + e); },
+        [&](bool in, int q, int64_t, uint32_t col) {
+          uint32_t pc = __shfl_up_sync(0xffffffffu, col, 1);
+          int pq = __shfl_up_sync(0xffffffffu, q, 1);
+          if (lane == 0) {
+            pc = prev_c;
+            pq = prev_q;
+          }
+          prev_c = __shfl_sync(0xffffffffu, col, 31);
+          prev_q = __shfl_sync(0xffffffffu, q, 31);
+          if (!in) return;
+          bad |= col >= nc;
+          if (pq == q) {
+            down |= col < pc;
+            equal |= col == pc;
+          }
+          if (DIAG && col < nc) hist_add32(h, diag, col - (uint32_t)(r0 + q) + (uint32_t)(nrows - 1));
+        });
+  }
+  const int bits = (bad ? COO_BAD_INDEX : 0) | (offsets ? COO_BAD_OFFSETS : 0) | (down ? COO_UNSORTED : 0) |
+                   (equal ? COO_DUPLICATE : 0);
+  if (bits) atomicOr(&s_bits, bits);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_bits) atomicOr(seen, s_bits);
+  if constexpr (DIAG) hist_flush(h, diag);
+}
+
 // ---- selection of bins -----------------------------------------------------
 __global__ void __launch_bounds__(SCAN_THREADS) bin_tile_sums(const int32_t* __restrict__ counts, int64_t nb,
                                                               int32_t thr, int64_t* __restrict__ sums,
@@ -868,6 +920,18 @@ int coo_pass(const int32_t* rows, const int32_t* cols, int64_t n, int64_t nrows,
     coo_pass_kernel<false, true><<<grid, 256, 0, s>>>(rows, cols, n, nrows, ncols, vec, &d->seen, diag, start);
   else
     coo_pass_kernel<false, false><<<grid, 256, 0, s>>>(rows, cols, n, nrows, ncols, vec, &d->seen, diag, start);
+  MGB_LAUNCH_CHECK();
+  return MGB_SUCCESS;
+}
+
+int csr_pass(const int32_t* ro, const int32_t* cols, int64_t n, int64_t nrows, int64_t ncols, Words* d,
+             int32_t* diag, cudaStream_t s) {
+  const int64_t nb = nrows + ncols - 1;
+  if (diag != nullptr && nb > 0) MGB_CUDA_CHECK(cudaMemsetAsync(diag, 0, sizeof(int32_t) * nb, s));
+  if (nrows <= 0) return MGB_SUCCESS;
+  const unsigned grid = blocks_for(nrows, 256, (int64_t)num_sms() * 8);
+  if (diag != nullptr) csr_pass_kernel<true><<<grid, 256, 0, s>>>(ro, cols, n, nrows, ncols, &d->seen, diag);
+  else csr_pass_kernel<false><<<grid, 256, 0, s>>>(ro, cols, n, nrows, ncols, &d->seen, diag);
   MGB_LAUNCH_CHECK();
   return MGB_SUCCESS;
 }

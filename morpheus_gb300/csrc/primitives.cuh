@@ -96,6 +96,7 @@ constexpr int32_t COO_BAD_INDEX = 1;      // a row outside [0, nrows) or a colum
 constexpr int32_t COO_ROWS_UNSORTED = 2;  // a row smaller than the one before it
 constexpr int32_t COO_UNSORTED = 4;       // a (row, column) smaller than the one before it
 constexpr int32_t COO_DUPLICATE = 8;      // a (row, column) equal to the one before it
+constexpr int32_t COO_BAD_OFFSETS = 16;   // CSR row offsets that do not rise from 0 to the number of entries
 struct Words {
   int64_t total, total2;  // plan sizes
   int32_t seen;           // COO_* bits
@@ -112,6 +113,11 @@ int words_read(const Words* d, Words* h, cudaStream_t s);         // synchronise
 // reported and not counted.
 int coo_pass(const int32_t* rows, const int32_t* cols, int64_t n, int64_t nrows, int64_t ncols, Words* d,
              int32_t* diag, int32_t* start, cudaStream_t s);
+
+// The same for the entries of a CSR matrix (its rows are in order), one read
+// of the columns; d->seen also COO_BAD_OFFSETS.
+int csr_pass(const int32_t* ro, const int32_t* cols, int64_t n, int64_t nrows, int64_t ncols, Words* d,
+             int32_t* diag, cudaStream_t s);
 
 // The bins with counts[b] >= threshold, in order: how many to *d_total, their
 // counts' sum to *d_sum (if not null), and tile prefixes in sums
@@ -217,38 +223,63 @@ __device__ __forceinline__ void hist_flush(CtaHist h, int32_t* global) {
 }
 
 // ---- entries of CSR rows, one warp per 32 rows ------------------------------
-// Visits every entry of the rows [r0, min(r0 + 32, nrows)), 128 consecutive
-// entries at a time and four per lane, however long the rows are: the offsets
-// of the 32 rows lie in shared memory (s_ro, 33 per warp), a lane finds the
-// row of its first entry by a 5-step search and moves on from there.  For each
-// group of four, e0 a multiple of 4: load(e0, lo, hi), then f(k, r) for every k in
-// [lo, hi) (entry e0 + k, row r), then store(e0, lo, hi); entries outside
-// [lo, hi) belong to other warps.
-template <typename LOAD, typename F, typename STORE>
-__device__ __forceinline__ void warp_row_quads(const int32_t* __restrict__ ro, int64_t r0, int64_t nrows,
-                                               int32_t* s_ro, int lane, LOAD load, F f, STORE store) {
+// Visits the entries of the rows [r0, min(r0 + 32, nrows)) in groups of 32
+// consecutive ones, a lane per entry, however long the rows are.  The rows'
+// first entries are marked in a bitmap of 1,024 entries at a time; an entry's
+// row is the number of marks up to it (one population count), through a list
+// of the rows that are not empty.  v = load(e) for four groups ahead of their
+// f(in, q, e, v), which every lane of the warp calls (in: the lane holds entry
+// e, of row r0 + q).  The warps that share the rows take every `step`th group
+// from `first` on.  Searching every fourth entry's row among the offsets and
+// moving on from there took 160 instructions per 128 entries; this takes 30.
+struct WarpRows {
+  uint32_t bits[32];
+  int32_t row[32];
+};
+template <typename LOAD, typename F>
+__device__ __forceinline__ void warp_row_walk(const int32_t* __restrict__ ro, int64_t r0, int64_t nrows, WarpRows& w,
+                                              int lane, int first, int step, LOAD load, F f) {
+  constexpr unsigned ALL = 0xffffffffu;
+  const int32_t a = ro[min(r0 + lane, nrows)], z = ro[min(r0 + lane + 1, nrows)];
+  const int64_t b = __shfl_sync(ALL, a, 0), t = __shfl_sync(ALL, z, 31);
+  const bool some = z > a;
+  const unsigned m = __ballot_sync(ALL, some);
+  const unsigned upto = ALL >> (31 - lane);
   __syncwarp();
-  s_ro[lane] = ro[min(r0 + lane, nrows)];
-  if (lane == 0) s_ro[32] = ro[min(r0 + 32, nrows)];
-  __syncwarp();
-  const int32_t b = s_ro[0], t = s_ro[32];
-  for (int64_t at = (int64_t)(b & ~3) + 4 * lane; at < t; at += 128) {
-    const int32_t e0 = (int32_t)at;
-    const int lo = max(b - e0, 0), hi = min(t - e0, 4);
-    if (lo >= hi) continue;
-    load(e0, lo, hi);
-    int q = 0;
+  if (some) w.row[__popc(m & (upto >> 1))] = lane;
+  for (int64_t c0 = b; c0 < t; c0 += 1024) {
+    w.bits[lane] = 0;
+    __syncwarp();
+    const int64_t at = a - c0;
+    if (some && at >= 0 && at < 1024) atomicOr(w.bits + (at >> 5), 1u << (at & 31));
+    __syncwarp();
+    const uint32_t word = w.bits[lane];
+    int pre = __popc(word);
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1)
-      if (s_ro[q + d] <= e0 + lo) q += d;
-    int32_t next = s_ro[q + 1];
+    for (int d = 1; d < 32; d <<= 1) {
+      const int u = __shfl_up_sync(ALL, pre, d);
+      if (lane >= d) pre += u;
+    }
+    pre += __popc(__ballot_sync(ALL, some && a < c0)) - __popc(word) - 1;
+    const int groups = (int)min((t - c0 + 31) >> 5, (int64_t)32);
+    for (int j = first; j < groups; j += 4 * step) {
+      decltype(load((int64_t)0)) v[4];
 #pragma unroll
-    for (int k = 0; k < 4; k++)
-      if (k >= lo && k < hi) {
-        while (q < 31 && e0 + k >= next) next = s_ro[++q + 1];
-        f(k, r0 + q);
+      for (int u = 0; u < 4; u++) {
+        const int g = j + u * step;
+        const int64_t e = c0 + 32 * g + lane;
+        if (g < groups && e < t) v[u] = load(e);
       }
-    store(e0, lo, hi);
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int g = j + u * step;
+        if (g >= groups) break;
+        const int64_t e = c0 + 32 * g + lane;
+        const int k = (__shfl_sync(ALL, pre, g) + __popc(__shfl_sync(ALL, word, g) & upto)) & 31;
+        f(e < t, m == ALL ? k : w.row[k], e, v[u]);
+      }
+    }
+    __syncwarp();
   }
 }
 

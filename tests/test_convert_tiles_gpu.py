@@ -156,3 +156,61 @@ def test_row_sort_tiles(cuda, N, lens, dtype):
     mgb.sort_by_row_and_column(A, stream=side)
     side.synchronize()
     assert_same_matrix(mgb.matrix_to_host(A), om.to_host())
+
+
+def _csr_host(coo):
+    ro = np.zeros(coo["nrows"] + 1, np.int32)
+    np.cumsum(np.bincount(coo["row_indices"], minlength=coo["nrows"]), out=ro[1:])
+    return {"format": 1, "nrows": coo["nrows"], "ncols": coo["ncols"], "nnz": coo["nnz"], "row_offsets": ro,
+            "column_indices": coo["column_indices"], "values": coo["values"]}
+
+
+# the entries of a CSR matrix without its row indices: empty rows, rows longer than the 1,024 entries that a warp marks
+# at a time, other shapes; and what goes through COO instead (columns out of order, repeated, non-square HDC)
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("fmt", [2, 3, 4, 5])
+@pytest.mark.parametrize("case", ["diagonals", "long", "empty_rows", "wide", "unsorted", "repeated"])
+def test_csr_without_row_indices(cuda, case, fmt, dtype):
+    import morpheus_gb300 as mgb
+    rng = np.random.default_rng(7)
+    if case == "diagonals":
+        A = _csr_host(diagonals(777, 777, 90, seed=3, dtype=dtype))
+    elif case == "long":
+        A = gen.random_lengths_csr(70, 3000, np.resize([2, 2900, 0, 1023, 1025, 1], 70), seed=4, dtype=dtype)
+    elif case == "empty_rows":
+        A = gen.random_csr(3001, 3001, 0.0004, seed=5, dtype=dtype, empty_row_frac=0.5)
+    elif case == "wide":
+        A = gen.random_csr(301, 900, 0.02, seed=6, dtype=dtype)
+    else:
+        A = gen.random_csr(200, 200, 0.05, seed=8, dtype=dtype)
+        cols, ro = A["column_indices"].copy(), A["row_offsets"]
+        for r in np.flatnonzero(np.diff(ro) > 1)[::3]:
+            if case == "unsorted":
+                cols[ro[r]:ro[r + 1]] = cols[ro[r]:ro[r + 1]][::-1]
+            else:
+                cols[ro[r] + 1] = cols[ro[r]]
+        A["column_indices"] = cols
+    om = O.OracleMatrix.from_host(A)
+    dyn = mgb.DynamicMatrix(mgb.matrix_from_host(A))
+    status = mgb.convert(dyn, fmt)
+    try:
+        want = om.convert(fmt).to_host()
+    except O.OracleError:
+        assert status == mgb.conversion_error_e.PROXY_TO_DYNAMIC and dyn.active_index() == 1
+        return
+    assert status == mgb.conversion_error_e.CONV_SUCCESS
+    assert_same_matrix(mgb.matrix_to_host(dyn.active()), want)
+
+
+def test_csr_with_offsets_that_do_not_span_its_entries(cuda):
+    """Such a matrix converts as its COO form does."""
+    import torch
+
+    import morpheus_gb300 as mgb
+    ro = torch.tensor([0, 2, 3, 3], dtype=torch.int32)
+    A = mgb.CsrMatrix(3, 3, 5, ro, torch.tensor([0, 1, 2, 1, 2], dtype=torch.int32),
+                      torch.arange(1, 6, dtype=torch.float64))
+    for fmt in (2, 3, 4, 5):
+        dyn = mgb.DynamicMatrix(A)
+        assert mgb.convert(dyn, fmt) == mgb.conversion_error_e.CONV_SUCCESS
+        assert_same_matrix(mgb.matrix_to_host(dyn.active()), mgb.matrix_to_host(mgb.from_coo(mgb.to_coo(A), fmt)))
