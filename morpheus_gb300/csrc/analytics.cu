@@ -26,6 +26,7 @@ using prim::Scratch;
 
 inline unsigned grid_for(int64_t n) { return blocks_for(n, 256, (int64_t)num_sms() * 16); }
 // counting kernels: the resident CTAs (a CTA's table is flushed once)
+inline unsigned csr_grid(int64_t n) { return blocks_for(n, 256, (int64_t)num_sms() * prim::DIAG_CTAS); }
 inline unsigned diag_grid(int64_t n) { return blocks_for(n, 256, (int64_t)num_sms() * 8); }
 
 // Row lengths: from CSR row offsets, or from a per-row count array.
@@ -101,7 +102,7 @@ __global__ void row_stats_kernel(LEN lens, int64_t nrows, int64_t hyb_w,
 // 32 rows, a lane per entry.  Bound by the issue slots of the counting beside
 // the column indices (HBM).  A thread per row read its columns uncoalesced:
 // 606 us on the 27-point stencil at 160^3.
-__global__ void __launch_bounds__(256) csr_diag_kernel(const int32_t* __restrict__ ro, const int32_t* __restrict__ ci,
+__global__ void __launch_bounds__(256, prim::DIAG_CTAS) csr_diag_kernel(const int32_t* __restrict__ ro, const int32_t* __restrict__ ci,
                                                        int64_t nrows, int64_t ncols, int32_t* lens,
                                                        int32_t* counts) {
   MGB_CTA_HIST(h);
@@ -111,16 +112,17 @@ __global__ void __launch_bounds__(256) csr_diag_kernel(const int32_t* __restrict
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const bool wide = nrows + ncols > (int64_t)INT_MAX;  // bins past 32 bits
   const uint32_t nc = (uint32_t)min(ncols, (int64_t)1 << 31);
-  for (int64_t r0 = ((int64_t)blockIdx.x * 8 + w) * 32; r0 < nrows; r0 += (int64_t)gridDim.x * 256)
+  for (int64_t r0 = ((int64_t)blockIdx.x * 8 + w) * 32; r0 < nrows; r0 += (int64_t)gridDim.x * 256) {
+    const uint32_t diag0 = (uint32_t)(nrows - 1 - r0);
     prim::warp_row_walk(
-        ro, r0, nrows, s_rows[w], lane, 0, 1, [&](int64_t e) { return (uint32_t)__ldcs(ci + e); },
-        [&](bool in, int q, int64_t, uint32_t c) {
+        ro, r0, nrows, s_rows[w], lane, 0, 1, [&](int64_t c0, int i) { return (uint32_t)__ldcs(ci + c0 + i); },
+        [&](bool in, bool, int q, int64_t, int, uint32_t c) {
           if (!in || c >= nc) return;
-          const int64_t r = r0 + q;
-          if (lens != nullptr) prim::warp_merged_add(lens, r);
-          if (wide) prim::hist_add(h, counts, (uint64_t)(c - r + nrows - 1));
-          else prim::hist_add32(h, counts, c - (uint32_t)r + (uint32_t)(nrows - 1));
+          if (lens != nullptr) prim::warp_merged_add(lens, r0 + q);
+          if (wide) prim::hist_add(h, counts, (uint64_t)(c - (r0 + q) + nrows - 1));
+          else prim::hist_add32(h, counts, c - q + diag0);
         });
+  }
   __syncthreads();
   prim::hist_flush(h, counts);
 }
@@ -323,7 +325,7 @@ struct CsrPass : FormPass {
   const int32_t* row_offsets() const override { return A->row_offsets; }
   int run(int32_t*, int32_t* counts, cudaStream_t s) const override {
     if (A->nnz == 0) return MGB_SUCCESS;
-    csr_diag_kernel<<<diag_grid(A->nrows), 256, 0, s>>>(A->row_offsets, A->column_indices, A->nrows, A->ncols,
+    csr_diag_kernel<<<csr_grid(A->nrows), 256, 0, s>>>(A->row_offsets, A->column_indices, A->nrows, A->ncols,
                                                         nullptr, counts);
     MGB_LAUNCH_CHECK();
     return MGB_SUCCESS;
@@ -386,7 +388,7 @@ struct HdcPass : FormPass {
   int run(int32_t* lens, int32_t* counts, cudaStream_t s) const override {
     if (int st = dia.run(lens, counts, s)) return st;
     if (csr->nnz == 0) return MGB_SUCCESS;
-    csr_diag_kernel<<<diag_grid(csr->nrows), 256, 0, s>>>(csr->row_offsets, csr->column_indices, csr->nrows,
+    csr_diag_kernel<<<csr_grid(csr->nrows), 256, 0, s>>>(csr->row_offsets, csr->column_indices, csr->nrows,
                                                           csr->ncols, lens, counts);
     MGB_LAUNCH_CHECK();
     return MGB_SUCCESS;

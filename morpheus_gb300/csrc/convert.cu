@@ -122,9 +122,9 @@ __global__ void __launch_bounds__(256) expand_rows(const int32_t* __restrict__ r
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int32_t* out = rows + shift;
   for (int64_t r0 = ((int64_t)blockIdx.x * 8 + w) * 32; r0 < nrows; r0 += (int64_t)gridDim.x * 256)
-    prim::warp_row_walk(ro, r0, nrows, s_rows[w], lane, 0, 1, [](int64_t) { return 0; },
-                        [&](bool in, int q, int64_t e, int) {
-                          if (in && e >= 0 && e < nnz) __stcs(out + e, (int32_t)(r0 + q));
+    prim::warp_row_walk(ro, r0, nrows, s_rows[w], lane, 0, 1, [](int64_t, int) { return 0; },
+                        [&](bool in, bool, int q, int64_t c0, int i, int) {
+                          if (in && c0 + i >= 0 && c0 + i < nnz) __stcs(out + c0 + i, (int32_t)(r0 + q));
                         });
   const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x, nt = (int64_t)gridDim.x * 256;
   const int64_t first = min((int64_t)ro[0], nnz), last = max((int64_t)ro[nrows], (int64_t)0);
@@ -298,61 +298,60 @@ __global__ void dia_place(const int32_t* __restrict__ r, const int32_t* __restri
 // in shared memory while they are few (DIA_HASH_DIAGS), else in the bin ->
 // slot array.
 constexpr int DIA_TILE_THREADS = 128;
-constexpr int DIA_TILE_BYTES = 32 * 1024;
+constexpr int DIA_TILE_BYTES = 16 * 1024;
 constexpr int DIA_TILE_ROWS = 512;  // at most
 constexpr int DIA_HASH_DIAGS = 256;  // at most a quarter of the table's slots
-constexpr int DIA_HASH_SLOTS = 1024;
+constexpr int DIA_HASH_LOG2 = 10;
+constexpr int DIA_HASH_SLOTS = 1 << DIA_HASH_LOG2;
 constexpr int32_t DIA_HASH_FREE = INT32_MIN;  // no offset: |offset| < 2^31 - 1
 
 struct DiaTable {
-  int32_t *key, *slot;  // diagonal offset (DIA_HASH_FREE: none) and its slot
+  int2* e;  // x: diagonal offset (DIA_HASH_FREE: none), y: its slot
 };
 __device__ __forceinline__ unsigned dia_hash(int32_t d) {
-  return (((uint32_t)d * 0x9E3779B1u) >> 16) & (DIA_HASH_SLOTS - 1);
+  return ((uint32_t)d * 0x9E3779B1u) >> (32 - DIA_HASH_LOG2);
 }
 
 // every thread; the caller synchronises.  Equal offsets keep the lowest slot.
 __device__ __forceinline__ void dia_table_clear(DiaTable t) {
-  for (int i = threadIdx.x; i < DIA_HASH_SLOTS; i += blockDim.x) {
-    t.key[i] = DIA_HASH_FREE;
-    t.slot[i] = INT32_MAX;
-  }
+  for (int i = threadIdx.x; i < DIA_HASH_SLOTS; i += blockDim.x) t.e[i] = make_int2(DIA_HASH_FREE, INT32_MAX);
 }
 __device__ __forceinline__ void dia_table_fill(DiaTable t, const int32_t* __restrict__ offs, int nd) {
   for (int k = threadIdx.x; k < nd; k += blockDim.x) {
     const int32_t d = offs[k];
     unsigned h = dia_hash(d);
     for (int p = 0; p < DIA_HASH_SLOTS; p++) {
-      const int32_t was = atomicCAS(t.key + h, DIA_HASH_FREE, d);
+      const int32_t was = atomicCAS(&t.e[h].x, DIA_HASH_FREE, d);
       if (was == DIA_HASH_FREE || was == d) break;
       h = (h + 1) & (DIA_HASH_SLOTS - 1);
     }
-    atomicMin(t.slot + h, k);
+    atomicMin(&t.e[h].y, k);
   }
 }
 __device__ __forceinline__ int dia_table_find(DiaTable t, int32_t d) {
   unsigned h = dia_hash(d);
-  int32_t k;
-  while ((k = t.key[h]) != d) {
-    if (k == DIA_HASH_FREE) return -1;
+  int2 e = t.e[h];
+  while (e.x != d) {
+    if (e.x == DIA_HASH_FREE) return -1;
     h = (h + 1) & (DIA_HASH_SLOTS - 1);
+    e = t.e[h];
   }
-  return t.slot[h];
+  return e.y;
 }
 
 // REM (HDC): also rem[row] = the row's entries on no stored diagonal.
 template <typename T, bool REM>
-__global__ void __launch_bounds__(DIA_TILE_THREADS)
+__global__ void __launch_bounds__(DIA_TILE_THREADS, 10)
 dia_fill_tiles(const int32_t* __restrict__ c, const T* __restrict__ v, const int32_t* __restrict__ start,
                int64_t nrows, int64_t pitch, int nd, const int32_t* __restrict__ offs,
                const int32_t* __restrict__ bin_slot, T* __restrict__ out, int32_t* __restrict__ rem, int R, int D) {
   constexpr int WARPS = DIA_TILE_THREADS / 32;
   extern __shared__ __align__(16) unsigned char dia_smem[];
   T* tile = reinterpret_cast<T*>(dia_smem);
-  __shared__ int32_t h_key[DIA_HASH_SLOTS], h_slot[DIA_HASH_SLOTS];
+  __shared__ int2 h_table[DIA_HASH_SLOTS];
   __shared__ int32_t s_rem[REM ? DIA_TILE_ROWS : 1];
   __shared__ prim::WarpRows s_rows[WARPS];
-  const DiaTable table{h_key, h_slot};
+  const DiaTable table{h_table};
   const bool hashed = nd <= DIA_HASH_DIAGS;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, S = R + 1;
   const int groups = R / 32;                              // of 32 rows
@@ -378,10 +377,10 @@ dia_fill_tiles(const int32_t* __restrict__ c, const T* __restrict__ v, const int
         if (g0 >= nrows) break;
         prim::warp_row_walk(
             start, g0, nrows, s_rows[w], lane, w % share, share,
-            [&](int64_t e) { return Entry{__ldcs(c + e), __ldcs(v + e)}; },
-            [&](bool in, int q, int64_t, Entry x) {
+            [&](int64_t c0, int i) { return Entry{__ldcs(c + c0 + i), __ldcs(v + c0 + i)}; },
+            [&](bool in, bool, int q, int64_t, int, Entry x) {
               if (!in) return;
-              const int32_t d = x.col - (int32_t)(g0 + q);
+              const int32_t d = x.col - (int32_t)g0 - q;
               const int found = hashed ? dia_table_find(table, d) : bin_slot[(int64_t)d + nrows - 1];
               const int s = found - d0;
               if (s >= 0 && s < dn) tile[s * S + 32 * g + q] = x.val;
@@ -415,7 +414,7 @@ void dia_tile_shape(int64_t nd, int* R, int* D) {
 }
 // More groups than this (thousands of diagonals) and the entries are placed
 // one by one instead.
-constexpr int64_t DIA_TILE_GROUPS = 16;
+constexpr int64_t DIA_TILE_GROUPS = 32;
 
 template <typename T>
 int launch_dia_fill(const mgb_coo* src, const int32_t* start, int64_t pitch, int64_t nd, const int32_t* offs,
@@ -423,7 +422,9 @@ int launch_dia_fill(const mgb_coo* src, const int32_t* start, int64_t pitch, int
   int R, D;
   dia_tile_shape<T>(nd, &R, &D);
   const size_t smem = sizeof(T) * (size_t)D * (R + 1);
-  const unsigned grid = blocks_for((pitch + R - 1) / R, 1, (int64_t)num_sms() * 16);
+  // one resident wave: every CTA sets its table up once
+  const int64_t per_sm = std::min<int64_t>(10, (200 * 1024) / (int64_t)(smem + 12 * 1024));
+  const unsigned grid = blocks_for((pitch + R - 1) / R, 1, (int64_t)num_sms() * std::max<int64_t>(1, per_sm));
   const T* v = static_cast<const T*>(src->values);
   if (rem != nullptr)
     dia_fill_tiles<T, true><<<grid, DIA_TILE_THREADS, smem, s>>>(src->column_indices, v, start, src->nrows, pitch,
@@ -1192,9 +1193,9 @@ hdc_remainder(const int32_t* __restrict__ c, const T* __restrict__ v, const int3
               const int32_t* __restrict__ base, int64_t nrows, int nd, const int32_t* __restrict__ offs,
               const int32_t* __restrict__ bin_slot, int64_t limit, int32_t* __restrict__ ocol,
               T* __restrict__ oval) {
-  __shared__ int32_t h_key[DIA_HASH_SLOTS], h_slot[DIA_HASH_SLOTS];
+  __shared__ int2 h_table[DIA_HASH_SLOTS];
   __shared__ prim::WarpRows s_rows[8];
-  const DiaTable table{h_key, h_slot};
+  const DiaTable table{h_table};
   const bool hashed = nd <= DIA_HASH_DIAGS;
   if (hashed) dia_table_clear(table);
   __syncthreads();
@@ -1205,15 +1206,15 @@ hdc_remainder(const int32_t* __restrict__ c, const T* __restrict__ v, const int3
     int64_t to = base[r0];
     if (to == base[min(r0 + 32, nrows)]) continue;  // every entry on a stored diagonal
     prim::warp_row_walk(
-        start, r0, nrows, s_rows[w], lane, 0, 1, [&](int64_t e) { return __ldcs(c + e); },
-        [&](bool in, int q, int64_t e, int32_t col) {
+        start, r0, nrows, s_rows[w], lane, 0, 1, [&](int64_t c0, int i) { return __ldcs(c + c0 + i); },
+        [&](bool in, bool, int q, int64_t c0, int i, int32_t col) {
           const int32_t d = col - (int32_t)(r0 + q);
           const bool miss = in && (hashed ? dia_table_find(table, d) : bin_slot[(int64_t)d + nrows - 1]) < 0;
           const unsigned m = __ballot_sync(0xffffffffu, miss);
           const int64_t p = to + __popc(m & ((1u << lane) - 1));
           if (miss && p < limit) {
             ocol[p] = col;
-            oval[p] = v[e];
+            oval[p] = v[c0 + i];
           }
           to += __popc(m);
         });

@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(256) coo_pass_kernel(const int32_t* __restrict
 }
 
 template <bool DIAG>
-__global__ void __launch_bounds__(256) csr_pass_kernel(const int32_t* __restrict__ ro, const int32_t* __restrict__ c,
+__global__ void __launch_bounds__(256, DIAG_CTAS) csr_pass_kernel(const int32_t* __restrict__ ro, const int32_t* __restrict__ c,
                                                        int64_t n, int64_t nrows, int64_t ncols, int32_t* seen,
                                                        int32_t* __restrict__ diag) {
   __shared__ uint32_t h_keys[DIAG ? HIST_SLOTS : 1];
@@ -279,26 +279,19 @@ __global__ void __launch_bounds__(256) csr_pass_kernel(const int32_t* __restrict
       offsets |= a > z || a < 0 || z > n || (r == 0 && a != 0) || (r == nrows - 1 && z != n);
     }
     if (__any_sync(0xffffffffu, offsets)) break;  // nothing of such rows is read
-    int32_t prev_q = -1;
-    uint32_t prev_c = 0;  // of the group before
-    prim::warp_row_walk(
-        ro, r0, nrows, s_rows[w], lane, 0, 1, [&](int64_t e) { return (uint32_t)__ldcs(c + e); },
-        [&](bool in, int q, int64_t, uint32_t col) {
-          uint32_t pc = __shfl_up_sync(0xffffffffu, col, 1);
-          int pq = __shfl_up_sync(0xffffffffu, q, 1);
-          if (lane == 0) {
-            pc = prev_c;
-            pq = prev_q;
-          }
-          prev_c = __shfl_sync(0xffffffffu, col, 31);
-          prev_q = __shfl_sync(0xffffffffu, q, 31);
+    uint32_t last = 0;  // column of the entry before the group
+    const uint32_t diag0 = (uint32_t)(nrows - 1 - r0);
+    warp_row_walk(
+        ro, r0, nrows, s_rows[w], lane, 0, 1, [&](int64_t c0, int i) { return (uint32_t)__ldcs(c + c0 + i); },
+        [&](bool in, bool head, int q, int64_t, int, uint32_t col) {
+          uint32_t before = __shfl_up_sync(0xffffffffu, col, 1);
+          if (lane == 0) before = last;
+          last = __shfl_sync(0xffffffffu, col, 31);
           if (!in) return;
           bad |= col >= nc;
-          if (pq == q) {
-            down |= col < pc;
-            equal |= col == pc;
-          }
-          if (DIAG && col < nc) hist_add32(h, diag, col - (uint32_t)(r0 + q) + (uint32_t)(nrows - 1));
+          down |= !head && col < before;
+          equal |= !head && col == before;
+          if (DIAG && col < nc) hist_add32(h, diag, col - q + diag0);
         });
   }
   const int bits = (bad ? COO_BAD_INDEX : 0) | (offsets ? COO_BAD_OFFSETS : 0) | (down ? COO_UNSORTED : 0) |
@@ -929,7 +922,7 @@ int csr_pass(const int32_t* ro, const int32_t* cols, int64_t n, int64_t nrows, i
   const int64_t nb = nrows + ncols - 1;
   if (diag != nullptr && nb > 0) MGB_CUDA_CHECK(cudaMemsetAsync(diag, 0, sizeof(int32_t) * nb, s));
   if (nrows <= 0) return MGB_SUCCESS;
-  const unsigned grid = blocks_for(nrows, 256, (int64_t)num_sms() * 8);
+  const unsigned grid = blocks_for(nrows, 256, (int64_t)num_sms() * DIAG_CTAS);
   if (diag != nullptr) csr_pass_kernel<true><<<grid, 256, 0, s>>>(ro, cols, n, nrows, ncols, &d->seen, diag);
   else csr_pass_kernel<false><<<grid, 256, 0, s>>>(ro, cols, n, nrows, ncols, &d->seen, diag);
   MGB_LAUNCH_CHECK();

@@ -160,6 +160,10 @@ constexpr int HIST_SLOTS = 1 << HIST_SLOTS_LOG2;
 constexpr int HIST_PROBES = 8;
 constexpr uint32_t HIST_EMPTY = ~0u;  // no key of the table (keys from here on are counted globally)
 
+// Resident CTAs of 256 threads per SM of the kernels that walk CSR rows into a
+// table: their grid is one wave (a CTA's table is set up and flushed once).
+constexpr int DIAG_CTAS = 6;
+
 struct CtaHist {
   uint32_t* keys;   // HIST_SLOTS keys, HIST_EMPTY where free
   int32_t* counts;  // HIST_SLOTS counts
@@ -227,11 +231,12 @@ __device__ __forceinline__ void hist_flush(CtaHist h, int32_t* global) {
 // consecutive ones, a lane per entry, however long the rows are.  The rows'
 // first entries are marked in a bitmap of 1,024 entries at a time; an entry's
 // row is the number of marks up to it (one population count), through a list
-// of the rows that are not empty.  v = load(e) for four groups ahead of their
-// f(in, q, e, v), which every lane of the warp calls (in: the lane holds entry
-// e, of row r0 + q).  The warps that share the rows take every `step`th group
-// from `first` on.  Searching every fourth entry's row among the offsets and
-// moving on from there took 160 instructions per 128 entries; this takes 30.
+// of the rows that are not empty.  Entry e = c0 + i: v = load(c0, i) for four
+// groups ahead of their f(in, head, q, c0, i, v), which every lane of the warp
+// calls (in: the lane holds an entry, of row r0 + q; head: the row's first; full
+// groups are compiled with in = true).  The warps that share the rows take every
+// `step`th group from `first` on.  Searching every fourth entry's row among
+// the offsets and moving on from there took 160 instructions per 128 entries.
 struct WarpRows {
   uint32_t bits[32];
   int32_t row[32];
@@ -261,23 +266,25 @@ __device__ __forceinline__ void warp_row_walk(const int32_t* __restrict__ ro, in
       if (lane >= d) pre += u;
     }
     pre += __popc(__ballot_sync(ALL, some && a < c0)) - __popc(word) - 1;
-    const int groups = (int)min((t - c0 + 31) >> 5, (int64_t)32);
-    for (int j = first; j < groups; j += 4 * step) {
-      decltype(load((int64_t)0)) v[4];
+    const int n = (int)min(t - c0, (int64_t)1024);
+    auto emit = [&](bool in, int g, auto v) {
+      const uint32_t marks = __shfl_sync(ALL, word, g);
+      const int k = (__shfl_sync(ALL, pre, g) + __popc(marks & upto)) & 31;
+      f(in, (marks >> lane) & 1, m == ALL ? k : w.row[k], c0, 32 * g + lane, v);
+    };
+    int j = first;
+    for (; j + 3 * step < (n >> 5); j += 4 * step) {
+      decltype(load(c0, 0)) v[4];
 #pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const int g = j + u * step;
-        const int64_t e = c0 + 32 * g + lane;
-        if (g < groups && e < t) v[u] = load(e);
-      }
+      for (int u = 0; u < 4; u++) v[u] = load(c0, 32 * (j + u * step) + lane);
 #pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const int g = j + u * step;
-        if (g >= groups) break;
-        const int64_t e = c0 + 32 * g + lane;
-        const int k = (__shfl_sync(ALL, pre, g) + __popc(__shfl_sync(ALL, word, g) & upto)) & 31;
-        f(e < t, m == ALL ? k : w.row[k], e, v[u]);
-      }
+      for (int u = 0; u < 4; u++) emit(true, j + u * step, v[u]);
+    }
+    for (; 32 * j < n; j += step) {
+      decltype(load(c0, 0)) v{};
+      const bool in = 32 * j + lane < n;
+      if (in) v = load(c0, 32 * j + lane);
+      emit(in, j, v);
     }
     __syncwarp();
   }
