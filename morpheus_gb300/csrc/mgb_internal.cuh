@@ -28,6 +28,24 @@ unsigned long long current_ctx_id();
 // Stream-ordered scratch from the library's pool (freed with cudaFreeAsync).
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
 
+// 64 bytes of page-locked host memory that kernels on the current device can
+// write (ok(): there was one free); given back when it goes out of scope, so
+// the stream has to be synchronised before that.
+class HostWord {
+ public:
+  HostWord();
+  ~HostWord();
+  HostWord(const HostWord&) = delete;
+  HostWord& operator=(const HostWord&) = delete;
+  bool ok() const { return host_ != nullptr; }
+  void* host() const { return host_; }
+  void* device() const { return device_; }
+
+ private:
+  void *host_ = nullptr, *device_ = nullptr;
+  int dev_ = 0, index_ = 0;
+};
+
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 }  // namespace mgb

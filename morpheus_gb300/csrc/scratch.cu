@@ -109,6 +109,54 @@ cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
   return pool != nullptr ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
 }
 
+// Host words: one page per device, 64 words of 64 bytes.  A context that went
+// away took its page with it; words still out of an older page are forgotten.
+namespace {
+struct HostPage {
+  unsigned long long ctx_id;
+  char *host, *device;
+  uint64_t used;  // a bit per word
+};
+HostPage g_page[64] = {};
+}  // namespace
+
+HostWord::HostWord() {
+  if (cudaGetDevice(&dev_) != cudaSuccess || dev_ < 0 || dev_ >= 64) {
+    (void)cudaGetLastError();
+    return;
+  }
+  const unsigned long long id = current_ctx_id();
+  if (id == 0) return;
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  HostPage& page = g_page[dev_];
+  if (page.host == nullptr || page.ctx_id != id) {
+    void *h = nullptr, *d = nullptr;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // another thread's capture is not disturbed
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
+    cudaError_t e = cudaHostAlloc(&h, 64 * 64, cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer(&d, h, 0);
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) {
+      (void)cudaGetLastError();
+      if (h != nullptr) (void)cudaFreeHost(h);
+      return;
+    }
+    page = HostPage{id, static_cast<char*>(h), static_cast<char*>(d), 0};
+  }
+  if (page.used == ~0ull) return;
+  index_ = __builtin_ctzll(~page.used);
+  page.used |= 1ull << index_;
+  host_ = page.host + 64 * index_;
+  device_ = page.device + 64 * index_;
+}
+
+HostWord::~HostWord() {
+  if (host_ == nullptr) return;
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  HostPage& page = g_page[dev_];
+  if (static_cast<char*>(host_) == page.host + 64 * index_) page.used &= ~(1ull << index_);
+}
+
 }  // namespace mgb
 
 extern "C" int mgb_scratch_release(void) {

@@ -17,6 +17,8 @@
 // shuffles, and a one-CTA kernel sums the per-CTA partials.  The partials live
 // in stream-ordered scratch, so no global state is shared
 // between calls or streams.
+#include <cooperative_groups.h>
+
 #include "mgb_internal.cuh"
 
 namespace mgb {
@@ -185,6 +187,63 @@ __global__ void __launch_bounds__(1024) sum_partials(int n, const T* __restrict_
   if (threadIdx.x == 0) *out = s;
 }
 
+// Short vectors: one cluster of SMALL_CTAS CTAs reduces them and writes the
+// result, in one launch and without scratch (two kernels and an allocation
+// otherwise; latency is all there is).  The CTAs' sums meet in the first one's
+// shared memory, in a fixed order.
+constexpr int SMALL_CTAS = 8;
+constexpr int SMALL_THREADS = 512;
+constexpr int64_t SMALL_N = 1 << 17;
+
+template <typename T, int MODE>
+__global__ void __cluster_dims__(SMALL_CTAS, 1, 1) __launch_bounds__(SMALL_THREADS)
+reduce_small(int64_t n, const T* __restrict__ x, const T* __restrict__ y, T* __restrict__ out) {
+  __shared__ T s_cta[SMALL_CTAS];
+  constexpr int V = 16 / sizeof(T);
+  constexpr int U = 4;
+  const int64_t tid = (int64_t)blockIdx.x * SMALL_THREADS + threadIdx.x;
+  constexpr int64_t nth = (int64_t)SMALL_CTAS * SMALL_THREADS;
+  T acc[4] = {T(0), T(0), T(0), T(0)};
+  const bool vec = (reinterpret_cast<uintptr_t>(x) % 16 == 0) && (MODE != 0 || reinterpret_cast<uintptr_t>(y) % 16 == 0);
+  const int64_t nv = vec ? n / V : 0;
+  for (int64_t i = tid; i < nv; i += U * nth) {
+    T a[U][V], b[U][V];
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (i + u * nth < nv) {
+        ld16(x, i + u * nth, a[u]);
+        if constexpr (MODE == 0) ld16(y, i + u * nth, b[u]);
+      }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (i + u * nth < nv) {
+#pragma unroll
+        for (int k = 0; k < V; k++) {
+          T& t = acc[(u * V + k) & 3];
+          if constexpr (MODE == 0) t = fmadd(a[u][k], b[u][k], t);
+          else if constexpr (MODE == 1) t = fmadd(a[u][k], a[u][k], t);
+          else t += a[u][k];
+        }
+      }
+  }
+  for (int64_t i = nv * V + tid; i < n; i += nth) {
+    const T a = __ldcs(x + i);
+    if constexpr (MODE == 0) acc[0] = fmadd(a, __ldcs(y + i), acc[0]);
+    else if constexpr (MODE == 1) acc[0] = fmadd(a, a, acc[0]);
+    else acc[0] += a;
+  }
+  const T t = block_sum((acc[0] + acc[1]) + (acc[2] + acc[3]));
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  if (threadIdx.x == 0) *cluster.map_shared_rank(s_cta + blockIdx.x, 0) = t;
+  cluster.sync();
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    T sum = s_cta[0];
+#pragma unroll
+    for (int i = 1; i < SMALL_CTAS; i++) sum += s_cta[i];
+    *out = sum;
+  }
+}
+
 template <typename T, int MODE>
 int launch_reduce(int64_t n, const T* x, const T* y, T* d_result, cudaStream_t s) {
   MGB_REQUIRE(n >= 0 && d_result != nullptr, MGB_ERR_BAD_ARGUMENT);
@@ -193,6 +252,11 @@ int launch_reduce(int64_t n, const T* x, const T* y, T* d_result, cudaStream_t s
     return MGB_SUCCESS;
   }
   MGB_REQUIRE(x != nullptr && (MODE != 0 || y != nullptr), MGB_ERR_BAD_ARGUMENT);
+  if (n <= SMALL_N) {
+    reduce_small<T, MODE><<<SMALL_CTAS, SMALL_THREADS, 0, s>>>(n, x, y, d_result);
+    MGB_LAUNCH_CHECK();
+    return MGB_SUCCESS;
+  }
   int64_t blocks = (n + RED_THREADS * 8 - 1) / (RED_THREADS * 8);
   const int64_t cap = (int64_t)num_sms() * 4;
   if (blocks > cap) blocks = cap;
@@ -213,6 +277,14 @@ int launch_reduce(int64_t n, const T* x, const T* y, T* d_result, cudaStream_t s
 template <typename T, int MODE>
 int reduce_to_host(int64_t n, const T* x, const T* y, T* result, cudaStream_t s) {
   MGB_REQUIRE(result != nullptr, MGB_ERR_BAD_ARGUMENT);
+  // the kernel writes the result into mapped host memory: no copy to wait for
+  if (HostWord word; n > 0 && word.ok()) {
+    const int st = launch_reduce<T, MODE>(n, x, y, static_cast<T*>(word.device()), s);
+    if (st != MGB_SUCCESS) return st;
+    MGB_CUDA_CHECK(cudaStreamSynchronize(s));
+    *result = *static_cast<const volatile T*>(word.host());
+    return MGB_SUCCESS;
+  }
   T* d = nullptr;
   MGB_CUDA_CHECK(scratch_alloc((void**)&d, sizeof(T), s));
   int st = launch_reduce<T, MODE>(n, x, y, d, s);

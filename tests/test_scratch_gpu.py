@@ -65,3 +65,23 @@ def test_scratch_under_capture(cuda):
         g.replay()
         torch.cuda.synchronize()
         assert np.array_equal(y.cpu().numpy(), want.cpu().numpy())
+
+
+# around the one-launch limit (131,072), fewer elements than threads or vectors, and views that 16-byte loads cannot take
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("n", [1, 3, 8, 4095, 16387, 131071, 131072, 131073])
+def test_short_reductions(cuda, n, dtype):
+    import math
+    rng = np.random.default_rng(n)
+    x, y = (rng.uniform(-1, 1, n + 1).astype(dtype) for _ in range(2))
+    xt, yt = torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda()
+    # a thread adds at most 16 elements of each of 4 sums, then 2 + 5 + 4 + 7 levels: 64 roundings at most
+    tol = 64 * np.finfo(dtype).eps
+    for a, b in ((0, n), (1, n + 1)):
+        u, v = x[a:b].astype(np.float64), y[a:b].astype(np.float64)
+        ut, vt = xt[a:b], yt[a:b]
+        size = math.fsum(np.abs(u * v))
+        assert abs(mgb.dot(n, ut, vt) - math.fsum(u * v)) <= tol * size
+        assert abs(mgb.dot(n, ut, ut) - math.fsum(u * u)) <= tol * math.fsum(u * u)
+        assert abs(mgb.reduce(ut, n) - math.fsum(u)) <= tol * math.fsum(np.abs(u))
+        assert mgb.dot(n, ut, vt) == mgb.dot(n, ut, vt)
