@@ -10,13 +10,8 @@
 // with init, then the COO part accumulating into y.
 //
 // Layout: slot (i, n) at [i + pitch * n], pitch = nrows (column-major, the
-// reference's CUDA LayoutLeft).  A thread owns RPT = 4 consecutive rows and
-// reads each slot column with one 16-byte load of their column indices
-// (int4) and, only where one of the 4 slots holds an entry, 16-byte loads of
-// the values (two double2 / one float4): padding values are never read, and
-// a warp whose 128 rows are all padding at slot n skips the value sectors.
-// Pitches or pointers that do not allow 16-byte loads take 2 or 1 rows per
-// thread.
+// reference's CUDA LayoutLeft).  Padding values are never read.  Three
+// kernels; the rule and the figures are at launch_ell.
 #include "mgb_internal.cuh"
 
 namespace mgb {
@@ -32,19 +27,9 @@ template <> struct EllVec<double, 4> {
     o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
   }
 };
-template <> struct EllVec<float, 4> {
-  static __device__ __forceinline__ void load(const float* p, float* o) {
-    const float4 v = __ldcs(reinterpret_cast<const float4*>(p)); o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
-  }
-};
 template <> struct EllVec<double, 2> {
   static __device__ __forceinline__ void load(const double* p, double* o) {
     const double2 v = __ldcs(reinterpret_cast<const double2*>(p)); o[0] = v.x; o[1] = v.y;
-  }
-};
-template <> struct EllVec<float, 2> {
-  static __device__ __forceinline__ void load(const float* p, float* o) {
-    const float2 v = __ldcs(reinterpret_cast<const float2*>(p)); o[0] = v.x; o[1] = v.y;
   }
 };
 template <typename T> struct EllVec<T, 1> {
@@ -66,6 +51,9 @@ template <> struct IdxVec<1> {
   static __device__ __forceinline__ void load(const int32_t* p, int32_t* o) { o[0] = __ldcs(p); }
 };
 
+// RPT consecutive rows per thread, a slot at a time.  RPT = 4: one 16-byte load
+// of the indices and, only where one of the 4 slots holds an entry, two of the
+// values (RPT = 2: half of each); pitch and pointers have to allow it.
 // MINB: resident CTAs of 256 threads per SM the kernel is compiled for (0:
 // no register cap); the launcher picks it.
 template <typename T, int RPT, int MINB>
@@ -112,24 +100,81 @@ spmv_ell_rows(int64_t nrows, int64_t ncols, int64_t width, int64_t pitch,
   }
 }
 
+// A thread per row, B slots at a time: their indices are loaded a step ahead,
+// their values and x elements are in flight together, and a slot that no row
+// of the warp fills takes no FMA (the FP64 pipe is busy for the slot even
+// where no lane has work).  The sums run in slot order.
+constexpr int ELL_PAIR_THREADS = 128;
+
+template <typename T, int B>
+__global__ void __launch_bounds__(ELL_PAIR_THREADS, 16)
+spmv_ell_pairs(int64_t nrows, int64_t ncols, int64_t width, int64_t pitch, const int32_t* __restrict__ ci,
+               const T* __restrict__ va, const T* __restrict__ x, T* __restrict__ y, int init) {
+  const int64_t row = (int64_t)blockIdx.x * ELL_PAIR_THREADS + threadIdx.x;
+  if (row >= nrows) return;
+  T acc = init ? T(0) : y[row];
+  const int32_t* cp = ci + row;
+  const T* vp = va + row;
+  int32_t c[B];
+#pragma unroll
+  for (int u = 0; u < B; u++) c[u] = u < width ? __ldcs(cp + u * pitch) : -1;
+  for (int64_t k0 = 0; k0 < width; k0 += B, vp += B * pitch) {
+    cp += B * pitch;
+    int32_t next[B];
+#pragma unroll
+    for (int u = 0; u < B; u++) next[u] = k0 + B + u < width ? __ldcs(cp + u * pitch) : -1;
+    T v[B], xv[B];
+#pragma unroll
+    for (int u = 0; u < B; u++)
+      if ((uint64_t)(int64_t)c[u] < (uint64_t)ncols) {
+        v[u] = __ldcs(vp + u * pitch);
+        xv[u] = __ldg(x + c[u]);
+      }
+#pragma unroll
+    for (int u = 0; u < B; u++) {
+      const bool in = (uint64_t)(int64_t)c[u] < (uint64_t)ncols;
+      if (__any_sync(__activemask(), in)) {
+        if (in) acc = fmadd(v[u], xv[u], acc);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < B; u++) c[u] = next[u];
+  }
+  y[row] = acc;
+}
+
 }  // namespace
 
-template <typename T, int MINB>
-int launch_ell_rows(const mgb_ell* A, const T* x, T* y, int init, cudaStream_t s, int64_t blocks, int rpt) {
-  const T* va = static_cast<const T*>(A->values);
-  if (rpt == 4)
-    spmv_ell_rows<T, 4, MINB><<<(unsigned)blocks, ELL_THREADS, 0, s>>>(
-        A->nrows, A->ncols, A->width, A->pitch, A->column_indices, va, x, y, init);
-  else if (rpt == 2)
-    spmv_ell_rows<T, 2, MINB><<<(unsigned)blocks, ELL_THREADS, 0, s>>>(
-        A->nrows, A->ncols, A->width, A->pitch, A->column_indices, va, x, y, init);
-  else
-    spmv_ell_rows<T, 1, MINB><<<(unsigned)blocks, ELL_THREADS, 0, s>>>(
-        A->nrows, A->ncols, A->width, A->pitch, A->column_indices, va, x, y, init);
+template <typename T, int RPT, int MINB>
+int launch_ell_rows(const mgb_ell* A, const T* x, T* y, int init, cudaStream_t s) {
+  const int64_t groups = (A->nrows + RPT - 1) / RPT;
+  int64_t blocks = (groups + ELL_THREADS - 1) / ELL_THREADS;
+  const int64_t cap = (int64_t)num_sms() * 64;
+  if (blocks > cap) blocks = cap;
+  spmv_ell_rows<T, RPT, MINB><<<(unsigned)blocks, ELL_THREADS, 0, s>>>(
+      A->nrows, A->ncols, A->width, A->pitch, A->column_indices, static_cast<const T*>(A->values), x, y, init);
   MGB_LAUNCH_CHECK();
   return MGB_SUCCESS;
 }
 
+// Which kernel (us on one GB300; p: pairs, 1 / 4: rows per thread of spmv_ell_rows):
+//                                     FP64   p     1     4        FP32   p     1     4
+//   27-point stencil, 195,112 rows        16.4  18.4  39.7          16.4  15.2  29.9
+//                     1,000,000           63.8  65.6  87.8          58.7  41.2  48.7
+//                     4,096,000          236   246   241           212   154   173
+//   power-law HYB part, width 34 -> 64 (with its COO part)
+//                        50,000 rows      34.9  39.0  48.2          30.7  24.6  44.6
+//                       400,000           86.5 101    92.2          86.9  62.4  90.3
+//                     1,234,567          206   228    -            192   145    -
+//                     2,000,000          297   330   279           278   204   240
+//   5-point stencil,    202,500 rows      16.8  20.5  20.5          16.0  14.9  16.3
+//                     1,000,000           61.7  69.8  47.0          49.8  30.7  30.8
+//                     4,194,304          232   256   145           182   107   109
+//   9-point stencil,  2,254,502           128    -    96 (2 rows)   -     64    90 (2 rows)
+// FP32: one row per thread everywhere (8 CTAs per SM).  FP64: pairs, except
+// mostly-padding slabs of more rows than threads fit the GPU, where four rows
+// per thread (two where the pitch is not a multiple of 4) read the padding's
+// indices in the fewest instructions.
 template <typename T>
 int launch_ell(const mgb_ell* A, const T* x, T* y, int init, cudaStream_t s) {
   MGB_REQUIRE(A != nullptr, MGB_ERR_BAD_ARGUMENT);
@@ -138,27 +183,24 @@ int launch_ell(const mgb_ell* A, const T* x, T* y, int init, cudaStream_t s) {
   MGB_REQUIRE(y != nullptr, MGB_ERR_BAD_ARGUMENT);
   MGB_REQUIRE(A->width == 0 || (A->pitch >= A->nrows && A->column_indices && A->values && x),
               MGB_ERR_BAD_ARGUMENT);
-  // 16-byte loads need every slot column (row0 + pitch * n, row0 a multiple
-  // of RPT) 16-byte aligned: pitch a multiple of 4 and 16-byte base pointers
-  const uintptr_t ap = reinterpret_cast<uintptr_t>(A->values), ai = reinterpret_cast<uintptr_t>(A->column_indices);
-  const bool vec4 = (A->pitch % 4 == 0) && (ap % 16 == 0) && (ai % 16 == 0);
-  const bool vec2 = (A->pitch % 2 == 0) && (ap % (2 * sizeof(T)) == 0) && (ai % 8 == 0);
-  const int rpt = vec4 ? 4 : (vec2 ? 2 : 1);
-  const int64_t groups = (A->nrows + rpt - 1) / rpt;
-  int64_t blocks = (groups + ELL_THREADS - 1) / ELL_THREADS;
-  const int64_t cap = (int64_t)num_sms() * 64;
-  if (blocks > cap) blocks = cap;
-  // Register caps (measured, 27-point stencil in ELL / power-law HYB at the
-  // p90 width): FP32 at 8 CTAs per SM, 178 -> 173 us / 252 -> 240 us.  FP64
-  // at 6 CTAs per SM where at least half the slots hold entries (FMA-heavy:
-  // stencil 258 -> 241 us), uncapped for mostly-padding slabs (HYB p90: 277
-  // us uncapped, 297 us at 6 CTAs).
   if constexpr (sizeof(T) == 4) {
-    return launch_ell_rows<T, 8>(A, x, y, init, s, blocks, rpt);
+    return launch_ell_rows<T, 1, 8>(A, x, y, init, s);
   } else {
-    const bool dense = 2 * A->nnz >= A->nrows * A->width;
-    if (dense) return launch_ell_rows<T, 6>(A, x, y, init, s, blocks, rpt);
-    return launch_ell_rows<T, 0>(A, x, y, init, s, blocks, rpt);
+    const uintptr_t ap = reinterpret_cast<uintptr_t>(A->values), ai = reinterpret_cast<uintptr_t>(A->column_indices);
+    const bool vec4 = (A->pitch % 4 == 0) && (ap % 16 == 0) && (ai % 16 == 0);
+    const bool padded = 2 * A->nnz < A->nrows * A->width;
+    const int64_t ctas = (A->nrows + ELL_PAIR_THREADS - 1) / ELL_PAIR_THREADS;
+    const bool vec2 = (A->pitch % 2 == 0) && (ap % 16 == 0) && (ai % 8 == 0);
+    if (padded && A->nrows > (int64_t)num_sms() * 2048) {
+      if (vec4) return launch_ell_rows<T, 4, 0>(A, x, y, init, s);
+      if (vec2) return launch_ell_rows<T, 2, 0>(A, x, y, init, s);
+    }
+    if (ctas > 0x7fffffffLL) return launch_ell_rows<T, 1, 0>(A, x, y, init, s);
+    spmv_ell_pairs<T, 2><<<(unsigned)ctas, ELL_PAIR_THREADS, 0, s>>>(A->nrows, A->ncols, A->width, A->pitch,
+                                                                     A->column_indices,
+                                                                     static_cast<const T*>(A->values), x, y, init);
+    MGB_LAUNCH_CHECK();
+    return MGB_SUCCESS;
   }
 }
 

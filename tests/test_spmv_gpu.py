@@ -401,3 +401,56 @@ def test_power_law_full_size(cuda):
     ref = O.OracleMatrix.from_host(A).multiply(x, threads=O.max_threads())
     y = gpu_multiply(A, x, np.zeros(A["nrows"]), True)
     assert rel_err(y, ref) <= 1e-12
+
+
+# ELL rows of very unequal length, odd and even pitches: gaps between a row's
+# slots, empty rows, sizes that leave part of a warp's rows, columns outside the matrix
+@pytest.mark.parametrize("init", [True, False])
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("N,lens", [(1, [0, 50]), (31, [0, 1, 40, 41]), (33, [90, 1, 1, 2]), (64, [0] * 40 + [33]),
+                                    (1000, [1, 1, 1, 34, 2, 0]), (4097, [3, 1, 0, 2, 70])])
+def test_ell_unequal_rows(cuda, N, lens, dtype, init):
+    rng = np.random.default_rng(N)
+    A = gen.csr_to_ell_host(gen.random_lengths_csr(N, 500, np.resize(np.asarray(lens), N), seed=N, dtype=dtype),
+                            width=max(lens) if N > 1 else 50)
+    ci, va = A["column_indices"].reshape(-1, N), A["values"].reshape(-1, N)
+    if A["width"] > A["entries_per_row"] + 2:  # leave a gap and put a stray column into the padding
+        ci[2:A["entries_per_row"] + 2], va[2:A["entries_per_row"] + 2] = \
+            ci[:A["entries_per_row"]].copy(), va[:A["entries_per_row"]].copy()
+        ci[:2], va[:2] = -1, 0
+        ci[1, ::3], va[1, ::3] = 500, 7.0
+    M = mgb.matrix_from_host(A)
+    x, y0 = rng.uniform(-1, 1, 500).astype(dtype), rng.uniform(-1, 1, N).astype(dtype)
+    y = torch.from_numpy(y0).cuda()
+    mgb.multiply(M, torch.from_numpy(x).cuda(), y, init=init)
+    valid = (ci >= 0) & (ci < 500)
+    prod = np.where(valid, va.astype(np.float64) * x.astype(np.float64)[np.where(valid, ci, 0)], 0.0)
+    want = prod.sum(0) + (0.0 if init else y0.astype(np.float64))
+    # a row's sum has at most 100 roundings in sequence
+    bound = 100 * np.finfo(dtype).eps * (np.abs(prod).sum(0) + np.abs(y0))
+    assert np.all(np.abs(y.cpu().numpy() - want) <= bound)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("extra", [0, 1, 2])
+def test_ell_more_rows_than_threads(cuda, extra, dtype):
+    """Mostly-padding slabs on both sides of the four-rows-per-thread rule, by size and by pitch."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for N in (sms * 2048 - 4 + extra, sms * 2048 + 4 + extra):
+        A = gen.csr_to_ell_host(_short_rows(N, dtype), width=2)
+        x = gen.x_vector(N, seed=2, dtype=dtype)
+        y = torch.empty(N, dtype=torch.float64 if dtype == np.float64 else torch.float32, device="cuda")
+        mgb.multiply(mgb.matrix_from_host(A), torch.from_numpy(x).cuda(), y)
+        ci, va = A["column_indices"].reshape(-1, N), A["values"].reshape(-1, N).astype(np.float64)
+        prod = np.where(ci >= 0, va * x.astype(np.float64)[np.maximum(ci, 0)], 0.0)
+        assert np.all(np.abs(y.cpu().numpy() - prod.sum(0)) <= 4 * np.finfo(dtype).eps * np.abs(prod).sum(0))
+
+
+def _short_rows(N, dtype):
+    """CSR rows of 1, 0 and 2 entries in turn."""
+    rng = np.random.default_rng(N)
+    lens = np.resize(np.array([1, 0, 2]), N)
+    rows = np.repeat(np.arange(N, dtype=np.int64), lens)
+    cols = rng.integers(0, N // 2, rows.size) + (np.arange(rows.size) % 2) * (N // 2)
+    order = np.lexsort((cols, rows))
+    return gen.csr_from_sorted_keys(N, N, rows, cols[order], rng.standard_normal(rows.size).astype(dtype))
