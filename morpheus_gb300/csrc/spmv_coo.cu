@@ -11,7 +11,7 @@
 // Design: fixed chunks of COO_CHUNK consecutive entries, one warp each, cut
 // into 32 contiguous lane ranges (the lane-segment scheme of spmv_csr.cu, so
 // every FP64 FMA is issued by all 32 lanes).  Row indices, columns and values
-// are staged through padded shared memory with coalesced loads; a lane
+// are copied into padded shared memory a step ahead (cp.async, two buffers); a lane
 // detects row ends by comparing consecutive row indices.  Rows that cross
 // lanes are combined by one segmented shuffle scan per chunk.  The first and
 // last row of a chunk may continue in a neighbouring chunk, so their sums are
@@ -19,12 +19,13 @@
 // chunk order; interior rows are stored directly: deterministic, no atomics,
 // no searches.  With init, rows without entries are zero-filled by the lane
 // that sees the gap, so y is written once per row.
-#include "mgb_internal.cuh"
+#include "csr_chunk.cuh"
 
 namespace mgb {
 namespace {
 
-constexpr int COO_WARPS = 8;
+constexpr int COO_WARPS = 4;
+constexpr int COO_CTAS = 5;                 // register budget per SM (shared memory allows 2 to 4)
 constexpr int COO_SEG = 8;                  // entries per lane per staging step
 constexpr int COO_PAD = COO_SEG + 1;        // padded lane stride in shared memory
 constexpr int64_t COO_CHUNK = 2048;         // entries per warp chunk (largest)
@@ -34,7 +35,7 @@ constexpr int64_t COO_CHUNK = 2048;         // entries per warp chunk (largest)
 // spread over every SM.
 inline int64_t coo_chunk_size(int64_t nnz) {
   int64_t chunk = COO_CHUNK;
-  const int64_t resident = (int64_t)num_sms() * COO_WARPS * 3;
+  const int64_t resident = (int64_t)num_sms() * 24;
   while (chunk > 256 && nnz / chunk < resident) chunk >>= 1;
   return chunk;
 }
@@ -47,19 +48,15 @@ __device__ __forceinline__ T gather_x(const T* __restrict__ x, int32_t c, int64_
 // IDX: entry and row index type inside the kernel (int32_t when nnz < 2^31 -
 // 4096: measured on GB300, power-law COO 252 -> 221 us, same arithmetic).
 template <typename T, typename IDX>
-__global__ void __launch_bounds__(COO_WARPS * 32, 3)
+__global__ void __launch_bounds__(COO_WARPS * 32, COO_CTAS)
 spmv_coo_segments(int64_t nrows, int64_t ncols, int64_t nnz, int64_t chunk, const int32_t* __restrict__ ri,
                   const int32_t* __restrict__ ci, const T* __restrict__ va, const T* __restrict__ x,
                   T* __restrict__ y, int init, int32_t* __restrict__ carry_row, T* __restrict__ carry_val) {
-  __shared__ T s_val[COO_WARPS][32 * COO_PAD];
-  __shared__ int32_t s_col[COO_WARPS][32 * COO_PAD];
-  __shared__ int32_t s_row[COO_WARPS][32 * COO_PAD];
+  __shared__ T s_val[COO_WARPS][2][32 * COO_PAD];
+  __shared__ int32_t s_col[COO_WARPS][2][32 * COO_PAD];
+  __shared__ int32_t s_row[COO_WARPS][2][32 * COO_PAD];
   const int lane = threadIdx.x & 31;
   const int w = threadIdx.x >> 5;
-  T* sv = s_val[w];
-  int32_t* sc = s_col[w];
-  int32_t* sr = s_row[w];
-
   const IDX nchunks = (nnz + chunk - 1) / chunk;
   const IDX KW = chunk / 32;  // entries per lane, a multiple of COO_SEG
   for (IDX k = (IDX)blockIdx.x * COO_WARPS + w; k < nchunks; k += (IDX)gridDim.x * COO_WARPS) {
@@ -98,19 +95,33 @@ spmv_coo_segments(int64_t nrows, int64_t ncols, int64_t nnz, int64_t chunk, cons
     IDX hrow = -1;
     T hval = T(0), acc = T(0);
 
-    for (IDX st = 0; st < KW; st += COO_SEG) {
-      __syncwarp();
+    // step s + 1 is copied (cp.async) while step s's x reads are in flight
+    auto stage = [&](IDX st, int b) {
+      if (st < KW) {
 #pragma unroll
-      for (int q = 0; q < COO_SEG; q++) {
-        const int f = q * 32 + lane;
-        const int L = f / COO_SEG, j = f % COO_SEG;
-        const IDX e = base + (IDX)L * KW + st + j;
-        const bool in = e < cend;
-        sr[L * COO_PAD + j] = in ? ldg_stream(ri + e) : -1;
-        sc[L * COO_PAD + j] = in ? ldg_stream(ci + e) : 0;
-        sv[L * COO_PAD + j] = in ? ldg_stream(va + e) : T(0);
+        for (int q = 0; q < COO_SEG; q++) {
+          const int f = q * 32 + lane;
+          const int L = f / COO_SEG, j = f % COO_SEG;
+          const IDX e = base + (IDX)L * KW + st + j;
+          const bool in = e < cend;
+          csr::copy_or_zero(s_row[w][b] + L * COO_PAD + j, ri + (in ? e : base), in);
+          csr::copy_or_zero(s_col[w][b] + L * COO_PAD + j, ci + (in ? e : base), in);
+          csr::copy_or_zero(s_val[w][b] + L * COO_PAD + j, va + (in ? e : base), in);
+        }
       }
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    __syncwarp();  // the chunk before is done with the buffers
+    stage(0, 0);
+    int buf = 0;
+    for (IDX st = 0; st < KW; st += COO_SEG, buf ^= 1) {
+      __syncwarp();  // the reads of the buffer filled next are done
+      stage(st + COO_SEG, buf ^ 1);
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
       __syncwarp();
+      const T* sv = s_val[w][buf];
+      const int32_t* sc = s_col[w][buf];
+      const int32_t* sr = s_row[w][buf];
       T v[COO_SEG], xv[COO_SEG];
       int32_t rw[COO_SEG];
 #pragma unroll
@@ -163,6 +174,16 @@ spmv_coo_segments(int64_t nrows, int64_t ncols, int64_t nnz, int64_t chunk, cons
   }
 }
 
+// Shared-memory carve-out of the kernel above (power-law matrix, 2e6 rows, FP64 /
+// FP32; single staging with 24 warps per SM: 223 / 200 us):
+// 35 %: 280 / 208, 45: 226 / 194, 60 and 70: 213 / 186 (12 / 16 warps per SM).
+constexpr int COO_CARVEOUT = 60;
+template <typename T>
+int coo_carveout() {
+  static std::atomic<bool> done[64];
+  return csr::set_carveout_once(spmv_coo_segments<T, int32_t>, done, COO_CARVEOUT);
+}
+
 // Adds the carries of each row in chunk order.  carry_row is non-decreasing.
 template <typename T>
 __global__ void coo_carry_fixup(int64_t ncarry, int64_t nrows,
@@ -192,6 +213,7 @@ int launch_coo(const mgb_coo* A, const T* x, T* y, int init, cudaStream_t s) {
     return MGB_SUCCESS;
   }
   MGB_REQUIRE(A->row_indices && A->column_indices && A->values && x, MGB_ERR_BAD_ARGUMENT);
+  if (int st = coo_carveout<T>()) return st;
   const int64_t chunk = coo_chunk_size(A->nnz);
   const int64_t nchunks = (A->nnz + chunk - 1) / chunk;
   const int64_t ncarry = 2 * nchunks;
@@ -323,6 +345,7 @@ int launch_coo_noalloc_f64(const mgb_coo* A, const double* x, double* y, int ini
     return MGB_SUCCESS;
   }
   MGB_REQUIRE(A->row_indices && A->column_indices && A->values && x, MGB_ERR_BAD_ARGUMENT);
+  if (int st = coo_carveout<double>()) return st;
   void* scratch = nullptr;
   int st = noalloc_scratch(&scratch);
   if (st != MGB_SUCCESS) return st;
