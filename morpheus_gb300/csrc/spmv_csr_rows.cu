@@ -173,6 +173,104 @@ spmv_csr_rowtile(int64_t nrows, int64_t ncols, const int32_t* __restrict__ ro, c
   }
 }
 
+// Short rows with neighbouring columns: a thread per row, straight from global
+// memory.  The entries of 32 rows are a few hundred consecutive bytes, so the
+// uncoalesced loads of a warp hit the same L1 lines over the U entries that
+// are read together, no staging comes between the row offsets and the x reads
+// (three memory latencies per row instead of four, and no waits for copies),
+// and 48 to 64 warps fit an SM.  What bounds it is L1's line lookups, so longer
+// rows go to the staged tiles: direct_kernel.  The sums run in row order as there.
+constexpr int DIRECT_THREADS = 128;
+
+template <typename T, bool DOT, int U, int MINB>
+__global__ void __launch_bounds__(DIRECT_THREADS, MINB)
+spmv_csr_rowdirect(int64_t nrows, int64_t ncols, const int32_t* __restrict__ ro, const int32_t* __restrict__ ci,
+                   const T* __restrict__ va, const T* __restrict__ x, T* __restrict__ y, int init,
+                   T* __restrict__ partials) {
+  T part = T(0);
+  for (int64_t r = (int64_t)blockIdx.x * DIRECT_THREADS + threadIdx.x; r < nrows;
+       r += (int64_t)gridDim.x * DIRECT_THREADS) {
+    const int32_t b = __ldg(ro + r), e = __ldg(ro + r + 1);
+    T acc = init ? T(0) : y[r];
+    for (int32_t j = b; j < e; j += U) {
+      int32_t c[U];
+      T v[U], xv[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        c[u] = j + u < e ? __ldg(ci + j + u) : -1;
+        v[u] = j + u < e ? __ldg(va + j + u) : T(0);
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) xv[u] = (uint64_t)(int64_t)c[u] < (uint64_t)ncols ? __ldg(x + c[u]) : T(0);
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (j + u < e) acc = fmadd(v[u], xv[u], acc);
+    }
+    y[r] = acc;
+    if (DOT) part = fmadd(x[r], acc, part);
+  }
+  if (DOT) {
+    __shared__ T s_part[DIRECT_THREADS / 32];
+    part = warp_sum(part);
+    if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = part;
+    __syncthreads();
+    if (threadIdx.x == 0) partials[blockIdx.x] = (s_part[0] + s_part[1]) + (s_part[2] + s_part[3]);
+  }
+}
+
+// Entries read together (U) and CTAs per SM (MINB) for rows of `mean` entries
+// on average, rounded up; 0: staged tiles.  U follows the row length (7 entries:
+// 4 + 3).  Measured (us, stencils of 1 to 4 million rows; staged, then direct as
+// U x MINB):
+//            FP64  staged  3x16  4x16  5x16  5x12  7x10     FP32  staged  3x16  4x16  5x16  7x10
+//    3 per row       55.3  41.0  41.4  45.6  50.8  62.2             51.4  32.7  32.5  31.1  38.5
+//    5               68.6  57.5  63.8  57.4  59.0  69.5             61.9  41.6  43.0  39.3  44.5
+//    7               67.7  62.7  59.4  66.4  67.6  63.8             57.4  43.0  41.6  42.6  42.6
+//    9               63.9  52.9  55.7  53.9  53.2  62.8             41.2  35.6  37.2  35.7  37.1
+//   13               71.7  75.9  71.1  71.5  67.7  68.1             47.2  47.4  47.4  46.4  43.4
+//   17               88.5  86.0  74.3  75.5  69.9  73.8             50.7  51.3  51.0  47.3  45.1
+//   19               88.8  91.9  77.9  77.6  73.1  74.4             48.8  54.7  53.2  49.7  47.6
+//   25               80.3   101  85.8  82.4  78.0  82.1             45.4  63.5  59.4  56.3  54.0
+// The fused dot's kernel holds more (16 CTAs per SM spill) and runs as one
+// wave: CG on the 2048^2 Laplacian, 24 iterations: 16 CTAs 4,157 us, 12 4,014,
+// 10 4,094 (staged tiles 4,346).
+constexpr int DIRECT_DOT_CTAS = 12;
+struct DirectShape {
+  int u, ctas;
+};
+template <typename T>
+DirectShape direct_shape(const mgb_csr* A) {
+  const int64_t mean = (A->nnz + A->nrows - 1) / (A->nrows > 0 ? A->nrows : 1);
+  if (mean <= 3) return {3, 16};
+  if (mean == 4) return {4, 16};
+  if (mean <= 6) return {5, 16};
+  if (mean <= 8) return {4, 16};
+  if constexpr (sizeof(T) == 8) {
+    if (mean <= 25) return {5, 12};
+  } else {
+    if (mean <= 10) return {5, 16};
+    if (mean <= 20) return {7, 10};
+  }
+  return {0, 0};
+}
+
+template <typename T, bool DOT>
+int launch_direct(const mgb_csr* A, const T* x, T* y, int init, cudaStream_t s, T* partials, DirectShape shape,
+                  unsigned blocks) {
+  const auto run = [&](auto kernel) {
+    kernel<<<blocks, DIRECT_THREADS, 0, s>>>(A->nrows, A->ncols, A->row_offsets, A->column_indices,
+                                             static_cast<const T*>(A->values), x, y, init, partials);
+  };
+  constexpr int MANY = DOT ? DIRECT_DOT_CTAS : 16;
+  if (shape.u == 3) run(spmv_csr_rowdirect<T, DOT, 3, MANY>);
+  else if (shape.u == 4) run(spmv_csr_rowdirect<T, DOT, 4, MANY>);
+  else if (shape.u == 5 && shape.ctas == 16) run(spmv_csr_rowdirect<T, DOT, 5, MANY>);
+  else if (sizeof(T) == 8) run(spmv_csr_rowdirect<T, DOT, 5, 12>);
+  else run(spmv_csr_rowdirect<T, DOT, 7, 10>);
+  MGB_LAUNCH_CHECK();
+  return MGB_SUCCESS;
+}
+
 // Row shape of a CSR matrix: shape[0] = longest row; over every 16th row r
 // (and row r + 1), shape[1] = entries k of the shorter of the two rows with
 // |col(r+1, k) - col(r, k) - 1| <= 2 (neighbouring rows reading neighbouring
@@ -289,6 +387,18 @@ int launch_rows_variant(const mgb_csr* A, const T* x, T* y, int init, cudaStream
 template <typename T>
 int launch_rows(const mgb_csr* A, const T* x, T* y, int init, cudaStream_t s, T* partials, int64_t* npartials,
                 bool gather) {
+  if (const DirectShape shape = direct_shape<T>(A); !gather && shape.u > 0) {
+    int64_t blocks = (A->nrows + DIRECT_THREADS - 1) / DIRECT_THREADS;
+    if (blocks > 0x7fffffffLL) blocks = 0x7fffffffLL;
+    if (npartials || partials) {  // the fused dot: one partial per CTA, grid capped at the resident CTAs
+      const int64_t resident = (int64_t)num_sms() * (shape.ctas < DIRECT_DOT_CTAS ? shape.ctas : DIRECT_DOT_CTAS);
+      if (blocks > resident) blocks = resident;
+      if (npartials) *npartials = blocks;
+    }
+    if (npartials && !partials) return take_device_query_error();
+    return partials ? launch_direct<T, true>(A, x, y, init, s, partials, shape, (unsigned)blocks)
+                    : launch_direct<T, false>(A, x, y, init, s, nullptr, shape, (unsigned)blocks);
+  }
   const int64_t ntiles = (A->nrows + 31) / 32;
   int64_t blocks = (ntiles + ROWS_WARPS - 1) / ROWS_WARPS;
   if (blocks > 0x7fffffffLL) blocks = 0x7fffffffLL;

@@ -454,3 +454,34 @@ def _short_rows(N, dtype):
     cols = rng.integers(0, N // 2, rows.size) + (np.arange(rows.size) % 2) * (N // 2)
     order = np.lexsort((cols, rows))
     return gen.csr_from_sorted_keys(N, N, rows, cols[order], rng.standard_normal(rows.size).astype(dtype))
+
+
+# rows read straight from global memory: every shape of the rule (3 to 25 entries per row and the first that is
+# staged), rows longer and shorter than the entries read together, more rows than one wave, bit for bit the same with
+# and without the fused dot
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("lens", [[1], [3, 2], [4], [5, 6, 4], [7, 8], [9, 10], [11, 12, 13], [20, 22], [25], [26, 27]])
+@pytest.mark.parametrize("N", [1, 129, 5000])
+def test_csr_short_rows(cuda, N, lens, dtype):
+    from morpheus_gb300 import solvers
+    hm = gen.random_lengths_csr(N, max(N, 40), np.resize(np.asarray(lens), N), seed=N + lens[0], dtype=dtype)
+    M = mgb.matrix_from_host(hm)
+    M._variant = mgb.CSR_ROWS
+    x = gen.x_vector(hm["ncols"], seed=1, dtype=dtype)
+    y0 = gen.x_vector(N, seed=2, dtype=dtype)
+    xt = torch.from_numpy(x).cuda()
+    prod = hm["values"].astype(np.float64) * x.astype(np.float64)[hm["column_indices"]]
+    rows = np.repeat(np.arange(N), np.diff(hm["row_offsets"]))
+    for init in (True, False):
+        y = torch.from_numpy(y0).cuda()
+        mgb.multiply(M, xt, y, init=init)
+        base = np.zeros(N) if init else y0.astype(np.float64)
+        want = base + np.bincount(rows, weights=prod, minlength=N)
+        bound = 40 * np.finfo(dtype).eps * (np.bincount(rows, weights=np.abs(prod), minlength=N) + np.abs(base))
+        assert np.all(np.abs(y.cpu().numpy() - want) <= bound)
+        y2 = torch.from_numpy(y0).cuda()
+        d = solvers.multiply_dot(M, xt, y2, init=init)
+        assert torch.equal(y, y2)
+        exact = float(x[:N].astype(np.float64) @ y.cpu().numpy().astype(np.float64))
+        scale = float(np.abs(x[:N].astype(np.float64)) @ np.abs(y.cpu().numpy().astype(np.float64)))
+        assert abs(float(d.item()) - exact) <= 64 * np.finfo(dtype).eps * scale
