@@ -65,15 +65,20 @@ PoolSlot g_pool[64] = {};
 // The current device's pool, made on first use (and again in a new context);
 // null where there is none to be had: the default pool serves then.
 cudaMemPool_t scratch_pool(cudaStream_t s, bool make) {
+  static thread_local PoolSlot last = {};  // a context's ID is never used again
+  const unsigned long long id = current_ctx_id();
+  if (id != 0 && last.ctx_id == id) return last.pool;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
     (void)cudaGetLastError();
     return nullptr;
   }
-  const unsigned long long id = current_ctx_id();
   std::lock_guard<std::mutex> lock(g_pool_mutex);
   PoolSlot& slot = g_pool[dev];
-  if (slot.pool != nullptr && id != 0 && slot.ctx_id == id) return slot.pool;
+  if (slot.pool != nullptr && id != 0 && slot.ctx_id == id) {
+    last = slot;
+    return slot.pool;
+  }
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   if (!make || id == 0 || cudaStreamIsCapturing(s, &capturing) != cudaSuccess ||
       capturing != cudaStreamCaptureStatusNone) {
@@ -99,6 +104,7 @@ cudaMemPool_t scratch_pool(cudaStream_t s, bool make) {
   }
   slot.pool = pool;
   slot.ctx_id = id;
+  last = slot;
   return pool;
 }
 

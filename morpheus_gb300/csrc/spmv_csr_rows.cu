@@ -275,33 +275,47 @@ int launch_direct(const mgb_csr* A, const T* x, T* y, int init, cudaStream_t s, 
 // (and row r + 1), shape[1] = entries k of the shorter of the two rows with
 // |col(r+1, k) - col(r, k) - 1| <= 2 (neighbouring rows reading neighbouring
 // columns), shape[2] = entries compared.
-__global__ void row_shape_kernel(const int32_t* __restrict__ ro, const int32_t* __restrict__ ci, int64_t nrows,
-                                 unsigned long long* shape) {
+// A warp compares a pair of rows 32 entries at a time, and a CTA adds to the
+// counters once: with a thread per pair and atomics per warp the choice took
+// longer than the multiply that followed it.
+__global__ void __launch_bounds__(256) row_shape_kernel(const int32_t* __restrict__ ro,
+                                                        const int32_t* __restrict__ ci, int64_t nrows,
+                                                        unsigned long long* shape) {
+  __shared__ int s_max[8];
+  __shared__ unsigned s_near[8], s_cmp[8];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int m = 0;
-  unsigned long long near = 0, cmp = 0;
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t a = ro[r], b = ro[r + 1];
-    m = max(m, b - a);
-    if ((r & 15) == 0 && r + 1 < nrows) {
-      const int32_t b2 = ro[r + 2];
-      const int32_t len = min(min(b - a, b2 - b), 64);
-      for (int32_t k = 0; k < len; k++) {
-        const int64_t d = (int64_t)ci[b + k] - (int64_t)ci[a + k] - 1;
-        near += (d >= -2 && d <= 2) ? 1u : 0u;
-      }
-      cmp += (unsigned long long)(len > 0 ? len : 0);
+  unsigned near = 0, cmp = 0;  // at most 64 per pair and lane: no overflow below 2^26 pairs per warp
+  for (int64_t r = (int64_t)blockIdx.x * 256 + threadIdx.x; r < nrows; r += (int64_t)gridDim.x * 256)
+    m = max(m, ro[r + 1] - ro[r]);
+  for (int64_t r = ((int64_t)blockIdx.x * 8 + w) * 16; r + 1 < nrows; r += (int64_t)gridDim.x * 128) {
+    const int32_t a = ro[r], b = ro[r + 1], b2 = ro[r + 2];
+    const int32_t len = min(min(b - a, b2 - b), 64);
+    for (int32_t k = lane; k < len; k += 32) {
+      const int64_t d = (int64_t)ci[b + k] - (int64_t)ci[a + k] - 1;
+      near += (d >= -2 && d <= 2) ? 1u : 0u;
+      cmp++;
     }
   }
   m = __reduce_max_sync(0xffffffffu, m);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    near += __shfl_xor_sync(0xffffffffu, near, o);
-    cmp += __shfl_xor_sync(0xffffffffu, cmp, o);
+  near = __reduce_add_sync(0xffffffffu, near);
+  cmp = __reduce_add_sync(0xffffffffu, cmp);
+  if (lane == 0) {
+    s_max[w] = m;
+    s_near[w] = near;
+    s_cmp[w] = cmp;
   }
-  if ((threadIdx.x & 31) == 0) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned long long n = 0, c = 0;
+    for (int i = 0; i < 8; i++) {
+      m = max(m, s_max[i]);
+      n += s_near[i];
+      c += s_cmp[i];
+    }
     atomicMax(shape, (unsigned long long)m);
-    atomicAdd(shape + 1, near);
-    atomicAdd(shape + 2, cmp);
+    atomicAdd(shape + 1, n);
+    atomicAdd(shape + 2, c);
   }
 }
 
