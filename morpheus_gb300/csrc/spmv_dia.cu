@@ -12,9 +12,9 @@
 // CSR-remainder entries, in that order, and writes y once.
 //
 // Layout: values(i, n) at values[i + pitch * n], pitch a multiple of 32, so a
-// thread owning RPT consecutive rows reads its slab entries with one 16-byte
-// (FP64, RPT = 2) or 16-byte (FP32, RPT = 4) vector load per diagonal; the
-// warp covers 32 * RPT consecutive rows, fully coalesced.  Offsets live in
+// thread owning RPT consecutive rows reads its slab entries with one element
+// load (RPT = 1) or 16-byte vector load (FP64 RPT = 2, FP32 RPT = 4) per diagonal;
+// the warp covers 32 * RPT consecutive rows, fully coalesced.  Offsets live in
 // shared memory (chunks of DIA_OFF_CHUNK diagonals).  x is read through the
 // read-only path: neighbouring diagonals hit the same lines in L1/L2.
 #include "mgb_internal.cuh"
@@ -24,18 +24,22 @@ namespace {
 
 constexpr int DIA_THREADS = 256;
 constexpr int DIA_OFF_CHUNK = 512;
-// FP64: pairs of diagonals whose slab and x loads are issued together
-// (measured 204 -> 197 us on the 27-point stencil at 160^3).  FP32: the plain
-// diagonal loop, which the compiler unrolls itself at 40 registers; explicit
-// groups of 2 or 4 raise the register count and lower occupancy (87 us
-// plain, 93-97 us grouped).
-template <typename T> constexpr int kDiaUnroll = sizeof(T) == 4 ? 1 : 2;
-// Resident CTAs of 256 threads per SM the kernel is compiled for (0: no
-// register cap).  FP64: 8 (32 registers, a few bytes of spills), the FP64
-// pipe fed by 64 warps: 27-point stencil DIA 197 -> 195 us, HDC 220 -> 209 us
-// (5 / 6 CTAs: 199 / 196 us).  FP32 is fastest uncapped (40 registers:
-// 87 us; capped at 5-8 CTAs: 88.5-95.6 us).
-template <typename T> constexpr int kDiaMinBlocks = sizeof(T) == 4 ? 0 : 8;
+// Rows per thread, diagonals whose slab and x loads are issued before their
+// FMAs (DU), and the register cap (resident CTAs of 256 threads per SM).
+// Measured (us; RPT x DU; 27 / 7 / 5 diagonals, HDC with 1 % off-band entries):
+//                          FP64 DIA  2x2   1x2   1x3   1x4   FP64 HDC  2x2   1x2   1x3   FP32 HDC  4x1   1x1
+//   27 diagonals,   512,000 rows    34.8  30.8  30.7  30.7            36.9  32.8  32.8           22.5  18.7
+//                 1,009,091         57.1  54.0  51.7  53.0            59.2  57.9  55.7           44.6  32.8
+//                 4,096,000        194.9 193.4 191.9 192.3           209.0 211.1 206.7          116.8 112.6
+//    7 diagonals, 3,375,000         49.2  49.2  47.1  49.2            56.1  59.6  57.4           37.3  43.0
+//    5 diagonals, 4,194,304         47.1  47.0  47.1  43.1            57.1  63.4  63.4           36.6  38.9
+// FP64 takes one row per thread and three diagonals (twice the threads: the
+// FP64 pipe is fed while they wait), HDC of few diagonals two rows: its rows'
+// remainders come one after the other and want fewer, longer threads.  FP32 DIA
+// is fastest with four rows and the plain loop, uncapped (87 us at 4,096,000
+// rows, one row 100 us), FP32 HDC of many diagonals with one.  FP64 caps at 8
+// CTAs (32 registers).
+constexpr int DIA_MANY = 16;  // diagonals from which HDC takes one row per thread
 
 template <typename T> struct Vec;
 template <> struct Vec<double> { using type = double2; static constexpr int n = 2; };
@@ -68,14 +72,13 @@ __device__ __forceinline__ void dia_load(const T* vp, int64_t row0, int64_t nrow
 
 // One thread = RPT consecutive rows (vector path, requires pitch % RPT == 0
 // and an aligned values pointer) or RPT = 1 (scalar path).
-template <typename T, int RPT, bool HDC>
-__global__ void __launch_bounds__(DIA_THREADS, kDiaMinBlocks<T>)
+template <typename T, int RPT, bool HDC, int DU, int MINB>
+__global__ void __launch_bounds__(DIA_THREADS, MINB)
 spmv_dia_rows(int64_t nrows, int64_t ncols, int ndiags, int64_t pitch,
               const int32_t* __restrict__ offs, const T* __restrict__ vals,
               const int32_t* __restrict__ cro, const int32_t* __restrict__ cci,
               const T* __restrict__ cva, int64_t csr_nnz,
               const T* __restrict__ x, T* __restrict__ y, int init) {
-  constexpr int DU = kDiaUnroll<T>;
   __shared__ int32_t s_off[DIA_OFF_CHUNK];
   const int64_t ngroups = (nrows + RPT - 1) / RPT;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -161,9 +164,9 @@ template <typename T, bool HDC>
 int launch_dia_rows(const mgb_dia* D, const mgb_csr* C, const T* x, T* y, int init,
                     cudaStream_t s) {
   constexpr int V = Vec<T>::n;
-  const bool vec_ok = (D->pitch % V == 0) &&
-                      (reinterpret_cast<uintptr_t>(D->values) % 16 == 0);
-  const int64_t rpt = vec_ok ? V : 1;
+  const bool vec_ok = (D->pitch % V == 0) && (reinterpret_cast<uintptr_t>(D->values) % 16 == 0);
+  const bool one = HDC ? D->ndiags >= DIA_MANY : sizeof(T) == 8;
+  const int64_t rpt = vec_ok && !one ? V : 1;
   const int64_t groups = (D->nrows + rpt - 1) / rpt;
   int64_t blocks = (groups + DIA_THREADS - 1) / DIA_THREADS;
   const int64_t cap = (int64_t)num_sms() * 64;
@@ -174,14 +177,17 @@ int launch_dia_rows(const mgb_dia* D, const mgb_csr* C, const T* x, T* y, int in
   const T* cva = HDC ? static_cast<const T*>(C->values) : nullptr;
   const int64_t cnnz = HDC ? C->nnz : 0;
   const T* vals = static_cast<const T*>(D->values);
-  if (vec_ok)
-    spmv_dia_rows<T, V, HDC><<<(unsigned)blocks, DIA_THREADS, 0, s>>>(
-        D->nrows, D->ncols, (int)D->ndiags, D->pitch, D->diagonal_offsets, vals,
-        cro, cci, cva, cnnz, x, y, init);
-  else
-    spmv_dia_rows<T, 1, HDC><<<(unsigned)blocks, DIA_THREADS, 0, s>>>(
-        D->nrows, D->ncols, (int)D->ndiags, D->pitch, D->diagonal_offsets, vals,
-        cro, cci, cva, cnnz, x, y, init);
+  const auto run = [&](auto kernel) {
+    kernel<<<(unsigned)blocks, DIA_THREADS, 0, s>>>(D->nrows, D->ncols, (int)D->ndiags, D->pitch, D->diagonal_offsets,
+                                                    vals, cro, cci, cva, cnnz, x, y, init);
+  };
+  if constexpr (sizeof(T) == 8) {
+    if (rpt == 1) run(spmv_dia_rows<T, 1, HDC, 3, 8>);
+    else run(spmv_dia_rows<T, V, HDC, 2, 8>);
+  } else {
+    if (rpt == 1) run(spmv_dia_rows<T, 1, HDC, 1, 0>);
+    else run(spmv_dia_rows<T, V, HDC, 1, 0>);
+  }
   MGB_LAUNCH_CHECK();
   return MGB_SUCCESS;
 }

@@ -485,3 +485,32 @@ def test_csr_short_rows(cuda, N, lens, dtype):
         exact = float(x[:N].astype(np.float64) @ y.cpu().numpy().astype(np.float64))
         scale = float(np.abs(x[:N].astype(np.float64)) @ np.abs(y.cpu().numpy().astype(np.float64)))
         assert abs(float(d.item()) - exact) <= 64 * np.finfo(dtype).eps * scale
+
+
+# diagonals read three at a time and their remainders; the number of diagonals from which HDC takes one row per thread
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("fmt", [2, 5])
+@pytest.mark.parametrize("nd", [1, 2, 3, 4, 15, 16, 17])
+@pytest.mark.parametrize("N", [31, 1000, 1025])
+def test_dia_hdc_diagonal_groups(cuda, N, nd, fmt, dtype):
+    rng = np.random.default_rng(N + nd)
+    offs = np.sort(rng.choice(np.arange(-N // 3, N // 3), min(nd, N // 2), replace=False))
+    r = np.arange(N)[:, None]
+    c = r + offs[None, :]
+    m = (c >= 0) & (c < N)
+    rows, cols = np.broadcast_to(r, c.shape)[m], c[m]
+    if fmt == 5:  # a few entries off the diagonals
+        extra = np.stack([rng.integers(0, N, 9), rng.integers(0, N, 9)])
+        key = np.unique(np.concatenate([rows * N + cols, extra[0] * N + extra[1]]))
+        rows, cols = key // N, key % N
+    vals = rng.uniform(-1, 1, rows.size).astype(dtype)
+    A = mgb.from_coo(mgb.CooMatrix(N, N, rows.size, rows.astype(np.int32), cols.astype(np.int32), vals,
+                                   dtype=torch.float64 if dtype == np.float64 else torch.float32), fmt)
+    x, y0 = rng.uniform(-1, 1, N).astype(dtype), rng.uniform(-1, 1, N).astype(dtype)
+    prod = vals.astype(np.float64) * x.astype(np.float64)[cols]
+    for init in (True, False):
+        y = torch.from_numpy(y0).cuda()
+        mgb.multiply(A, torch.from_numpy(x).cuda(), y, init=init)
+        base = np.zeros(N) if init else y0.astype(np.float64)
+        bound = 30 * np.finfo(dtype).eps * (np.bincount(rows, weights=np.abs(prod), minlength=N) + np.abs(base))
+        assert np.all(np.abs(y.cpu().numpy() - base - np.bincount(rows, weights=prod, minlength=N)) <= bound)
