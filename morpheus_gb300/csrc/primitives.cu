@@ -509,16 +509,23 @@ __device__ __forceinline__ uint64_t record_key(const RowRecord& r) {
 
 // rank[i] = how many entries of the row came to its counter before (any
 // order).  Lanes of a warp with the same row add once; the search for them is
-// left out where no neighbouring lanes share a row.
-__global__ void __launch_bounds__(256) row_ranks(const int32_t* __restrict__ rows, int64_t n, int32_t* counts,
-                                                 int32_t* __restrict__ rank) {
+// left out where no neighbouring lanes share a row.  *scattered = warps whose
+// rows fall by more than a quarter of the matrix from one lane to the next.
+__global__ void __launch_bounds__(256) row_ranks(const int32_t* __restrict__ rows, int64_t n, int64_t nrows,
+                                                 int32_t* counts, int32_t* __restrict__ rank, int32_t* scattered) {
+  __shared__ int32_t cta_falls;
+  if (threadIdx.x == 0) cta_falls = 0;
+  __syncthreads();
   const int lane = threadIdx.x & 31;
+  const int32_t far = (int32_t)(nrows >> 2);
+  int32_t falls = 0;
   for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;; i += (int64_t)gridDim.x * 256) {
     const bool in = i < n;
     const unsigned active = __ballot_sync(0xffffffffu, in);
     if (!active) break;
     const int32_t r = in ? __ldcs(rows + i) : -1;
     const int32_t up = __shfl_up_sync(0xffffffffu, r, 1);
+    falls += __any_sync(0xffffffffu, in && lane > 0 && up - r > far);
     if (!__any_sync(0xffffffffu, in && lane > 0 && up == r)) {
       if (in) rank[i] = atomicAdd(counts + r, 1);
       continue;
@@ -530,14 +537,37 @@ __global__ void __launch_bounds__(256) row_ranks(const int32_t* __restrict__ row
     base = __shfl_sync(0xffffffffu, base, leader);
     if (in) rank[i] = base + __popc(same & ((1u << lane) - 1));
   }
+  if (lane == 0 && falls) atomicAdd(&cta_falls, falls);
+  __syncthreads();
+  if (threadIdx.x == 0 && cta_falls) atomicAdd(scattered, cta_falls);
 }
 
-template <typename T>
+// Records to their rows.  Each is one 16-byte store, half a sector, to a
+// place that only its row tells: while the records stay within L2 (129 MB) the
+// other half of the sector arrives before the sector is written back.  Beyond
+// that, entries in arbitrary order are written for the lower and then the
+// upper half of the rows (PASS 1 and 2, each reads all of `rows`); entries
+// whose rows are near each other in most warps (*scattered tells) need no
+// second pass and pay an empty launch.  PASS 0: everything at once.
+// CSR from shuffled triplets, one pass -> two: 15.2M entries (power law) 960
+// -> 909 us, 19.3M (27 diagonals, FP32) 1,040 -> 943, 45M 3,200 -> 2,940;
+// 7.6M (121 MB) 501 -> 500, 4.6M 341 -> 354, which is why the line is at L2's
+// size; three passes were worth 0.5-2 % beyond 30M only.  Row-sorted triplets,
+// 16M: 508 in one pass, 517 with an empty second, 542 in two.
+constexpr int64_t SCATTER_L2 = (int64_t)128 << 20;
+template <typename T, int PASS>
 __global__ void __launch_bounds__(256) row_scatter(const int32_t* __restrict__ rows, const int32_t* __restrict__ cols,
                                                    const T* __restrict__ vals, const int32_t* __restrict__ start,
-                                                   const int32_t* __restrict__ rank, int64_t n, RowRecord* rec) {
+                                                   const int32_t* __restrict__ rank, int64_t n, int64_t nrows,
+                                                   const int32_t* __restrict__ scattered, RowRecord* rec) {
+  const bool halves = PASS != 0 && __ldg(scattered) > n / 64;
+  if (PASS == 2 && !halves) return;
+  const int32_t mid = (int32_t)(nrows >> 1);
   for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
-    const int64_t at = (int64_t)__ldg(start + __ldcs(rows + i)) + __ldcs(rank + i);
+    const int32_t r = __ldcs(rows + i);
+    if (PASS == 1 && halves && r >= mid) continue;
+    if (PASS == 2 && r < mid) continue;
+    const int64_t at = (int64_t)__ldg(start + r) + __ldcs(rank + i);
     const uint64_t v = bits_of(__ldcs(vals + i));
     reinterpret_cast<uint4*>(rec)[at] =
         make_uint4((unsigned)i, (unsigned)__ldcs(cols + i), (unsigned)v, (unsigned)(v >> 32));
@@ -1002,15 +1032,21 @@ int row_sort(const int32_t* rows, const int32_t* cols, const T* vals, int64_t n,
   MGB_SCRATCH(sc, tile_row, ntiles + 1);
   MGB_SCRATCH(sc, medium, n / SORT_SHORT + 1);
   MGB_SCRATCH(sc, large, n / SORT_MED + 1);
-  MGB_SCRATCH(sc, counters, 2);
+  MGB_SCRATCH(sc, counters, 3);  // medium rows, large rows, scattered warps
   MGB_CUDA_CHECK(cudaMemsetAsync(counts, 0, sizeof(int32_t) * (nrows + 1), s));
-  MGB_CUDA_CHECK(cudaMemsetAsync(counters, 0, 2 * sizeof(int32_t), s));
+  MGB_CUDA_CHECK(cudaMemsetAsync(counters, 0, 3 * sizeof(int32_t), s));
   const unsigned grid = blocks_for(n, 256, (int64_t)num_sms() * 8);
-  row_ranks<<<grid, 256, 0, s>>>(rows, n, counts, rank);
+  row_ranks<<<grid, 256, 0, s>>>(rows, n, nrows, counts, rank, counters + 2);
   MGB_LAUNCH_CHECK();
   int st = exclusive_scan<int32_t, int32_t>(counts, start, nrows + 1, s);
   if (st) return st;
-  row_scatter<T><<<grid, 256, 0, s>>>(rows, cols, vals, start, rank, n, rec);
+  if (n * (int64_t)sizeof(RowRecord) > SCATTER_L2) {
+    row_scatter<T, 1><<<grid, 256, 0, s>>>(rows, cols, vals, start, rank, n, nrows, counters + 2, rec);
+    MGB_LAUNCH_CHECK();
+    row_scatter<T, 2><<<grid, 256, 0, s>>>(rows, cols, vals, start, rank, n, nrows, counters + 2, rec);
+  } else {
+    row_scatter<T, 0><<<grid, 256, 0, s>>>(rows, cols, vals, start, rank, n, nrows, counters + 2, rec);
+  }
   MGB_LAUNCH_CHECK();
   sort_plan<<<blocks_for(nrows + 1, 256, (int64_t)num_sms() * 8), 256, 0, s>>>(start, nrows, ntiles, tile_row, medium,
                                                                                 large, counters);

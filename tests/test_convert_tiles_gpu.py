@@ -158,6 +158,31 @@ def test_row_sort_tiles(cuda, N, lens, dtype):
     assert_same_matrix(mgb.matrix_to_host(A), om.to_host())
 
 
+# more records than L2 holds: scattered in two halves (the middle row on either side, an odd number of rows) or, with
+# rows near each other, at once
+@pytest.mark.parametrize("N", [4098, 65537])
+@pytest.mark.parametrize("shuffled", [True, False])
+def test_row_sort_beyond_l2(cuda, N, shuffled):
+    import torch
+
+    import morpheus_gb300 as mgb
+    n = (1 << 23) + 77
+    rng = np.random.default_rng(N)
+    rows = rng.integers(0, N, n, dtype=np.int32)
+    if not shuffled:
+        rows.sort()
+    cols = rng.integers(0, 1 << 20, n, dtype=np.int32)
+    vals = np.arange(n, dtype=np.float32)
+    order = np.lexsort((cols, rows))
+    dev = [torch.from_numpy(a.copy()).cuda() for a in (rows, cols, vals)]
+    A = mgb.CooMatrix(N, 1 << 20, n, *dev, dtype=torch.float32, device="cuda")
+    mgb.sort_by_row_and_column(A)
+    got = mgb.matrix_to_host(A)
+    np.testing.assert_array_equal(got["row_indices"], rows[order])
+    np.testing.assert_array_equal(got["column_indices"], cols[order])
+    np.testing.assert_array_equal(got["values"], vals[order])
+
+
 def _csr_host(coo):
     ro = np.zeros(coo["nrows"] + 1, np.int32)
     np.cumsum(np.bincount(coo["row_indices"], minlength=coo["nrows"]), out=ro[1:])
