@@ -112,8 +112,14 @@ __global__ void __launch_bounds__(256, prim::DIAG_CTAS) csr_diag_kernel(const in
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const bool wide = nrows + ncols > (int64_t)INT_MAX;  // bins past 32 bits
   const uint32_t nc = (uint32_t)min(ncols, (int64_t)1 << 31);
+  prim::KeyRun run;
+  int misses = 0;
+  bool unused = false;
   for (int64_t r0 = ((int64_t)blockIdx.x * 8 + w) * 32; r0 < nrows; r0 += (int64_t)gridDim.x * 256) {
     const uint32_t diag0 = (uint32_t)(nrows - 1 - r0);
+    if (!wide && lens == nullptr &&
+        prim::warp_equal_rows<false>(ro, r0, nrows, ci, nc, lane, h, counts, run, misses, &unused, &unused, &unused))
+      continue;
     prim::warp_row_walk(
         ro, r0, nrows, s_rows[w], lane, 0, 1, [&](int64_t c0, int i) { return (uint32_t)__ldcs(ci + c0 + i); },
         [&](bool in, bool, int q, int64_t, int, uint32_t c) {
@@ -123,6 +129,7 @@ __global__ void __launch_bounds__(256, prim::DIAG_CTAS) csr_diag_kernel(const in
           else prim::hist_add32(h, counts, c - q + diag0);
         });
   }
+  prim::run_end(h, counts, run);
   __syncthreads();
   prim::hist_flush(h, counts);
 }

@@ -272,6 +272,8 @@ __global__ void __launch_bounds__(256, DIAG_CTAS) csr_pass_kernel(const int32_t*
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint32_t nc = (uint32_t)min(ncols, (int64_t)1 << 31);
   bool bad = false, offsets = false, down = false, equal = false;
+  KeyRun run;
+  int misses = 0;
   for (int64_t r0 = ((int64_t)blockIdx.x * 8 + w) * 32; r0 < nrows; r0 += (int64_t)gridDim.x * 256) {
     const int64_t r = r0 + lane;
     if (r < nrows) {
@@ -281,6 +283,7 @@ __global__ void __launch_bounds__(256, DIAG_CTAS) csr_pass_kernel(const int32_t*
     if (__any_sync(0xffffffffu, offsets)) break;  // nothing of such rows is read
     uint32_t last = 0;  // column of the entry before the group
     const uint32_t diag0 = (uint32_t)(nrows - 1 - r0);
+    if (DIAG && warp_equal_rows<true>(ro, r0, nrows, c, nc, lane, h, diag, run, misses, &bad, &down, &equal)) continue;
     warp_row_walk(
         ro, r0, nrows, s_rows[w], lane, 0, 1, [&](int64_t c0, int i) { return (uint32_t)__ldcs(c + c0 + i); },
         [&](bool in, bool head, int q, int64_t, int, uint32_t col) {
@@ -294,6 +297,7 @@ __global__ void __launch_bounds__(256, DIAG_CTAS) csr_pass_kernel(const int32_t*
           if (DIAG && col < nc) hist_add32(h, diag, col - q + diag0);
         });
   }
+  if constexpr (DIAG) run_end(h, diag, run);
   const int bits = (bad ? COO_BAD_INDEX : 0) | (offsets ? COO_BAD_OFFSETS : 0) | (down ? COO_UNSORTED : 0) |
                    (equal ? COO_DUPLICATE : 0);
   if (bits) atomicOr(&s_bits, bits);

@@ -181,23 +181,23 @@ __device__ __forceinline__ void hist_init(CtaHist h) {
 
 __device__ __forceinline__ unsigned hist_home(uint32_t key) { return (key * 0x9E3779B1u) >> (32 - HIST_SLOTS_LOG2); }
 
-// counts one occurrence of key < HIST_EMPTY (global[key] += 1, in the end).  MERGE: lanes
+// counts n occurrences of key < HIST_EMPTY (global[key] += n, in the end).  MERGE: lanes
 // that go to the global counter with the same key add once (runs of equal
-// keys: the rows of row-sorted entries).
+// keys: the rows of row-sorted entries; n = 1).
 template <bool MERGE = false>
-__device__ __forceinline__ void hist_add32(CtaHist h, int32_t* global, uint32_t key) {
+__device__ __forceinline__ void hist_add32(CtaHist h, int32_t* global, uint32_t key, int32_t n = 1) {
   unsigned slot = hist_home(key);
   volatile uint32_t* keys = h.keys;
   uint32_t k = keys[slot];
   if (k == key) {
-    atomicAdd(h.counts + slot, 1);
+    atomicAdd(h.counts + slot, n);
     return;
   }
   const int probes = *reinterpret_cast<volatile int*>(h.full) ? 2 : HIST_PROBES;
   for (int p = 0; p < probes; p++) {
     if (k == HIST_EMPTY) k = atomicCAS(h.keys + slot, HIST_EMPTY, key);
     if (k == HIST_EMPTY || k == key) {
-      atomicAdd(h.counts + slot, 1);
+      atomicAdd(h.counts + slot, n);
       return;
     }
     slot = (slot + 1) & (HIST_SLOTS - 1);
@@ -208,8 +208,26 @@ __device__ __forceinline__ void hist_add32(CtaHist h, int32_t* global, uint32_t 
     const unsigned same = __match_any_sync(__activemask(), key);
     if ((int)(threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(global + key, __popc(same));
   } else {
-    atomicAdd(global + key, 1);
+    atomicAdd(global + key, n);
   }
+}
+
+// A lane's keys, one after the other: equal ones in a row are counted in a
+// register.  run_end once, after the last key.
+struct KeyRun {
+  uint32_t key = HIST_EMPTY;
+  int32_t n = 0;
+};
+__device__ __forceinline__ void run_end(CtaHist h, int32_t* global, const KeyRun& k) {
+  if (k.n) hist_add32(h, global, k.key, k.n);
+}
+__device__ __forceinline__ void run_add(CtaHist h, int32_t* global, KeyRun& k, uint32_t key) {
+  if (key != k.key) {
+    run_end(h, global, k);
+    k.key = key;
+    k.n = 0;
+  }
+  k.n++;
 }
 
 // the same for keys that may not fit the table's 32 bits
@@ -288,6 +306,110 @@ __device__ __forceinline__ void warp_row_walk(const int32_t* __restrict__ ro, in
     }
     __syncwarp();
   }
+}
+
+// Counts the diagonals (bin column - row + nrows - 1) of the entries of the same
+// 32 rows so that a lane keeps its position in the row while the rows go by:
+// 32 / L rows of L entries at a time, which are consecutive entries too.  On a
+// stencil's or band's rows a lane's diagonal then stays the same from row to
+// row, and its KeyRun takes eight steps with one comparison of them all (six
+// instructions per step; a look into the table and a shared-memory atomic per
+// entry made it 70).  Where the diagonals change, each lane starts a run at the
+// first of the eight; if the others are not on it either, or a column is
+// outside the matrix, they go through the table one by one, and after four
+// eights in a row like that (columns that follow no diagonal) the warp is told
+// to walk its other rows.
+// ORDER: *down / *equal as for entries of one row that follow each other;
+// *bad: a column beyond the matrix.
+// False, and nothing counted, unless the lengths change so seldom that the
+// steps outweigh the changes (one costs about what 96 entries of the walk do),
+// no row is longer than the warp, and the offsets do not decrease.
+// 27-point stencil, 160^3, walk -> here: csr_pass 236 -> 148 us, csr_diag 193 ->
+// 136 (the columns at the copy rate: 66); entries one by one after each change
+// of length: 170 / 156; the next eight loaded ahead with four CTAs per SM: 151 /
+// 140, and rows that have to be walked 5-10 % slower than with six.
+template <bool ORDER>
+__device__ __forceinline__ bool warp_equal_rows(const int32_t* __restrict__ ro, int64_t r0, int64_t nrows,
+                                                const int32_t* __restrict__ c, uint32_t nc, int lane, CtaHist h,
+                                                int32_t* counts, KeyRun& run, int& misses, bool* bad, bool* down,
+                                                bool* equal) {
+  constexpr unsigned ALL = 0xffffffffu;
+  constexpr int STEPS = 8;
+  if (misses >= 4) return false;
+  const int32_t a = ro[min(r0 + lane, nrows)], len = ro[min(r0 + lane + 1, nrows)] - a;
+  const int32_t left = __shfl_up_sync(ALL, len, 1);
+  unsigned heads = __ballot_sync(ALL, lane == 0 || len != left);
+  const int32_t total = __shfl_sync(ALL, a + len, 31) - __shfl_sync(ALL, a, 0);
+  if (96 * __popc(heads) > total || __any_sync(ALL, (unsigned)len > 32u)) return false;
+  const uint32_t diag0 = (uint32_t)(nrows - 1 - r0);
+  while (heads) {
+    const int q0 = __ffs(heads) - 1;
+    heads &= heads - 1;
+    const int q1 = heads ? __ffs(heads) - 1 : 32;
+    const int L = __shfl_sync(ALL, len, q0);
+    const int32_t e0 = __shfl_sync(ALL, a, q0);
+    if (L == 0) continue;
+    const int P = 32 / L, sub = lane / L;
+    const bool inner = lane > sub * L;  // not the row's first
+    const int end = sub < P ? q1 : 0;
+    const int32_t* p = c + e0 + lane;
+    for (int q = q0; q < q1; q += STEPS * P, p += STEPS * P * L) {
+      uint32_t v[STEPS];
+#pragma unroll
+      for (int u = 0; u < STEPS; u++) v[u] = q + u * P + sub < end ? (uint32_t)__ldcs(p + u * P * L) : 0;
+      int32_t n = 0;
+      auto same = [&] {  // every entry on its lane's run
+        const uint32_t want = run.key - diag0 + (q + sub);
+        uint32_t other = 0, last = 0;
+        n = 0;
+#pragma unroll
+        for (int u = 0; u < STEPS; u++)
+          if (q + u * P + sub < end) {
+            other |= v[u] ^ (want + u * P);
+            last = v[u];
+            n++;
+          }
+        return !__any_sync(ALL, other != 0 || last >= nc || v[0] >= nc);
+      };
+      bool all = same();
+      if (!all) {  // runs start at the first of the steps
+        const uint32_t key = v[0] - (q + sub) + diag0;
+        if (n > 0 && v[0] < nc && key != run.key) {
+          run_end(h, counts, run);
+          run.key = key;
+          run.n = 0;
+        }
+        all = same();
+        misses += !all;
+      } else {
+        misses = 0;
+      }
+      if (all) {
+        run.n += n;
+        if constexpr (ORDER) {  // alike in all steps
+          const uint32_t before = __shfl_up_sync(ALL, v[0], 1);
+          *down |= n > 0 && inner && v[0] < before;
+          *equal |= n > 0 && inner && v[0] == before;
+        }
+        continue;
+      }
+#pragma unroll 1
+      for (int u = 0; u < STEPS && q + u * P < q1; u++) {
+        const int row = q + u * P + sub;
+        const bool in = row < end;
+        const uint32_t col = in ? (uint32_t)__ldg(p + u * P * L) : 0;
+        if constexpr (ORDER) {
+          const uint32_t before = __shfl_up_sync(ALL, col, 1);
+          *down |= in && inner && col < before;
+          *equal |= in && inner && col == before;
+        }
+        if (!in) continue;
+        if (col >= nc) *bad = true;
+        else run_add(h, counts, run, col - row + diag0);
+      }
+    }
+  }
+  return true;
 }
 
 // global[key] += 1 with the lanes of a warp holding the same key merged

@@ -239,3 +239,39 @@ def test_csr_with_offsets_that_do_not_span_its_entries(cuda):
         dyn = mgb.DynamicMatrix(A)
         assert mgb.convert(dyn, fmt) == mgb.conversion_error_e.CONV_SUCCESS
         assert_same_matrix(mgb.matrix_to_host(dyn.active()), mgb.matrix_to_host(mgb.from_coo(mgb.to_coo(A), fmt)))
+
+
+# rows that a warp walks several at a time (32 / L of them) and counts by lane: every remainder of 32 / L, lengths at and
+# past the warp's width, a change of length inside a warp's rows, a last warp that is not full; columns in order, with
+# one row of a run out of order or with a column twice
+@pytest.mark.parametrize("case", ["in_order", "unsorted", "repeated"])
+@pytest.mark.parametrize("L", [3, 5, 9, 16, 17, 27, 31, 32, 33])
+def test_csr_rows_of_equal_length(cuda, L, case):
+    import morpheus_gb300 as mgb
+    from morpheus_gb300 import analytics
+    N = 32 * 9 + 19
+    lens = np.full(N, L)
+    lens[40], lens[100:132], lens[200:220] = 1, 0, max(1, L - 2)
+    offs = np.array([d for k in range(17) for d in (-k, k + 1)][:L])
+    ro = np.zeros(N + 1, np.int32)
+    np.cumsum(lens, out=ro[1:])
+    cols = np.concatenate([np.sort((r + offs[:lens[r]]) % N) for r in range(N)]).astype(np.int32)
+    if case != "in_order":
+        r = 32 * 5 + 11
+        s = slice(ro[r], ro[r + 1])
+        cols[s] = cols[s][::-1] if case == "unsorted" else np.r_[cols[s][0], cols[s][:-1]]
+    A = {"format": 1, "nrows": N, "ncols": N, "nnz": cols.size, "row_offsets": ro, "column_indices": cols,
+         "values": np.random.default_rng(L).standard_normal(cols.size)}
+    om = O.OracleMatrix.from_host(A)
+    M = mgb.matrix_from_host(A, device="cuda")
+    assert np.array_equal(analytics.count_nnz_per_diagonal(M).cpu().numpy(), om.count_nnz_per_diagonal())
+    for fmt in (O.DIA, O.HDC):
+        dyn = mgb.DynamicMatrix(mgb.matrix_from_host(A, device="cuda"))
+        status = mgb.convert(dyn, fmt)
+        try:
+            want = om.convert(fmt).to_host()
+        except O.OracleError:
+            assert status == mgb.conversion_error_e.PROXY_TO_DYNAMIC
+            continue
+        assert status == mgb.conversion_error_e.CONV_SUCCESS
+        assert_same_matrix(mgb.matrix_to_host(dyn.active()), want)
