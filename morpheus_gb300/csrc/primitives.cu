@@ -107,15 +107,6 @@ __global__ void max_i32_kernel(const int32_t* __restrict__ in, int64_t n, int32_
   if ((threadIdx.x & 31) == 0) atomicMax(out, m);
 }
 
-__global__ void sum_i32_kernel(const int32_t* __restrict__ in, int64_t n, unsigned long long* out) {
-  int64_t sacc = 0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    sacc += in[i];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) sacc += __shfl_xor_sync(0xffffffffu, sacc, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(out, (unsigned long long)sacc);
-}
-
 // counts[k] += 1 for every key in [0, nbins); few hot keys per CTA are
 // counted in shared memory first (CtaHist)
 __global__ void histogram_kernel(const int32_t* __restrict__ keys, int64_t n, int32_t* counts, int64_t nbins) {
@@ -883,7 +874,6 @@ int exclusive_scan(const Tin* in, Tout* out, int64_t n, cudaStream_t s, int64_t*
 }
 
 template int exclusive_scan<int32_t, int32_t>(const int32_t*, int32_t*, int64_t, cudaStream_t, int64_t*);
-template int exclusive_scan<int32_t, int64_t>(const int32_t*, int64_t*, int64_t, cudaStream_t, int64_t*);
 template int exclusive_scan<uint8_t, int64_t>(const uint8_t*, int64_t*, int64_t, cudaStream_t, int64_t*);
 template int exclusive_scan<uint8_t, int32_t>(const uint8_t*, int32_t*, int64_t, cudaStream_t, int64_t*);
 
@@ -892,15 +882,6 @@ int reduce_max_i32(const int32_t* in, int64_t n, int32_t* d_out, cudaStream_t s)
   MGB_LAUNCH_CHECK();
   if (n <= 0) return MGB_SUCCESS;
   max_i32_kernel<<<blocks_for(n, 256, (int64_t)num_sms() * 8), 256, 0, s>>>(in, n, d_out);
-  MGB_LAUNCH_CHECK();
-  return MGB_SUCCESS;
-}
-
-int reduce_sum_i32(const int32_t* in, int64_t n, int64_t* d_out, cudaStream_t s) {
-  MGB_CUDA_CHECK(cudaMemsetAsync(d_out, 0, sizeof(int64_t), s));
-  if (n <= 0) return MGB_SUCCESS;
-  sum_i32_kernel<<<blocks_for(n, 256, (int64_t)num_sms() * 8), 256, 0, s>>>(
-      in, n, reinterpret_cast<unsigned long long*>(d_out));
   MGB_LAUNCH_CHECK();
   return MGB_SUCCESS;
 }

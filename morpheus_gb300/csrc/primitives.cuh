@@ -59,8 +59,6 @@ int exclusive_scan(const Tin* in, Tout* out, int64_t n, cudaStream_t s, int64_t*
 
 // Max over n int32 values into *d_out (device); n == 0 writes INT32_MIN.
 int reduce_max_i32(const int32_t* in, int64_t n, int32_t* d_out, cudaStream_t s);
-// Sum over n int32 values into *d_out (device, 64-bit).
-int reduce_sum_i32(const int32_t* in, int64_t n, int64_t* d_out, cudaStream_t s);
 
 // Counts of keys in [0, nbins) (out of range keys are ignored).
 int histogram(const int32_t* keys, int64_t n, int32_t* counts, int64_t nbins, cudaStream_t s);

@@ -25,11 +25,14 @@
 //    lane ranges of KW entries.  Lane l walks its range accumulating with one
 //    FMA per entry into the current row and flushing at row ends; every FMA
 //    instruction is issued by all 32 lanes together.
-//  * Staging.  Each step the warp loads 8 entries of every lane range
-//    (4 x 64-byte pieces per load instruction) into padded shared memory, so
+//  * Staging.  Each step the warp copies 8 entries of every lane range
+//    (4 x 64-byte pieces per instruction) into padded shared memory, so
 //    HBM reads stay sector-complete and shared-memory reads conflict-free.
-//    Row offsets of the chunk are staged too, so row-end tests never wait on
-//    global memory.
+//    The multiply copies the next step's entries with cp.async while the lanes
+//    work on this one's (two buffers, csr_rows_pipe); the multiply with a fused
+//    dot, and matrices of 2^31 - 256 rows and more, load and store them in turn
+//    (csr_chunk).  Row offsets of the chunk are staged too, so row-end tests
+//    never wait on global memory.
 //  * Rows crossing lanes.  A row that continues into the next lane leaves a
 //    tail partial; one 5-step segmented shuffle scan per chunk (keyed by row)
 //    forwards the partials, and the lane where the row ends adds them: 6
@@ -47,11 +50,12 @@ constexpr int CSR_WARPS = 8;  // warps per CTA
 
 // DOT: also x[0..nrows) . y of the finished rows, one partial per CTA in
 // partials[blockIdx.x] (the fused step of an iterative solver; the matrix is
-// square there; the launcher caps the grid at the resident CTAs).  With a chunk plan the warps read
-// their rows from it instead of searching the row offsets.  SMALL: 32-bit
-// indices in the chunk routine, 256 staged row offsets and 4 CTAs per SM
-// (64 registers) -- measured on GB300 faster for FP32 (power-law 183 ->
-// 164 us) and slower for FP64 (195 -> 206 us), so FP32 only.
+// square there; the launcher caps the grid at the resident CTAs).  With a
+// chunk plan the warps read their rows from it instead of searching the row
+// offsets.  Only these fused multiplies and matrices too tall for the pipelined
+// kernel come here.  SMALL: 32-bit indices in the chunk routine, 256 staged row
+// offsets and 4 CTAs per SM (64 registers) -- faster for FP32 (power-law
+// 183 -> 164 us) and slower for FP64 (195 -> 206 us), so FP32 only.
 template <typename T, bool DOT, bool SMALL = false>
 __global__ void __launch_bounds__(CSR_WARPS * 32, SMALL ? 4 : 3)
 spmv_csr_segments(int64_t nrows, int64_t ncols, int64_t nnz, int64_t nchunks, int64_t chunk,

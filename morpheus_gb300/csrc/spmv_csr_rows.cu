@@ -14,7 +14,11 @@
 //   MGB_CSR_ROWS_GATHER when their columns are scattered, else
 //   MGB_CSR_SEGMENTS    the lane-segment kernel of spmv_csr.cu (any structure).
 //
-// Row-tile kernel: one warp owns 32 consecutive rows.  The tile's entries are
+// Direct kernel: rows of up to 25 entries (FP32: 20) with neighbouring columns
+// are walked by a thread each, straight from global memory (spmv_csr_rowdirect;
+// the line is at direct_shape).
+//
+// Row-tile kernel, for the others: one warp owns 32 consecutive rows.  The tile's entries are
 // one contiguous range of the CSR arrays; up to TILE of them at a time are
 // staged into shared memory with cp.async (all in flight at once), then every
 // lane walks its own row from shared memory in lockstep with the others

@@ -14,9 +14,11 @@
 //
 // Reductions: a grid of at most 4 CTAs per SM accumulates with one FMA (dot)
 // or add (reduce) per element and 16-byte loads, reduces in-CTA with
-// shuffles, and a one-CTA kernel sums the per-CTA partials.  The partials live
-// in stream-ordered scratch, so no global state is shared
-// between calls or streams.
+// shuffles, and a one-CTA kernel sums the per-CTA partials.  Up to 131,072
+// elements one cluster does both (its CTAs' partials meet in the first one's
+// shared memory).  The partials live in stream-ordered scratch and a result
+// for the host in a mapped word of the call's own, so no global state is
+// shared between calls or streams.
 #include <cooperative_groups.h>
 
 #include "mgb_internal.cuh"
