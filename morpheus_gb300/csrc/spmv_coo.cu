@@ -31,12 +31,17 @@ constexpr int COO_PAD = COO_SEG + 1;        // padded lane stride in shared memo
 constexpr int64_t COO_CHUNK = 2048;         // entries per warp chunk (largest)
 
 // 2048 entries per chunk, halved (down to 256) while the matrix would give
-// fewer chunks than the GPU holds resident warps, so small matrices still
-// spread over every SM.
+// fewer than three chunks per resident warp (12 of FP64, 16 of FP32 per SM; two
+// left the last wave nearly empty at some sizes, smaller chunks pay more
+// carries).  Power-law matrices of 350,000 / 700,000 rows, us at two -> three:
+// FP64 49.5 -> 47.6 / 93.3 -> 88.8, FP32 43.1 -> 39.1 / 76.8 -> 77.3; COO part of
+// the HYB of 1.5 / 2.0 M rows with its ELL part: FP64 220.9 -> 214.6 / 287.8 -> 287.9,
+// FP32 159.1 -> 157.9 / 212.5 -> 205.1; five: FP64 219 / 286, FP32 160 / 205.
+template <typename T>
 inline int64_t coo_chunk_size(int64_t nnz) {
   int64_t chunk = COO_CHUNK;
-  const int64_t resident = (int64_t)num_sms() * 24;
-  while (chunk > 256 && nnz / chunk < resident) chunk >>= 1;
+  const int64_t enough = (int64_t)num_sms() * (sizeof(T) == 8 ? 36 : 48);
+  while (chunk > 256 && nnz / chunk < enough) chunk >>= 1;
   return chunk;
 }
 
@@ -214,7 +219,7 @@ int launch_coo(const mgb_coo* A, const T* x, T* y, int init, cudaStream_t s) {
   }
   MGB_REQUIRE(A->row_indices && A->column_indices && A->values && x, MGB_ERR_BAD_ARGUMENT);
   if (int st = coo_carveout<T>()) return st;
-  const int64_t chunk = coo_chunk_size(A->nnz);
+  const int64_t chunk = coo_chunk_size<T>(A->nnz);
   const int64_t nchunks = (A->nnz + chunk - 1) / chunk;
   const int64_t ncarry = 2 * nchunks;
   void* scratch = nullptr;
@@ -332,7 +337,7 @@ int noalloc_scratch(void** out) {
 int launch_coo_noalloc_f64(const mgb_coo* A, const double* x, double* y, int init, cudaStream_t s) {
   MGB_REQUIRE(A != nullptr, MGB_ERR_BAD_ARGUMENT);
   MGB_REQUIRE(!bad_sizes(A->nrows, A->ncols, A->nnz), MGB_ERR_BAD_ARGUMENT);
-  const int64_t chunk = coo_chunk_size(A->nnz);
+  const int64_t chunk = coo_chunk_size<double>(A->nnz);
   const int64_t nchunks = (A->nnz + chunk - 1) / chunk;
   const int64_t ncarry = 2 * nchunks;
   const size_t rows_bytes = ((sizeof(int32_t) * (size_t)ncarry + 255) / 256) * 256;
