@@ -26,8 +26,6 @@ namespace {
 
 constexpr int COO_WARPS = 4;
 constexpr int COO_CTAS = 5;                 // register budget per SM (shared memory allows 2 to 4)
-constexpr int COO_SEG = 8;                  // entries per lane per staging step
-constexpr int COO_PAD = COO_SEG + 1;        // padded lane stride in shared memory
 constexpr int64_t COO_CHUNK = 2048;         // entries per warp chunk (largest)
 
 // 2048 entries per chunk, halved (down to 256) while the matrix would give
@@ -52,18 +50,20 @@ __device__ __forceinline__ T gather_x(const T* __restrict__ x, int32_t c, int64_
 
 // IDX: entry and row index type inside the kernel (int32_t when nnz < 2^31 -
 // 4096: measured on GB300, power-law COO 252 -> 221 us, same arithmetic).
-template <typename T, typename IDX>
+// SEG: entries per lane per staging step.
+template <typename T, typename IDX, int SEG>
 __global__ void __launch_bounds__(COO_WARPS * 32, COO_CTAS)
 spmv_coo_segments(int64_t nrows, int64_t ncols, int64_t nnz, int64_t chunk, const int32_t* __restrict__ ri,
                   const int32_t* __restrict__ ci, const T* __restrict__ va, const T* __restrict__ x,
                   T* __restrict__ y, int init, int32_t* __restrict__ carry_row, T* __restrict__ carry_val) {
-  __shared__ T s_val[COO_WARPS][2][32 * COO_PAD];
-  __shared__ int32_t s_col[COO_WARPS][2][32 * COO_PAD];
-  __shared__ int32_t s_row[COO_WARPS][2][32 * COO_PAD];
+  constexpr int PAD = SEG + 1;  // padded lane stride in shared memory
+  __shared__ T s_val[COO_WARPS][2][32 * PAD];
+  __shared__ int32_t s_col[COO_WARPS][2][32 * PAD];
+  __shared__ int32_t s_row[COO_WARPS][2][32 * PAD];
   const int lane = threadIdx.x & 31;
   const int w = threadIdx.x >> 5;
   const IDX nchunks = (nnz + chunk - 1) / chunk;
-  const IDX KW = chunk / 32;  // entries per lane, a multiple of COO_SEG
+  const IDX KW = chunk / 32;  // entries per lane, a multiple of SEG
   for (IDX k = (IDX)blockIdx.x * COO_WARPS + w; k < nchunks; k += (IDX)gridDim.x * COO_WARPS) {
     const IDX base = k * chunk;
     const IDX cend = min(base + chunk, nnz);
@@ -104,14 +104,14 @@ spmv_coo_segments(int64_t nrows, int64_t ncols, int64_t nnz, int64_t chunk, cons
     auto stage = [&](IDX st, int b) {
       if (st < KW) {
 #pragma unroll
-        for (int q = 0; q < COO_SEG; q++) {
+        for (int q = 0; q < SEG; q++) {
           const int f = q * 32 + lane;
-          const int L = f / COO_SEG, j = f % COO_SEG;
+          const int L = f / SEG, j = f % SEG;
           const IDX e = base + (IDX)L * KW + st + j;
           const bool in = e < cend;
-          csr::copy_or_zero(s_row[w][b] + L * COO_PAD + j, ri + (in ? e : base), in);
-          csr::copy_or_zero(s_col[w][b] + L * COO_PAD + j, ci + (in ? e : base), in);
-          csr::copy_or_zero(s_val[w][b] + L * COO_PAD + j, va + (in ? e : base), in);
+          csr::copy_or_zero(s_row[w][b] + L * PAD + j, ri + (in ? e : base), in);
+          csr::copy_or_zero(s_col[w][b] + L * PAD + j, ci + (in ? e : base), in);
+          csr::copy_or_zero(s_val[w][b] + L * PAD + j, va + (in ? e : base), in);
         }
       }
       asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -119,25 +119,25 @@ spmv_coo_segments(int64_t nrows, int64_t ncols, int64_t nnz, int64_t chunk, cons
     __syncwarp();  // the chunk before is done with the buffers
     stage(0, 0);
     int buf = 0;
-    for (IDX st = 0; st < KW; st += COO_SEG, buf ^= 1) {
+    for (IDX st = 0; st < KW; st += SEG, buf ^= 1) {
       __syncwarp();  // the reads of the buffer filled next are done
-      stage(st + COO_SEG, buf ^ 1);
+      stage(st + SEG, buf ^ 1);
       asm volatile("cp.async.wait_group 1;\n" ::: "memory");
       __syncwarp();
       const T* sv = s_val[w][buf];
       const int32_t* sc = s_col[w][buf];
       const int32_t* sr = s_row[w][buf];
-      T v[COO_SEG], xv[COO_SEG];
-      int32_t rw[COO_SEG];
+      T v[SEG], xv[SEG];
+      int32_t rw[SEG];
 #pragma unroll
-      for (int kk = 0; kk < COO_SEG; kk++) {
+      for (int kk = 0; kk < SEG; kk++) {
         const bool valid = la + st + kk < lb;
-        rw[kk] = sr[lane * COO_PAD + kk];
-        v[kk] = valid ? sv[lane * COO_PAD + kk] : T(0);
-        xv[kk] = valid ? gather_x(x, sc[lane * COO_PAD + kk], ncols) : T(0);
+        rw[kk] = sr[lane * PAD + kk];
+        v[kk] = valid ? sv[lane * PAD + kk] : T(0);
+        xv[kk] = valid ? gather_x(x, sc[lane * PAD + kk], ncols) : T(0);
       }
 #pragma unroll
-      for (int kk = 0; kk < COO_SEG; kk++) {
+      for (int kk = 0; kk < SEG; kk++) {
         const IDX e = la + st + kk;
         if (e < lb && rw[kk] != cur) {  // a new row starts at e (or the lane's first row)
           if (cur >= 0) {
@@ -180,13 +180,37 @@ spmv_coo_segments(int64_t nrows, int64_t ncols, int64_t nnz, int64_t chunk, cons
 }
 
 // Shared-memory carve-out of the kernel above (power-law matrix, 2e6 rows, FP64 /
-// FP32; single staging with 24 warps per SM: 223 / 200 us):
-// 35 %: 280 / 208, 45: 226 / 194, 60 and 70: 213 / 186 (12 / 16 warps per SM).
-constexpr int COO_CARVEOUT = 60;
-template <typename T>
-int coo_carveout() {
+// FP32; single staging with 24 warps per SM: 223 / 200 us): 35 %: 280 / 208,
+// 45: 226 / 194, 60 and 70: 213 / 186 (12 / 16 warps per SM).
+// FP64 of fewer than COO_SHORT entries: four entries per step, so that a
+// carve-out of 45 % holds 16 warps and leaves L1 more lines.  Steps of eight at
+// 60 % -> four at 45 % (single staging), us: COO of 1.8 M entries 25.9 -> 22.6
+// (24.6), 5.3 M 48.8 -> 45.1 (48.5), 10.6 M 89.3 -> 88.4 (86.3), 15.2 M 121.7 ->
+// 126.5 (122.2), 30.4 M 214 -> 223 (222); HYB with a COO part of 4 M entries
+// 176.0 -> 171.5 (173.0), of 8 M 290.4 -> 283.5 (278.3).
+constexpr int64_t COO_SHORT = 12 << 20;
+
+template <typename T, typename IDX, int SEG, int PERCENT>
+int launch_segments(const mgb_coo* A, int64_t chunk, int64_t nchunks, const T* x, T* y, int init, int32_t* cr, T* cv,
+                    cudaStream_t s) {
   static std::atomic<bool> done[64];
-  return csr::set_carveout_once(spmv_coo_segments<T, int32_t>, done, COO_CARVEOUT);
+  if (int st = csr::set_carveout_once(spmv_coo_segments<T, IDX, SEG>, done, PERCENT)) return st;
+  const int64_t blocks = (nchunks + COO_WARPS - 1) / COO_WARPS;
+  spmv_coo_segments<T, IDX, SEG><<<(unsigned)blocks, COO_WARPS * 32, 0, s>>>(
+      A->nrows, A->ncols, A->nnz, chunk, A->row_indices, A->column_indices, static_cast<const T*>(A->values), x, y,
+      init, cr, cv);
+  MGB_LAUNCH_CHECK();
+  return MGB_SUCCESS;
+}
+template <typename T>
+int coo_segments(const mgb_coo* A, int64_t chunk, int64_t nchunks, const T* x, T* y, int init, int32_t* cr, T* cv,
+                 cudaStream_t s) {
+  if constexpr (sizeof(T) == 8) {
+    if (A->nnz < COO_SHORT) return launch_segments<T, int32_t, 4, 45>(A, chunk, nchunks, x, y, init, cr, cv, s);
+  }
+  if (A->nnz < ((int64_t)1 << 31) - 4096)
+    return launch_segments<T, int32_t, 8, 60>(A, chunk, nchunks, x, y, init, cr, cv, s);
+  return launch_segments<T, int64_t, 8, 60>(A, chunk, nchunks, x, y, init, cr, cv, s);
 }
 
 // Adds the carries of each row in chunk order.  carry_row is non-decreasing.
@@ -218,7 +242,6 @@ int launch_coo(const mgb_coo* A, const T* x, T* y, int init, cudaStream_t s) {
     return MGB_SUCCESS;
   }
   MGB_REQUIRE(A->row_indices && A->column_indices && A->values && x, MGB_ERR_BAD_ARGUMENT);
-  if (int st = coo_carveout<T>()) return st;
   const int64_t chunk = coo_chunk_size<T>(A->nnz);
   const int64_t nchunks = (A->nnz + chunk - 1) / chunk;
   const int64_t ncarry = 2 * nchunks;
@@ -227,21 +250,14 @@ int launch_coo(const mgb_coo* A, const T* x, T* y, int init, cudaStream_t s) {
   MGB_CUDA_CHECK(scratch_alloc(&scratch, rows_bytes + sizeof(T) * ncarry, s));
   int32_t* cr = static_cast<int32_t*>(scratch);
   T* cv = reinterpret_cast<T*>(static_cast<char*>(scratch) + rows_bytes);
-  const int64_t blocks = (nchunks + COO_WARPS - 1) / COO_WARPS;
-  if (A->nnz < ((int64_t)1 << 31) - 4096)
-    spmv_coo_segments<T, int32_t><<<(unsigned)blocks, COO_WARPS * 32, 0, s>>>(
-        A->nrows, A->ncols, A->nnz, chunk, A->row_indices, A->column_indices,
-        static_cast<const T*>(A->values), x, y, init, cr, cv);
-  else
-    spmv_coo_segments<T, int64_t><<<(unsigned)blocks, COO_WARPS * 32, 0, s>>>(
-        A->nrows, A->ncols, A->nnz, chunk, A->row_indices, A->column_indices,
-        static_cast<const T*>(A->values), x, y, init, cr, cv);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) {
+  int st = coo_segments<T>(A, chunk, nchunks, x, y, init, cr, cv, s);
+  cudaError_t e = cudaSuccess;
+  if (st == MGB_SUCCESS) {
     coo_carry_fixup<T><<<(unsigned)((ncarry + 255) / 256), 256, 0, s>>>(ncarry, A->nrows, cr, cv, y, init);
     e = cudaGetLastError();
   }
   cudaError_t ef = cudaFreeAsync(scratch, s);
+  if (st != MGB_SUCCESS) return st;
   if (e != cudaSuccess) return record_cuda_error(e);
   if (ef != cudaSuccess) return record_cuda_error(ef);
   return MGB_SUCCESS;
@@ -350,17 +366,13 @@ int launch_coo_noalloc_f64(const mgb_coo* A, const double* x, double* y, int ini
     return MGB_SUCCESS;
   }
   MGB_REQUIRE(A->row_indices && A->column_indices && A->values && x, MGB_ERR_BAD_ARGUMENT);
-  if (int st = coo_carveout<double>()) return st;
   void* scratch = nullptr;
   int st = noalloc_scratch(&scratch);
   if (st != MGB_SUCCESS) return st;
   int32_t* cr = static_cast<int32_t*>(scratch);
   double* cv = reinterpret_cast<double*>(static_cast<char*>(scratch) + rows_bytes);
-  const int64_t blocks = (nchunks + COO_WARPS - 1) / COO_WARPS;
-  spmv_coo_segments<double, int32_t><<<(unsigned)blocks, COO_WARPS * 32, 0, s>>>(  // nnz is far below 2^31 here
-      A->nrows, A->ncols, A->nnz, chunk, A->row_indices, A->column_indices,
-      static_cast<const double*>(A->values), x, y, init, cr, cv);
-  MGB_LAUNCH_CHECK();
+  st = coo_segments<double>(A, chunk, nchunks, x, y, init, cr, cv, s);  // nnz is far below 2^31 here
+  if (st != MGB_SUCCESS) return st;
   coo_carry_fixup<double><<<(unsigned)((ncarry + 255) / 256), 256, 0, s>>>(ncarry, A->nrows, cr, cv, y, init);
   MGB_LAUNCH_CHECK();
   return MGB_SUCCESS;

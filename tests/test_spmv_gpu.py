@@ -514,3 +514,22 @@ def test_dia_hdc_diagonal_groups(cuda, N, nd, fmt, dtype):
         base = np.zeros(N) if init else y0.astype(np.float64)
         bound = 30 * np.finfo(dtype).eps * (np.bincount(rows, weights=np.abs(prod), minlength=N) + np.abs(base))
         assert np.all(np.abs(y.cpu().numpy() - base - np.bincount(rows, weights=prod, minlength=N)) <= bound)
+
+
+# either side of the entries up to which FP64 COO stages four entries per lane and step (12 << 20), a last chunk of one
+# entry; row sums of integers, exact in FP64
+@pytest.mark.parametrize("nnz", [257, (12 << 20) - 1, 12 << 20, (12 << 20) + 1])
+@pytest.mark.parametrize("init", [True, False])
+def test_coo_staging_by_size(cuda, nnz, init):
+    N = max(3, nnz // 11)
+    rng = np.random.default_rng(nnz)
+    rows = np.sort(rng.integers(0, N, nnz)).astype(np.int32)
+    cols = rng.integers(0, N, nnz).astype(np.int32)
+    vals = rng.integers(-8, 9, nnz).astype(np.float64)
+    x, y0 = rng.integers(-8, 9, N).astype(np.float64), rng.integers(-8, 9, N).astype(np.float64)
+    want = np.bincount(rows, weights=vals * x[cols], minlength=N) + (0 if init else y0)
+    dev = [torch.from_numpy(a).cuda() for a in (rows, cols, vals)]
+    A = mgb.CooMatrix(N, N, nnz, *dev, dtype=torch.float64, device="cuda")
+    y = torch.from_numpy(y0.copy()).cuda()
+    mgb.multiply(A, torch.from_numpy(x).cuda(), y, init=init)
+    assert np.array_equal(y.cpu().numpy(), want)
