@@ -142,7 +142,7 @@ __device__ __forceinline__ RowRange csr_rows_x(RowRange rows, int64_t nrows, int
     } else {
       IDX lo = r_begin, hi = r_end;  // first i in [lo, hi] with ro[i] > e_lo
       while (lo < hi) {
-        const IDX mid = (lo + hi) >> 1;
+        const IDX mid = lo + ((hi - lo) >> 1);  // lo + hi may pass 2^31
         if (ro_at(mid) <= e_lo) lo = mid + 1; else hi = mid;
       }
       r = lo - 1;
@@ -289,7 +289,7 @@ __device__ __forceinline__ RowRange csr_rows_pipe(RowRange rows, int64_t nrows, 
     } else {
       IDX lo = r_begin, hi = r_end;  // first i in [lo, hi] with ro[i] > e_lo
       while (lo < hi) {
-        const IDX mid = (lo + hi) >> 1;
+        const IDX mid = lo + ((hi - lo) >> 1);  // lo + hi may pass 2^31
         if (ro_at(mid) <= e_lo) lo = mid + 1; else hi = mid;
       }
       r = lo - 1;

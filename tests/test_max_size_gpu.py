@@ -2,10 +2,13 @@
 kernels accept (2^31 - 4096), built on the device: every CSR kernel and the
 COO kernel give the exact window sums (values 1, column j of row r is
 (r + j) mod ncols), checked against an FP64 prefix-sum computation."""
+import ctypes as C
+
 import pytest
 import torch
 
 import morpheus_gb300 as mgb
+from morpheus_gb300 import _lib
 
 pytestmark = [pytest.mark.gpu, pytest.mark.slow]
 
@@ -61,3 +64,36 @@ def test_chooser_and_coo_at_int32_limit(big):
     torch.cuda.synchronize()
     err = (torch.linalg.norm(y - y_ref) / torch.linalg.norm(y_ref)).item()
     assert err <= 1e-12, err
+
+
+# More rows than 2^30, three entries in every 128 of them: the sum of two row
+# numbers passes 2^31.  Values and x are small integers, so row sums are exact.
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("planned", [True, False])
+def test_csr_beyond_2_30_rows(cuda, planned, dtype):
+    if torch.cuda.get_device_properties(0).total_memory < 120 * 2**30:
+        pytest.skip("needs a GPU with >= 120 GB")
+    dev, rows, ncols = torch.device("cuda"), (1 << 30) + (1 << 20) + 77, 1009
+    groups = rows // 128 + 1
+    r = torch.arange(rows + 1, device=dev, dtype=torch.int64)
+    ro = (r // 128 * 3 + (r % 128 > 3).int() + 2 * (r % 128 > 70).int()).to(torch.int32)
+    del r
+    nnz = int(ro[-1])
+    ci = (torch.arange(nnz, device=dev, dtype=torch.int64) * 7919 % ncols).to(torch.int32)
+    x = torch.arange(ncols, device=dev).to(dtype) - 500
+    A = mgb.CsrMatrix(rows, ncols, nnz, ro, ci, torch.ones(nnz, dtype=dtype, device=dev), dtype=dtype)
+    want = torch.zeros(groups * 128, dtype=dtype, device=dev)
+    xv = torch.cat([x[ci.long()], torch.zeros(3, dtype=dtype, device=dev)])
+    first = torch.arange(groups, device=dev, dtype=torch.int64) * 3
+    want[3::128] = xv[first.clamp(max=nnz)]
+    want[70::128] = xv[(first + 1).clamp(max=nnz)] + xv[(first + 2).clamp(max=nnz)]
+    want = want[:rows]
+    y = torch.full((rows,), 7, dtype=dtype, device=dev)
+    if planned:
+        A._variant = mgb.CSR_SEGMENTS
+        mgb.multiply(A, x, y)
+    else:
+        desc, name = A._desc(), "mgb_spmv_csr_" + ("f64" if dtype == torch.float64 else "f32")
+        _lib.call(name, C.byref(desc), x.data_ptr(), y.data_ptr(), 1, None)
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
