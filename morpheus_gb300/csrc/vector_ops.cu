@@ -201,6 +201,8 @@ template <typename T, int MODE>
 __global__ void __cluster_dims__(SMALL_CTAS, 1, 1) __launch_bounds__(SMALL_THREADS)
 reduce_small(int64_t n, const T* __restrict__ x, const T* __restrict__ y, T* __restrict__ out) {
   __shared__ T s_cta[SMALL_CTAS];
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  cluster.barrier_arrive();  // this CTA runs: the others may write its shared memory
   constexpr int V = 16 / sizeof(T);
   constexpr int U = 4;
   const int64_t tid = (int64_t)blockIdx.x * SMALL_THREADS + threadIdx.x;
@@ -235,7 +237,7 @@ reduce_small(int64_t n, const T* __restrict__ x, const T* __restrict__ y, T* __r
     else acc[0] += a;
   }
   const T t = block_sum((acc[0] + acc[1]) + (acc[2] + acc[3]));
-  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  cluster.barrier_wait();  // the first CTA has started (the loads above covered the wait)
   if (threadIdx.x == 0) *cluster.map_shared_rank(s_cta + blockIdx.x, 0) = t;
   cluster.sync();
   if (blockIdx.x == 0 && threadIdx.x == 0) {

@@ -85,3 +85,18 @@ def test_short_reductions(cuda, n, dtype):
         assert abs(mgb.dot(n, ut, ut) - math.fsum(u * u)) <= tol * math.fsum(u * u)
         assert abs(mgb.reduce(ut, n) - math.fsum(u)) <= tol * math.fsum(np.abs(u))
         assert mgb.dot(n, ut, vt) == mgb.dot(n, ut, vt)
+
+
+@pytest.mark.parametrize("n", [1, 31, 700])
+def test_short_reductions_beside_other_work(cuda, n):
+    """CTAs of the cluster that have nothing to add, started while other kernels hold most of the GPU."""
+    x = torch.arange(1, n + 1, dtype=torch.float64, device="cuda")
+    big, side = torch.ones(1 << 24, device="cuda"), torch.cuda.Stream()
+    out = torch.empty(200, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    for k in range(200):
+        big.mul_(1.0)
+        with torch.cuda.stream(side):
+            _lib.call("mgb_reduce_f64_async", x.data_ptr(), n, out[k:].data_ptr(), side.cuda_stream)
+    torch.cuda.synchronize()
+    assert torch.equal(out, torch.full_like(out, n * (n + 1) / 2))
