@@ -29,21 +29,25 @@ unsigned long long current_ctx_id();
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
 
 // 64 bytes of page-locked host memory that kernels on the current device can
-// write (ok(): there was one free); given back when it goes out of scope, so
-// the stream has to be synchronised before that.
+// write (ok(): there was one free), for one call on one stream.  Another call
+// gets them only once that stream has run: wait() synchronises it, and a call
+// that returns without (an error after a launch) synchronises on the way out.
 class HostWord {
  public:
-  HostWord();
+  explicit HostWord(cudaStream_t s);
   ~HostWord();
   HostWord(const HostWord&) = delete;
   HostWord& operator=(const HostWord&) = delete;
   bool ok() const { return host_ != nullptr; }
   void* host() const { return host_; }
   void* device() const { return device_; }
+  cudaError_t wait();
 
  private:
+  cudaStream_t s_;
   void *host_ = nullptr, *device_ = nullptr;
   int dev_ = 0, index_ = 0;
+  bool waited_ = false;
 };
 
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }

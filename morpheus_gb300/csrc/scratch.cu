@@ -126,7 +126,7 @@ struct HostPage {
 HostPage g_page[64] = {};
 }  // namespace
 
-HostWord::HostWord() {
+HostWord::HostWord(cudaStream_t s) : s_(s) {
   if (cudaGetDevice(&dev_) != cudaSuccess || dev_ < 0 || dev_ >= 64) {
     (void)cudaGetLastError();
     return;
@@ -156,8 +156,18 @@ HostWord::HostWord() {
   device_ = page.device + 64 * index_;
 }
 
+cudaError_t HostWord::wait() {
+  const cudaError_t e = cudaStreamSynchronize(s_);
+  waited_ = e == cudaSuccess;
+  return e;
+}
+
 HostWord::~HostWord() {
   if (host_ == nullptr) return;
+  if (!waited_ && wait() != cudaSuccess) {  // a kernel may still write the word: nobody gets it again
+    (void)cudaGetLastError();
+    return;
+  }
   std::lock_guard<std::mutex> lock(g_pool_mutex);
   HostPage& page = g_page[dev_];
   if (static_cast<char*>(host_) == page.host + 64 * index_) page.used &= ~(1ull << index_);

@@ -281,13 +281,16 @@ int launch_reduce(int64_t n, const T* x, const T* y, T* d_result, cudaStream_t s
 template <typename T, int MODE>
 int reduce_to_host(int64_t n, const T* x, const T* y, T* result, cudaStream_t s) {
   MGB_REQUIRE(result != nullptr, MGB_ERR_BAD_ARGUMENT);
+  MGB_REQUIRE(n >= 0 && (n == 0 || (x != nullptr && (MODE != 0 || y != nullptr))), MGB_ERR_BAD_ARGUMENT);
   // the kernel writes the result into mapped host memory: no copy to wait for
-  if (HostWord word; n > 0 && word.ok()) {
-    const int st = launch_reduce<T, MODE>(n, x, y, static_cast<T*>(word.device()), s);
-    if (st != MGB_SUCCESS) return st;
-    MGB_CUDA_CHECK(cudaStreamSynchronize(s));
-    *result = *static_cast<const volatile T*>(word.host());
-    return MGB_SUCCESS;
+  if (n > 0) {
+    if (HostWord word(s); word.ok()) {
+      const int st = launch_reduce<T, MODE>(n, x, y, static_cast<T*>(word.device()), s);
+      if (st != MGB_SUCCESS) return st;
+      MGB_CUDA_CHECK(word.wait());
+      *result = *static_cast<const volatile T*>(word.host());
+      return MGB_SUCCESS;
+    }
   }
   T* d = nullptr;
   MGB_CUDA_CHECK(scratch_alloc((void**)&d, sizeof(T), s));
