@@ -113,7 +113,7 @@ int mgb_version(void);
 /* Text of the last CUDA error seen by this thread (static storage). */
 const char* mgb_last_cuda_error_string(void);
 /* Gives back the device memory that the library's scratch pool of the current
- * device keeps between calls (at most 32 MiB).  Synchronises the device. */
+ * context keeps between calls (at most 32 MiB).  Synchronises the device. */
 int mgb_scratch_release(void);
 
 /* ---- SpMV: y = A*x (init != 0) or y += A*x (init == 0) ------------------

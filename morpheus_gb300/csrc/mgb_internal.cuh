@@ -46,7 +46,8 @@ class HostWord {
  private:
   cudaStream_t s_;
   void *host_ = nullptr, *device_ = nullptr;
-  int dev_ = 0, index_ = 0;
+  uint64_t* used_ = nullptr;
+  int index_ = 0;
   bool waited_ = false;
 };
 

@@ -5,7 +5,7 @@
 // default memory pool gives its free memory back to the system at every
 // synchronisation, so a call after a synchronisation maps it anew: 110 us for
 // one allocation, 220 us more for a COO multiply (452 against 230 us).  Scratch
-// therefore comes from a pool of the library's own, one per device, that
+// therefore comes from a pool of the library's own, one per context, that
 // keeps up to SCRATCH_KEEP bytes between calls; what exceeds it goes back at
 // the next synchronisation as before, and mgb_scratch_release() gives back
 // the rest.  Allocations stay ordered on their stream, so threads and streams
@@ -14,6 +14,7 @@
 #include <cuda.h>  // CUcontext / CUresult types only: the driver calls are resolved at run time
 
 #include <mutex>
+#include <new>
 
 #include "mgb_internal.cuh"
 
@@ -55,32 +56,54 @@ unsigned long long current_ctx_id() {
 
 namespace {
 
-struct PoolSlot {
-  unsigned long long ctx_id;  // unique ID of the context the pool belongs to (0: none)
+// What the library keeps per CUDA context: the scratch pool and a page of 64
+// mapped host words.  One entry for every context that called, found again when
+// a program changes between contexts; entries stay until the process ends (a
+// context that went away took its pool and page with it, and IDs are not used
+// again).
+struct ContextState {
+  unsigned long long ctx_id;
   cudaMemPool_t pool;
+  char *page, *page_device;
+  uint64_t used;  // host words handed out, a bit each
+  ContextState* next;
 };
-std::mutex g_pool_mutex;
-PoolSlot g_pool[64] = {};
+std::mutex g_mutex;
+ContextState* g_contexts = nullptr;
 
-// The current device's pool, made on first use (and again in a new context);
-// null where there is none to be had: the default pool serves then.
+// The current context's entry, made on first use; null without a context ID.
+// g_mutex held.
+ContextState* context_state(unsigned long long id) {
+  if (id == 0) return nullptr;
+  for (ContextState* c = g_contexts; c != nullptr; c = c->next)
+    if (c->ctx_id == id) return c;
+  ContextState* c = new (std::nothrow) ContextState{};
+  if (c == nullptr) return nullptr;
+  c->ctx_id = id;
+  c->next = g_contexts;
+  g_contexts = c;
+  return c;
+}
+
+// The current context's pool, made on first use; null where there is none to be
+// had: the default pool serves then.
 cudaMemPool_t scratch_pool(cudaStream_t s, bool make) {
-  static thread_local PoolSlot last = {};  // a context's ID is never used again
+  static thread_local struct {
+    unsigned long long ctx_id;
+    cudaMemPool_t pool;
+  } last = {};
   const unsigned long long id = current_ctx_id();
   if (id != 0 && last.ctx_id == id) return last.pool;
+  std::lock_guard<std::mutex> lock(g_mutex);
+  ContextState* c = context_state(id);
+  if (c == nullptr) return nullptr;
+  if (c->pool != nullptr) {
+    last = {id, c->pool};
+    return c->pool;
+  }
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
-    (void)cudaGetLastError();
-    return nullptr;
-  }
-  std::lock_guard<std::mutex> lock(g_pool_mutex);
-  PoolSlot& slot = g_pool[dev];
-  if (slot.pool != nullptr && id != 0 && slot.ctx_id == id) {
-    last = slot;
-    return slot.pool;
-  }
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-  if (!make || id == 0 || cudaStreamIsCapturing(s, &capturing) != cudaSuccess ||
+  if (!make || cudaGetDevice(&dev) != cudaSuccess || cudaStreamIsCapturing(s, &capturing) != cudaSuccess ||
       capturing != cudaStreamCaptureStatusNone) {
     (void)cudaGetLastError();
     return nullptr;
@@ -102,9 +125,8 @@ cudaMemPool_t scratch_pool(cudaStream_t s, bool make) {
     if (pool != nullptr) (void)cudaMemPoolDestroy(pool);
     return nullptr;
   }
-  slot.pool = pool;
-  slot.ctx_id = id;
-  last = slot;
+  c->pool = pool;
+  last = {id, pool};
   return pool;
 }
 
@@ -115,27 +137,12 @@ cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
   return pool != nullptr ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
 }
 
-// Host words: one page per device, 64 words of 64 bytes.  A context that went
-// away took its page with it; words still out of an older page are forgotten.
-namespace {
-struct HostPage {
-  unsigned long long ctx_id;
-  char *host, *device;
-  uint64_t used;  // a bit per word
-};
-HostPage g_page[64] = {};
-}  // namespace
-
 HostWord::HostWord(cudaStream_t s) : s_(s) {
-  if (cudaGetDevice(&dev_) != cudaSuccess || dev_ < 0 || dev_ >= 64) {
-    (void)cudaGetLastError();
-    return;
-  }
   const unsigned long long id = current_ctx_id();
-  if (id == 0) return;
-  std::lock_guard<std::mutex> lock(g_pool_mutex);
-  HostPage& page = g_page[dev_];
-  if (page.host == nullptr || page.ctx_id != id) {
+  std::lock_guard<std::mutex> lock(g_mutex);
+  ContextState* c = context_state(id);
+  if (c == nullptr) return;
+  if (c->page == nullptr) {
     void *h = nullptr, *d = nullptr;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // another thread's capture is not disturbed
     (void)cudaThreadExchangeStreamCaptureMode(&mode);
@@ -147,13 +154,15 @@ HostWord::HostWord(cudaStream_t s) : s_(s) {
       if (h != nullptr) (void)cudaFreeHost(h);
       return;
     }
-    page = HostPage{id, static_cast<char*>(h), static_cast<char*>(d), 0};
+    c->page = static_cast<char*>(h);
+    c->page_device = static_cast<char*>(d);
   }
-  if (page.used == ~0ull) return;
-  index_ = __builtin_ctzll(~page.used);
-  page.used |= 1ull << index_;
-  host_ = page.host + 64 * index_;
-  device_ = page.device + 64 * index_;
+  if (c->used == ~0ull) return;
+  index_ = __builtin_ctzll(~c->used);
+  c->used |= 1ull << index_;
+  used_ = &c->used;
+  host_ = c->page + 64 * index_;
+  device_ = c->page_device + 64 * index_;
 }
 
 cudaError_t HostWord::wait() {
@@ -168,9 +177,8 @@ HostWord::~HostWord() {
     (void)cudaGetLastError();
     return;
   }
-  std::lock_guard<std::mutex> lock(g_pool_mutex);
-  HostPage& page = g_page[dev_];
-  if (static_cast<char*>(host_) == page.host + 64 * index_) page.used &= ~(1ull << index_);
+  std::lock_guard<std::mutex> lock(g_mutex);
+  *used_ &= ~(1ull << index_);
 }
 
 }  // namespace mgb

@@ -119,6 +119,22 @@ int main() {
     HostWord w(nullptr);
     expect(w.ok() && w.host() != first, "a word that may still be written is not handed out");
   }
+  // two contexts used in turn keep one pool and one page each
+  void* from[2] = {nullptr, nullptr};
+  for (int k = 0; k < 20; k++) {
+    g_ctx = 1 + k % 2;
+    void* p = nullptr;
+    expect(mgb::scratch_alloc(&p, 256, nullptr) == cudaSuccess, "scratch");
+    expect(p != nullptr && (from[k % 2] == nullptr || from[k % 2] == p), "a context keeps its pool");
+    from[k % 2] = p;
+    HostWord w(nullptr);
+    expect(w.ok() && w.wait() == cudaSuccess, "a word in either context");
+  }
+  expect(from[0] != from[1] && g_pools.size() == 2 && g_host.size() == 2, "one pool and one page per context");
+  g_ctx = 0;  // no context: the default pool serves
+  void* p = &g_ctx;
+  expect(mgb::scratch_alloc(&p, 256, nullptr) == cudaSuccess && p == nullptr, "no context, no pool");
+  expect(!HostWord(nullptr).ok(), "no context, no word");
   std::printf("%d failed\n", g_failed);
   return g_failed != 0;
 }
