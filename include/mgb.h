@@ -446,13 +446,16 @@ int mgb_convert_coo_to_hdc_f32(const mgb_coo* src, mgb_hdc* dst, void* stream);
  * call takes fill_bytes of a second workspace (same alignment; null: it
  * allocates).  A plan is good for one fill of the same source, on a stream
  * ordered after the plan call's; the workspaces may be freed once that fill has
- * run. */
+ * run.  A planned call whose source is of another kind or other sizes than the
+ * plan's, or whose value type a CSR plan's fill does not take (the diagonals that
+ * fit are fewer in FP64), returns MGB_ERR_BAD_ARGUMENT before any launch. */
 typedef struct {
   int64_t sizes[3];
   int64_t fill_bytes;
   int32_t format;
-  int32_t seen;   /* internal */
-  void* parts[3]; /* internal: pointers into the workspace */
+  int32_t seen;      /* internal, as the rest */
+  int64_t source[4]; /* what the plan was made of: 1 COO / 2 CSR, nrows, ncols, nnz */
+  void* parts[3];    /* pointers into the workspace */
 } mgb_coo_plan;
 int mgb_convert_coo_workspace_bytes(const mgb_coo* src, int format, int64_t* bytes);
 int mgb_convert_coo_plan(const mgb_coo* src, int format, int64_t hyb_width, void* workspace, int64_t bytes,

@@ -57,7 +57,8 @@ class Hdc(C.Structure):
 
 
 class CooPlan(C.Structure):
-    _fields_ = [("sizes", i64 * 3), ("fill_bytes", i64), ("format", C.c_int32), ("seen", C.c_int32), ("parts", vp * 3)]
+    _fields_ = [("sizes", i64 * 3), ("fill_bytes", i64), ("format", C.c_int32), ("seen", C.c_int32), ("source", i64 * 4),
+                ("parts", vp * 3)]
 
 
 # name -> (restype, argtypes)

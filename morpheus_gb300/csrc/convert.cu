@@ -1428,6 +1428,14 @@ int coo_plan_bytes(const mgb_coo* src, int format, int64_t* bytes) {
   return MGB_SUCCESS;
 }
 
+enum { SOURCE_COO = 1, SOURCE_CSR = 2 };
+
+// The plan was made of a source of this kind and of src's sizes.
+bool plan_of(const mgb_coo_plan* plan, int64_t kind, const mgb_coo* src) {
+  return plan->source[0] == kind && plan->source[1] == src->nrows && plan->source[2] == src->ncols &&
+         plan->source[3] == src->nnz;
+}
+
 inline bool bad_workspace(const void* ws) { return reinterpret_cast<uintptr_t>(ws) % 256 != 0; }
 
 // The common part: src's entries with, for a CSR matrix, its offsets.
@@ -1437,6 +1445,8 @@ int plan_any(const mgb_coo* src, const int32_t* ro, int format, int64_t hyb_widt
               MGB_ERR_BAD_ARGUMENT);
   *plan = mgb_coo_plan{};
   plan->format = format;
+  const int64_t made_of[4] = {ro ? SOURCE_CSR : SOURCE_COO, src->nrows, src->ncols, src->nnz};
+  std::copy(made_of, made_of + 4, plan->source);
   Scratch sc(s, ws, (size_t)bytes);
   int st;
   if (format == PLAN_CSR) {
@@ -1485,9 +1495,9 @@ int coo_plan(const mgb_coo* src, int format, int64_t hyb_width, void* ws, int64_
   return plan_any(src, nullptr, format, hyb_width, ws, bytes, plan, s);
 }
 
+// src: the plan's source, or the entries of its CSR matrix.
 template <typename T>
-int coo_planned(const mgb_coo* src, const mgb_coo_plan* plan, void* dst, void* ws, int64_t bytes, cudaStream_t s) {
-  MGB_REQUIRE(plan != nullptr && dst != nullptr && src != nullptr, MGB_ERR_BAD_ARGUMENT);
+int fill_planned(const mgb_coo* src, const mgb_coo_plan* plan, void* dst, void* ws, int64_t bytes, cudaStream_t s) {
   auto* counts = static_cast<int32_t*>(plan->parts[0]);
   auto* start = static_cast<int32_t*>(plan->parts[1]);
   auto* sums = static_cast<int64_t*>(plan->parts[2]);
@@ -1522,6 +1532,14 @@ int coo_planned(const mgb_coo* src, const mgb_coo_plan* plan, void* dst, void* w
   MGB_REQUIRE(plan->format == PLAN_HYB, MGB_ERR_BAD_ARGUMENT);
   p.h.total = plan->sizes[1];
   return hyb_fill<T>(src, p, plan->sizes[0], static_cast<mgb_hyb*>(dst), s);
+}
+
+template <typename T>
+int coo_planned(const mgb_coo* src, const mgb_coo_plan* plan, void* dst, void* ws, int64_t bytes, cudaStream_t s) {
+  MGB_REQUIRE(plan != nullptr && dst != nullptr, MGB_ERR_BAD_ARGUMENT);
+  if (int st = check_coo_args(src, plan->format != PLAN_CSR)) return st;
+  MGB_REQUIRE(plan_of(plan, SOURCE_COO, src), MGB_ERR_BAD_ARGUMENT);
+  return fill_planned<T>(src, plan, dst, ws, bytes, s);
 }
 
 // The entries of a CSR matrix without row indices: every routine that fills
@@ -1572,9 +1590,15 @@ int csr_source_plan(const mgb_csr* src, int format, int64_t hyb_width, void* ws,
 
 template <typename T>
 int csr_source_planned(const mgb_csr* src, const mgb_coo_plan* plan, void* dst, cudaStream_t s) {
-  MGB_REQUIRE(src != nullptr && plan != nullptr && plan->format >= PLAN_DIA, MGB_ERR_BAD_ARGUMENT);
+  MGB_REQUIRE(src != nullptr && plan != nullptr && dst != nullptr && plan->format >= PLAN_DIA, MGB_ERR_BAD_ARGUMENT);
   const mgb_coo e = csr_entries(src);
-  return coo_planned<T>(&e, plan, dst, nullptr, 0, s);
+  MGB_REQUIRE(src->row_offsets != nullptr && (src->nnz == 0 || (src->column_indices && src->values)),
+              MGB_ERR_BAD_ARGUMENT);
+  // the fills below read no row indices: only what csr_source_plan<T> lets through may come here
+  MGB_REQUIRE(plan_of(plan, SOURCE_CSR, &e) && plan->parts[1] == src->row_offsets &&
+                  csr_fillable<T>(src, plan->format, *plan),
+              MGB_ERR_BAD_ARGUMENT);
+  return fill_planned<T>(&e, plan, dst, nullptr, 0, s);
 }
 
 // ---------------------------------------------------------------- sort API
