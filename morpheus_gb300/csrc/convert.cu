@@ -808,54 +808,77 @@ int place_ell(const mgb_coo* src, mgb_ell* e, int64_t W, const int32_t* slot, ui
   return MGB_SUCCESS;
 }
 
-// ELL slab of row-sorted entries: a CTA takes R rows, brings their entries
-// (one contiguous range) through shared memory and writes every slot column
-// of the rows, padding included, in consecutive rows: the slab is written once
-// in full sectors and not cleared before.  Rows whose entries do not fit
-// ELL_TILE are read where they lie.  A pad after every 32 staged entries
-// spreads rows of even length over the banks.  Placing each entry alone into
-// a cleared slab: see the figures at launch_ell_fill.
+// ELL slab of row-sorted entries: a CTA takes R rows and a segment of the slot
+// columns, brings the rows' entries through shared memory and writes every slot
+// of the segment, padding included, in consecutive rows: the slab is written
+// once in full sectors and not cleared before.  Where the rows' entries (one
+// contiguous range) do not fit ELL_TILE, ELL_TILE / R slots of every row at a
+// time are staged.  A pad after every 32 staged entries spreads rows of even
+// length over the banks.  Segments (grid y) divide the width where the rows
+// alone are too few CTAs: 33 rows of 1e6 entries 68,000 -> 1,070 us.  Placing
+// each entry alone into a cleared slab: 27-point stencil on 120 x 120 x 121, COO
+// -> ELL in all 2,667 us, this way 525.
 constexpr int ELL_TILE = 2048;
 constexpr int ELL_TILE_ROWS = 256;
+constexpr int ELL_SEGMENT = 64;  // slot columns of a segment at least
 __device__ __forceinline__ int ell_pad(int i) { return i + (i >> 5); }
 
 template <typename T>
 __global__ void __launch_bounds__(256)
 ell_fill_tiles(const int32_t* __restrict__ c, const T* __restrict__ v, const int32_t* __restrict__ start,
                int64_t nrows, int64_t pitch, int64_t width, int64_t W, int32_t* __restrict__ eci, T* __restrict__ ev,
-               int R) {
+               int R, int64_t segment) {
   __shared__ T s_v[ELL_TILE + ELL_TILE / 32];
   __shared__ int32_t s_c[ELL_TILE + ELL_TILE / 32];
   __shared__ int32_t s_start[ELL_TILE_ROWS + 1];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t ntiles = (pitch + R - 1) / R;
+  const int64_t k_begin = blockIdx.y * segment, k_end = min(k_begin + segment, width);
+  const int block = ELL_TILE / R;  // a power of two, as R
+  // slots [k0, k1) of the tile's rows; at(q, k): where entry k of row q is staged
+  auto write = [&](int64_t r0, int64_t k0, int64_t k1, auto at) {
+    for (int q = lane; q < R; q += 32) {
+      const int64_t row = r0 + q;
+      if (row >= pitch) break;
+      const int64_t len = min((int64_t)(s_start[q + 1] - s_start[q]), W);
+      for (int64_t k = k0 + w; k < k1; k += 8) {
+        int32_t col = MGB_INVALID_INDEX;
+        T val = T(0);
+        if (k < len) {
+          const int i = at(q, k);
+          col = s_c[ell_pad(i)];
+          val = s_v[ell_pad(i)];
+        }
+        __stcs(eci + row + pitch * k, col);
+        __stcs(ev + row + pitch * k, val);
+      }
+    }
+  };
   for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int64_t r0 = t * R;
     for (int q = threadIdx.x; q <= R; q += 256) s_start[q] = start[min(r0 + q, nrows)];
     __syncthreads();
     const int32_t e0 = s_start[0], n = s_start[R] - e0;
-    const bool staged = n <= ELL_TILE;
-    if (staged)
+    if (n <= ELL_TILE) {
       for (int i = threadIdx.x; i < n; i += 256) {
         s_c[ell_pad(i)] = __ldcs(c + e0 + i);
         s_v[ell_pad(i)] = __ldcs(v + e0 + i);
       }
-    __syncthreads();
-    for (int q = lane; q < R; q += 32) {
-      const int64_t row = r0 + q;
-      if (row >= pitch) break;
-      const int32_t b = s_start[q];
-      const int64_t len = min((int64_t)(s_start[q + 1] - b), W);
-      for (int64_t k = w; k < width; k += 8) {
-        int32_t col = MGB_INVALID_INDEX;
-        T val = T(0);
-        if (k < len) {
-          const int i = b - e0 + (int)k;
-          col = staged ? s_c[ell_pad(i)] : __ldg(c + e0 + i);
-          val = staged ? s_v[ell_pad(i)] : __ldg(v + e0 + i);
+      __syncthreads();
+      write(r0, k_begin, k_end, [&](int q, int64_t k) { return s_start[q] - e0 + (int)k; });
+    } else {
+      for (int64_t k0 = k_begin; k0 < k_end; k0 += block) {
+        for (int i = threadIdx.x; i < ELL_TILE; i += 256) {
+          const int q = i / block;
+          const int64_t k = k0 + i % block;
+          if (k < s_start[q + 1] - s_start[q]) {
+            s_c[ell_pad(i)] = __ldcs(c + s_start[q] + k);
+            s_v[ell_pad(i)] = __ldcs(v + s_start[q] + k);
+          }
         }
-        __stcs(eci + row + pitch * k, col);
-        __stcs(ev + row + pitch * k, val);
+        __syncthreads();
+        write(r0, k0, min(k0 + block, k_end), [&](int q, int64_t k) { return q * block + (int)(k - k0); });
+        __syncthreads();
       }
     }
     __syncthreads();
@@ -869,9 +892,15 @@ int launch_ell_fill(const mgb_coo* src, const int32_t* start, mgb_ell* e, int64_
   const int64_t mean = src->nnz / std::max<int64_t>(1, src->nrows) + 1;
   int R = ELL_TILE_ROWS;
   while (R > 32 && R * mean > ELL_TILE * 5 / 8) R >>= 1;
-  ell_fill_tiles<T><<<blocks_for((e->pitch + R - 1) / R, 1, (int64_t)num_sms() * 8), 256, 0, s>>>(
-      src->column_indices, static_cast<const T*>(src->values), start, src->nrows, e->pitch, e->width, W,
-      e->column_indices, static_cast<T*>(e->values), R);
+  const int64_t resident = (int64_t)num_sms() * 8;
+  const unsigned tiles = blocks_for((e->pitch + R - 1) / R, 1, resident);
+  // segments of whole staging blocks (multiples of ELL_SEGMENT, as ELL_TILE / R divides it), about one wave of CTAs
+  const int64_t parts = std::max<int64_t>(1, std::min(resident / tiles, e->width / ELL_SEGMENT));
+  const int64_t segment = ((e->width + parts - 1) / parts + ELL_SEGMENT - 1) / ELL_SEGMENT * ELL_SEGMENT;
+  const dim3 grid(tiles, (unsigned)((e->width + segment - 1) / segment));
+  ell_fill_tiles<T><<<grid, 256, 0, s>>>(src->column_indices, static_cast<const T*>(src->values), start, src->nrows,
+                                         e->pitch, e->width, W, e->column_indices, static_cast<T*>(e->values), R,
+                                         segment);
   MGB_LAUNCH_CHECK();
   return MGB_SUCCESS;
 }

@@ -80,6 +80,19 @@ def test_ell_and_hyb_tiles(cuda, N, lens, width, dtype):
         assert_same_matrix(got, ref, f"{fmt} width {w}:")
 
 
+# slabs too wide for their rows: several segments of the slot columns, rows beyond the staging (whole blocks of their
+# slots, a last block that is not full), one long row among short ones
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("N,lens,width", [(1, [70000], 0), (33, [9001, 8990, 9008], 0), (64, [5000], 4999),
+                                          (300, [3] * 299 + [12345], 700), (257, [2] * 100 + [4097] + [7] * 156, 64)])
+def test_wide_slabs(cuda, N, lens, width, dtype):
+    A = gen.random_lengths_csr(N, 80000, np.resize(np.asarray(lens), N), seed=N, dtype=dtype)
+    coo = gen.csr_to_coo_host(A)
+    for fmt, w in ((O.ELL, 0), (O.HYB, 0), (O.HYB, width)):
+        got, ref = both(coo, fmt, hyb_width=w)
+        assert_same_matrix(got, ref, f"{fmt} width {w}:")
+
+
 # all, some or none of the entries on true diagonals; more true diagonals than the lookup table takes
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 @pytest.mark.parametrize("N,nd,keep", [(3, 3, 1.0), (64, 5, 0.9), (513, 40, 0.6), (700, 500, 0.5), (1200, 1500, 0.4),
