@@ -907,7 +907,10 @@ int launch_ell_fill(const mgb_coo* src, const int32_t* start, mgb_ell* e, int64_
 
 // HYB's COO part of row-sorted entries: excess[r] = the row's entries past
 // the ELL width; with their exclusive scan, one warp per 32 rows copies the
-// rows that have some.
+// rows that have some.  Rows with more than EXCESS_PIECE of them are listed in
+// pieces of that many, and a CTA copies each piece (a row of 500,000 entries
+// took its warp 7,000 us).
+constexpr int EXCESS_PIECE = 2048;
 __global__ void row_excess(const int32_t* __restrict__ start, int64_t nrows, int64_t W, int32_t* excess) {
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += (int64_t)gridDim.x * blockDim.x)
     excess[r] = (int32_t)max((int64_t)(start[r + 1] - start[r]) - W, (int64_t)0);
@@ -916,7 +919,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 copy_excess(const int32_t* __restrict__ c, const T* __restrict__ v, const int32_t* __restrict__ start,
             const int32_t* __restrict__ base, int64_t nrows, int64_t W, int32_t* __restrict__ orow,
-            int32_t* __restrict__ ocol, T* __restrict__ oval) {
+            int32_t* __restrict__ ocol, T* __restrict__ oval, int2* __restrict__ pieces, int32_t* npieces) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * 8;
   for (int64_t r0 = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * 32; r0 < nrows; r0 += warps * 32) {
@@ -931,11 +934,36 @@ copy_excess(const int32_t* __restrict__ c, const T* __restrict__ v, const int32_
       const int j = __ffs(m) - 1;
       const int32_t f = __shfl_sync(0xffffffffu, from, j), k = __shfl_sync(0xffffffffu, n, j);
       const int32_t o = __shfl_sync(0xffffffffu, to, j);
+      if (k > EXCESS_PIECE) {
+        const int32_t np = (int32_t)(((int64_t)k + EXCESS_PIECE - 1) / EXCESS_PIECE);
+        int32_t at = 0;
+        if (lane == 0) at = atomicAdd(npieces, np);
+        at = __shfl_sync(0xffffffffu, at, 0);
+        for (int32_t i = lane; i < np; i += 32) pieces[at + i] = make_int2((int32_t)(r0 + j), i);
+        continue;
+      }
       for (int32_t i = lane; i < k; i += 32) {
         orow[o + i] = (int32_t)(r0 + j);
         ocol[o + i] = c[f + i];
         oval[o + i] = v[f + i];
       }
+    }
+  }
+}
+template <typename T>
+__global__ void __launch_bounds__(256)
+copy_excess_pieces(const int32_t* __restrict__ c, const T* __restrict__ v, const int32_t* __restrict__ start,
+                   const int32_t* __restrict__ base, int64_t W, int32_t* __restrict__ orow, int32_t* __restrict__ ocol,
+                   T* __restrict__ oval, const int2* __restrict__ pieces, const int32_t* __restrict__ npieces) {
+  for (int32_t p = blockIdx.x; p < *npieces; p += gridDim.x) {
+    const int2 piece = pieces[p];
+    const int64_t skip = (int64_t)piece.y * EXCESS_PIECE;
+    const int64_t f = start[piece.x] + W + skip, o = base[piece.x] + skip;
+    const int n = (int)min((int64_t)EXCESS_PIECE, start[piece.x + 1] - f);
+    for (int i = threadIdx.x; i < n; i += 256) {
+      orow[o + i] = piece.x;
+      ocol[o + i] = c[f + i];
+      oval[o + i] = v[f + i];
     }
   }
 }
@@ -1115,9 +1143,19 @@ int hyb_fill(const mgb_coo* src, const RowPlan& p, int64_t W, mgb_hyb* dst, cuda
     MGB_LAUNCH_CHECK();
     st = prim::exclusive_scan<int32_t, int32_t>(excess, base, src->nrows, s);
     if (st) return st;
-    copy_excess<T><<<grid_for(src->nrows), 256, 0, s>>>(
-        src->column_indices, static_cast<const T*>(src->values), p.start, base, src->nrows, W, c->row_indices,
-        c->column_indices, static_cast<T*>(c->values));
+    int2* pieces;
+    int32_t* npieces;
+    MGB_SCRATCH(sc, npieces, 1);
+    MGB_SCRATCH(sc, pieces, 2 * (cn / EXCESS_PIECE) + 1);  // at least half of EXCESS_PIECE in a listed row's pieces on average
+    MGB_CUDA_CHECK(cudaMemsetAsync(npieces, 0, sizeof(int32_t), s));
+    const T* v = static_cast<const T*>(src->values);
+    T* ov = static_cast<T*>(c->values);
+    copy_excess<T><<<grid_for(src->nrows), 256, 0, s>>>(src->column_indices, v, p.start, base, src->nrows, W,
+                                                        c->row_indices, c->column_indices, ov, pieces, npieces);
+    MGB_LAUNCH_CHECK();
+    if (cn <= EXCESS_PIECE) return MGB_SUCCESS;
+    copy_excess_pieces<T><<<blocks_for(cn, EXCESS_PIECE, (int64_t)num_sms() * 8), 256, 0, s>>>(
+        src->column_indices, v, p.start, base, W, c->row_indices, c->column_indices, ov, pieces, npieces);
     MGB_LAUNCH_CHECK();
     return MGB_SUCCESS;
   }

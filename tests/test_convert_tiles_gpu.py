@@ -93,6 +93,16 @@ def test_wide_slabs(cuda, N, lens, width, dtype):
         assert_same_matrix(got, ref, f"{fmt} width {w}:")
 
 
+# rows whose entries past the ELL width are one piece, one more, several pieces, the whole COO part
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("lens,width", [([2048 + 5], 5), ([2049 + 5, 3], 5), ([1, 30000, 0, 9, 4101], 5), ([40960 + 1], 1),
+                                        ([6, 9, 4], 4)])
+def test_hyb_long_rows(cuda, lens, width, dtype):
+    A = gen.random_lengths_csr(len(lens), 50000, np.asarray(lens), seed=width, dtype=dtype)
+    got, ref = both(gen.csr_to_coo_host(A), O.HYB, hyb_width=width)
+    assert_same_matrix(got, ref)
+
+
 # all, some or none of the entries on true diagonals; more true diagonals than the lookup table takes
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 @pytest.mark.parametrize("N,nd,keep", [(3, 3, 1.0), (64, 5, 0.9), (513, 40, 0.6), (700, 500, 0.5), (1200, 1500, 0.4),
