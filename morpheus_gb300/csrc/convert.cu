@@ -157,9 +157,11 @@ int csr_plan(const mgb_coo* src, CsrPlan* p, Scratch& sc, cudaStream_t s) {
   Words* dw;
   int st = words_alloc(sc, &dw, s);
   if (st) return st;
+  int32_t* gaps;
   MGB_SCRATCH(sc, p->start, src->nrows + 1);
+  MGB_SCRATCH(sc, gaps, prim::gap_words(src->nrows));
   st = prim::coo_pass(src->row_indices, src->column_indices, src->nnz, src->nrows, src->ncols, dw, nullptr, p->start,
-                      s);
+                      gaps, s);
   if (st) return st;
   st = words_read(dw, &p->h, s);
   if (st) return st;
@@ -462,10 +464,14 @@ int index_pass(const mgb_coo* src, const int32_t* ro, bool starts, Words* dw, in
     *start = ro;
     return prim::csr_pass(ro, src->column_indices, src->nnz, src->nrows, src->ncols, dw, diag, s);
   }
-  int32_t* own = nullptr;
-  if (starts) MGB_SCRATCH(sc, own, src->nrows + 1);
+  int32_t *own = nullptr, *gaps = nullptr;
+  if (starts) {
+    MGB_SCRATCH(sc, own, src->nrows + 1);
+    MGB_SCRATCH(sc, gaps, prim::gap_words(src->nrows));
+  }
   *start = own;
-  return prim::coo_pass(src->row_indices, src->column_indices, src->nnz, src->nrows, src->ncols, dw, diag, own, s);
+  return prim::coo_pass(src->row_indices, src->column_indices, src->nnz, src->nrows, src->ncols, dw, diag, own, gaps,
+                        s);
 }
 
 // COO -> DIA sizes: one pass over the indices counts the diagonals, checks
@@ -1480,7 +1486,8 @@ int coo_to_hdc(const mgb_coo* src, mgb_hdc* dst, cudaStream_t s) {
 enum { PLAN_CSR = 1, PLAN_DIA = 2, PLAN_ELL = 3, PLAN_HYB = 4, PLAN_HDC = 5 };  // formats_e
 
 size_t plan_bytes(int64_t nrows, int64_t ncols, int format) {
-  size_t b = Scratch::padded(sizeof(Words)) + Scratch::padded(sizeof(int32_t) * (size_t)(nrows + 1));
+  size_t b = Scratch::padded(sizeof(Words)) + Scratch::padded(sizeof(int32_t) * (size_t)(nrows + 1)) +
+             Scratch::padded(sizeof(int32_t) * (size_t)prim::gap_words(nrows));
   const int64_t nb = std::max<int64_t>(1, nrows + ncols - 1);
   if (format == PLAN_DIA || format == PLAN_HDC)
     b += Scratch::padded(sizeof(int32_t) * (size_t)nb) + Scratch::padded(sizeof(int64_t) * (size_t)prim::bin_tiles(nb));
@@ -1682,7 +1689,7 @@ int coo_sort(mgb_coo* A, void* ws, int64_t bytes, cudaStream_t s) {
   st = prim::reduce_max_i32(A->row_indices, A->nnz, &dw->maxv, s);
   if (st) return st;
   // rows and columns must be >= 0 (the counting sort indexes by them)
-  st = prim::coo_pass(A->row_indices, A->column_indices, A->nnz, INT32_MAX, INT32_MAX, dw, nullptr, nullptr, s);
+  st = prim::coo_pass(A->row_indices, A->column_indices, A->nnz, INT32_MAX, INT32_MAX, dw, nullptr, nullptr, nullptr, s);
   if (st) return st;
   Words hw;
   st = words_read(dw, &hw, s);

@@ -142,25 +142,33 @@ __global__ void sorted_flags_kernel(const int32_t* __restrict__ r, const int32_t
 // (five kernels before: 480 us of index reads and an intermediate bin array
 // on the 27-point stencil at 160^3; the HBM floor of the pass is 131 us).
 // Row starts: the entry where the row changes from p to q is the start of
-// the rows p + 1..q; gaps longer than PASS_GAP are left to the whole CTA at
-// the end, and the rows before the first and after the last entry to the grid.
+// the rows p + 1..q; gaps longer than PASS_GAP are listed by their entry and
+// filled by fill_gaps, a warp each, those beyond PASS_HUGE by its whole grid (by
+// the CTA that met them, 10,000 entries in 5e7 rows took the conversion to CSR
+// 3,256 us); the rows before the first and after the last entry are left to
+// this kernel's grid.
 // Rows that go down make the starts useless, and entries in random order have
 // gaps of a third of the matrix each: the first such row that a CTA sees stops
 // the writing of starts in that CTA at once and in the others at their next
 // tile.
 constexpr uint32_t PASS_GAP = 256;
-constexpr int PASS_GAPS = 256;
+constexpr uint32_t PASS_HUGE = 1 << 16;
+constexpr int PASS_GAPS = 1024;  // listed per CTA before the global list
+// of non-decreasing rows at most so many gaps
+__host__ __device__ inline int64_t max_gaps(int64_t nrows) { return nrows / PASS_GAP + 1; }
+__host__ __device__ inline int64_t max_huge(int64_t nrows) { return nrows / PASS_HUGE + 1; }
 
 template <bool DIAG, bool STARTS>
 __global__ void __launch_bounds__(256) coo_pass_kernel(const int32_t* __restrict__ r, const int32_t* __restrict__ c,
                                                        int64_t n, int64_t nrows, int64_t ncols, bool vec,
-                                                       int32_t* seen, int32_t* __restrict__ diag,
-                                                       int32_t* __restrict__ start) {
+                                                       Words* d, int32_t* __restrict__ diag,
+                                                       int32_t* __restrict__ start, int32_t* __restrict__ gaps) {
+  int32_t* seen = &d->seen;
   __shared__ uint32_t h_keys[DIAG ? HIST_SLOTS : 1];
   __shared__ int32_t h_counts[DIAG ? HIST_SLOTS : 1];
   __shared__ int h_full;
-  __shared__ int32_t gap_from[STARTS ? PASS_GAPS : 1], gap_to[STARTS ? PASS_GAPS : 1], gap_at[STARTS ? PASS_GAPS : 1];
-  __shared__ int ngaps, s_bits, s_stop;
+  __shared__ int32_t gap_at[STARTS ? PASS_GAPS : 1];
+  __shared__ int ngaps, s_bits, s_stop, s_base;
   volatile int* stop = &s_stop;
   const CtaHist h{h_keys, h_counts, &h_full};
   if constexpr (DIAG) hist_init(h);
@@ -214,12 +222,17 @@ __global__ void __launch_bounds__(256) coo_pass_kernel(const int32_t* __restrict
             if (rr[k] < nr) start[rr[k]] = (int32_t)(i0 + k);
           } else if (rr[k] > pr && rr[k] < nr && !*stop) {
             const int32_t at = (int32_t)(i0 + k);
-            int g = PASS_GAPS;
-            if (rr[k] - pr > PASS_GAP) g = atomicAdd(&ngaps, 1);
-            if (g < PASS_GAPS) {
-              gap_from[g] = (int32_t)(pr + 1);
-              gap_to[g] = (int32_t)rr[k];
-              gap_at[g] = at;
+            if (rr[k] - pr > PASS_HUGE) {
+              const int64_t g = atomicAdd(&d->huge, 1);
+              if (g < max_huge(nrows)) gaps[max_gaps(nrows) + g] = at;
+            } else if (rr[k] - pr > PASS_GAP) {
+              const int g = atomicAdd(&ngaps, 1);
+              if (g < PASS_GAPS) {
+                gap_at[g] = at;
+              } else {
+                const int64_t all = atomicAdd(&d->gaps, 1);
+                if (all < max_gaps(nrows)) gaps[all] = at;
+              }
             } else {
               for (uint32_t q = pr + 1; q <= rr[k]; q++) start[q] = at;
             }
@@ -238,13 +251,36 @@ __global__ void __launch_bounds__(256) coo_pass_kernel(const int32_t* __restrict
   if (threadIdx.x == 0 && s_bits) atomicOr(seen, s_bits);
   if constexpr (DIAG) hist_flush(h, diag);
   if constexpr (STARTS) {
-    for (int g = 0; g < (s_stop ? 0 : min(ngaps, PASS_GAPS)); g++)
-      for (int64_t q = (int64_t)gap_from[g] + threadIdx.x; q <= gap_to[g]; q += 256) start[q] = gap_at[g];
+    const int listed = s_stop ? 0 : min(ngaps, PASS_GAPS);
+    if (listed > 0) {
+      if (threadIdx.x == 0) s_base = atomicAdd(&d->gaps, listed);
+      __syncthreads();
+      for (int g = threadIdx.x; g < listed; g += 256)
+        if ((int64_t)s_base + g < max_gaps(nrows)) gaps[s_base + g] = gap_at[g];
+    }
     const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x, nt = (int64_t)gridDim.x * 256;
     const int64_t first = n > 0 ? min((int64_t)r[0], nrows) : nrows;
     const int64_t last = n > 0 ? max((int64_t)r[n - 1], (int64_t)-1) : nrows;
     for (int64_t q = t; q <= first; q += nt) start[q] = 0;
     for (int64_t q = last + 1 + t; q <= nrows; q += nt) start[q] = (int32_t)n;
+  }
+}
+
+// The rows of the listed gaps start at the entry behind the gap.
+__global__ void __launch_bounds__(256) fill_gaps(const int32_t* __restrict__ r, int64_t nrows, const Words* d,
+                                                 const int32_t* __restrict__ gaps, int32_t* __restrict__ start) {
+  if (d->seen & (COO_BAD_INDEX | COO_ROWS_UNSORTED)) return;  // no starts
+  const int64_t warps = (int64_t)gridDim.x * 8, n = min((int64_t)d->gaps, max_gaps(nrows));
+  for (int64_t g = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); g < n; g += warps) {
+    const int32_t at = gaps[g];
+    for (int64_t q = (int64_t)r[at - 1] + 1 + (threadIdx.x & 31); q <= r[at]; q += 32) start[q] = at;
+  }
+  const int64_t huge = min((int64_t)d->huge, max_huge(nrows));
+  for (int64_t g = 0; g < huge; g++) {
+    const int32_t at = gaps[max_gaps(nrows) + g];
+    const int64_t first = (int64_t)r[at - 1] + 1, last = r[at];
+    for (int64_t q = first + (int64_t)blockIdx.x * 256 + threadIdx.x; q <= last; q += (int64_t)gridDim.x * 256)
+      start[q] = at;
   }
 }
 
@@ -913,22 +949,28 @@ int words_alloc(Scratch& sc, Words** d, cudaStream_t s) {
 
 int words_read(const Words* d, Words* h, cudaStream_t s) { return to_host(d, h, s); }
 
+int64_t gap_words(int64_t nrows) { return max_gaps(nrows) + max_huge(nrows); }
+
 int coo_pass(const int32_t* rows, const int32_t* cols, int64_t n, int64_t nrows, int64_t ncols, Words* d,
-             int32_t* diag, int32_t* start, cudaStream_t s) {
+             int32_t* diag, int32_t* start, int32_t* gaps, cudaStream_t s) {
   const int64_t nb = nrows + ncols - 1;
   if (diag != nullptr && nb > 0) MGB_CUDA_CHECK(cudaMemsetAsync(diag, 0, sizeof(int32_t) * nb, s));
   if (n <= 0 && start == nullptr) return MGB_SUCCESS;
   const bool vec = (reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(cols)) % 16 == 0;
   const unsigned grid = blocks_for(n / 4 + 1, 256, (int64_t)num_sms() * 8);
   if (diag != nullptr && start != nullptr)
-    coo_pass_kernel<true, true><<<grid, 256, 0, s>>>(rows, cols, n, nrows, ncols, vec, &d->seen, diag, start);
+    coo_pass_kernel<true, true><<<grid, 256, 0, s>>>(rows, cols, n, nrows, ncols, vec, d, diag, start, gaps);
   else if (diag != nullptr)
-    coo_pass_kernel<true, false><<<grid, 256, 0, s>>>(rows, cols, n, nrows, ncols, vec, &d->seen, diag, start);
+    coo_pass_kernel<true, false><<<grid, 256, 0, s>>>(rows, cols, n, nrows, ncols, vec, d, diag, start, gaps);
   else if (start != nullptr)
-    coo_pass_kernel<false, true><<<grid, 256, 0, s>>>(rows, cols, n, nrows, ncols, vec, &d->seen, diag, start);
+    coo_pass_kernel<false, true><<<grid, 256, 0, s>>>(rows, cols, n, nrows, ncols, vec, d, diag, start, gaps);
   else
-    coo_pass_kernel<false, false><<<grid, 256, 0, s>>>(rows, cols, n, nrows, ncols, vec, &d->seen, diag, start);
+    coo_pass_kernel<false, false><<<grid, 256, 0, s>>>(rows, cols, n, nrows, ncols, vec, d, diag, start, gaps);
   MGB_LAUNCH_CHECK();
+  if (start != nullptr && n > 1 && nrows > PASS_GAP) {
+    fill_gaps<<<blocks_for(nrows, 1024, (int64_t)num_sms() * 8), 256, 0, s>>>(rows, nrows, d, gaps, start);
+    MGB_LAUNCH_CHECK();
+  }
   return MGB_SUCCESS;
 }
 

@@ -98,7 +98,8 @@ constexpr int32_t COO_BAD_OFFSETS = 16;   // CSR row offsets that do not rise fr
 struct Words {
   int64_t total, total2;  // plan sizes
   int32_t seen;           // COO_* bits
-  int32_t maxv, pad[2];
+  int32_t maxv;
+  int32_t gaps, huge;     // of the row starts, still to be filled
 };
 int words_alloc(Scratch& sc, Words** d, cudaStream_t s);          // zeroed
 int words_read(const Words* d, Words* h, cudaStream_t s);         // synchronises
@@ -107,10 +108,11 @@ int words_read(const Words* d, Words* h, cudaStream_t s);         // synchronise
 // d->seen |= the COO_* bits; diag != nullptr (nrows + ncols - 1 counters,
 // zeroed here): the entries on each diagonal, bin column - row + nrows - 1;
 // start != nullptr (nrows + 1 entries): the first entry of every row, valid
-// when the rows are in range and non-decreasing.  Entries out of range are
-// reported and not counted.
+// when the rows are in range and non-decreasing, with gaps = gap_words(nrows)
+// words of scratch.  Entries out of range are reported and not counted.
+int64_t gap_words(int64_t nrows);
 int coo_pass(const int32_t* rows, const int32_t* cols, int64_t n, int64_t nrows, int64_t ncols, Words* d,
-             int32_t* diag, int32_t* start, cudaStream_t s);
+             int32_t* diag, int32_t* start, int32_t* gaps, cudaStream_t s);
 
 // The same for the entries of a CSR matrix (its rows are in order), one read
 // of the columns; d->seen also COO_BAD_OFFSETS.

@@ -64,6 +64,22 @@ def test_row_starts_over_gaps(cuda, gap, shift):
         assert_same_matrix(mgb.matrix_to_host(mgb.from_coo(A, fmt)), want)
 
 
+# gaps that are listed: more than a CTA's list holds, around the length from which the whole grid fills them, both kinds
+@pytest.mark.parametrize("gaps", [[258] * 2100, [65535, 65536, 65537, 65538], [65537] * 3 + [257, 300000, 1, 256] * 2,
+                                  [1] * 1023 + [70000] + [1] * 1024 + [5000]])
+def test_row_starts_over_long_gaps(cuda, gaps):
+    rng = np.random.default_rng(len(gaps))
+    rows = 3 + np.cumsum(np.asarray([0] + gaps))
+    rows = np.repeat(rows, rng.integers(1, 3, rows.size))
+    n, N = rows.size, int(rows[-1]) + 5
+    order = np.lexsort((np.arange(n) % 2, rows))
+    hm = {"format": 0, "nrows": N, "ncols": 7, "nnz": n, "row_indices": rows.astype(np.int32),
+          "column_indices": (np.arange(n)[order] % 2 + 1).astype(np.int32), "values": rng.standard_normal(n)}
+    for fmt in (O.CSR, O.ELL, O.HYB):
+        got, ref = both(hm, fmt)
+        assert_same_matrix(got, ref, f"{fmt}:")
+
+
 def test_stencil_tiles(cuda):
     check_all_targets(gen.stencil_27pt(23, seed=5))
 
