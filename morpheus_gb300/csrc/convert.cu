@@ -462,7 +462,9 @@ int index_pass(const mgb_coo* src, const int32_t* ro, bool starts, Words* dw, in
                Scratch& sc, cudaStream_t s) {
   if (ro != nullptr) {
     *start = ro;
-    return prim::csr_pass(ro, src->column_indices, src->nnz, src->nrows, src->ncols, dw, diag, s);
+    int2* pieces;
+    MGB_SCRATCH(sc, pieces, prim::max_row_pieces(src->nnz));
+    return prim::csr_pass(ro, src->column_indices, src->nnz, src->nrows, src->ncols, dw, diag, pieces, s);
   }
   int32_t *own = nullptr, *gaps = nullptr;
   if (starts) {
@@ -1485,9 +1487,10 @@ int coo_to_hdc(const mgb_coo* src, mgb_hdc* dst, cudaStream_t s) {
 // row indices are neither made nor read.
 enum { PLAN_CSR = 1, PLAN_DIA = 2, PLAN_ELL = 3, PLAN_HYB = 4, PLAN_HDC = 5 };  // formats_e
 
-size_t plan_bytes(int64_t nrows, int64_t ncols, int format) {
+size_t plan_bytes(int64_t nrows, int64_t ncols, int64_t nnz, int format) {
   size_t b = Scratch::padded(sizeof(Words)) + Scratch::padded(sizeof(int32_t) * (size_t)(nrows + 1)) +
-             Scratch::padded(sizeof(int32_t) * (size_t)prim::gap_words(nrows));
+             Scratch::padded(sizeof(int32_t) * (size_t)prim::gap_words(nrows)) +
+             Scratch::padded(sizeof(int2) * (size_t)prim::max_row_pieces(nnz));
   const int64_t nb = std::max<int64_t>(1, nrows + ncols - 1);
   if (format == PLAN_DIA || format == PLAN_HDC)
     b += Scratch::padded(sizeof(int32_t) * (size_t)nb) + Scratch::padded(sizeof(int64_t) * (size_t)prim::bin_tiles(nb));
@@ -1498,7 +1501,7 @@ int coo_plan_bytes(const mgb_coo* src, int format, int64_t* bytes) {
   MGB_REQUIRE(bytes != nullptr && format >= PLAN_CSR && format <= PLAN_HDC, MGB_ERR_BAD_ARGUMENT);
   int st = check_coo_args(src, format != PLAN_CSR);
   if (st) return st;
-  *bytes = (int64_t)plan_bytes(src->nrows, src->ncols, format);
+  *bytes = (int64_t)plan_bytes(src->nrows, src->ncols, src->nnz, format);
   return MGB_SUCCESS;
 }
 
@@ -1515,7 +1518,7 @@ inline bool bad_workspace(const void* ws) { return reinterpret_cast<uintptr_t>(w
 // The common part: src's entries with, for a CSR matrix, its offsets.
 int plan_any(const mgb_coo* src, const int32_t* ro, int format, int64_t hyb_width, void* ws, int64_t bytes,
              mgb_coo_plan* plan, cudaStream_t s) {
-  MGB_REQUIRE(ws != nullptr && !bad_workspace(ws) && bytes >= (int64_t)plan_bytes(src->nrows, src->ncols, format),
+  MGB_REQUIRE(ws != nullptr && !bad_workspace(ws) && bytes >= (int64_t)plan_bytes(src->nrows, src->ncols, src->nnz, format),
               MGB_ERR_BAD_ARGUMENT);
   *plan = mgb_coo_plan{};
   plan->format = format;
@@ -1626,7 +1629,7 @@ int csr_source_bytes(const mgb_csr* src, int format, int64_t* bytes) {
   MGB_REQUIRE(src != nullptr && bytes != nullptr && format >= PLAN_DIA && format <= PLAN_HDC, MGB_ERR_BAD_ARGUMENT);
   MGB_REQUIRE(!bad_sizes(src->nrows, src->ncols, src->nnz), MGB_ERR_BAD_ARGUMENT);
   MGB_REQUIRE(src->nrows + src->ncols < INT32_MAX, MGB_ERR_INVALID_INPUT);
-  *bytes = (int64_t)plan_bytes(src->nrows, src->ncols, format);
+  *bytes = (int64_t)plan_bytes(src->nrows, src->ncols, src->nnz, format);
   return MGB_SUCCESS;
 }
 

@@ -100,6 +100,7 @@ struct Words {
   int32_t seen;           // COO_* bits
   int32_t maxv;
   int32_t gaps, huge;     // of the row starts, still to be filled
+  int32_t pieces, pad;    // of long rows
 };
 int words_alloc(Scratch& sc, Words** d, cudaStream_t s);          // zeroed
 int words_read(const Words* d, Words* h, cudaStream_t s);         // synchronises
@@ -115,9 +116,10 @@ int coo_pass(const int32_t* rows, const int32_t* cols, int64_t n, int64_t nrows,
              int32_t* diag, int32_t* start, int32_t* gaps, cudaStream_t s);
 
 // The same for the entries of a CSR matrix (its rows are in order), one read
-// of the columns; d->seen also COO_BAD_OFFSETS.
+// of the columns; d->seen also COO_BAD_OFFSETS.  pieces: max_row_pieces(n) of
+// scratch.
 int csr_pass(const int32_t* ro, const int32_t* cols, int64_t n, int64_t nrows, int64_t ncols, Words* d,
-             int32_t* diag, cudaStream_t s);
+             int32_t* diag, int2* pieces, cudaStream_t s);
 
 // The bins with counts[b] >= threshold, in order: how many to *d_total, their
 // counts' sum to *d_sum (if not null), and tile prefixes in sums
@@ -305,6 +307,67 @@ __device__ __forceinline__ void warp_row_walk(const int32_t* __restrict__ ro, in
       emit(in, j, v);
     }
     __syncwarp();
+  }
+}
+
+// Rows too long for one warp: listed in pieces of ROW_PIECE entries (x: row, y:
+// piece), which a second kernel takes by CTAs.  At most nnz / LONG_ROW + 1
+// pieces for valid offsets; what would not fit is dropped.
+constexpr int LONG_ROW = 512;
+constexpr int ROW_PIECE = 2048;
+struct RowPieces {
+  int2* list;
+  int32_t* count;  // zeroed
+  int64_t limit;
+};
+inline int64_t max_row_pieces(int64_t nnz) { return nnz / LONG_ROW + 1; }
+
+// The rows [r0, min(r0 + 32, nrows)) where one of them is long: lists the long
+// ones and calls f(in, q, e, first) for 32 entries e of a short row r0 + q at a
+// time (first: the row's first entry), every lane of the warp.  False, and
+// nothing done, where all are short.
+template <typename F>
+__device__ __forceinline__ bool warp_rows_apart(const int32_t* __restrict__ ro, int64_t r0, int64_t nrows,
+                                                RowPieces pieces, int lane, F f) {
+  constexpr unsigned ALL = 0xffffffffu;
+  const int32_t a = ro[min(r0 + lane, nrows)], z = ro[min(r0 + lane + 1, nrows)];
+  const int64_t len = (int64_t)z - a;
+  const unsigned longs = __ballot_sync(ALL, len > LONG_ROW);
+  if (!longs) return false;
+  const int32_t np = len > LONG_ROW ? (int32_t)((len + ROW_PIECE - 1) / ROW_PIECE) : 0;
+  int32_t upto = np;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int32_t u = __shfl_up_sync(ALL, upto, d);
+    if (lane >= d) upto += u;
+  }
+  int32_t base = 0;
+  if (lane == 31) base = atomicAdd(pieces.count, upto);
+  base = __shfl_sync(ALL, base, 31);
+  for (int q = 0; q < 32; q++) {
+    const int64_t n = __shfl_sync(ALL, len, q);
+    const int32_t first = __shfl_sync(ALL, a, q);
+    if ((longs >> q) & 1) {
+      const int32_t k = __shfl_sync(ALL, np, q), at = base + __shfl_sync(ALL, upto, q) - k;
+      for (int32_t i = lane; i < k; i += 32)
+        if ((int64_t)at + i < pieces.limit) pieces.list[at + i] = make_int2((int32_t)(r0 + q), i);
+    } else {
+      for (int64_t j = 0; j < n; j += 32) f(j + lane < n, q, (int32_t)(first + j + lane), first);
+    }
+  }
+  return true;
+}
+
+// Calls f(row, e, first) for every entry e of the listed pieces, a thread each;
+// CTAs of 256 threads.
+template <typename F>
+__device__ __forceinline__ void for_row_pieces(const int32_t* __restrict__ ro, RowPieces pieces, F f) {
+  const int64_t n = min((int64_t)*pieces.count, pieces.limit);
+  for (int64_t p = blockIdx.x; p < n; p += gridDim.x) {
+    const int2 piece = pieces.list[p];
+    const int32_t first = ro[piece.x], end = ro[piece.x + 1];
+    const int64_t e0 = first + (int64_t)piece.y * ROW_PIECE, e1 = min(e0 + ROW_PIECE, (int64_t)end);
+    for (int64_t e = e0 + threadIdx.x; e < e1; e += 256) f(piece.x, (int32_t)e, first);
   }
 }
 

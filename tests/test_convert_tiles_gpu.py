@@ -266,6 +266,37 @@ def test_csr_without_row_indices(cuda, case, fmt, dtype):
     assert_same_matrix(mgb.matrix_to_host(dyn.active()), want)
 
 
+# rows that a warp leaves to other CTAs: at the length limit (512), at a piece's end (2,048) and past it, among short and
+# empty rows; two entries out of order or equal across a piece's border
+@pytest.mark.parametrize("fmt", [2, 3, 4, 5])
+@pytest.mark.parametrize("case", ["in_order", "unsorted", "repeated", "outside"])
+@pytest.mark.parametrize("lens", [[512], [513], [2, 2048, 2049, 0, 33], [5000] + [7] * 70 + [513]])
+def test_csr_long_rows(cuda, lens, case, fmt):
+    import morpheus_gb300 as mgb
+    A = gen.random_lengths_csr(len(lens), 6000, np.asarray(lens), seed=fmt, dtype=np.float64)
+    cols, r = A["column_indices"].copy(), int(np.argmax(lens))
+    b = A["row_offsets"][r] + (2048 if lens[r] > 2048 else lens[r] // 2)
+    if case == "unsorted":
+        cols[b - 1:b + 1] = cols[b - 1:b + 1][::-1]
+    elif case == "repeated":
+        cols[b] = cols[b - 1]
+    elif case == "outside":
+        cols[A["row_offsets"][r + 1] - 1] = 6000
+    A["column_indices"] = cols
+    dyn = mgb.DynamicMatrix(mgb.matrix_from_host(A))
+    status = mgb.convert(dyn, fmt)
+    if case == "outside":
+        assert status == mgb.conversion_error_e.PROXY_TO_DYNAMIC and dyn.active_index() == 1
+        return
+    try:
+        want = O.OracleMatrix.from_host(A).convert(fmt).to_host()
+    except O.OracleError:
+        assert status == mgb.conversion_error_e.PROXY_TO_DYNAMIC
+        return
+    assert status == mgb.conversion_error_e.CONV_SUCCESS
+    assert_same_matrix(mgb.matrix_to_host(dyn.active()), want)
+
+
 def test_csr_with_offsets_that_do_not_span_its_entries(cuda):
     """Such a matrix converts as its COO form does."""
     import torch
