@@ -102,9 +102,9 @@ __global__ void row_stats_kernel(LEN lens, int64_t nrows, int64_t hyb_w,
 // 32 rows, a lane per entry.  Bound by the issue slots of the counting beside
 // the column indices (HBM).  A thread per row read its columns uncoalesced:
 // 606 us on the 27-point stencil at 160^3.
-__global__ void __launch_bounds__(256, prim::DIAG_CTAS) csr_diag_kernel(const int32_t* __restrict__ ro, const int32_t* __restrict__ ci,
-                                                       int64_t nrows, int64_t ncols, int32_t* lens,
-                                                       int32_t* counts) {
+__global__ void __launch_bounds__(256, prim::DIAG_CTAS)
+csr_diag_kernel(const int32_t* __restrict__ ro, const int32_t* __restrict__ ci, int64_t nrows, int64_t ncols,
+                int32_t* lens, int32_t* counts, bool apart, prim::RowPieces pieces) {
   MGB_CTA_HIST(h);
   __shared__ prim::WarpRows s_rows[8];
   prim::hist_init(h);
@@ -120,6 +120,15 @@ __global__ void __launch_bounds__(256, prim::DIAG_CTAS) csr_diag_kernel(const in
     if (!wide && lens == nullptr &&
         prim::warp_equal_rows<false>(ro, r0, nrows, ci, nc, lane, h, counts, run, misses, &unused, &unused, &unused))
       continue;
+    if (apart && prim::warp_rows_apart(ro, r0, nrows, pieces, lane, [&](bool in, int q, int32_t e, int32_t) {
+          const uint32_t c = in ? (uint32_t)__ldcs(ci + e) : nc;
+          const unsigned m = __ballot_sync(0xffffffffu, c < nc);
+          if (lens != nullptr && lane == 0 && m) atomicAdd(lens + r0 + q, __popc(m));
+          if (c >= nc) return;
+          if (wide) prim::hist_add(h, counts, (uint64_t)(c - (r0 + q) + nrows - 1));
+          else prim::hist_add32(h, counts, c - q + diag0);
+        }))
+      continue;
     prim::warp_row_walk(
         ro, r0, nrows, s_rows[w], lane, 0, 1, [&](int64_t c0, int i) { return (uint32_t)__ldcs(ci + c0 + i); },
         [&](bool in, bool, int q, int64_t, int, uint32_t c) {
@@ -132,6 +141,41 @@ __global__ void __launch_bounds__(256, prim::DIAG_CTAS) csr_diag_kernel(const in
   prim::run_end(h, counts, run);
   __syncthreads();
   prim::hist_flush(h, counts);
+}
+
+// The entries of the rows that the warps above listed (64 rows of 500,000: the
+// statistics took 190,000 us by threads and 230,000 by warps).
+__global__ void __launch_bounds__(256) csr_diag_pieces(const int32_t* __restrict__ ro, const int32_t* __restrict__ ci,
+                                                       int64_t nrows, int64_t ncols, int32_t* lens, int32_t* counts,
+                                                       prim::RowPieces pieces) {
+  const uint32_t nc = (uint32_t)min(ncols, (int64_t)1 << 31);
+  prim::for_row_pieces(ro, pieces, [&](int32_t row, int32_t e, int32_t) {
+    const uint32_t c = __ldg(ci + e);
+    if (c >= nc) return;
+    if (lens != nullptr) prim::warp_merged_add(lens, row);
+    atomicAdd(counts + ((int64_t)c - row + nrows - 1), 1);
+  });
+}
+
+int csr_diags(const mgb_csr* A, int32_t* lens, int32_t* counts, cudaStream_t s) {
+  Scratch sc(s);
+  prim::RowPieces pieces{nullptr, nullptr, 0};
+  const bool apart = A->nnz > prim::LONG_ROW;
+  if (apart) {
+    pieces.limit = prim::max_row_pieces(A->nnz);
+    MGB_SCRATCH(sc, pieces.list, pieces.limit);
+    MGB_SCRATCH(sc, pieces.count, 1);
+    MGB_CUDA_CHECK(cudaMemsetAsync(pieces.count, 0, sizeof(int32_t), s));
+  }
+  csr_diag_kernel<<<csr_grid(A->nrows), 256, 0, s>>>(A->row_offsets, A->column_indices, A->nrows, A->ncols, lens,
+                                                     counts, apart, pieces);
+  MGB_LAUNCH_CHECK();
+  if (apart) {
+    csr_diag_pieces<<<blocks_for(pieces.limit, 1, (int64_t)num_sms() * 8), 256, 0, s>>>(
+        A->row_offsets, A->column_indices, A->nrows, A->ncols, lens, counts, pieces);
+    MGB_LAUNCH_CHECK();
+  }
+  return MGB_SUCCESS;
 }
 
 // Diagonal summary: occupied diagonals, true diagonals and their entries,
@@ -331,11 +375,7 @@ struct CsrPass : FormPass {
   explicit CsrPass(const mgb_csr* a) : A(a) {}
   const int32_t* row_offsets() const override { return A->row_offsets; }
   int run(int32_t*, int32_t* counts, cudaStream_t s) const override {
-    if (A->nnz == 0) return MGB_SUCCESS;
-    csr_diag_kernel<<<csr_grid(A->nrows), 256, 0, s>>>(A->row_offsets, A->column_indices, A->nrows, A->ncols,
-                                                        nullptr, counts);
-    MGB_LAUNCH_CHECK();
-    return MGB_SUCCESS;
+    return A->nnz == 0 ? MGB_SUCCESS : csr_diags(A, nullptr, counts, s);
   }
 };
 
@@ -394,11 +434,7 @@ struct HdcPass : FormPass {
   explicit HdcPass(const mgb_hdc* a) : dia(&a->dia), csr(&a->csr) {}
   int run(int32_t* lens, int32_t* counts, cudaStream_t s) const override {
     if (int st = dia.run(lens, counts, s)) return st;
-    if (csr->nnz == 0) return MGB_SUCCESS;
-    csr_diag_kernel<<<csr_grid(csr->nrows), 256, 0, s>>>(csr->row_offsets, csr->column_indices, csr->nrows,
-                                                          csr->ncols, lens, counts);
-    MGB_LAUNCH_CHECK();
-    return MGB_SUCCESS;
+    return csr->nnz == 0 ? MGB_SUCCESS : csr_diags(csr, lens, counts, s);
   }
 };
 

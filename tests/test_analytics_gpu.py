@@ -118,3 +118,18 @@ def test_selector_choice_independent_of_active_format(cuda):
         choices.add(selector.select_format(dyn))
     assert len(choices) == 1
     _ = torch
+
+
+# rows that a warp leaves to other CTAs (more than 512 entries, pieces of 2,048) among short and empty ones
+@pytest.mark.parametrize("lens", [[513], [512, 2049, 0, 6], [5000] + [7] * 70 + [513]])
+def test_statistics_of_long_rows(cuda, lens):
+    full = np.ones(6000, np.int64)
+    full[100:100 + len(lens)] = lens
+    A = gen.random_lengths_csr(6000, 6000, full, seed=48)
+    diags = O.OracleMatrix.from_host(A).count_nnz_per_diagonal()
+    for hm in (A, O.OracleMatrix.from_host(A).convert(O.HDC).to_host()):
+        st = analytics.analyze(mgb.matrix_from_host(hm, device="cuda"))
+        assert st["count_diagonals"] == np.count_nonzero(diags)
+        assert (st["max_nnnz"], st["min_nnnz"]) == (full.max(), full.min())
+        assert st["average_nnnz"] == full.sum() / 6000
+        assert st["bandwidth"] == np.abs(np.flatnonzero(diags) - 5999).max()
