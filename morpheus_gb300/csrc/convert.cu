@@ -341,12 +341,25 @@ __device__ __forceinline__ int dia_table_find(DiaTable t, int32_t d) {
   return e.y;
 }
 
-// REM (HDC): also rem[row] = the row's entries on no stored diagonal.
+// First position in [b, e) with c[position] >= col, columns in order.
+__device__ __forceinline__ int64_t lower_column(const int32_t* __restrict__ c, int64_t b, int64_t e, int64_t col) {
+  while (b < e) {
+    const int64_t mid = (b + e) >> 1;
+    if (__ldg(c + mid) < col) b = mid + 1; else e = mid;
+  }
+  return b;
+}
+
+// REM (HDC): also rem[row] = the row's entries on no stored diagonal.  Rows of
+// more than `longest` entries, most of them on none, are not walked: the stored
+// diagonals' entries are searched in them (a row of 1e6 entries kept its warp
+// for 8,000 us).
 template <typename T, bool REM>
 __global__ void __launch_bounds__(DIA_TILE_THREADS, 10)
 dia_fill_tiles(const int32_t* __restrict__ c, const T* __restrict__ v, const int32_t* __restrict__ start,
                int64_t nrows, int64_t pitch, int nd, const int32_t* __restrict__ offs,
-               const int32_t* __restrict__ bin_slot, T* __restrict__ out, int32_t* __restrict__ rem, int R, int D) {
+               const int32_t* __restrict__ bin_slot, T* __restrict__ out, int32_t* __restrict__ rem, int R, int D,
+               int longest) {
   constexpr int WARPS = DIA_TILE_THREADS / 32;
   extern __shared__ __align__(16) unsigned char dia_smem[];
   T* tile = reinterpret_cast<T*>(dia_smem);
@@ -377,17 +390,43 @@ dia_fill_tiles(const int32_t* __restrict__ c, const T* __restrict__ v, const int
       for (int g = w / share; g < groups; g += WARPS / share) {
         const int64_t g0 = r0 + 32 * g;
         if (g0 >= nrows) break;
-        prim::warp_row_walk(
-            start, g0, nrows, s_rows[w], lane, w % share, share,
-            [&](int64_t c0, int i) { return Entry{__ldcs(c + c0 + i), __ldcs(v + c0 + i)}; },
-            [&](bool in, bool, int q, int64_t, int, Entry x) {
-              if (!in) return;
-              const int32_t d = x.col - (int32_t)g0 - q;
-              const int found = hashed ? dia_table_find(table, d) : bin_slot[(int64_t)d + nrows - 1];
-              const int s = found - d0;
-              if (s >= 0 && s < dn) tile[s * S + 32 * g + q] = x.val;
-              if (REM && found < 0 && d0 == 0) atomicAdd(s_rem + 32 * g + q, 1);
-            });
+        unsigned longs = 0;
+        if constexpr (REM)
+          longs = __ballot_sync(0xffffffffu,
+                                start[min(g0 + lane + 1, nrows)] - start[min(g0 + lane, nrows)] > longest);
+        for (int64_t p = g0;;) {  // the rows up to the next long one, and that one
+          const int64_t end = longs ? g0 + __ffs(longs) - 1 : min(g0 + 32, nrows);
+          const int q0 = (int)(p - g0);
+          if (!REM || p < end)
+            prim::warp_row_walk(
+                start, p, REM ? end : nrows, s_rows[w], lane, w % share, share,
+                [&](int64_t c0, int i) { return Entry{__ldcs(c + c0 + i), __ldcs(v + c0 + i)}; },
+                [&](bool in, bool, int q, int64_t, int, Entry x) {
+                  if (!in) return;
+                  q += q0;
+                  const int32_t d = x.col - (int32_t)g0 - q;
+                  const int found = hashed ? dia_table_find(table, d) : bin_slot[(int64_t)d + nrows - 1];
+                  const int s = found - d0;
+                  if (s >= 0 && s < dn) tile[s * S + 32 * g + q] = x.val;
+                  if (REM && found < 0 && d0 == 0) atomicAdd(s_rem + 32 * g + q, 1);
+                });
+          if (!REM || !longs) break;
+          const int64_t b = start[end], e = start[end + 1];
+          const int q = 32 * g + (int)(end - g0);
+          int hits = 0;
+          for (int d = (d0 == 0 ? 0 : d0) + 32 * (w % share) + lane; d < (d0 == 0 ? nd : d0 + dn); d += 32 * share) {
+            const int64_t col = end + offs[d], at = lower_column(c, b, e, col);
+            if (at == e || c[at] != col) continue;
+            hits++;
+            if (d < d0 + dn) tile[(d - d0) * S + q] = v[at];
+          }
+          if (REM && d0 == 0) {
+            hits = __reduce_add_sync(0xffffffffu, hits);
+            if (lane == 0) atomicAdd(s_rem + q, (w % share == 0 ? (int)(e - b) : 0) - hits);
+          }
+          longs &= longs - 1;
+          p = end + 1;
+        }
       }
       __syncthreads();
       if (REM && d0 == 0)
@@ -428,12 +467,14 @@ int launch_dia_fill(const mgb_coo* src, const int32_t* start, int64_t pitch, int
   const int64_t per_sm = std::min<int64_t>(10, (200 * 1024) / (int64_t)(smem + 12 * 1024));
   const unsigned grid = blocks_for((pitch + R - 1) / R, 1, (int64_t)num_sms() * std::max<int64_t>(1, per_sm));
   const T* v = static_cast<const T*>(src->values);
+  // a search of 32 diagonals costs about what 1,500 entries of the walk do
+  const int longest = 2048 * (int)((nd + 31) / 32);
   if (rem != nullptr)
     dia_fill_tiles<T, true><<<grid, DIA_TILE_THREADS, smem, s>>>(src->column_indices, v, start, src->nrows, pitch,
-                                                                 (int)nd, offs, bin_slot, out, rem, R, D);
+                                                                 (int)nd, offs, bin_slot, out, rem, R, D, longest);
   else
     dia_fill_tiles<T, false><<<grid, DIA_TILE_THREADS, smem, s>>>(src->column_indices, v, start, src->nrows, pitch,
-                                                                  (int)nd, offs, bin_slot, out, nullptr, R, D);
+                                                                  (int)nd, offs, bin_slot, out, nullptr, R, D, longest);
   MGB_LAUNCH_CHECK();
   return MGB_SUCCESS;
 }
@@ -1261,13 +1302,14 @@ __global__ void hdc_dia_place(const int32_t* __restrict__ r, const T* __restrict
 // CSR remainder of row-sorted entries: base = the exclusive scan of the rows'
 // remainders.  Entries are row-sorted, so those of 32 rows that lie on no
 // stored diagonal go, in order, to the consecutive places from base[first
-// row] on: one warp per 32 rows, ranks by ballot.
+// row] on: one warp per 32 rows, ranks by ballot.  Long rows are left in pieces
+// to hdc_remainder_pieces.
 template <typename T>
 __global__ void __launch_bounds__(256)
 hdc_remainder(const int32_t* __restrict__ c, const T* __restrict__ v, const int32_t* __restrict__ start,
               const int32_t* __restrict__ base, int64_t nrows, int nd, const int32_t* __restrict__ offs,
               const int32_t* __restrict__ bin_slot, int64_t limit, int32_t* __restrict__ ocol,
-              T* __restrict__ oval) {
+              T* __restrict__ oval, prim::RowPieces pieces) {
   __shared__ int2 h_table[DIA_HASH_SLOTS];
   __shared__ prim::WarpRows s_rows[8];
   const DiaTable table{h_table};
@@ -1280,19 +1322,90 @@ hdc_remainder(const int32_t* __restrict__ c, const T* __restrict__ v, const int3
   for (int64_t r0 = ((int64_t)blockIdx.x * 8 + w) * 32; r0 < nrows; r0 += (int64_t)gridDim.x * 256) {
     int64_t to = base[r0];
     if (to == base[min(r0 + 32, nrows)]) continue;  // every entry on a stored diagonal
+    auto place = [&](bool in, int q, int64_t e, int32_t col) {
+      const int32_t d = col - (int32_t)(r0 + q);
+      const bool miss = in && (hashed ? dia_table_find(table, d) : bin_slot[(int64_t)d + nrows - 1]) < 0;
+      const unsigned m = __ballot_sync(0xffffffffu, miss);
+      const int64_t p = to + __popc(m & ((1u << lane) - 1));
+      if (miss && p < limit) {
+        ocol[p] = col;
+        oval[p] = v[e];
+      }
+      to += __popc(m);
+    };
+    if (prim::warp_rows_apart(start, r0, nrows, pieces, lane, [&](bool in, int q, int32_t e, int32_t first) {
+          if (e - lane == first) to = base[r0 + q];
+          place(in, q, e, in ? __ldcs(c + e) : (int32_t)(r0 + q));
+        }))
+      continue;
     prim::warp_row_walk(
         start, r0, nrows, s_rows[w], lane, 0, 1, [&](int64_t c0, int i) { return __ldcs(c + c0 + i); },
-        [&](bool in, bool, int q, int64_t c0, int i, int32_t col) {
-          const int32_t d = col - (int32_t)(r0 + q);
-          const bool miss = in && (hashed ? dia_table_find(table, d) : bin_slot[(int64_t)d + nrows - 1]) < 0;
-          const unsigned m = __ballot_sync(0xffffffffu, miss);
-          const int64_t p = to + __popc(m & ((1u << lane) - 1));
-          if (miss && p < limit) {
-            ocol[p] = col;
-            oval[p] = v[c0 + i];
-          }
-          to += __popc(m);
-        });
+        [&](bool in, bool, int q, int64_t c0, int i, int32_t col) { place(in, q, c0 + i, col); });
+  }
+}
+
+// A CTA per piece of a long row.  The row's entries before the piece that lie on
+// a stored diagonal are counted by searching for every diagonal's column below
+// the piece's first one; within the piece, a warp per 256 entries.
+template <typename T>
+__global__ void __launch_bounds__(256)
+hdc_remainder_pieces(const int32_t* __restrict__ c, const T* __restrict__ v, const int32_t* __restrict__ start,
+                     const int32_t* __restrict__ base, int64_t nrows, int nd, const int32_t* __restrict__ offs,
+                     const int32_t* __restrict__ bin_slot, int64_t limit, int32_t* __restrict__ ocol,
+                     T* __restrict__ oval, prim::RowPieces pieces) {
+  constexpr int PER_WARP = prim::ROW_PIECE / 8, STEPS = PER_WARP / 32;
+  __shared__ int2 h_table[DIA_HASH_SLOTS];
+  __shared__ int s_hits[8], s_misses[8];
+  const DiaTable table{h_table};
+  const bool hashed = nd <= DIA_HASH_DIAGS;
+  if (hashed) dia_table_clear(table);
+  __syncthreads();
+  if (hashed) dia_table_fill(table, offs, nd);
+  __syncthreads();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t n = min((int64_t)*pieces.count, pieces.limit);
+  for (int64_t piece = blockIdx.x; piece < n; piece += gridDim.x) {
+    const int32_t row = pieces.list[piece].x;
+    const int64_t b = start[row], e = start[row + 1], e0 = b + (int64_t)pieces.list[piece].y * prim::ROW_PIECE;
+    const int64_t first = __ldg(c + e0);
+    int hits = 0;
+    for (int d = threadIdx.x; d < nd; d += 256) {
+      const int64_t col = (int64_t)row + offs[d];
+      if (col >= first) continue;
+      const int64_t at = lower_column(c, b, e0, col);
+      hits += at < e0 && c[at] == col;
+    }
+    hits = __reduce_add_sync(0xffffffffu, hits);
+    const int64_t w0 = e0 + (int64_t)w * PER_WARP;
+    int32_t col[STEPS];
+    unsigned miss[STEPS];
+    int misses = 0;
+#pragma unroll
+    for (int k = 0; k < STEPS; k++) {
+      const int64_t at = w0 + 32 * k + lane;
+      col[k] = at < e ? __ldg(c + at) : row;
+      const int32_t d = col[k] - row;
+      const bool out = at < e && (hashed ? dia_table_find(table, d) : bin_slot[(int64_t)d + nrows - 1]) < 0;
+      miss[k] = __ballot_sync(0xffffffffu, out);
+      misses += __popc(miss[k]);
+    }
+    if (lane == 0) {
+      s_hits[w] = hits;
+      s_misses[w] = misses;
+    }
+    __syncthreads();
+    int64_t to = base[row] + (e0 - b);
+    for (int i = 0; i < 8; i++) to += (i < w ? s_misses[i] : 0) - s_hits[i];
+#pragma unroll
+    for (int k = 0; k < STEPS; k++) {
+      const int64_t p = to + __popc(miss[k] & ((1u << lane) - 1));
+      if (((miss[k] >> lane) & 1) && p < limit) {
+        ocol[p] = col[k];
+        oval[p] = v[w0 + 32 * k + lane];
+      }
+      to += __popc(miss[k]);
+    }
+    __syncthreads();  // the next piece's counts
   }
 }
 
@@ -1399,9 +1512,18 @@ int hdc_fill(const mgb_coo* src, const HdcPlan& p, mgb_hdc* dst, cudaStream_t s)
       if (st) return st;
       st = prim::exclusive_scan<int32_t, int32_t>(rem, C->row_offsets, N + 1, s);
       if (st || cn == 0) return st;
+      prim::RowPieces pieces{nullptr, nullptr, prim::max_row_pieces(n)};
+      MGB_SCRATCH(sc, pieces.list, pieces.limit);
+      MGB_SCRATCH(sc, pieces.count, 1);
+      MGB_CUDA_CHECK(cudaMemsetAsync(pieces.count, 0, sizeof(int32_t), s));
       hdc_remainder<T><<<blocks_for(N, 256, (int64_t)num_sms() * 8), 256, 0, s>>>(
           src->column_indices, v, p.start, C->row_offsets, N, (int)nd, D->diagonal_offsets, p.counts, cn,
-          C->column_indices, static_cast<T*>(C->values));
+          C->column_indices, static_cast<T*>(C->values), pieces);
+      MGB_LAUNCH_CHECK();
+      if (n <= prim::LONG_ROW) return MGB_SUCCESS;
+      hdc_remainder_pieces<T><<<blocks_for(pieces.limit, 1, (int64_t)num_sms() * 8), 256, 0, s>>>(
+          src->column_indices, v, p.start, C->row_offsets, N, (int)nd, D->diagonal_offsets, p.counts, cn,
+          C->column_indices, static_cast<T*>(C->values), pieces);
       MGB_LAUNCH_CHECK();
       return MGB_SUCCESS;
     }

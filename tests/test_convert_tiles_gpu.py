@@ -128,6 +128,28 @@ def test_hdc_tiles(cuda, N, nd, keep, dtype):
     assert_same_matrix(got, ref)
 
 
+# rows with more entries off the diagonals than a warp walks or compacts itself (512; pieces of 2,048; 2,048 per 32
+# diagonals): first, last, neighbouring, beside short and empty rows
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("nd", [1, 3, 40, 300])
+@pytest.mark.parametrize("rows,length", [([0], 513), ([5999], 6000), ([31, 32, 33], 2100), ([100, 101, 4000], 5000)])
+def test_hdc_long_rows(cuda, rows, length, nd, dtype):
+    N = 6000
+    rng = np.random.default_rng(nd + length)
+    hm = diagonals(N, N, nd, seed=nd, dtype=dtype, keep=1.0)
+    if nd == 3:  # offsets near the middle: every diagonal is a long one
+        r = np.arange(1, N - 1)
+        key = np.unique(np.concatenate([r * N + r + d for d in (-1, 0, 1)]))
+    else:
+        key = hm["row_indices"].astype(np.int64) * N + hm["column_indices"]
+    key = np.unique(np.concatenate([key] + [r * N + np.sort(rng.choice(N, length, replace=False)) for r in rows]))
+    key = key[(key // N != 34) & (key // N != 4001)]  # empty rows
+    hm = {"format": 0, "nrows": N, "ncols": N, "nnz": key.size, "row_indices": (key // N).astype(np.int32),
+          "column_indices": (key % N).astype(np.int32), "values": rng.standard_normal(key.size).astype(dtype)}
+    got, ref = both(hm, O.HDC)
+    assert_same_matrix(got, ref)
+
+
 def _two_call(A, fmt, like):
     """The conversion through its own *_plan and fill entry points, into a container of `like`'s sizes."""
     import ctypes as C
