@@ -448,7 +448,7 @@ int mgb_convert_coo_to_hdc_f32(const mgb_coo* src, mgb_hdc* dst, void* stream);
  * ordered after the plan call's; the workspaces may be freed once that fill has
  * run.  A planned call whose source is of another kind or other sizes than the
  * plan's, or whose value type a CSR plan's fill does not take (the diagonals that
- * fit are fewer in FP64), returns MGB_ERR_BAD_ARGUMENT before any launch. */
+ * an HDC fill takes are fewer in FP64), returns MGB_ERR_BAD_ARGUMENT before any launch. */
 typedef struct {
   int64_t sizes[3];
   int64_t fill_bytes;
@@ -468,7 +468,7 @@ int mgb_convert_coo_planned_f32(const mgb_coo* src, const mgb_coo_plan* plan, vo
 /* The same for the entries of a CSR matrix, DIA / ELL / HYB / HDC (formats_e 2..5):
  * what a conversion through its COO form gives, without its row indices.  A plan
  * whose format comes back as 0 was not made (offsets that do not rise from 0 to
- * nnz, columns out of order or repeated in a row for DIA and HDC, thousands of
+ * nnz, columns out of order or repeated in a row for DIA and HDC, hundreds of
  * diagonals, no rows): convert through COO. */
 int mgb_convert_csr_workspace_bytes(const mgb_csr* src, int format, int64_t* bytes);
 int mgb_convert_csr_plan_f64(const mgb_csr* src, int format, int64_t hyb_width, void* workspace, int64_t bytes,

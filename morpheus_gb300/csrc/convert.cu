@@ -453,9 +453,21 @@ void dia_tile_shape(int64_t nd, int* R, int* D) {
   while (*R > 32 && nd * (*R + 1) * (int64_t)sizeof(T) > DIA_TILE_BYTES) *R >>= 1;
   *D = (int)std::min<int64_t>(nd, DIA_TILE_BYTES / ((*R + 1) * (int64_t)sizeof(T)));
 }
-// More groups than this (thousands of diagonals) and the entries are placed
-// one by one instead.
-constexpr int64_t DIA_TILE_GROUPS = 32;
+// More diagonals and the entries are placed one by one instead (a COO source) or
+// made a COO first (CSR): every group of D diagonals reads the rows' entries
+// again, and beyond DIA_HASH_DIAGS each looks its slot up in global memory.  Whole
+// conversions, us, tiles / placed (150,000 rows, half of the slots filled; HDC 100,000):
+//   diagonals     63         125        187        249        373          497
+//   FP64 COO      165 / 132  210 / 205  285 / 270  378 / 340   793 /  488  1336 /  647
+//        CSR      183 / 301  322 / 462  441 / 603  624 / 777  1593 / 1162  2620 / 1545
+//   FP64 HDC COO  202 / 266  263 / 551  342 / 735  472 / 909  1149 / 1282  1836 / 1645
+//        HDC CSR  222 / 411  298 / 743  420 / 980  563 /1190  1279 / 1648  1997 / 2110
+//   FP32 CSR         -       283 / 395     -       495 / 646   978 /  942  1514 / 1248
+//   FP32 HDC COO  177 / 261  231 / 516  269 / 693  367 / 845   688 / 1180  1068 / 1507
+// and, 1,200,000 rows, one group: FP64 62 diagonals 561 / 973, FP32 124 995 / 1728
+// (slabs beyond L2 are where placing costs most).  HDC's other way also reads the
+// entries several times, so its line is later.
+constexpr int64_t HDC_TILE_GROUPS = 6;
 
 template <typename T>
 int launch_dia_fill(const mgb_coo* src, const int32_t* start, int64_t pitch, int64_t nd, const int32_t* offs,
@@ -478,12 +490,13 @@ int launch_dia_fill(const mgb_coo* src, const int32_t* start, int64_t pitch, int
   MGB_LAUNCH_CHECK();
   return MGB_SUCCESS;
 }
+inline bool dia_tiled(int64_t nd) { return nd > 0 && nd <= DIA_HASH_DIAGS; }
 template <typename T>
-bool dia_tiled(int64_t nd) {
+bool hdc_tiled(int64_t nd) {
   if (nd == 0) return false;
   int R, D;
   dia_tile_shape<T>(nd, &R, &D);
-  return (nd + D - 1) / D <= DIA_TILE_GROUPS;
+  return (nd + D - 1) / D <= HDC_TILE_GROUPS;
 }
 
 // Argument checks of a COO source (the index range checks are queued with
@@ -578,7 +591,7 @@ int dia_fill(const mgb_coo* src, const DiaPlan& p, mgb_dia* dst, cudaStream_t s)
   const T* v = static_cast<const T*>(src->values);
   T* out = static_cast<T*>(dst->values);
   const bool distinct = words_distinct(p.h);
-  if (distinct && dia_tiled<T>(nd))
+  if (distinct && dia_tiled(nd))
     return launch_dia_fill<T>(src, p.start, dst->pitch, nd, dst->diagonal_offsets, slot, out, nullptr, s);
   MGB_CUDA_CHECK(cudaMemsetAsync(dst->values, 0, sizeof(T) * dst->pitch * nd, s));
   if (distinct) {
@@ -1503,7 +1516,7 @@ int hdc_fill(const mgb_coo* src, const HdcPlan& p, mgb_hdc* dst, cudaStream_t s)
       MGB_CUDA_CHECK(cudaMemcpyAsync(C->values, v, sizeof(T) * n, cudaMemcpyDeviceToDevice, s));
       return MGB_SUCCESS;
     }
-    if (dia_tiled<T>(nd)) {
+    if (hdc_tiled<T>(nd)) {
       int32_t* rem;
       MGB_SCRATCH(sc, rem, N + 1);
       MGB_CUDA_CHECK(cudaMemsetAsync(rem + N, 0, sizeof(int32_t), s));
@@ -1766,7 +1779,7 @@ bool csr_fillable(const mgb_csr* src, int format, const mgb_coo_plan& p) {
   Words h{};
   h.seen = p.seen;
   if (!words_distinct(h) || (format == PLAN_HDC && src->nrows != src->ncols)) return false;
-  return p.sizes[0] == 0 || dia_tiled<T>(p.sizes[0]);
+  return p.sizes[0] == 0 || (format == PLAN_DIA ? dia_tiled(p.sizes[0]) : hdc_tiled<T>(p.sizes[0]));
 }
 
 template <typename T>

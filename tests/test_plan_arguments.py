@@ -10,7 +10,7 @@ N, NNZ = 5000, 12000
 AT = 1 << 20  # an address that nothing reads
 
 
-def _plan(kind, fmt=2, sizes=(3000, 0, 0), seen=0, n=N, nnz=NNZ):
+def _plan(kind, fmt=2, sizes=(100, 0, 0), seen=0, n=N, nnz=NNZ):
     return _lib.CooPlan((C.c_int64 * 3)(*sizes), 0, fmt, seen, (C.c_int64 * 4)(kind, n, n, nnz), (C.c_void_p * 3)(AT, AT, AT))
 
 
@@ -28,17 +28,17 @@ ROWS_DOWN, UNSORTED, DUPLICATE, BAD_OFFSETS = 2, 4, 8, 16
 @pytest.mark.parametrize("dt", ["f64", "f32"])
 @pytest.mark.parametrize("plan", [_plan(1), _plan(2, n=N + 1), _plan(2, nnz=NNZ - 1), _plan(2, seen=UNSORTED),
                                   _plan(2, seen=DUPLICATE), _plan(2, seen=BAD_OFFSETS), _plan(2, fmt=0),
-                                  _plan(2, fmt=1), _plan(2, fmt=6), _plan(2, sizes=(3969, 0, 0)),
+                                  _plan(2, fmt=1), _plan(2, fmt=6), _plan(2, sizes=(257, 0, 0)), _plan(2, fmt=5, sizes=(745, 0, 0)),
                                   _plan(2, fmt=5, seen=UNSORTED)])
 def test_csr_plan_of_another_source(lib_built, plan, dt):
     assert _call(f"mgb_convert_csr_planned_{dt}", CSR, plan) == BAD_ARGUMENT
 
 
-@pytest.mark.parametrize("fmt", [2, 5])
-def test_csr_plan_of_the_other_value_type(lib_built, fmt):
-    """3,000 diagonals fit the FP32 tiles (32 groups of 124) and not the FP64 ones (of 62)."""
-    assert _call("mgb_convert_csr_planned_f64", CSR, _plan(2, fmt=fmt)) == BAD_ARGUMENT
-    assert _call("mgb_convert_csr_planned_f32", CSR, _plan(2, fmt=fmt)) != BAD_ARGUMENT  # dst's sizes are refused later
+def test_csr_plan_of_the_other_value_type(lib_built):
+    """500 diagonals are 5 groups of an HDC's FP32 tiles and 9 of its FP64 ones: 6 are taken."""
+    plan = _plan(2, fmt=5, sizes=(500, 0, 0))
+    assert _call("mgb_convert_csr_planned_f64", CSR, plan) == BAD_ARGUMENT
+    assert _call("mgb_convert_csr_planned_f32", CSR, plan) != BAD_ARGUMENT  # dst's sizes are refused later
 
 
 def test_csr_plan_of_other_offsets(lib_built):
