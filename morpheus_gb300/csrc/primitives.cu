@@ -1,6 +1,7 @@
 // primitives.cu -- scan, reductions, histograms and sorts used by convert.cu.
 #include <climits>
 #include <type_traits>
+#include <utility>
 
 #include "primitives.cuh"
 
@@ -747,108 +748,87 @@ sort_tiles(const RowRecord* __restrict__ rec, const int32_t* __restrict__ start,
   }
 }
 
-// bitonic sort of m (power of two) records in shared memory
-template <bool COLS>
-__device__ void bitonic_records(RowRecord* sk, int m) {
-  for (int k = 2; k <= m; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = threadIdx.x; i < m; i += blockDim.x) {
-        const int p = i ^ j;
-        if (p > i) {
-          const RowRecord a = sk[i], b = sk[p];
-          const bool up = ((i & k) == 0);
-          if ((record_key<COLS>(a) > record_key<COLS>(b)) == up) { sk[i] = b; sk[p] = a; }
-        }
-      }
-      __syncthreads();
-    }
-  }
-}
-// past the last record (no entry has this column and position)
-__device__ __forceinline__ RowRecord record_max() { return RowRecord{~0u, -1, 0}; }
-
-template <typename T>
-__device__ __forceinline__ void write_records(const RowRecord* src, int64_t b, int64_t n, int32_t row, int32_t* orow,
-                                              int32_t* ocol, T* oval) {
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-    if (orow != nullptr) orow[b + i] = row;
-    ocol[b + i] = src[i].col;
-    oval[b + i] = value_of<T>(src[i].val);
-  }
-}
-
 constexpr int SORT_LONG_THREADS = 512;
 constexpr int SORT_RUN = 128;
 
-// One CTA per row of SORT_SHORT < length <= SORT_MED.  Every thread keeps its
-// records in registers and only moves keys: the place in a run of SORT_RUN by
-// counting, then doubled runs by one binary search of the neighbouring run
-// per level.  (A bitonic network over 16-byte records: 129 us where a few rows
-// of thousands of entries are all there is.)
+// The order of up to SORT_MED records by one CTA: mine[k] (record
+// k * SORT_LONG_THREADS + threadIdx.x of rec) belongs at pos[k].  Every thread
+// keeps its records in registers and only moves keys: the place in a run of
+// SORT_RUN by counting, then doubled runs by one binary search of the
+// neighbouring run per level.  (A bitonic network over 16-byte records: 129 us
+// where a few rows of thousands of entries are all there is.)
+constexpr int SORT_LONG_PER = SORT_MED / SORT_LONG_THREADS;
+template <bool COLS>
+using SortKey = typename std::conditional<COLS, uint64_t, uint32_t>::type;
+
+template <bool COLS>
+__device__ __forceinline__ void order_records(const RowRecord* __restrict__ rec, int len, RowRecord* mine, int* pos,
+                                              SortKey<COLS>* from, SortKey<COLS>* to) {
+  using Key = SortKey<COLS>;
+#pragma unroll
+  for (int k = 0; k < SORT_LONG_PER; k++) {
+    const int e = k * SORT_LONG_THREADS + threadIdx.x;
+    if (e < len) {
+      mine[k] = load_record(rec + e);
+      from[e] = (Key)record_key<COLS>(mine[k]);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < SORT_LONG_PER; k++) {
+    const int e = k * SORT_LONG_THREADS + threadIdx.x;
+    if (e < len) {
+      const int c0 = e & ~(SORT_RUN - 1), c1 = min(c0 + SORT_RUN, len);
+      const Key key = (Key)record_key<COLS>(mine[k]);
+      int at = c0;
+#pragma unroll 8
+      for (int j = c0; j < c1; j++) at += from[j] < key ? 1 : 0;
+      pos[k] = at;
+      to[at] = key;
+    }
+  }
+  __syncthreads();
+  for (int width = SORT_RUN; width < len; width <<= 1) {
+    Key* t = from;
+    from = to;
+    to = t;
+#pragma unroll
+    for (int k = 0; k < SORT_LONG_PER; k++) {
+      const int e = k * SORT_LONG_THREADS + threadIdx.x;
+      if (e < len) {
+        const Key key = (Key)record_key<COLS>(mine[k]);
+        const int own = pos[k] & ~(width - 1), other = own ^ width;
+        int lo = min(other, len), hi = min(other + width, len);
+        const int first = lo;
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (from[mid] < key) lo = mid + 1; else hi = mid;
+        }
+        pos[k] = min(own, other) + (pos[k] - own) + (lo - first);
+        to[pos[k]] = key;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// One CTA per row of SORT_SHORT < length <= SORT_MED.
 template <typename T, bool COLS>
 __global__ void __launch_bounds__(SORT_LONG_THREADS)
 sort_medium_rows(const RowRecord* __restrict__ rec, const int32_t* __restrict__ start,
                  const int32_t* __restrict__ list, const int32_t* __restrict__ count, int32_t* __restrict__ orow,
                  int32_t* __restrict__ ocol, T* __restrict__ oval) {
-  using Key = typename std::conditional<COLS, uint64_t, uint32_t>::type;
-  constexpr int PER = SORT_MED / SORT_LONG_THREADS;
   extern __shared__ __align__(16) unsigned char sort_smem[];
-  Key* from = reinterpret_cast<Key*>(sort_smem);
-  Key* to = from + SORT_MED;
+  SortKey<COLS>* keys = reinterpret_cast<SortKey<COLS>*>(sort_smem);
   for (int64_t w = blockIdx.x; w < *count; w += gridDim.x) {
     const int32_t r = list[w];
     const int32_t b = start[r], len = start[r + 1] - b;
-    RowRecord mine[PER];
-    int pos[PER];
+    RowRecord mine[SORT_LONG_PER];
+    int pos[SORT_LONG_PER];
+    order_records<COLS>(rec + b, len, mine, pos, keys, keys + SORT_MED);
 #pragma unroll
-    for (int k = 0; k < PER; k++) {
-      const int e = k * SORT_LONG_THREADS + threadIdx.x;
-      if (e < len) {
-        mine[k] = load_record(rec + b + e);
-        from[e] = (Key)record_key<COLS>(mine[k]);
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < PER; k++) {
-      const int e = k * SORT_LONG_THREADS + threadIdx.x;
-      if (e < len) {
-        const int c0 = e & ~(SORT_RUN - 1), c1 = min(c0 + SORT_RUN, len);
-        const Key key = (Key)record_key<COLS>(mine[k]);
-        int at = c0;
-#pragma unroll 8
-        for (int j = c0; j < c1; j++) at += from[j] < key ? 1 : 0;
-        pos[k] = at;
-        to[at] = key;
-      }
-    }
-    __syncthreads();
-    for (int width = SORT_RUN; width < len; width <<= 1) {
-      Key* t = from;
-      from = to;
-      to = t;
-#pragma unroll
-      for (int k = 0; k < PER; k++) {
-        const int e = k * SORT_LONG_THREADS + threadIdx.x;
-        if (e < len) {
-          const Key key = (Key)record_key<COLS>(mine[k]);
-          const int own = pos[k] & ~(width - 1), other = own ^ width;
-          int lo = min(other, len), hi = min(other + width, len);
-          const int first = lo;
-          while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (from[mid] < key) lo = mid + 1; else hi = mid;
-          }
-          pos[k] = min(own, other) + (pos[k] - own) + (lo - first);
-          to[pos[k]] = key;
-        }
-      }
-      __syncthreads();
-    }
-#pragma unroll
-    for (int k = 0; k < PER; k++) {
-      const int e = k * SORT_LONG_THREADS + threadIdx.x;
-      if (e < len) {
+    for (int k = 0; k < SORT_LONG_PER; k++) {
+      if (k * SORT_LONG_THREADS + (int)threadIdx.x < len) {
         if (orow != nullptr) orow[b + pos[k]] = r;
         ocol[b + pos[k]] = mine[k].col;
         oval[b + pos[k]] = value_of<T>(mine[k].val);
@@ -858,11 +838,55 @@ sort_medium_rows(const RowRecord* __restrict__ rec, const int32_t* __restrict__ 
   }
 }
 
-// large rows: sort chunks of SORT_MED in shared memory, then merge runs pairwise
-// (merge path: each thread emits a contiguous slice of the output)
+// Rows beyond SORT_MED, in pieces of SORT_MED records (x: row, y: piece) that
+// CTAs take: each piece is ordered by itself, then runs of doubled length are
+// merged, one launch per level, a CTA per piece of the output.  (One CTA per row
+// for all of it: 118 ms for a row of 2e6 records, 26 ms for one of 500,000.)
+// The runs alternate between rec and tmp; a row is done, where it is then, when
+// it is one run.
+__device__ __forceinline__ int merge_levels(int64_t len) {
+  int n = 0;
+  for (int64_t width = SORT_MED; width < len; width <<= 1) n++;
+  return n;
+}
+
+__global__ void list_sort_pieces(const int32_t* __restrict__ start, const int32_t* __restrict__ list,
+                                 const int32_t* __restrict__ count, int2* pieces, int32_t* npieces) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < *count; w += warps) {
+    const int32_t r = list[w];
+    const int32_t n = (int32_t)(((int64_t)start[r + 1] - start[r] + SORT_MED - 1) / SORT_MED);
+    int32_t at = 0;
+    if (lane == 0) at = atomicAdd(npieces, n);
+    at = __shfl_sync(0xffffffffu, at, 0);
+    for (int32_t i = lane; i < n; i += 32) pieces[at + i] = make_int2(r, i);
+  }
+}
+
+template <bool COLS>
+__global__ void __launch_bounds__(SORT_LONG_THREADS)
+sort_pieces(RowRecord* rec, const int32_t* __restrict__ start, const int2* __restrict__ pieces,
+            const int32_t* __restrict__ npieces) {
+  extern __shared__ __align__(16) unsigned char sort_smem[];
+  SortKey<COLS>* keys = reinterpret_cast<SortKey<COLS>*>(sort_smem);
+  for (int32_t p = blockIdx.x; p < *npieces; p += gridDim.x) {
+    const int2 piece = pieces[p];
+    const int64_t b = start[piece.x] + (int64_t)piece.y * SORT_MED;
+    const int len = (int)min((int64_t)SORT_MED, start[piece.x + 1] - b);
+    RowRecord mine[SORT_LONG_PER];
+    int pos[SORT_LONG_PER];
+    order_records<COLS>(rec + b, len, mine, pos, keys, keys + SORT_MED);
+#pragma unroll
+    for (int k = 0; k < SORT_LONG_PER; k++)
+      if (k * SORT_LONG_THREADS + (int)threadIdx.x < len) rec[b + pos[k]] = mine[k];
+    __syncthreads();  // the next piece's keys
+  }
+}
+
+// number of records taken from a among the first k of a and b merged
 template <bool COLS>
 __device__ int64_t merge_corank(const RowRecord* a, int64_t na, const RowRecord* b, int64_t nb, int64_t k) {
-  // number of elements taken from a among the first k outputs
   int64_t lo = k > nb ? k - nb : 0, hi = k < na ? k : na;
   while (lo < hi) {
     const int64_t mid = (lo + hi) >> 1;
@@ -871,50 +895,68 @@ __device__ int64_t merge_corank(const RowRecord* a, int64_t na, const RowRecord*
   return lo;
 }
 
-template <typename T, bool COLS>
+template <bool COLS>
 __global__ void __launch_bounds__(SORT_LONG_THREADS)
-sort_large_rows(RowRecord* rec, RowRecord* tmp, const int32_t* __restrict__ start, const int32_t* __restrict__ list,
-                const int32_t* __restrict__ count, int32_t* __restrict__ orow, int32_t* __restrict__ ocol,
-                T* __restrict__ oval) {
-  extern __shared__ RowRecord sk[];
-  for (int64_t w = blockIdx.x; w < *count; w += gridDim.x) {
-    const int32_t r = list[w];
-    const int64_t b = start[r], len = start[r + 1] - b;
-    RowRecord* src = rec + b;
-    RowRecord* dst = tmp + b;
-    for (int64_t c0 = 0; c0 < len; c0 += SORT_MED) {
-      const int cl = (int)min((int64_t)SORT_MED, len - c0);
-      __syncthreads();
-      for (int i = threadIdx.x; i < SORT_MED; i += blockDim.x) sk[i] = i < cl ? src[c0 + i] : record_max();
-      __syncthreads();
-      bitonic_records<COLS>(sk, SORT_MED);
-      for (int i = threadIdx.x; i < cl; i += blockDim.x) src[c0 + i] = sk[i];
-    }
+merge_pieces(const RowRecord* __restrict__ src, RowRecord* __restrict__ dst, const int32_t* __restrict__ start,
+             const int2* __restrict__ pieces, const int32_t* __restrict__ npieces, int64_t width) {
+  __shared__ SortKey<COLS> s_key[SORT_MED];
+  __shared__ int64_t s_from[2];
+  for (int32_t p = blockIdx.x; p < *npieces; p += gridDim.x) {
+    const int2 piece = pieces[p];
+    const int64_t b = start[piece.x], len = start[piece.x + 1] - b;
+    if (len <= width) continue;
+    const int64_t k0 = (int64_t)piece.y * SORT_MED, k1 = min(k0 + SORT_MED, len);
+    const int64_t a0 = k0 / (2 * width) * (2 * width);  // the pair of runs that the piece lies in
+    const int64_t na = min(width, len - a0), nb = max((int64_t)0, min(width, len - a0 - width));
+    const RowRecord *A = src + b + a0, *B = A + na;
+    if (threadIdx.x < 2) s_from[threadIdx.x] = merge_corank<COLS>(A, na, B, nb, (threadIdx.x ? k1 : k0) - a0);
     __syncthreads();
-    bool in_src = true;
-    for (int64_t width = SORT_MED; width < len; width <<= 1) {
-      const RowRecord* from = in_src ? src : dst;
-      RowRecord* to = in_src ? dst : src;
-      for (int64_t a0 = 0; a0 < len; a0 += 2 * width) {
-        const int64_t na = min(width, len - a0);
-        const int64_t nb = max((int64_t)0, min(width, len - a0 - width));
-        const int64_t tot = na + nb;
-        const int64_t per = (tot + blockDim.x - 1) / blockDim.x;
-        const int64_t k0 = min(tot, (int64_t)threadIdx.x * per), k1 = min(tot, k0 + per);
-        const RowRecord* A = from + a0;
-        const RowRecord* B = from + a0 + na;
-        int64_t ia = merge_corank<COLS>(A, na, B, nb, k0);
-        int64_t ib = k0 - ia;
-        for (int64_t k = k0; k < k1; k++) {
-          if (ib >= nb || (ia < na && record_key<COLS>(A[ia]) <= record_key<COLS>(B[ib]))) to[a0 + k] = A[ia++];
-          else to[a0 + k] = B[ib++];
-        }
+    const int64_t ia = s_from[0], ib = k0 - a0 - ia;
+    const int m = (int)(k1 - k0), ma = (int)(s_from[1] - ia);  // records of the piece, those from A
+    RowRecord mine[SORT_LONG_PER];
+#pragma unroll
+    for (int k = 0; k < SORT_LONG_PER; k++) {
+      const int e = k * SORT_LONG_THREADS + threadIdx.x;
+      if (e < m) {
+        mine[k] = load_record(e < ma ? A + ia + e : B + ib + (e - ma));
+        s_key[e] = (SortKey<COLS>)record_key<COLS>(mine[k]);
       }
-      __syncthreads();
-      in_src = !in_src;
     }
-    write_records<T>(in_src ? src : dst, b, len, r, orow, ocol, oval);
     __syncthreads();
+#pragma unroll
+    for (int k = 0; k < SORT_LONG_PER; k++) {
+      const int e = k * SORT_LONG_THREADS + threadIdx.x;
+      if (e < m) {
+        const SortKey<COLS> key = (SortKey<COLS>)record_key<COLS>(mine[k]);
+        int lo = e < ma ? ma : 0, hi = e < ma ? m : ma;
+        const int first = lo;
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (s_key[mid] < key) lo = mid + 1; else hi = mid;
+        }
+        dst[b + k0 + (e < ma ? e : e - ma) + (lo - first)] = mine[k];
+      }
+    }
+    __syncthreads();  // the next piece's keys
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(SORT_LONG_THREADS)
+write_pieces(const RowRecord* __restrict__ rec, const RowRecord* __restrict__ tmp, const int32_t* __restrict__ start,
+             const int2* __restrict__ pieces, const int32_t* __restrict__ npieces, int32_t* __restrict__ orow,
+             int32_t* __restrict__ ocol, T* __restrict__ oval) {
+  for (int32_t p = blockIdx.x; p < *npieces; p += gridDim.x) {
+    const int2 piece = pieces[p];
+    const int64_t b = start[piece.x], end = start[piece.x + 1];
+    const RowRecord* from = merge_levels(end - b) & 1 ? tmp : rec;
+    const int64_t k0 = b + (int64_t)piece.y * SORT_MED, k1 = min(k0 + SORT_MED, end);
+    for (int64_t k = k0 + threadIdx.x; k < k1; k += SORT_LONG_THREADS) {
+      const RowRecord x = load_record(from + k);
+      if (orow != nullptr) orow[k] = piece.x;
+      ocol[k] = x.col;
+      oval[k] = value_of<T>(x.val);
+    }
   }
 }
 
@@ -1121,9 +1163,8 @@ int row_sort(const int32_t* rows, const int32_t* cols, const T* vals, int64_t n,
   }
   sort_tiles<T, COLS><<<(unsigned)ntiles, 256, 0, s>>>(rec, start, tile_row, orow, ocol, oval);
   MGB_LAUNCH_CHECK();
-  constexpr int smem = SORT_MED * (int)sizeof(RowRecord);
+  constexpr int keys = 2 * SORT_MED * (int)sizeof(SortKey<COLS>);
   if (h[0] > 0) {
-    constexpr int keys = 2 * SORT_MED * (COLS ? 8 : 4);
     MGB_CUDA_CHECK(cudaFuncSetAttribute(sort_medium_rows<T, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, keys));
     sort_medium_rows<T, COLS><<<(unsigned)min((int64_t)h[0], (int64_t)num_sms() * 3), SORT_LONG_THREADS, keys, s>>>(
         rec, start, medium, counters, orow, ocol, oval);
@@ -1131,10 +1172,27 @@ int row_sort(const int32_t* rows, const int32_t* cols, const T* vals, int64_t n,
   }
   if (h[1] > 0) {
     RowRecord* tmp;
+    int2* pieces;
+    int32_t* npieces;
+    const int64_t most = 2 * (n / SORT_MED);  // a row's pieces are at least half full on average
     MGB_SCRATCH(sc, tmp, n);
-    MGB_CUDA_CHECK(cudaFuncSetAttribute(sort_large_rows<T, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    sort_large_rows<T, COLS><<<(unsigned)min((int64_t)h[1], (int64_t)num_sms() * 3), SORT_LONG_THREADS, smem, s>>>(
-        rec, tmp, start, large, counters + 1, orow, ocol, oval);
+    MGB_SCRATCH(sc, pieces, most);
+    MGB_SCRATCH(sc, npieces, 1);
+    MGB_CUDA_CHECK(cudaMemsetAsync(npieces, 0, sizeof(int32_t), s));
+    list_sort_pieces<<<blocks_for(h[1], 8, (int64_t)num_sms() * 8), 256, 0, s>>>(start, large, counters + 1, pieces,
+                                                                                npieces);
+    MGB_LAUNCH_CHECK();
+    const unsigned pgrid = blocks_for(most, 1, (int64_t)num_sms() * 4);
+    MGB_CUDA_CHECK(cudaFuncSetAttribute(sort_pieces<COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, keys));
+    sort_pieces<COLS><<<pgrid, SORT_LONG_THREADS, keys, s>>>(rec, start, pieces, npieces);
+    MGB_LAUNCH_CHECK();
+    RowRecord *from = rec, *to = tmp;
+    for (int64_t width = SORT_MED; width < n; width <<= 1) {
+      merge_pieces<COLS><<<pgrid, SORT_LONG_THREADS, 0, s>>>(from, to, start, pieces, npieces, width);
+      MGB_LAUNCH_CHECK();
+      std::swap(from, to);
+    }
+    write_pieces<T><<<pgrid, SORT_LONG_THREADS, 0, s>>>(rec, tmp, start, pieces, npieces, orow, ocol, oval);
     MGB_LAUNCH_CHECK();
   }
   return MGB_SUCCESS;

@@ -219,6 +219,27 @@ def test_row_sort_tiles(cuda, N, lens, dtype):
     assert_same_matrix(mgb.matrix_to_host(A), om.to_host())
 
 
+# rows that several CTAs sort in pieces (4,096): one entry past a piece, full pieces, odd and even numbers of merge levels,
+# a last run without a neighbour, rows of different levels together; many equal columns
+@pytest.mark.parametrize("ncols", [50, 1 << 20])
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("lens", [[4097], [8192], [8193, 0, 3], [12289, 40000, 600, 4096], [70001, 2, 16384, 16385]])
+def test_row_sort_pieces(cuda, lens, ncols, dtype):
+    import morpheus_gb300 as mgb
+    rng = np.random.default_rng(len(lens))
+    rows = rng.permutation(np.repeat(np.arange(len(lens), dtype=np.int32), lens))
+    cols = rng.integers(0, ncols, rows.size).astype(np.int32)
+    hm = {"format": 0, "nrows": len(lens), "ncols": ncols, "nnz": rows.size, "row_indices": rows,
+          "column_indices": cols, "values": rng.standard_normal(rows.size).astype(dtype)}
+    got, ref = both(hm, O.CSR)
+    assert_same_matrix(got, ref)
+    A = mgb.matrix_from_host(hm)
+    mgb.sort_by_row_and_column(A)
+    om = O.OracleMatrix.from_host(hm)
+    om.sort_by_row_and_column()
+    assert_same_matrix(mgb.matrix_to_host(A), om.to_host())
+
+
 # more records than L2 holds: scattered in two halves (the middle row on either side, an odd number of rows) or, with
 # rows near each other, at once
 @pytest.mark.parametrize("N", [4098, 65537])
