@@ -214,17 +214,33 @@ int coo_segments(const mgb_coo* A, int64_t chunk, int64_t nchunks, const T* x, T
 }
 
 // Adds the carries of each row in chunk order.  carry_row is non-decreasing.
+// The sum is one thread's, but sixteen carries are read at a time: a row of
+// 500,000 entries has 4,000 of them (one read after the other: 470 us).
 template <typename T>
 __global__ void coo_carry_fixup(int64_t ncarry, int64_t nrows,
                                 const int32_t* __restrict__ cr,
                                 const T* __restrict__ cv, T* __restrict__ y,
                                 int init) {
+  constexpr int U = 16;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= ncarry) return;
   const int32_t r = cr[i];
   if (i > 0 && cr[i - 1] == r) return;
-  T s = T(0);
-  for (int64_t j = i; j < ncarry && cr[j] == r; j++) s += cv[j];
+  T s = cv[i];
+  bool more = i + 1 < ncarry && cr[i + 1] == r;
+  for (int64_t j = i + 1; more; j += U) {
+    T v[U];
+    bool in[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      in[u] = j + u < ncarry && cr[j + u] == r;
+      v[u] = j + u < ncarry ? cv[j + u] : T(0);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (in[u]) s += v[u];
+    more = in[U - 1];
+  }
   if (r >= 0 && r < nrows) y[r] = init ? s : y[r] + s;
 }
 
