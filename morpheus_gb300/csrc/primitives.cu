@@ -814,7 +814,7 @@ __device__ __forceinline__ void order_records(const RowRecord* __restrict__ rec,
 
 // One CTA per row of SORT_SHORT < length <= SORT_MED.
 template <typename T, bool COLS>
-__global__ void __launch_bounds__(SORT_LONG_THREADS)
+__global__ void __launch_bounds__(SORT_LONG_THREADS, 2)
 sort_medium_rows(const RowRecord* __restrict__ rec, const int32_t* __restrict__ start,
                  const int32_t* __restrict__ list, const int32_t* __restrict__ count, int32_t* __restrict__ orow,
                  int32_t* __restrict__ ocol, T* __restrict__ oval) {
@@ -865,7 +865,7 @@ __global__ void list_sort_pieces(const int32_t* __restrict__ start, const int32_
 }
 
 template <bool COLS>
-__global__ void __launch_bounds__(SORT_LONG_THREADS)
+__global__ void __launch_bounds__(SORT_LONG_THREADS, 2)
 sort_pieces(RowRecord* rec, const int32_t* __restrict__ start, const int2* __restrict__ pieces,
             const int32_t* __restrict__ npieces) {
   extern __shared__ __align__(16) unsigned char sort_smem[];
