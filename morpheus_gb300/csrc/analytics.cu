@@ -97,6 +97,22 @@ __global__ void row_stats_kernel(LEN lens, int64_t nrows, int64_t hyb_w,
   }
 }
 
+// Rows of a long group; false where they are walked as any.
+__device__ __noinline__ bool diag_rows_apart(const int32_t* __restrict__ ro, const int32_t* __restrict__ ci,
+                                             int64_t r0, int64_t nrows, uint32_t nc, bool wide, int lane,
+                                             prim::CtaHist h, int32_t* lens, int32_t* counts,
+                                             prim::RowPieces pieces) {
+  return prim::warp_rows_apart(ro, r0, nrows, pieces, lane, [&](bool in, int q, int32_t e, int32_t) {
+    const uint32_t c = in ? (uint32_t)__ldcs(ci + e) : nc;
+    const unsigned m = __ballot_sync(0xffffffffu, c < nc);
+    if (lens != nullptr && lane == 0 && m) atomicAdd(lens + r0 + q, __popc(m));
+    if (c >= nc) return;
+    const uint64_t bin = c - (r0 + q) + nrows - 1;
+    if (wide) prim::hist_add(h, counts, bin);
+    else prim::hist_add32(h, counts, (uint32_t)bin);
+  });
+}
+
 // Diagonal bin (c - r + nrows - 1) of every entry, and (lens != nullptr) its
 // row's length increased by the row's entries inside the matrix: one warp per
 // 32 rows, a lane per entry.  Bound by the issue slots of the counting beside
@@ -120,14 +136,8 @@ csr_diag_kernel(const int32_t* __restrict__ ro, const int32_t* __restrict__ ci, 
     if (!wide && lens == nullptr &&
         prim::warp_equal_rows<false>(ro, r0, nrows, ci, nc, lane, h, counts, run, misses, &unused, &unused, &unused))
       continue;
-    if (apart && prim::warp_rows_apart(ro, r0, nrows, pieces, lane, [&](bool in, int q, int32_t e, int32_t) {
-          const uint32_t c = in ? (uint32_t)__ldcs(ci + e) : nc;
-          const unsigned m = __ballot_sync(0xffffffffu, c < nc);
-          if (lens != nullptr && lane == 0 && m) atomicAdd(lens + r0 + q, __popc(m));
-          if (c >= nc) return;
-          if (wide) prim::hist_add(h, counts, (uint64_t)(c - (r0 + q) + nrows - 1));
-          else prim::hist_add32(h, counts, c - q + diag0);
-        }))
+    if (apart && prim::long_group(ro, r0, nrows) &&
+        diag_rows_apart(ro, ci, r0, nrows, nc, wide, lane, h, lens, counts, pieces))
       continue;
     prim::warp_row_walk(
         ro, r0, nrows, s_rows[w], lane, 0, 1, [&](int64_t c0, int i) { return (uint32_t)__ldcs(ci + c0 + i); },
@@ -143,8 +153,9 @@ csr_diag_kernel(const int32_t* __restrict__ ro, const int32_t* __restrict__ ci, 
   prim::hist_flush(h, counts);
 }
 
-// The entries of the rows that the warps above listed (64 rows of 500,000: the
-// statistics took 190,000 us by threads and 230,000 by warps).
+// The entries of the rows that the warps above listed (statistics of 64 rows of
+// 500,000 entries: 190,000 us with a thread per row, 230,000 with a warp per 32
+// rows, 217 with pieces).
 __global__ void __launch_bounds__(256) csr_diag_pieces(const int32_t* __restrict__ ro, const int32_t* __restrict__ ci,
                                                        int64_t nrows, int64_t ncols, int32_t* lens, int32_t* counts,
                                                        prim::RowPieces pieces) {
@@ -157,21 +168,15 @@ __global__ void __launch_bounds__(256) csr_diag_pieces(const int32_t* __restrict
   });
 }
 
-int csr_diags(const mgb_csr* A, int32_t* lens, int32_t* counts, cudaStream_t s) {
-  Scratch sc(s);
-  prim::RowPieces pieces{nullptr, nullptr, 0};
-  const bool apart = A->nnz > prim::LONG_ROW;
-  if (apart) {
-    pieces.limit = prim::max_row_pieces(A->nnz);
-    MGB_SCRATCH(sc, pieces.list, pieces.limit);
-    MGB_SCRATCH(sc, pieces.count, 1);
-    MGB_CUDA_CHECK(cudaMemsetAsync(pieces.count, 0, sizeof(int32_t), s));
-  }
+// pieces.limit: csr_pieces(A)
+int64_t csr_pieces(const mgb_csr* A) { return A->nnz > prim::LONG_GROUP ? prim::max_row_pieces(A->nnz) : 0; }
+int csr_diags(const mgb_csr* A, int32_t* lens, int32_t* counts, prim::RowPieces pieces, cudaStream_t s) {
+  const bool apart = pieces.limit > 0;
   csr_diag_kernel<<<csr_grid(A->nrows), 256, 0, s>>>(A->row_offsets, A->column_indices, A->nrows, A->ncols, lens,
                                                      counts, apart, pieces);
   MGB_LAUNCH_CHECK();
   if (apart) {
-    csr_diag_pieces<<<blocks_for(pieces.limit, 1, (int64_t)num_sms() * 8), 256, 0, s>>>(
+    csr_diag_pieces<<<blocks_for(pieces.limit, 1, (int64_t)num_sms() * 4), 256, 0, s>>>(
         A->row_offsets, A->column_indices, A->nrows, A->ncols, lens, counts, pieces);
     MGB_LAUNCH_CHECK();
   }
@@ -284,7 +289,7 @@ __global__ void coo_form_ell(const int32_t* __restrict__ ci, int64_t width, int6
 }
 
 __global__ void init_stats(unsigned long long* u, double* d, int* i) {
-  u[0] = 0; u[1] = 0; u[2] = 0; u[3] = 0; u[4] = 0;
+  u[0] = 0; u[1] = 0; u[2] = 0; u[3] = 0; u[4] = 0; u[5] = 0;
   d[0] = 0.0;
   i[0] = 0;        // max len
   i[1] = INT_MAX;  // min len
@@ -301,7 +306,8 @@ bool exceeds_tolerance(double num_rows, double num_entries, double num_columns) 
 // has row offsets) and the diagonal histogram (counts, zeroed).
 struct FormPass {
   virtual ~FormPass() = default;
-  virtual int run(int32_t* lens, int32_t* counts, cudaStream_t s) const = 0;
+  virtual int run(int32_t* lens, int32_t* counts, prim::RowPieces pieces, cudaStream_t s) const = 0;
+  virtual int64_t pieces() const { return 0; }  // of long CSR rows, at most
   virtual const int32_t* row_offsets() const { return nullptr; }  // lengths straight from CSR offsets
 };
 
@@ -316,10 +322,13 @@ int analyze_pass(int64_t N, int64_t M, int64_t nnz_meta, const FormPass& pass, d
   int* iv;
   int32_t* counts;
   int32_t* lens = nullptr;
-  MGB_SCRATCH(sc, u, 5);
+  MGB_SCRATCH(sc, u, 6);  // the last: pieces of long rows
   MGB_SCRATCH(sc, d, 1);
   MGB_SCRATCH(sc, iv, 3);
-  MGB_SCRATCH(sc, counts, nb);
+  const int64_t limit = pass.pieces();  // their list lies behind the counts: one allocation
+  MGB_SCRATCH(sc, counts, (nb + 1) / 2 * 2 + 2 * limit);
+  const prim::RowPieces pieces{reinterpret_cast<int2*>(counts + (nb + 1) / 2 * 2), reinterpret_cast<int32_t*>(u + 5),
+                               limit};
   const int32_t* ro = pass.row_offsets();
   if (ro == nullptr) {
     MGB_SCRATCH(sc, lens, N);
@@ -328,7 +337,7 @@ int analyze_pass(int64_t N, int64_t M, int64_t nnz_meta, const FormPass& pass, d
   init_stats<<<1, 1, 0, s>>>(u, d, iv);
   MGB_LAUNCH_CHECK();
   MGB_CUDA_CHECK(cudaMemsetAsync(counts, 0, sizeof(int32_t) * nb, s));
-  if (int st = pass.run(lens, counts, s)) return st;
+  if (int st = pass.run(lens, counts, pieces, s)) return st;
   if (ro != nullptr)
     row_stats_kernel<<<grid_for(N), 256, 0, s>>>(LensFromOffsets{ro}, N, hyb_w, u, d, iv, iv + 1, u + 4);
   else
@@ -374,15 +383,16 @@ struct CsrPass : FormPass {
   const mgb_csr* A;
   explicit CsrPass(const mgb_csr* a) : A(a) {}
   const int32_t* row_offsets() const override { return A->row_offsets; }
-  int run(int32_t*, int32_t* counts, cudaStream_t s) const override {
-    return A->nnz == 0 ? MGB_SUCCESS : csr_diags(A, nullptr, counts, s);
+  int64_t pieces() const override { return csr_pieces(A); }
+  int run(int32_t*, int32_t* counts, prim::RowPieces pieces, cudaStream_t s) const override {
+    return A->nnz == 0 ? MGB_SUCCESS : csr_diags(A, nullptr, counts, pieces, s);
   }
 };
 
 struct CooPass : FormPass {
   const mgb_coo* A;
   explicit CooPass(const mgb_coo* a) : A(a) {}
-  int run(int32_t* lens, int32_t* counts, cudaStream_t s) const override {
+  int run(int32_t* lens, int32_t* counts, prim::RowPieces pieces, cudaStream_t s) const override {
     if (A->nnz == 0) return MGB_SUCCESS;
     coo_form_coo<<<diag_grid(A->nnz), 256, 0, s>>>(A->row_indices, A->column_indices, A->nnz, A->nrows, A->ncols,
                                                   lens, counts);
@@ -395,7 +405,7 @@ template <typename T>
 struct DiaPass : FormPass {
   const mgb_dia* A;
   explicit DiaPass(const mgb_dia* a) : A(a) {}
-  int run(int32_t* lens, int32_t* counts, cudaStream_t s) const override {
+  int run(int32_t* lens, int32_t* counts, prim::RowPieces pieces, cudaStream_t s) const override {
     if (A->ndiags == 0) return MGB_SUCCESS;
     coo_form_dia<T><<<grid_for(A->nrows), 256, 0, s>>>(A->diagonal_offsets, A->ndiags, A->pitch,
                                                        static_cast<const T*>(A->values), A->nrows, A->ncols, lens,
@@ -408,7 +418,7 @@ struct DiaPass : FormPass {
 struct EllPass : FormPass {
   const mgb_ell* A;
   explicit EllPass(const mgb_ell* a) : A(a) {}
-  int run(int32_t* lens, int32_t* counts, cudaStream_t s) const override {
+  int run(int32_t* lens, int32_t* counts, prim::RowPieces pieces, cudaStream_t s) const override {
     if (A->width == 0) return MGB_SUCCESS;
     coo_form_ell<<<diag_grid(A->nrows), 256, 0, s>>>(A->column_indices, A->width, A->pitch, A->nrows, A->ncols, lens,
                                                     counts);
@@ -421,9 +431,9 @@ struct HybPass : FormPass {
   EllPass ell;
   CooPass coo;
   explicit HybPass(const mgb_hyb* a) : ell(&a->ell), coo(&a->coo) {}
-  int run(int32_t* lens, int32_t* counts, cudaStream_t s) const override {
-    if (int st = ell.run(lens, counts, s)) return st;
-    return coo.run(lens, counts, s);
+  int run(int32_t* lens, int32_t* counts, prim::RowPieces pieces, cudaStream_t s) const override {
+    if (int st = ell.run(lens, counts, pieces, s)) return st;
+    return coo.run(lens, counts, pieces, s);
   }
 };
 
@@ -431,10 +441,11 @@ template <typename T>
 struct HdcPass : FormPass {
   DiaPass<T> dia;
   const mgb_csr* csr;
+  int64_t pieces() const override { return csr_pieces(csr); }
   explicit HdcPass(const mgb_hdc* a) : dia(&a->dia), csr(&a->csr) {}
-  int run(int32_t* lens, int32_t* counts, cudaStream_t s) const override {
-    if (int st = dia.run(lens, counts, s)) return st;
-    return csr->nnz == 0 ? MGB_SUCCESS : csr_diags(csr, lens, counts, s);
+  int run(int32_t* lens, int32_t* counts, prim::RowPieces pieces, cudaStream_t s) const override {
+    if (int st = dia.run(lens, counts, pieces, s)) return st;
+    return csr->nnz == 0 ? MGB_SUCCESS : csr_diags(csr, lens, counts, pieces, s);
   }
 };
 

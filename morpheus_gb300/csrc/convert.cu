@@ -161,10 +161,11 @@ int csr_plan(const mgb_coo* src, CsrPlan* p, Scratch& sc, cudaStream_t s) {
   MGB_SCRATCH(sc, p->start, src->nrows + 1);
   MGB_SCRATCH(sc, gaps, prim::gap_words(src->nrows));
   st = prim::coo_pass(src->row_indices, src->column_indices, src->nnz, src->nrows, src->ncols, dw, nullptr, p->start,
-                      gaps, s);
+                      gaps, false, s);
   if (st) return st;
   st = words_read(dw, &p->h, s);
   if (st) return st;
+  if (prim::gaps_left(p->h)) return prim::coo_pass_gaps(src->row_indices, src->nrows, dw, gaps, p->start, s);
   return words_valid(p->h) ? MGB_SUCCESS : MGB_ERR_INVALID_INPUT;
 }
 
@@ -350,11 +351,12 @@ __device__ __forceinline__ int64_t lower_column(const int32_t* __restrict__ c, i
   return b;
 }
 
-// REM (HDC): also rem[row] = the row's entries on no stored diagonal.  Rows of
-// more than `longest` entries, most of them on none, are not walked: the stored
-// diagonals' entries are searched in them (a row of 1e6 entries kept its warp
-// for 8,000 us).
-template <typename T, bool REM>
+// REM (HDC): also rem[row] = the row's entries on no stored diagonal.  LONGS:
+// rows of more than `longest` entries, most of them on none, are not walked, the
+// stored diagonals' entries are searched in them (a tridiagonal matrix of 1e6
+// rows with a full last one: the conversion 19,600 us with a warp per row here
+// and in the remainder, 250).
+template <typename T, bool REM, bool LONGS>
 __global__ void __launch_bounds__(DIA_TILE_THREADS, 10)
 dia_fill_tiles(const int32_t* __restrict__ c, const T* __restrict__ v, const int32_t* __restrict__ start,
                int64_t nrows, int64_t pitch, int nd, const int32_t* __restrict__ offs,
@@ -391,26 +393,26 @@ dia_fill_tiles(const int32_t* __restrict__ c, const T* __restrict__ v, const int
         const int64_t g0 = r0 + 32 * g;
         if (g0 >= nrows) break;
         unsigned longs = 0;
-        if constexpr (REM)
+        if constexpr (LONGS)
           longs = __ballot_sync(0xffffffffu,
                                 start[min(g0 + lane + 1, nrows)] - start[min(g0 + lane, nrows)] > longest);
         for (int64_t p = g0;;) {  // the rows up to the next long one, and that one
           const int64_t end = longs ? g0 + __ffs(longs) - 1 : min(g0 + 32, nrows);
           const int q0 = (int)(p - g0);
-          if (!REM || p < end)
+          if (!LONGS || p < end)
             prim::warp_row_walk(
-                start, p, REM ? end : nrows, s_rows[w], lane, w % share, share,
+                start, p, LONGS ? end : nrows, s_rows[w], lane, w % share, share,
                 [&](int64_t c0, int i) { return Entry{__ldcs(c + c0 + i), __ldcs(v + c0 + i)}; },
                 [&](bool in, bool, int q, int64_t, int, Entry x) {
                   if (!in) return;
-                  q += q0;
+                  if (LONGS) q += q0;
                   const int32_t d = x.col - (int32_t)g0 - q;
                   const int found = hashed ? dia_table_find(table, d) : bin_slot[(int64_t)d + nrows - 1];
                   const int s = found - d0;
                   if (s >= 0 && s < dn) tile[s * S + 32 * g + q] = x.val;
                   if (REM && found < 0 && d0 == 0) atomicAdd(s_rem + 32 * g + q, 1);
                 });
-          if (!REM || !longs) break;
+          if (!LONGS || !longs) break;
           const int64_t b = start[end], e = start[end + 1];
           const int q = 32 * g + (int)(end - g0);
           int hits = 0;
@@ -420,7 +422,7 @@ dia_fill_tiles(const int32_t* __restrict__ c, const T* __restrict__ v, const int
             hits++;
             if (d < d0 + dn) tile[(d - d0) * S + q] = v[at];
           }
-          if (REM && d0 == 0) {
+          if (d0 == 0) {
             hits = __reduce_add_sync(0xffffffffu, hits);
             if (lane == 0) atomicAdd(s_rem + q, (w % share == 0 ? (int)(e - b) : 0) - hits);
           }
@@ -471,7 +473,7 @@ constexpr int64_t HDC_TILE_GROUPS = 6;
 
 template <typename T>
 int launch_dia_fill(const mgb_coo* src, const int32_t* start, int64_t pitch, int64_t nd, const int32_t* offs,
-                    const int32_t* bin_slot, T* out, int32_t* rem, cudaStream_t s) {
+                    const int32_t* bin_slot, T* out, int32_t* rem, bool longs, cudaStream_t s) {
   int R, D;
   dia_tile_shape<T>(nd, &R, &D);
   const size_t smem = sizeof(T) * (size_t)D * (R + 1);
@@ -481,12 +483,13 @@ int launch_dia_fill(const mgb_coo* src, const int32_t* start, int64_t pitch, int
   const T* v = static_cast<const T*>(src->values);
   // a search of 32 diagonals costs about what 1,500 entries of the walk do
   const int longest = 2048 * (int)((nd + 31) / 32);
-  if (rem != nullptr)
-    dia_fill_tiles<T, true><<<grid, DIA_TILE_THREADS, smem, s>>>(src->column_indices, v, start, src->nrows, pitch,
-                                                                 (int)nd, offs, bin_slot, out, rem, R, D, longest);
-  else
-    dia_fill_tiles<T, false><<<grid, DIA_TILE_THREADS, smem, s>>>(src->column_indices, v, start, src->nrows, pitch,
-                                                                  (int)nd, offs, bin_slot, out, nullptr, R, D, longest);
+  const auto run = [&](auto kernel) {
+    kernel<<<grid, DIA_TILE_THREADS, smem, s>>>(src->column_indices, v, start, src->nrows, pitch, (int)nd, offs,
+                                                bin_slot, out, rem, R, D, longest);
+  };
+  if (rem == nullptr) run(dia_fill_tiles<T, false, false>);
+  else if (!longs) run(dia_fill_tiles<T, true, false>);
+  else run(dia_fill_tiles<T, true, true>);
   MGB_LAUNCH_CHECK();
   return MGB_SUCCESS;
 }
@@ -510,24 +513,41 @@ int check_coo_args(const mgb_coo* src, bool diagonals = true) {
 }
 
 // One pass over the entries' indices into *dw (and the diagonal counts unless
-// null); *start: a CSR matrix's offsets, else, if asked for, row starts in
+// null); start: a CSR matrix's offsets, else, if asked for, row starts in
 // scratch.
-int index_pass(const mgb_coo* src, const int32_t* ro, bool starts, Words* dw, int32_t* diag, const int32_t** start,
+struct IndexPass {
+  const int32_t* start = nullptr;
+  int32_t *own = nullptr, *gaps = nullptr;
+};
+int index_pass(const mgb_coo* src, const int32_t* ro, bool starts, bool huge, Words* dw, int32_t* diag, IndexPass* p,
                Scratch& sc, cudaStream_t s) {
   if (ro != nullptr) {
-    *start = ro;
+    p->start = ro;
     int2* pieces;
     MGB_SCRATCH(sc, pieces, prim::max_row_pieces(src->nnz));
     return prim::csr_pass(ro, src->column_indices, src->nnz, src->nrows, src->ncols, dw, diag, pieces, s);
   }
-  int32_t *own = nullptr, *gaps = nullptr;
   if (starts) {
-    MGB_SCRATCH(sc, own, src->nrows + 1);
-    MGB_SCRATCH(sc, gaps, prim::gap_words(src->nrows));
+    MGB_SCRATCH(sc, p->own, src->nrows + 1);
+    MGB_SCRATCH(sc, p->gaps, prim::gap_words(src->nrows));
   }
-  *start = own;
-  return prim::coo_pass(src->row_indices, src->column_indices, src->nnz, src->nrows, src->ncols, dw, diag, own, gaps,
-                        s);
+  p->start = p->own;
+  return prim::coo_pass(src->row_indices, src->column_indices, src->nnz, src->nrows, src->ncols, dw, diag, p->own,
+                        p->gaps, huge, s);
+}
+
+// The pass, then the sizes (queued by `sizes`) and one host read; sizes and read
+// again where the pass left long gaps.
+template <typename SIZES>
+int pass_and_sizes(const mgb_coo* src, const int32_t* ro, bool starts, bool huge, Words* dw, int32_t* diag,
+                   IndexPass* p, Words* h, Scratch& sc, cudaStream_t s, SIZES sizes) {
+  int st = index_pass(src, ro, starts, huge, dw, diag, p, sc, s);
+  for (;;) {
+    if (!st) st = sizes();
+    if (!st) st = words_read(dw, h, s);
+    if (st || !prim::gaps_left(*h)) return st;
+    st = prim::coo_pass_gaps(src->row_indices, src->nrows, dw, p->gaps, p->own, s);
+  }
 }
 
 // COO -> DIA sizes: one pass over the indices counts the diagonals, checks
@@ -549,15 +569,13 @@ int dia_plan(const mgb_coo* src, const int32_t* ro, bool starts, DiaPlan* p, Scr
   if (st) return st;
   const int64_t nb = src->nrows + src->ncols - 1;
   MGB_SCRATCH(sc, p->counts, nb > 0 ? nb : 1);
-  st = index_pass(src, ro, starts, dw, p->counts, &p->start, sc, s);
+  if (src->nnz > 0 && nb > 0) MGB_SCRATCH(sc, p->sums, prim::bin_tiles(nb));
+  IndexPass pass;
+  st = pass_and_sizes(src, ro, starts, false, dw, p->counts, &pass, &p->h, sc, s, [&] {
+    return p->sums ? prim::select_bins(p->counts, nb, 1, p->sums, &dw->total, nullptr, s) : MGB_SUCCESS;
+  });
   if (st) return st;
-  if (src->nnz > 0 && nb > 0) {
-    MGB_SCRATCH(sc, p->sums, prim::bin_tiles(nb));
-    st = prim::select_bins(p->counts, nb, 1, p->sums, &dw->total, nullptr, s);
-    if (st) return st;
-  }
-  st = words_read(dw, &p->h, s);
-  if (st) return st;
+  p->start = pass.start;
   if (!words_valid(p->h)) return MGB_ERR_INVALID_INPUT;
   if (exceeds_tolerance(src->nrows, src->nnz, p->h.total)) return MGB_ERR_FORMAT_CONVERSION;
   return MGB_SUCCESS;
@@ -592,7 +610,7 @@ int dia_fill(const mgb_coo* src, const DiaPlan& p, mgb_dia* dst, cudaStream_t s)
   T* out = static_cast<T*>(dst->values);
   const bool distinct = words_distinct(p.h);
   if (distinct && dia_tiled(nd))
-    return launch_dia_fill<T>(src, p.start, dst->pitch, nd, dst->diagonal_offsets, slot, out, nullptr, s);
+    return launch_dia_fill<T>(src, p.start, dst->pitch, nd, dst->diagonal_offsets, slot, out, nullptr, false, s);
   MGB_CUDA_CHECK(cudaMemsetAsync(dst->values, 0, sizeof(T) * dst->pitch * nd, s));
   if (distinct) {
     dia_place<T><<<grid_for(n), 256, 0, s>>>(src->row_indices, src->column_indices, v, n, src->nrows, slot,
@@ -877,7 +895,8 @@ int place_ell(const mgb_coo* src, mgb_ell* e, int64_t W, const int32_t* slot, ui
 // contiguous range) do not fit ELL_TILE, ELL_TILE / R slots of every row at a
 // time are staged.  A pad after every 32 staged entries spreads rows of even
 // length over the banks.  Segments (grid y) divide the width where the rows
-// alone are too few CTAs: 33 rows of 1e6 entries 68,000 -> 1,070 us.  Placing
+// alone are too few CTAs (COO -> ELL of 33 rows of 1e6 entries: 68,000 us with
+// whole rows per CTA, 520 with segments).  Placing
 // each entry alone into a cleared slab: 27-point stencil on 120 x 120 x 121, COO
 // -> ELL in all 2,667 us, this way 525.
 constexpr int ELL_TILE = 2048;
@@ -885,8 +904,40 @@ constexpr int ELL_TILE_ROWS = 256;
 constexpr int ELL_SEGMENT = 64;  // slot columns of a segment at least
 __device__ __forceinline__ int ell_pad(int i) { return i + (i >> 5); }
 
+// The tile's rows whose entries do not fit: blocks of their slots (out of line,
+// for the registers of the kernel).
 template <typename T>
-__global__ void __launch_bounds__(256)
+__device__ __noinline__ void ell_fill_long(const int32_t* __restrict__ c, const T* __restrict__ v,
+                                           const int32_t* s_start, int32_t* s_c, T* s_v, int64_t r0, int64_t pitch,
+                                           int64_t k_begin, int64_t k_end, int64_t W, int32_t* __restrict__ eci,
+                                           T* __restrict__ ev, int R) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int block = ELL_TILE / R;  // a power of two, as R
+  for (int64_t k0 = k_begin; k0 < k_end; k0 += block) {
+    for (int i = threadIdx.x; i < ELL_TILE; i += 256) {
+      const int q = i / block;
+      const int64_t k = k0 + i % block;
+      if (k < s_start[q + 1] - s_start[q]) {
+        s_c[ell_pad(i)] = __ldcs(c + s_start[q] + k);
+        s_v[ell_pad(i)] = __ldcs(v + s_start[q] + k);
+      }
+    }
+    __syncthreads();
+    const int64_t k1 = min(k0 + block, k_end);
+    for (int q = lane; q < R && r0 + q < pitch; q += 32) {
+      const int64_t len = min((int64_t)(s_start[q + 1] - s_start[q]), W);
+      for (int64_t k = k0 + w; k < k1; k += 8) {
+        const int i = ell_pad(q * block + (int)(k - k0));
+        __stcs(eci + r0 + q + pitch * k, k < len ? s_c[i] : MGB_INVALID_INDEX);
+        __stcs(ev + r0 + q + pitch * k, k < len ? s_v[i] : T(0));
+      }
+    }
+    __syncthreads();
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256, 8)
 ell_fill_tiles(const int32_t* __restrict__ c, const T* __restrict__ v, const int32_t* __restrict__ start,
                int64_t nrows, int64_t pitch, int64_t width, int64_t W, int32_t* __restrict__ eci, T* __restrict__ ev,
                int R, int64_t segment) {
@@ -896,51 +947,35 @@ ell_fill_tiles(const int32_t* __restrict__ c, const T* __restrict__ v, const int
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t ntiles = (pitch + R - 1) / R;
   const int64_t k_begin = blockIdx.y * segment, k_end = min(k_begin + segment, width);
-  const int block = ELL_TILE / R;  // a power of two, as R
-  // slots [k0, k1) of the tile's rows; at(q, k): where entry k of row q is staged
-  auto write = [&](int64_t r0, int64_t k0, int64_t k1, auto at) {
-    for (int q = lane; q < R; q += 32) {
-      const int64_t row = r0 + q;
-      if (row >= pitch) break;
-      const int64_t len = min((int64_t)(s_start[q + 1] - s_start[q]), W);
-      for (int64_t k = k0 + w; k < k1; k += 8) {
-        int32_t col = MGB_INVALID_INDEX;
-        T val = T(0);
-        if (k < len) {
-          const int i = at(q, k);
-          col = s_c[ell_pad(i)];
-          val = s_v[ell_pad(i)];
-        }
-        __stcs(eci + row + pitch * k, col);
-        __stcs(ev + row + pitch * k, val);
-      }
-    }
-  };
   for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int64_t r0 = t * R;
     for (int q = threadIdx.x; q <= R; q += 256) s_start[q] = start[min(r0 + q, nrows)];
     __syncthreads();
     const int32_t e0 = s_start[0], n = s_start[R] - e0;
-    if (n <= ELL_TILE) {
-      for (int i = threadIdx.x; i < n; i += 256) {
-        s_c[ell_pad(i)] = __ldcs(c + e0 + i);
-        s_v[ell_pad(i)] = __ldcs(v + e0 + i);
-      }
-      __syncthreads();
-      write(r0, k_begin, k_end, [&](int q, int64_t k) { return s_start[q] - e0 + (int)k; });
-    } else {
-      for (int64_t k0 = k_begin; k0 < k_end; k0 += block) {
-        for (int i = threadIdx.x; i < ELL_TILE; i += 256) {
-          const int q = i / block;
-          const int64_t k = k0 + i % block;
-          if (k < s_start[q + 1] - s_start[q]) {
-            s_c[ell_pad(i)] = __ldcs(c + s_start[q] + k);
-            s_v[ell_pad(i)] = __ldcs(v + s_start[q] + k);
-          }
+    if (n > ELL_TILE) {
+      ell_fill_long<T>(c, v, s_start, s_c, s_v, r0, pitch, k_begin, k_end, W, eci, ev, R);
+      continue;
+    }
+    for (int i = threadIdx.x; i < n; i += 256) {
+      s_c[ell_pad(i)] = __ldcs(c + e0 + i);
+      s_v[ell_pad(i)] = __ldcs(v + e0 + i);
+    }
+    __syncthreads();
+    for (int q = lane; q < R; q += 32) {
+      const int64_t row = r0 + q;
+      if (row >= pitch) break;
+      const int32_t b = s_start[q];
+      const int64_t len = min((int64_t)(s_start[q + 1] - b), W);
+      for (int64_t k = k_begin + w; k < k_end; k += 8) {
+        int32_t col = MGB_INVALID_INDEX;
+        T val = T(0);
+        if (k < len) {
+          const int i = ell_pad(b - e0 + (int)k);
+          col = s_c[i];
+          val = s_v[i];
         }
-        __syncthreads();
-        write(r0, k0, min(k0 + block, k_end), [&](int q, int64_t k) { return q * block + (int)(k - k0); });
-        __syncthreads();
+        __stcs(eci + row + pitch * k, col);
+        __stcs(ev + row + pitch * k, val);
       }
     }
     __syncthreads();
@@ -969,9 +1004,9 @@ int launch_ell_fill(const mgb_coo* src, const int32_t* start, mgb_ell* e, int64_
 
 // HYB's COO part of row-sorted entries: excess[r] = the row's entries past
 // the ELL width; with their exclusive scan, one warp per 32 rows copies the
-// rows that have some.  Rows with more than EXCESS_PIECE of them are listed in
-// pieces of that many, and a CTA copies each piece (a row of 500,000 entries
-// took its warp 7,000 us).
+// rows that have some.  Rows with HUGE_ROW of them or more, where the index pass
+// saw such a row, are listed in pieces, and a CTA copies each piece (1e6 short
+// rows and one of 500,000: the conversion 8,180 us with a warp per row, 330).
 constexpr int EXCESS_PIECE = 2048;
 __global__ void row_excess(const int32_t* __restrict__ start, int64_t nrows, int64_t W, int32_t* excess) {
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += (int64_t)gridDim.x * blockDim.x)
@@ -996,7 +1031,7 @@ copy_excess(const int32_t* __restrict__ c, const T* __restrict__ v, const int32_
       const int j = __ffs(m) - 1;
       const int32_t f = __shfl_sync(0xffffffffu, from, j), k = __shfl_sync(0xffffffffu, n, j);
       const int32_t o = __shfl_sync(0xffffffffu, to, j);
-      if (k > EXCESS_PIECE) {
+      if (k >= prim::HUGE_ROW && pieces != nullptr) {
         const int32_t np = (int32_t)(((int64_t)k + EXCESS_PIECE - 1) / EXCESS_PIECE);
         int32_t at = 0;
         if (lane == 0) at = atomicAdd(npieces, np);
@@ -1004,6 +1039,7 @@ copy_excess(const int32_t* __restrict__ c, const T* __restrict__ v, const int32_
         for (int32_t i = lane; i < np; i += 32) pieces[at + i] = make_int2((int32_t)(r0 + j), i);
         continue;
       }
+#pragma unroll 4
       for (int32_t i = lane; i < k; i += 32) {
         orow[o + i] = (int32_t)(r0 + j);
         ocol[o + i] = c[f + i];
@@ -1081,13 +1117,15 @@ int row_plan(const mgb_coo* src, const int32_t* ro, int64_t width, RowPlan* p, S
   Words* dw;
   int st = words_alloc(sc, &dw, s);
   if (st) return st;
-  st = index_pass(src, ro, true, dw, nullptr, &p->start, sc, s);
-  if (st) return st;
   const unsigned grid = blocks_for(N, 256, (int64_t)num_sms() * 8);
-  row_sizes<<<grid, 256, 0, s>>>(RowsFromStart{p->start}, N, width, dw);
-  MGB_LAUNCH_CHECK();
-  st = words_read(dw, &p->h, s);
+  IndexPass pass;
+  st = pass_and_sizes(src, ro, true, true, dw, nullptr, &pass, &p->h, sc, s, [&] {
+    row_sizes<<<grid, 256, 0, s>>>(RowsFromStart{pass.start}, N, width, dw);
+    MGB_LAUNCH_CHECK();
+    return (int)MGB_SUCCESS;
+  });
   if (st) return st;
+  p->start = pass.start;
   if (!words_valid(p->h)) return MGB_ERR_INVALID_INPUT;
   if (words_rows_sorted(p->h)) return MGB_SUCCESS;
   const int32_t seen = p->h.seen;
@@ -1205,17 +1243,20 @@ int hyb_fill(const mgb_coo* src, const RowPlan& p, int64_t W, mgb_hyb* dst, cuda
     MGB_LAUNCH_CHECK();
     st = prim::exclusive_scan<int32_t, int32_t>(excess, base, src->nrows, s);
     if (st) return st;
-    int2* pieces;
-    int32_t* npieces;
-    MGB_SCRATCH(sc, npieces, 1);
-    MGB_SCRATCH(sc, pieces, 2 * (cn / EXCESS_PIECE) + 1);  // at least half of EXCESS_PIECE in a listed row's pieces on average
-    MGB_CUDA_CHECK(cudaMemsetAsync(npieces, 0, sizeof(int32_t), s));
+    const bool longs = (p.h.seen & prim::COO_HUGE_ROW) && cn >= prim::HUGE_ROW;
+    int2* pieces = nullptr;
+    int32_t* npieces = nullptr;
+    if (longs) {
+      MGB_SCRATCH(sc, npieces, 1);
+      MGB_SCRATCH(sc, pieces, 2 * (cn / EXCESS_PIECE) + 1);  // listed rows' pieces are more than half full
+      MGB_CUDA_CHECK(cudaMemsetAsync(npieces, 0, sizeof(int32_t), s));
+    }
     const T* v = static_cast<const T*>(src->values);
     T* ov = static_cast<T*>(c->values);
     copy_excess<T><<<grid_for(src->nrows), 256, 0, s>>>(src->column_indices, v, p.start, base, src->nrows, W,
                                                         c->row_indices, c->column_indices, ov, pieces, npieces);
     MGB_LAUNCH_CHECK();
-    if (cn <= EXCESS_PIECE) return MGB_SUCCESS;
+    if (!longs) return MGB_SUCCESS;
     copy_excess_pieces<T><<<blocks_for(cn, EXCESS_PIECE, (int64_t)num_sms() * 8), 256, 0, s>>>(
         src->column_indices, v, p.start, base, W, c->row_indices, c->column_indices, ov, pieces, npieces);
     MGB_LAUNCH_CHECK();
@@ -1317,7 +1358,7 @@ __global__ void hdc_dia_place(const int32_t* __restrict__ r, const T* __restrict
 // stored diagonal go, in order, to the consecutive places from base[first
 // row] on: one warp per 32 rows, ranks by ballot.  Long rows are left in pieces
 // to hdc_remainder_pieces.
-template <typename T>
+template <typename T, bool LONGS>
 __global__ void __launch_bounds__(256)
 hdc_remainder(const int32_t* __restrict__ c, const T* __restrict__ v, const int32_t* __restrict__ start,
               const int32_t* __restrict__ base, int64_t nrows, int nd, const int32_t* __restrict__ offs,
@@ -1346,7 +1387,8 @@ hdc_remainder(const int32_t* __restrict__ c, const T* __restrict__ v, const int3
       }
       to += __popc(m);
     };
-    if (prim::warp_rows_apart(start, r0, nrows, pieces, lane, [&](bool in, int q, int32_t e, int32_t first) {
+    if (LONGS && prim::long_group(start, r0, nrows) &&
+        prim::warp_rows_apart(start, r0, nrows, pieces, lane, [&](bool in, int q, int32_t e, int32_t first) {
           if (e - lane == first) to = base[r0 + q];
           place(in, q, e, in ? __ldcs(c + e) : (int32_t)(r0 + q));
         }))
@@ -1379,6 +1421,7 @@ hdc_remainder_pieces(const int32_t* __restrict__ c, const T* __restrict__ v, con
   const int64_t n = min((int64_t)*pieces.count, pieces.limit);
   for (int64_t piece = blockIdx.x; piece < n; piece += gridDim.x) {
     const int32_t row = pieces.list[piece].x;
+    if (row < 0) continue;
     const int64_t b = start[row], e = start[row + 1], e0 = b + (int64_t)pieces.list[piece].y * prim::ROW_PIECE;
     const int64_t first = __ldg(c + e0);
     int hits = 0;
@@ -1445,12 +1488,12 @@ int hdc_plan(const mgb_coo* src, const int32_t* ro, bool starts, HdcPlan* p, Scr
   if (st) return st;
   MGB_SCRATCH(sc, p->counts, nb);
   MGB_SCRATCH(sc, p->sums, prim::bin_tiles(nb));
-  st = index_pass(src, ro, starts, dw, p->counts, &p->start, sc, s);
+  IndexPass pass;
+  st = pass_and_sizes(src, ro, starts, true, dw, p->counts, &pass, &p->h, sc, s, [&] {
+    return prim::select_bins(p->counts, nb, p->min_elem, p->sums, &dw->total, &dw->total2, s);
+  });
   if (st) return st;
-  st = prim::select_bins(p->counts, nb, p->min_elem, p->sums, &dw->total, &dw->total2, s);
-  if (st) return st;
-  st = words_read(dw, &p->h, s);
-  if (st) return st;
+  p->start = pass.start;
   if (!words_valid(p->h)) return MGB_ERR_INVALID_INPUT;
   if (exceeds_tolerance(src->nrows, p->h.total2, p->h.total)) return MGB_ERR_FORMAT_CONVERSION;
   return MGB_SUCCESS;
@@ -1517,23 +1560,28 @@ int hdc_fill(const mgb_coo* src, const HdcPlan& p, mgb_hdc* dst, cudaStream_t s)
       return MGB_SUCCESS;
     }
     if (hdc_tiled<T>(nd)) {
+      // rows that one warp has too much with: 32 of less than HUGE_ROW do as little as the mean allows
+      const bool longs = (p.h.seen & prim::COO_HUGE_ROW) || n / N > prim::LONG_GROUP / 32;
       int32_t* rem;
       MGB_SCRATCH(sc, rem, N + 1);
       MGB_CUDA_CHECK(cudaMemsetAsync(rem + N, 0, sizeof(int32_t), s));
       st = launch_dia_fill<T>(src, p.start, D->pitch, nd, D->diagonal_offsets, p.counts, static_cast<T*>(D->values),
-                              rem, s);
+                              rem, longs, s);
       if (st) return st;
       st = prim::exclusive_scan<int32_t, int32_t>(rem, C->row_offsets, N + 1, s);
       if (st || cn == 0) return st;
       prim::RowPieces pieces{nullptr, nullptr, prim::max_row_pieces(n)};
-      MGB_SCRATCH(sc, pieces.list, pieces.limit);
-      MGB_SCRATCH(sc, pieces.count, 1);
-      MGB_CUDA_CHECK(cudaMemsetAsync(pieces.count, 0, sizeof(int32_t), s));
-      hdc_remainder<T><<<blocks_for(N, 256, (int64_t)num_sms() * 8), 256, 0, s>>>(
-          src->column_indices, v, p.start, C->row_offsets, N, (int)nd, D->diagonal_offsets, p.counts, cn,
-          C->column_indices, static_cast<T*>(C->values), pieces);
+      if (longs)
+        if (int e = prim::row_pieces_alloc(&pieces, sc, s)) return e;
+      const auto run = [&](auto kernel) {
+        kernel<<<blocks_for(N, 256, (int64_t)num_sms() * 8), 256, 0, s>>>(
+            src->column_indices, v, p.start, C->row_offsets, N, (int)nd, D->diagonal_offsets, p.counts, cn,
+            C->column_indices, static_cast<T*>(C->values), pieces);
+      };
+      if (longs) run(hdc_remainder<T, true>);
+      else run(hdc_remainder<T, false>);
       MGB_LAUNCH_CHECK();
-      if (n <= prim::LONG_ROW) return MGB_SUCCESS;
+      if (!longs) return MGB_SUCCESS;
       hdc_remainder_pieces<T><<<blocks_for(pieces.limit, 1, (int64_t)num_sms() * 8), 256, 0, s>>>(
           src->column_indices, v, p.start, C->row_offsets, N, (int)nd, D->diagonal_offsets, p.counts, cn,
           C->column_indices, static_cast<T*>(C->values), pieces);
@@ -1827,7 +1875,7 @@ int coo_sort(mgb_coo* A, void* ws, int64_t bytes, cudaStream_t s) {
   st = prim::reduce_max_i32(A->row_indices, A->nnz, &dw->maxv, s);
   if (st) return st;
   // rows and columns must be >= 0 (the counting sort indexes by them)
-  st = prim::coo_pass(A->row_indices, A->column_indices, A->nnz, INT32_MAX, INT32_MAX, dw, nullptr, nullptr, nullptr, s);
+  st = prim::coo_pass(A->row_indices, A->column_indices, A->nnz, INT32_MAX, INT32_MAX, dw, nullptr, nullptr, nullptr, false, s);
   if (st) return st;
   Words hw;
   st = words_read(dw, &hw, s);

@@ -144,9 +144,9 @@ __global__ void sorted_flags_kernel(const int32_t* __restrict__ r, const int32_t
 // on the 27-point stencil at 160^3; the HBM floor of the pass is 131 us).
 // Row starts: the entry where the row changes from p to q is the start of
 // the rows p + 1..q; gaps longer than PASS_GAP are listed by their entry and
-// filled by fill_gaps, a warp each, those beyond PASS_HUGE by its whole grid (by
-// the CTA that met them, 10,000 entries in 5e7 rows took the conversion to CSR
-// 3,256 us); the rows before the first and after the last entry are left to
+// filled by fill_gaps, a warp each, those beyond PASS_HUGE by its whole grid (COO
+// -> CSR of 10,000 entries in 5e7 rows: 3,260 us with the CTA that met the gap
+// filling it, 195); the rows before the first and after the last entry are left to
 // this kernel's grid.
 // Rows that go down make the starts useless, and entries in random order have
 // gaps of a third of the matrix each: the first such row that a CTA sees stops
@@ -154,13 +154,19 @@ __global__ void sorted_flags_kernel(const int32_t* __restrict__ r, const int32_t
 // tile.
 constexpr uint32_t PASS_GAP = 256;
 constexpr uint32_t PASS_HUGE = 1 << 16;
-constexpr int PASS_GAPS = 1024;  // listed per CTA before the global list
 // of non-decreasing rows at most so many gaps
 __host__ __device__ inline int64_t max_gaps(int64_t nrows) { return nrows / PASS_GAP + 1; }
 __host__ __device__ inline int64_t max_huge(int64_t nrows) { return nrows / PASS_HUGE + 1; }
 
-template <bool DIAG, bool STARTS>
-__global__ void __launch_bounds__(256) coo_pass_kernel(const int32_t* __restrict__ r, const int32_t* __restrict__ c,
+// out of line: the pass has no registers to spare for it
+__device__ __noinline__ void list_gap(Words* d, int32_t* gaps, int64_t nrows, int32_t at, bool huge) {
+  const int64_t g = atomicAdd(huge ? &d->huge : &d->gaps, 1);
+  if (g < (huge ? max_huge(nrows) : max_gaps(nrows))) gaps[(huge ? max_gaps(nrows) : 0) + g] = at;
+}
+
+// HUGE: looks for rows of HUGE_ROW entries (COO_HUGE_ROW).
+template <bool DIAG, bool STARTS, bool HUGE>
+__global__ void __launch_bounds__(256, STARTS ? (DIAG && HUGE ? 6 : 8) : 1) coo_pass_kernel(const int32_t* __restrict__ r, const int32_t* __restrict__ c,
                                                        int64_t n, int64_t nrows, int64_t ncols, bool vec,
                                                        Words* d, int32_t* __restrict__ diag,
                                                        int32_t* __restrict__ start, int32_t* __restrict__ gaps) {
@@ -168,13 +174,11 @@ __global__ void __launch_bounds__(256) coo_pass_kernel(const int32_t* __restrict
   __shared__ uint32_t h_keys[DIAG ? HIST_SLOTS : 1];
   __shared__ int32_t h_counts[DIAG ? HIST_SLOTS : 1];
   __shared__ int h_full;
-  __shared__ int32_t gap_at[STARTS ? PASS_GAPS : 1];
-  __shared__ int ngaps, s_bits, s_stop, s_base;
+  __shared__ int s_bits, s_stop;
   volatile int* stop = &s_stop;
   const CtaHist h{h_keys, h_counts, &h_full};
   if constexpr (DIAG) hist_init(h);
   if (threadIdx.x == 0) {
-    ngaps = 0;
     s_bits = 0;
     s_stop = 0;
   }
@@ -184,7 +188,7 @@ __global__ void __launch_bounds__(256) coo_pass_kernel(const int32_t* __restrict
   // negative indices upset do not matter, such a matrix is refused)
   const uint32_t nr = (uint32_t)min(nrows, (int64_t)1 << 31), nc = (uint32_t)min(ncols, (int64_t)1 << 31);
   const uint32_t mid = (uint32_t)(nrows - 1);
-  bool bad = false, rows_down = false, down = false, equal = false;
+  int bits = 0;
   for (int64_t base = (int64_t)blockIdx.x * 1024; base < n; base += (int64_t)gridDim.x * 1024) {
     const int64_t i0 = base + (int64_t)threadIdx.x * 4;
     const int m = (int)min((int64_t)4, n - i0);  // this thread's entries (<= 0: none)
@@ -202,17 +206,20 @@ __global__ void __launch_bounds__(256) coo_pass_kernel(const int32_t* __restrict
     uint32_t pr = __shfl_up_sync(0xffffffffu, rr[3], 1), pc = __shfl_up_sync(0xffffffffu, cc[3], 1);
     if (lane == 0 && m > 0 && i0 > 0) { pr = r[i0 - 1]; pc = c[i0 - 1]; }
     if (i0 == 0) { pr = rr[0]; pc = 0; }  // the first entry: nothing before it
+    // a row of HUGE_ROW entries has two that are HUGE_ROW - 1024 apart, the first at a multiple of 1024
+    if (HUGE && threadIdx.x == 0 && base + HUGE_ROW - 1024 < n && r[base + HUGE_ROW - 1024] == (int32_t)rr[0])
+      bits |= COO_HUGE_ROW;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       if (k >= m) break;
       const bool ok = rr[k] < nr && cc[k] < nc;
-      bad |= !ok;
+      if (!ok) bits |= COO_BAD_INDEX;
       if (rr[k] == pr) {
-        down |= cc[k] < pc;
-        equal |= cc[k] == pc && (k > 0 || i0 > 0);
+        if (cc[k] < pc) bits |= COO_UNSORTED;
+        if (cc[k] == pc && (k > 0 || i0 > 0)) bits |= COO_DUPLICATE;
       } else {
         if (rr[k] < pr) {
-          rows_down = true;
+          bits |= COO_ROWS_UNSORTED | COO_UNSORTED;
           if (STARTS && !*stop) {
             *stop = 1;
             atomicOr(seen, COO_ROWS_UNSORTED);
@@ -223,17 +230,8 @@ __global__ void __launch_bounds__(256) coo_pass_kernel(const int32_t* __restrict
             if (rr[k] < nr) start[rr[k]] = (int32_t)(i0 + k);
           } else if (rr[k] > pr && rr[k] < nr && !*stop) {
             const int32_t at = (int32_t)(i0 + k);
-            if (rr[k] - pr > PASS_HUGE) {
-              const int64_t g = atomicAdd(&d->huge, 1);
-              if (g < max_huge(nrows)) gaps[max_gaps(nrows) + g] = at;
-            } else if (rr[k] - pr > PASS_GAP) {
-              const int g = atomicAdd(&ngaps, 1);
-              if (g < PASS_GAPS) {
-                gap_at[g] = at;
-              } else {
-                const int64_t all = atomicAdd(&d->gaps, 1);
-                if (all < max_gaps(nrows)) gaps[all] = at;
-              }
+            if (rr[k] - pr > PASS_GAP) {
+              list_gap(d, gaps, nrows, at, rr[k] - pr > PASS_HUGE);
             } else {
               for (uint32_t q = pr + 1; q <= rr[k]; q++) start[q] = at;
             }
@@ -245,20 +243,11 @@ __global__ void __launch_bounds__(256) coo_pass_kernel(const int32_t* __restrict
       pc = cc[k];
     }
   }
-  const int bits = (bad ? COO_BAD_INDEX : 0) | (rows_down ? COO_ROWS_UNSORTED | COO_UNSORTED : 0) |
-                   (down ? COO_UNSORTED : 0) | (equal ? COO_DUPLICATE : 0);
   if (bits) atomicOr(&s_bits, bits);
   __syncthreads();
   if (threadIdx.x == 0 && s_bits) atomicOr(seen, s_bits);
   if constexpr (DIAG) hist_flush(h, diag);
   if constexpr (STARTS) {
-    const int listed = s_stop ? 0 : min(ngaps, PASS_GAPS);
-    if (listed > 0) {
-      if (threadIdx.x == 0) s_base = atomicAdd(&d->gaps, listed);
-      __syncthreads();
-      for (int g = threadIdx.x; g < listed; g += 256)
-        if ((int64_t)s_base + g < max_gaps(nrows)) gaps[s_base + g] = gap_at[g];
-    }
     const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x, nt = (int64_t)gridDim.x * 256;
     const int64_t first = n > 0 ? min((int64_t)r[0], nrows) : nrows;
     const int64_t last = n > 0 ? max((int64_t)r[n - 1], (int64_t)-1) : nrows;
@@ -267,10 +256,10 @@ __global__ void __launch_bounds__(256) coo_pass_kernel(const int32_t* __restrict
   }
 }
 
-// The rows of the listed gaps start at the entry behind the gap.
+// The rows of the listed gaps start at the entry behind the gap (valid and
+// non-decreasing rows).
 __global__ void __launch_bounds__(256) fill_gaps(const int32_t* __restrict__ r, int64_t nrows, const Words* d,
                                                  const int32_t* __restrict__ gaps, int32_t* __restrict__ start) {
-  if (d->seen & (COO_BAD_INDEX | COO_ROWS_UNSORTED)) return;  // no starts
   const int64_t warps = (int64_t)gridDim.x * 8, n = min((int64_t)d->gaps, max_gaps(nrows));
   for (int64_t g = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); g < n; g += warps) {
     const int32_t at = gaps[g];
@@ -283,6 +272,23 @@ __global__ void __launch_bounds__(256) fill_gaps(const int32_t* __restrict__ r, 
     for (int64_t q = first + (int64_t)blockIdx.x * 256 + threadIdx.x; q <= last; q += (int64_t)gridDim.x * 256)
       start[q] = at;
   }
+}
+
+// Rows of a long group: their COO_* bits, -1 where they are walked as any.
+template <bool DIAG>
+__device__ __noinline__ int csr_pass_apart(const int32_t* __restrict__ ro, const int32_t* __restrict__ c, int64_t r0,
+                                           int64_t nrows, uint32_t nc, int lane, CtaHist h, int32_t* diag,
+                                           RowPieces pieces) {
+  int bits = COO_HUGE_ROW;
+  const bool apart = warp_rows_apart(ro, r0, nrows, pieces, lane, [&](bool in, int q, int32_t e, int32_t first) {
+    if (!in) return;
+    const uint32_t col = c[e], before = e > first ? c[e - 1] : 0;
+    if (col >= nc) bits |= COO_BAD_INDEX;
+    if (col < before) bits |= COO_UNSORTED;
+    if (e > first && col == before) bits |= COO_DUPLICATE;
+    if (DIAG && col < nc) hist_add32(h, diag, col - (uint32_t)(r0 + q) + (uint32_t)(nrows - 1));
+  });
+  return apart ? bits : -1;
 }
 
 template <bool DIAG>
@@ -300,6 +306,7 @@ __global__ void __launch_bounds__(256, DIAG_CTAS) csr_pass_kernel(const int32_t*
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint32_t nc = (uint32_t)min(ncols, (int64_t)1 << 31);
   bool bad = false, offsets = false, down = false, equal = false;
+  int longs = 0;
   KeyRun run;
   int misses = 0;
   for (int64_t r0 = ((int64_t)blockIdx.x * 8 + w) * 32; r0 < nrows; r0 += (int64_t)gridDim.x * 256) {
@@ -312,15 +319,13 @@ __global__ void __launch_bounds__(256, DIAG_CTAS) csr_pass_kernel(const int32_t*
     uint32_t last = 0;  // column of the entry before the group
     const uint32_t diag0 = (uint32_t)(nrows - 1 - r0);
     if (DIAG && warp_equal_rows<true>(ro, r0, nrows, c, nc, lane, h, diag, run, misses, &bad, &down, &equal)) continue;
-    if (n > LONG_ROW && warp_rows_apart(ro, r0, nrows, pieces, lane, [&](bool in, int q, int32_t e, int32_t first) {
-          if (!in) return;
-          const uint32_t col = c[e], before = e > first ? c[e - 1] : 0;
-          bad |= col >= nc;
-          down |= col < before;
-          equal |= e > first && col == before;
-          if (DIAG && col < nc) hist_add32(h, diag, col - q + diag0);
-        }))
-      continue;
+    if (long_group(ro, r0, nrows)) {
+      const int b = csr_pass_apart<DIAG>(ro, c, r0, nrows, nc, lane, h, diag, pieces);
+      if (b >= 0) {
+        longs |= b;
+        continue;
+      }
+    }
     warp_row_walk(
         ro, r0, nrows, s_rows[w], lane, 0, 1, [&](int64_t c0, int i) { return (uint32_t)__ldcs(c + c0 + i); },
         [&](bool in, bool head, int q, int64_t, int, uint32_t col) {
@@ -336,7 +341,7 @@ __global__ void __launch_bounds__(256, DIAG_CTAS) csr_pass_kernel(const int32_t*
   }
   if constexpr (DIAG) run_end(h, diag, run);
   const int bits = (bad ? COO_BAD_INDEX : 0) | (offsets ? COO_BAD_OFFSETS : 0) | (down ? COO_UNSORTED : 0) |
-                   (equal ? COO_DUPLICATE : 0);
+                   (equal ? COO_DUPLICATE : 0) | longs;
   if (bits) atomicOr(&s_bits, bits);
   __syncthreads();
   if (threadIdx.x == 0 && s_bits) atomicOr(seen, s_bits);
@@ -344,13 +349,13 @@ __global__ void __launch_bounds__(256, DIAG_CTAS) csr_pass_kernel(const int32_t*
 }
 
 // The entries of the long rows: most of them alone on their diagonals, so they
-// are counted globally.  64 rows of 500,000 entries: the conversion to ELL took
-// 27,089 us through COO, 95,410 with a warp per 32 rows.
+// are counted globally.  CSR -> ELL of 64 rows of 500,000 entries: 27,100 us
+// through COO, 95,400 with a warp per 32 rows, 350 with pieces.
 template <bool DIAG>
 __global__ void __launch_bounds__(256) csr_pass_pieces(const int32_t* __restrict__ ro, const int32_t* __restrict__ c,
                                                        int64_t nrows, int64_t ncols, int32_t* seen,
                                                        int32_t* __restrict__ diag, RowPieces pieces) {
-  if (*reinterpret_cast<volatile int32_t*>(seen) & COO_BAD_OFFSETS) return;
+  if (*pieces.count == 0 || (*reinterpret_cast<volatile int32_t*>(seen) & COO_BAD_OFFSETS)) return;
   const uint32_t nc = (uint32_t)min(ncols, (int64_t)1 << 31);
   bool bad = false, down = false, equal = false;
   for_row_pieces(ro, pieces, [&](int32_t row, int32_t e, int32_t first) {
@@ -841,7 +846,7 @@ sort_medium_rows(const RowRecord* __restrict__ rec, const int32_t* __restrict__ 
 // Rows beyond SORT_MED, in pieces of SORT_MED records (x: row, y: piece) that
 // CTAs take: each piece is ordered by itself, then runs of doubled length are
 // merged, one launch per level, a CTA per piece of the output.  (One CTA per row
-// for all of it: 118 ms for a row of 2e6 records, 26 ms for one of 500,000.)
+// for all of it: sorting a row of 2e6 entries 118 ms, with pieces 0.8.)
 // The runs alternate between rec and tmp; a row is done, where it is then, when
 // it is one run.
 __device__ __forceinline__ int merge_levels(int64_t len) {
@@ -1024,25 +1029,21 @@ int words_read(const Words* d, Words* h, cudaStream_t s) { return to_host(d, h, 
 int64_t gap_words(int64_t nrows) { return max_gaps(nrows) + max_huge(nrows); }
 
 int coo_pass(const int32_t* rows, const int32_t* cols, int64_t n, int64_t nrows, int64_t ncols, Words* d,
-             int32_t* diag, int32_t* start, int32_t* gaps, cudaStream_t s) {
+             int32_t* diag, int32_t* start, int32_t* gaps, bool huge, cudaStream_t s) {
   const int64_t nb = nrows + ncols - 1;
   if (diag != nullptr && nb > 0) MGB_CUDA_CHECK(cudaMemsetAsync(diag, 0, sizeof(int32_t) * nb, s));
   if (n <= 0 && start == nullptr) return MGB_SUCCESS;
   const bool vec = (reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(cols)) % 16 == 0;
   const unsigned grid = blocks_for(n / 4 + 1, 256, (int64_t)num_sms() * 8);
-  if (diag != nullptr && start != nullptr)
-    coo_pass_kernel<true, true><<<grid, 256, 0, s>>>(rows, cols, n, nrows, ncols, vec, d, diag, start, gaps);
-  else if (diag != nullptr)
-    coo_pass_kernel<true, false><<<grid, 256, 0, s>>>(rows, cols, n, nrows, ncols, vec, d, diag, start, gaps);
-  else if (start != nullptr)
-    coo_pass_kernel<false, true><<<grid, 256, 0, s>>>(rows, cols, n, nrows, ncols, vec, d, diag, start, gaps);
-  else
-    coo_pass_kernel<false, false><<<grid, 256, 0, s>>>(rows, cols, n, nrows, ncols, vec, d, diag, start, gaps);
+  const auto run = [&](auto kernel) {
+    kernel<<<grid, 256, 0, s>>>(rows, cols, n, nrows, ncols, vec, d, diag, start, gaps);
+  };
+  if (diag != nullptr && start != nullptr && huge) run(coo_pass_kernel<true, true, true>);
+  else if (diag != nullptr && start != nullptr) run(coo_pass_kernel<true, true, false>);
+  else if (diag != nullptr) run(coo_pass_kernel<true, false, false>);
+  else if (start != nullptr) run(coo_pass_kernel<false, true, true>);
+  else run(coo_pass_kernel<false, false, false>);
   MGB_LAUNCH_CHECK();
-  if (start != nullptr && n > 1 && nrows > PASS_GAP) {
-    fill_gaps<<<blocks_for(nrows, 1024, (int64_t)num_sms() * 8), 256, 0, s>>>(rows, nrows, d, gaps, start);
-    MGB_LAUNCH_CHECK();
-  }
   return MGB_SUCCESS;
 }
 
@@ -1056,11 +1057,19 @@ int csr_pass(const int32_t* ro, const int32_t* cols, int64_t n, int64_t nrows, i
   if (diag != nullptr) csr_pass_kernel<true><<<grid, 256, 0, s>>>(ro, cols, n, nrows, ncols, &d->seen, diag, longs);
   else csr_pass_kernel<false><<<grid, 256, 0, s>>>(ro, cols, n, nrows, ncols, &d->seen, diag, longs);
   MGB_LAUNCH_CHECK();
-  if (n <= LONG_ROW) return MGB_SUCCESS;
-  const unsigned cap = blocks_for(longs.limit, 1, (int64_t)num_sms() * 8);
-  if (diag != nullptr) csr_pass_pieces<true><<<cap, 256, 0, s>>>(ro, cols, nrows, ncols, &d->seen, diag, longs);
-  else csr_pass_pieces<false><<<cap, 256, 0, s>>>(ro, cols, nrows, ncols, &d->seen, diag, longs);
+  if (n <= LONG_GROUP) return MGB_SUCCESS;
+  const unsigned pgrid = blocks_for(longs.limit, 1, (int64_t)num_sms() * 4);
+  if (diag != nullptr) csr_pass_pieces<true><<<pgrid, 256, 0, s>>>(ro, cols, nrows, ncols, &d->seen, diag, longs);
+  else csr_pass_pieces<false><<<pgrid, 256, 0, s>>>(ro, cols, nrows, ncols, &d->seen, diag, longs);
   MGB_LAUNCH_CHECK();
+  return MGB_SUCCESS;
+}
+
+int coo_pass_gaps(const int32_t* rows, int64_t nrows, Words* d, const int32_t* gaps, int32_t* start, cudaStream_t s) {
+  fill_gaps<<<blocks_for(nrows, 1024, (int64_t)num_sms() * 8), 256, 0, s>>>(rows, nrows, d, gaps, start);
+  MGB_LAUNCH_CHECK();
+  MGB_CUDA_CHECK(cudaMemsetAsync(&d->total, 0, 2 * sizeof(int64_t), s));
+  MGB_CUDA_CHECK(cudaMemsetAsync(&d->maxv, 0, 3 * sizeof(int32_t), s));  // and gaps, huge
   return MGB_SUCCESS;
 }
 

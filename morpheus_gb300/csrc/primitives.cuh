@@ -95,6 +95,8 @@ constexpr int32_t COO_ROWS_UNSORTED = 2;  // a row smaller than the one before i
 constexpr int32_t COO_UNSORTED = 4;       // a (row, column) smaller than the one before it
 constexpr int32_t COO_DUPLICATE = 8;      // a (row, column) equal to the one before it
 constexpr int32_t COO_BAD_OFFSETS = 16;   // CSR row offsets that do not rise from 0 to the number of entries
+constexpr int32_t COO_HUGE_ROW = 32;      // where it is looked for: maybe a row of HUGE_ROW entries or more (never missed)
+constexpr int HUGE_ROW = 4096;
 struct Words {
   int64_t total, total2;  // plan sizes
   int32_t seen;           // COO_* bits
@@ -110,10 +112,18 @@ int words_read(const Words* d, Words* h, cudaStream_t s);         // synchronise
 // zeroed here): the entries on each diagonal, bin column - row + nrows - 1;
 // start != nullptr (nrows + 1 entries): the first entry of every row, valid
 // when the rows are in range and non-decreasing, with gaps = gap_words(nrows)
-// words of scratch.  Entries out of range are reported and not counted.
+// words of scratch, and once coo_pass_gaps has filled the long gaps where the
+// words read back say that there are some (gaps_left); huge: also COO_HUGE_ROW.
+// Entries out of range are reported and not counted.
 int64_t gap_words(int64_t nrows);
 int coo_pass(const int32_t* rows, const int32_t* cols, int64_t n, int64_t nrows, int64_t ncols, Words* d,
-             int32_t* diag, int32_t* start, int32_t* gaps, cudaStream_t s);
+             int32_t* diag, int32_t* start, int32_t* gaps, bool huge, cudaStream_t s);
+
+inline bool gaps_left(const Words& h) {
+  return !(h.seen & (COO_BAD_INDEX | COO_ROWS_UNSORTED)) && (h.gaps | h.huge) != 0;
+}
+// also clears the gaps and the sizes (total, total2, maxv) in *d
+int coo_pass_gaps(const int32_t* rows, int64_t nrows, Words* d, const int32_t* gaps, int32_t* start, cudaStream_t s);
 
 // The same for the entries of a CSR matrix (its rows are in order), one read
 // of the columns; d->seen also COO_BAD_OFFSETS.  pieces: max_row_pieces(n) of
@@ -310,9 +320,12 @@ __device__ __forceinline__ void warp_row_walk(const int32_t* __restrict__ ro, in
   }
 }
 
-// Rows too long for one warp: listed in pieces of ROW_PIECE entries (x: row, y:
-// piece), which a second kernel takes by CTAs.  At most nnz / LONG_ROW + 1
-// pieces for valid offsets; what would not fit is dropped.
+// Groups of 32 rows with more than LONG_GROUP entries have too many for one warp.
+// Their rows of more than LONG_ROW: listed in pieces of ROW_PIECE entries (x: row, or
+// -1 for none, y: piece), which a second kernel takes by CTAs.  The list is
+// bounded (512 KB): rows beyond it stay with their warps, of which so many long
+// rows keep enough busy.
+constexpr int LONG_GROUP = 8192;
 constexpr int LONG_ROW = 512;
 constexpr int ROW_PIECE = 2048;
 struct RowPieces {
@@ -320,19 +333,35 @@ struct RowPieces {
   int32_t* count;  // zeroed
   int64_t limit;
 };
-inline int64_t max_row_pieces(int64_t nnz) { return nnz / LONG_ROW + 1; }
+inline int64_t max_row_pieces(int64_t nnz) {
+  const int64_t n = nnz / LONG_ROW + 1;
+  return n < 65536 ? n : 65536;
+}
 
-// The rows [r0, min(r0 + 32, nrows)) where one of them is long: lists the long
-// ones and calls f(in, q, e, first) for 32 entries e of a short row r0 + q at a
-// time (first: the row's first entry), every lane of the warp.  False, and
-// nothing done, where all are short.
+// The list (limit set) and its count, from sc.
+inline int row_pieces_alloc(RowPieces* p, Scratch& sc, cudaStream_t s) {
+  MGB_SCRATCH(sc, p->list, p->limit + 1);
+  p->count = reinterpret_cast<int32_t*>(p->list + p->limit);
+  MGB_CUDA_CHECK(cudaMemsetAsync(p->count, 0, sizeof(int32_t), s));
+  return MGB_SUCCESS;
+}
+
+// Asked before warp_rows_apart, which kernels call out of line: few groups need
+// it, and inlined it costs the others registers.
+__device__ __forceinline__ bool long_group(const int32_t* __restrict__ ro, int64_t r0, int64_t nrows) {
+  return (int64_t)ro[min(r0 + 32, nrows)] - ro[r0] > LONG_GROUP;
+}
+// The rows [r0, min(r0 + 32, nrows)) of a long group, where one of them is long:
+// lists the long ones and calls f(in, q, e, first) for 32 entries e of another
+// row r0 + q at a time (first: the row's first entry), every lane of the warp.
+// Otherwise false, and nothing is done.
 template <typename F>
 __device__ __forceinline__ bool warp_rows_apart(const int32_t* __restrict__ ro, int64_t r0, int64_t nrows,
                                                 RowPieces pieces, int lane, F f) {
   constexpr unsigned ALL = 0xffffffffu;
   const int32_t a = ro[min(r0 + lane, nrows)], z = ro[min(r0 + lane + 1, nrows)];
   const int64_t len = (int64_t)z - a;
-  const unsigned longs = __ballot_sync(ALL, len > LONG_ROW);
+  unsigned longs = __ballot_sync(ALL, len > LONG_ROW);
   if (!longs) return false;
   const int32_t np = len > LONG_ROW ? (int32_t)((len + ROW_PIECE - 1) / ROW_PIECE) : 0;
   int32_t upto = np;
@@ -341,16 +370,21 @@ __device__ __forceinline__ bool warp_rows_apart(const int32_t* __restrict__ ro, 
     const int32_t u = __shfl_up_sync(ALL, upto, d);
     if (lane >= d) upto += u;
   }
+  const int32_t total = __shfl_sync(ALL, upto, 31);
   int32_t base = 0;
-  if (lane == 31) base = atomicAdd(pieces.count, upto);
-  base = __shfl_sync(ALL, base, 31);
+  if (lane == 0) base = *reinterpret_cast<volatile int32_t*>(pieces.count) >= pieces.limit
+                            ? (int32_t)pieces.limit : atomicAdd(pieces.count, total);
+  base = __shfl_sync(ALL, base, 0);
+  if ((int64_t)base + total > pieces.limit) {  // full: the places left hold nothing
+    for (int64_t i = base + lane; i < pieces.limit; i += 32) pieces.list[i] = make_int2(-1, 0);
+    longs = 0;
+  }
   for (int q = 0; q < 32; q++) {
     const int64_t n = __shfl_sync(ALL, len, q);
     const int32_t first = __shfl_sync(ALL, a, q);
     if ((longs >> q) & 1) {
       const int32_t k = __shfl_sync(ALL, np, q), at = base + __shfl_sync(ALL, upto, q) - k;
-      for (int32_t i = lane; i < k; i += 32)
-        if ((int64_t)at + i < pieces.limit) pieces.list[at + i] = make_int2((int32_t)(r0 + q), i);
+      for (int32_t i = lane; i < k; i += 32) pieces.list[at + i] = make_int2((int32_t)(r0 + q), i);
     } else {
       for (int64_t j = 0; j < n; j += 32) f(j + lane < n, q, (int32_t)(first + j + lane), first);
     }
@@ -365,6 +399,7 @@ __device__ __forceinline__ void for_row_pieces(const int32_t* __restrict__ ro, R
   const int64_t n = min((int64_t)*pieces.count, pieces.limit);
   for (int64_t p = blockIdx.x; p < n; p += gridDim.x) {
     const int2 piece = pieces.list[p];
+    if (piece.x < 0) continue;
     const int32_t first = ro[piece.x], end = ro[piece.x + 1];
     const int64_t e0 = first + (int64_t)piece.y * ROW_PIECE, e1 = min(e0 + ROW_PIECE, (int64_t)end);
     for (int64_t e = e0 + threadIdx.x; e < e1; e += 256) f(piece.x, (int32_t)e, first);

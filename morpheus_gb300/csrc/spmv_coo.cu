@@ -215,7 +215,8 @@ int coo_segments(const mgb_coo* A, int64_t chunk, int64_t nchunks, const T* x, T
 
 // Adds the carries of each row in chunk order.  carry_row is non-decreasing.
 // The sum is one thread's, but sixteen carries are read at a time: a row of
-// 500,000 entries has 4,000 of them (one read after the other: 470 us).
+// 500,000 entries has 4,000 of them (the multiply of 2e6 entries with such a row
+// 590 us with one read after the other, 345 this way).
 template <typename T>
 __global__ void coo_carry_fixup(int64_t ncarry, int64_t nrows,
                                 const int32_t* __restrict__ cr,

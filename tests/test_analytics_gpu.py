@@ -120,8 +120,9 @@ def test_selector_choice_independent_of_active_format(cuda):
     _ = torch
 
 
-# rows that a warp leaves to other CTAs (more than 512 entries, pieces of 2,048) among short and empty ones
-@pytest.mark.parametrize("lens", [[513], [512, 2049, 0, 6], [5000] + [7] * 70 + [513]])
+# rows that a warp leaves to other CTAs (of 32 rows with more than 8,192 entries those with more than 512, in pieces of
+# 2,048) among short and empty ones
+@pytest.mark.parametrize("lens", [[513] * 40, [512, 4097, 0, 4096, 6], [6000, 5000] + [7] * 70 + [513]])
 def test_statistics_of_long_rows(cuda, lens):
     full = np.ones(6000, np.int64)
     full[100:100 + len(lens)] = lens

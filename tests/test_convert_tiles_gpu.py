@@ -109,10 +109,10 @@ def test_wide_slabs(cuda, N, lens, width, dtype):
         assert_same_matrix(got, ref, f"{fmt} width {w}:")
 
 
-# rows whose entries past the ELL width are one piece, one more, several pieces, the whole COO part
+# rows whose entries past the ELL width are at the limit of a warp's copy (4,096), several pieces, the whole COO part
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
-@pytest.mark.parametrize("lens,width", [([2048 + 5], 5), ([2049 + 5, 3], 5), ([1, 30000, 0, 9, 4101], 5), ([40960 + 1], 1),
-                                        ([6, 9, 4], 4)])
+@pytest.mark.parametrize("lens,width", [([4095 + 5], 5), ([4096 + 5, 3], 5), ([1, 30000, 0, 9, 4101], 5), ([40960 + 1], 1),
+                                        ([2040] * 3 + [4096] + [4097] * 2, 1), ([6, 9, 4], 4)])
 def test_hyb_long_rows(cuda, lens, width, dtype):
     A = gen.random_lengths_csr(len(lens), 50000, np.asarray(lens), seed=width, dtype=dtype)
     got, ref = both(gen.csr_to_coo_host(A), O.HYB, hyb_width=width)
@@ -128,11 +128,12 @@ def test_hdc_tiles(cuda, N, nd, keep, dtype):
     assert_same_matrix(got, ref)
 
 
-# rows with more entries off the diagonals than a warp walks or compacts itself (512; pieces of 2,048; 2,048 per 32
-# diagonals): first, last, neighbouring, beside short and empty rows
+# rows with more entries off the diagonals than a warp walks or compacts itself (512 or 4,096; pieces of 2,048; 2,048 per
+# 32 diagonals): first, last, neighbouring, beside short and empty rows
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 @pytest.mark.parametrize("nd", [1, 3, 40, 300])
-@pytest.mark.parametrize("rows,length", [([0], 513), ([5999], 6000), ([31, 32, 33], 2100), ([100, 101, 4000], 5000)])
+@pytest.mark.parametrize("rows,length", [([0], 513), ([5999], 6000), ([31, 32, 33], 2100), ([100, 101, 4000], 5000),
+                                         (list(range(64, 128)), 4096)])
 def test_hdc_long_rows(cuda, rows, length, nd, dtype):
     N = 6000
     rng = np.random.default_rng(nd + length)
@@ -309,14 +310,15 @@ def test_csr_without_row_indices(cuda, case, fmt, dtype):
     assert_same_matrix(mgb.matrix_to_host(dyn.active()), want)
 
 
-# rows that a warp leaves to other CTAs: at the length limit (512), at a piece's end (2,048) and past it, among short and
-# empty rows; two entries out of order or equal across a piece's border
+# rows that a warp leaves to other CTAs: 32 rows at the limit (8,192 entries) and past it, rows at the length limit (512),
+# at a piece's end (2,048) and past it, among short and empty rows; entries out of order or equal across a piece's border
 @pytest.mark.parametrize("fmt", [2, 3, 4, 5])
 @pytest.mark.parametrize("case", ["in_order", "unsorted", "repeated", "outside"])
-@pytest.mark.parametrize("lens", [[512], [513], [2, 2048, 2049, 0, 33], [5000] + [7] * 70 + [513]])
+@pytest.mark.parametrize("lens", [[8192], [8193], [512] * 15 + [513], [512] * 16 + [513] * 16,
+                                  [2, 4096, 4097, 0, 33], [8900] + [7] * 70 + [513]])
 def test_csr_long_rows(cuda, lens, case, fmt):
     import morpheus_gb300 as mgb
-    A = gen.random_lengths_csr(len(lens), 6000, np.asarray(lens), seed=fmt, dtype=np.float64)
+    A = gen.random_lengths_csr(len(lens), 9000, np.asarray(lens), seed=fmt, dtype=np.float64)
     cols, r = A["column_indices"].copy(), int(np.argmax(lens))
     b = A["row_offsets"][r] + (2048 if lens[r] > 2048 else lens[r] // 2)
     if case == "unsorted":
@@ -324,7 +326,7 @@ def test_csr_long_rows(cuda, lens, case, fmt):
     elif case == "repeated":
         cols[b] = cols[b - 1]
     elif case == "outside":
-        cols[A["row_offsets"][r + 1] - 1] = 6000
+        cols[A["row_offsets"][r + 1] - 1] = 9000
     A["column_indices"] = cols
     dyn = mgb.DynamicMatrix(mgb.matrix_from_host(A))
     status = mgb.convert(dyn, fmt)
