@@ -213,36 +213,53 @@ int coo_segments(const mgb_coo* A, int64_t chunk, int64_t nchunks, const T* x, T
   return launch_segments<T, int64_t, 8, 60>(A, chunk, nchunks, x, y, init, cr, cv, s);
 }
 
-// Adds the carries of each row in chunk order.  carry_row is non-decreasing.
-// The sum is one thread's, but sixteen carries are read at a time: a row of
-// 500,000 entries has 4,000 of them (the multiply of 2e6 entries with such a row
-// 590 us with one read after the other, 345 this way).
+// Adds the carries of each row.  carry_row is non-decreasing.  A thread adds the
+// few carries of most rows in chunk order; a row of many (5e6 entries: 39,000) is
+// added by the CTA that its first one falls to, in an order that the matrix alone
+// fixes.  One thread for all of them: the multiply of 2e7 entries with such a row
+// 3,390 us, with a CTA 264.
+constexpr int FIXUP_FEW = 32;
 template <typename T>
-__global__ void coo_carry_fixup(int64_t ncarry, int64_t nrows,
-                                const int32_t* __restrict__ cr,
-                                const T* __restrict__ cv, T* __restrict__ y,
-                                int init) {
-  constexpr int U = 16;
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= ncarry) return;
-  const int32_t r = cr[i];
-  if (i > 0 && cr[i - 1] == r) return;
-  T s = cv[i];
-  bool more = i + 1 < ncarry && cr[i + 1] == r;
-  for (int64_t j = i + 1; more; j += U) {
-    T v[U];
-    bool in[U];
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      in[u] = j + u < ncarry && cr[j + u] == r;
-      v[u] = j + u < ncarry ? cv[j + u] : T(0);
+__global__ void __launch_bounds__(256) coo_carry_fixup(int64_t ncarry, int64_t nrows,
+                                                       const int32_t* __restrict__ cr, const T* __restrict__ cv,
+                                                       T* __restrict__ y, int init) {
+  __shared__ int64_t s_head[256 / FIXUP_FEW + 1];  // heads of many are more than FIXUP_FEW apart
+  __shared__ T s_part[8];
+  __shared__ int s_heads;
+  if (threadIdx.x == 0) s_heads = 0;
+  __syncthreads();
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  const int32_t r = i < ncarry ? cr[i] : -1;
+  if (i < ncarry && (i == 0 || cr[i - 1] != r)) {
+    if (i + FIXUP_FEW < ncarry && cr[i + FIXUP_FEW] == r) {
+      s_head[atomicAdd(&s_heads, 1)] = i;
+    } else {
+      T s = T(0);
+      for (int64_t j = i; j < ncarry && cr[j] == r; j++) s += cv[j];
+      if (r >= 0 && r < nrows) y[r] = init ? s : y[r] + s;
     }
-#pragma unroll
-    for (int u = 0; u < U; u++)
-      if (in[u]) s += v[u];
-    more = in[U - 1];
   }
-  if (r >= 0 && r < nrows) y[r] = init ? s : y[r] + s;
+  __syncthreads();
+  for (int k = 0; k < s_heads; k++) {
+    const int64_t head = s_head[k];
+    const int32_t row = cr[head];
+    int64_t end = ncarry;  // the first carry of another row
+    for (int64_t lo = head + FIXUP_FEW + 1; lo < end;) {
+      const int64_t mid = (lo + end) >> 1;
+      if (cr[mid] == row) lo = mid + 1; else end = mid;
+    }
+    T s = T(0);
+#pragma unroll 8
+    for (int64_t j = head + threadIdx.x; j < end; j += 256) s += cv[j];
+    s = warp_sum(s);
+    if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0 && row >= 0 && row < nrows) {
+      for (int w = 1; w < 8; w++) s += s_part[w];
+      y[row] = init ? s : y[row] + s;
+    }
+    __syncthreads();  // the next row's parts
+  }
 }
 
 }  // namespace

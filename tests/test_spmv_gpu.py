@@ -538,7 +538,8 @@ def test_coo_staging_by_size(cuda, nnz, init):
 # a row of many chunks: more carries than are read at a time, at their border, alone and between others
 @pytest.mark.parametrize("init", [True, False])
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
-@pytest.mark.parametrize("lens", [[40000], [3, 2048 + 17, 1], [5] * 300 + [30000, 0, 4400] + [2] * 50])
+@pytest.mark.parametrize("lens", [[40000], [3, 2048 + 17, 1], [5] * 300 + [30000, 0, 4400] + [2] * 50,
+                                  [256 * 15 + 1, 256 * 16 - 1, 256 * 16, 256 * 16 + 1, 256 * 17] * 4])
 def test_coo_long_row_carries(cuda, lens, dtype, init):
     A = gen.csr_to_coo_host(gen.random_lengths_csr(len(lens), 50000, np.asarray(lens), seed=len(lens), dtype=dtype))
     x, y0 = gen.x_vector(50000, seed=3, dtype=dtype), gen.x_vector(len(lens), seed=4, dtype=dtype)
@@ -547,6 +548,6 @@ def test_coo_long_row_carries(cuda, lens, dtype, init):
     prod = A["values"].astype(np.float64) * x.astype(np.float64)[A["column_indices"]]
     want = np.bincount(A["row_indices"], weights=prod, minlength=len(lens)) + (0.0 if init else y0.astype(np.float64))
     size = np.bincount(A["row_indices"], weights=np.abs(prod), minlength=len(lens)) + np.abs(y0)
-    # a lane adds at most 64 products, a warp 32 lanes' sums, the carries one after the other (two per 256 entries)
+    # a lane adds at most 64 products, a warp 32 lanes' sums, and the carries (two per 256 entries) at most one by one
     bound = (64 + 32 + 2 * max(lens) / 256 + 2) * np.finfo(dtype).eps * size
     assert np.all(np.abs(y.cpu().numpy() - want) <= bound)
