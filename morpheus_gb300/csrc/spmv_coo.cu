@@ -8,7 +8,7 @@
 // Serial multiply (impl/Coo/Serial/Morpheus_Multiply_Impl.hpp:38-59):
 // y = 0 if init, then y[I[n]] += V[n] * x[J[n]].
 //
-// Design: fixed chunks of COO_CHUNK consecutive entries, one warp each, cut
+// Design: fixed chunks of up to COO_CHUNK consecutive entries, one warp each, cut
 // into 32 contiguous lane ranges (the lane-segment scheme of spmv_csr.cu, so
 // every FP64 FMA is issued by all 32 lanes).  Row indices, columns and values
 // are copied into padded shared memory a step ahead (cp.async, two buffers); a lane
@@ -26,19 +26,25 @@ namespace {
 
 constexpr int COO_WARPS = 4;
 constexpr int COO_CTAS = 5;                 // register budget per SM (shared memory allows 2 to 4)
-constexpr int64_t COO_CHUNK = 2048;         // entries per warp chunk (largest)
+constexpr int64_t COO_CHUNK = 2048;         // entries per warp chunk at most
 
-// 2048 entries per chunk, halved (down to 256) while the matrix would give
-// fewer than three chunks per resident warp (12 of FP64, 16 of FP32 per SM; two
-// left the last wave nearly empty at some sizes, smaller chunks pay more
-// carries).  Power-law matrices of 350,000 / 700,000 rows, us at two -> three:
-// FP64 49.5 -> 47.6 / 93.3 -> 88.8, FP32 43.1 -> 39.1 / 76.8 -> 77.3; COO part of
-// the HYB of 1.5 / 2.0 M rows with its ELL part: FP64 220.9 -> 214.6 / 287.8 -> 287.9,
-// FP32 159.1 -> 157.9 / 212.5 -> 205.1; five: FP64 219 / 286, FP32 160 / 205.
+// Entries per chunk.  FP64: 256 below COO_SHORT (steps of four entries, 16 warps
+// per SM), 512 from there on.  Larger chunks leave the last wave nearly empty at
+// some sizes; smaller ones pay carries.  Power-law COO of 350,000 / 700,000 / 1.0 M
+// / 1.6 M rows (5.3 to 24 M entries), us at 256: 43.1 / 77.8 / 101.5 / 153.5, 512: 45.1
+// / 80.2 / 107.1 / 160.2, 1024: 50.9 / 88.7, 2048: 51.8 / 90.0.  From COO_SHORT on (steps
+// of eight), 2.0 M rows and 27-point stencils on 100^3 and 160^3: 256: 231 / 189 / 758,
+// 512: 209 / 145 / 554, 1024: 220 / 160, 2048: 214 / 166 / 607.
+// FP32: 2048, halved (down to 256) while there are fewer than three chunks per
+// resident warp (16 per SM).  350,000 / 700,000 rows, us at two -> three: 43.1 -> 39.1 /
+// 76.8 -> 77.3; COO part of the HYB of 1.5 / 2.0 M rows with its ELL part: 159.1 ->
+// 157.9 / 212.5 -> 205.1; five: 160 / 205.
+constexpr int64_t COO_SHORT = 24 << 20;
 template <typename T>
 inline int64_t coo_chunk_size(int64_t nnz) {
+  if (sizeof(T) == 8) return nnz < COO_SHORT ? 256 : 512;
   int64_t chunk = COO_CHUNK;
-  const int64_t enough = (int64_t)num_sms() * (sizeof(T) == 8 ? 36 : 48);
+  const int64_t enough = (int64_t)num_sms() * 48;
   while (chunk > 256 && nnz / chunk < enough) chunk >>= 1;
   return chunk;
 }
@@ -184,12 +190,11 @@ spmv_coo_segments(int64_t nrows, int64_t ncols, int64_t nnz, int64_t chunk, cons
 // 45: 226 / 194, 60 and 70: 213 / 186 (12 / 16 warps per SM).
 // FP64 of fewer than COO_SHORT entries: four entries per step, so that a
 // carve-out of 45 % holds 16 warps and leaves L1 more lines.  Steps of eight at
-// 60 % -> four at 45 % (single staging), us: COO of 1.8 M entries 25.9 -> 22.6
-// (24.6), 5.3 M 48.8 -> 45.1 (48.5), 10.6 M 89.3 -> 88.4 (86.3), 15.2 M 121.7 ->
-// 126.5 (122.2), 30.4 M 214 -> 223 (222); HYB with a COO part of 4 M entries
-// 176.0 -> 171.5 (173.0), of 8 M 290.4 -> 283.5 (278.3).
-constexpr int64_t COO_SHORT = 12 << 20;
-
+// 60 % / four at 45 % (single staging before), us, each with its chunks: power-law
+// COO of 7.6 M entries 65.6 / 61.1 (76.8), 12 M 94.1 / 85.3 (91.2), 13.7 M 103.1 / 93.8
+// (100.7), 15 M 112.8 / 101.5 (122.4), 24 M 171.4 / 153.5 (176.3), 30 M 209.4 / 231.4
+// (220.8); 5-point rows, 20 M 132.4 / 120.9 (158.7), 27-point, 26 M 145.1 / 189.4 (164.7);
+// HYB with a COO part of 8 M entries 288 / 278 (277 to 279).
 template <typename T, typename IDX, int SEG, int PERCENT>
 int launch_segments(const mgb_coo* A, int64_t chunk, int64_t nchunks, const T* x, T* y, int init, int32_t* cr, T* cv,
                     cudaStream_t s) {
@@ -328,8 +333,9 @@ int mgb_spmv_coo_f32(const mgb_coo* A, const float* x, float* y, int init, void*
 // Limits and rules:
 //  * The array is COO_NOALLOC_BYTES (4 MiB) of device memory that every GPU
 //    which loads this library holds until the process exits.  It holds two
-//    carries (int32 row + double value) per 2048-entry chunk, so A->nnz may be
-//    at most 357,892,096; larger matrices get MGB_ERR_INVALID_INPUT before any
+//    carries (int32 row + double value) per chunk of up to 2048 entries (chunks
+//    grow with the matrix until their carries fit), so A->nnz may be at most
+//    357,892,096; larger matrices get MGB_ERR_INVALID_INPUT before any
 //    work is queued.
 //  * The first call on a device looks up the array's device address with
 //    cudaGetSymbolAddress (once per device, with that device current) and
@@ -387,11 +393,15 @@ int noalloc_scratch(void** out) {
 int launch_coo_noalloc_f64(const mgb_coo* A, const double* x, double* y, int init, cudaStream_t s) {
   MGB_REQUIRE(A != nullptr, MGB_ERR_BAD_ARGUMENT);
   MGB_REQUIRE(!bad_sizes(A->nrows, A->ncols, A->nnz), MGB_ERR_BAD_ARGUMENT);
-  const int64_t chunk = coo_chunk_size<double>(A->nnz);
-  const int64_t nchunks = (A->nnz + chunk - 1) / chunk;
-  const int64_t ncarry = 2 * nchunks;
-  const size_t rows_bytes = ((sizeof(int32_t) * (size_t)ncarry + 255) / 256) * 256;
-  MGB_REQUIRE(rows_bytes + sizeof(double) * (size_t)ncarry <= COO_NOALLOC_BYTES, MGB_ERR_INVALID_INPUT);
+  int64_t chunk = coo_chunk_size<double>(A->nnz), nchunks, ncarry;
+  size_t rows_bytes;
+  for (;; chunk <<= 1) {  // chunks as large as the array needs them, up to COO_CHUNK
+    nchunks = (A->nnz + chunk - 1) / chunk;
+    ncarry = 2 * nchunks;
+    rows_bytes = ((sizeof(int32_t) * (size_t)ncarry + 255) / 256) * 256;
+    if (rows_bytes + sizeof(double) * (size_t)ncarry <= COO_NOALLOC_BYTES) break;
+    MGB_REQUIRE(chunk < COO_CHUNK, MGB_ERR_INVALID_INPUT);
+  }
   MGB_REQUIRE(A->nrows < ((int64_t)1 << 31), MGB_ERR_INVALID_INPUT);
   if (A->nrows == 0) return MGB_SUCCESS;
   MGB_REQUIRE(y != nullptr, MGB_ERR_BAD_ARGUMENT);

@@ -551,3 +551,25 @@ def test_coo_long_row_carries(cuda, lens, dtype, init):
     # a lane adds at most 64 products, a warp 32 lanes' sums, and the carries (two per 256 entries) at most one by one
     bound = (64 + 32 + 2 * max(lens) / 256 + 2) * np.finfo(dtype).eps * size
     assert np.all(np.abs(y.cpu().numpy() - want) <= bound)
+
+
+# both sides of the entry count from which FP64 takes longer steps and chunks, and beyond what the allocation-free entry
+# point's carries allow for those chunks
+@pytest.mark.parametrize("nnz", [(24 << 20) - 1, 24 << 20, 90_000_000])
+def test_coo_chunk_limits(cuda, nnz):
+    import ctypes as C
+
+    from morpheus_gb300 import _lib
+    N, dev = nnz // 5 + 1, torch.device("cuda")
+    rows = (torch.arange(nnz, device=dev, dtype=torch.int64) // 5).int()
+    cols = (torch.arange(nnz, device=dev, dtype=torch.int64) * 7919 % 1009).int()
+    vals = torch.ones(nnz, dtype=torch.float64, device=dev)
+    x = torch.arange(1009, device=dev, dtype=torch.float64) - 500  # integers: every sum is exact
+    want = torch.zeros(N, dtype=torch.float64, device=dev).index_add_(0, rows, x[cols.long()])
+    A = mgb.CooMatrix(N, 1009, nnz, rows, cols, vals)
+    desc = A._desc()
+    for name in ("mgb_spmv_coo_f64", "mgb_spmv_coo_f64_noalloc"):
+        y = torch.full((N,), 3.0, dtype=torch.float64, device=dev)
+        _lib.call(name, C.byref(desc), x.data_ptr(), y.data_ptr(), 1, None)
+        torch.cuda.synchronize()
+        assert torch.equal(y, want), name
