@@ -502,8 +502,8 @@ bool hdc_tiled(int64_t nd) {
   return (nd + D - 1) / D <= HDC_TILE_GROUPS;
 }
 
-// Argument checks of a COO source (the index range checks are queued with
-// validate_async and read with the caller's other words).
+// Argument checks of a COO source (the index pass checks the index ranges, read
+// back with the caller's other words).
 int check_coo_args(const mgb_coo* src, bool diagonals = true) {
   MGB_REQUIRE(src != nullptr, MGB_ERR_BAD_ARGUMENT);
   MGB_REQUIRE(src->nrows >= 0 && src->ncols >= 0 && src->nnz >= 0, MGB_ERR_BAD_ARGUMENT);

@@ -182,7 +182,7 @@ spmv_csr_rowtile(int64_t nrows, int64_t ncols, const int32_t* __restrict__ ro, c
 // uncoalesced loads of a warp hit the same L1 lines over the U entries that
 // are read together, no staging comes between the row offsets and the x reads
 // (three memory latencies per row instead of four, and no waits for copies),
-// and 48 to 64 warps fit an SM.  What bounds it is L1's line lookups, so longer
+// and 40 to 64 warps fit an SM.  What bounds it is L1's line lookups, so longer
 // rows go to the staged tiles: direct_kernel.  The sums run in row order as there.
 constexpr int DIRECT_THREADS = 128;
 
@@ -364,8 +364,6 @@ int launch_rows_cfg(const mgb_csr* A, const T* x, T* y, int init, cudaStream_t s
 // 180 KB in FP64, 215 KB in FP32 -- the 27-point stencil in FP32, 896 x 6:
 // 185.0 us, 896 x 7: 172.5 us; 135 KB for scattered columns: L1 for the
 // misses in flight), at most 12.  Measured on GB300 (us per SpMV, FP64, TILE x CTAs):
-//   5-point Laplacian 2048^2:      224 x 12  69.6
-//   band of 13, N = 2M:            448 x 10  78.5   448 x 8  71.7
 //   27-point stencil 160^3:        896 x 5  342.8   896 x 4  319.7   896 x 3  388.7
 //   scattered, 12 per row, N = 2M: 448 x 10 213.4   224 x 10 108.6   448 x 6 109.7
 //   scattered, 20 per row:         896 x 5  263.3   224 x 10 160.2   896 x 3 147.5
@@ -379,7 +377,9 @@ constexpr int rows_ctas(int tile, bool gather) {
 
 // Staging size: the smallest of 224 / 448 / 896 entries that holds a tile of
 // 32 rows of the mean length (longer tiles are processed in pieces, so this
-// is a performance choice only).  Returns the CTAs per SM of the choice.
+// is a performance choice only); rows with neighbouring columns that are short
+// enough for less than 896 take the direct kernel.  Returns the CTAs per SM of
+// the choice.
 template <typename T>
 int rows_config(const mgb_csr* A, bool gather, int* tile) {
   const int64_t tile_entries = 32 * (A->nnz / (A->nrows > 0 ? A->nrows : 1)) + 8;
@@ -390,15 +390,13 @@ int rows_config(const mgb_csr* A, bool gather, int* tile) {
 template <typename T, bool DOT>
 int launch_rows_variant(const mgb_csr* A, const T* x, T* y, int init, cudaStream_t s, T* partials,
                         unsigned blocks, bool gather) {
-  int tile = 0;
-  rows_config<T>(A, gather, &tile);
   if (gather) {
+    int tile = 0;
+    rows_config<T>(A, true, &tile);
     if (tile == 224) return launch_rows_cfg<T, DOT, 224, rows_ctas<T>(224, true)>(A, x, y, init, s, partials, blocks);
     if (tile == 448) return launch_rows_cfg<T, DOT, 448, rows_ctas<T>(448, true)>(A, x, y, init, s, partials, blocks);
     return launch_rows_cfg<T, DOT, 896, rows_ctas<T>(896, true)>(A, x, y, init, s, partials, blocks);
   }
-  if (tile == 224) return launch_rows_cfg<T, DOT, 224, rows_ctas<T>(224, false)>(A, x, y, init, s, partials, blocks);
-  if (tile == 448) return launch_rows_cfg<T, DOT, 448, rows_ctas<T>(448, false)>(A, x, y, init, s, partials, blocks);
   return launch_rows_cfg<T, DOT, 896, rows_ctas<T>(896, false)>(A, x, y, init, s, partials, blocks);
 }
 

@@ -182,8 +182,14 @@ int launch_dia_rows(const mgb_dia* D, const mgb_csr* C, const T* x, T* y, int in
                                                     vals, cro, cci, cva, cnnz, x, y, init);
   };
   if constexpr (sizeof(T) == 8) {
-    if (rpt == 1) run(spmv_dia_rows<T, 1, HDC, 3, 8>);
-    else run(spmv_dia_rows<T, V, HDC, 2, 8>);
+    if constexpr (HDC) {
+      if (rpt != 1) {
+        run(spmv_dia_rows<T, V, true, 2, 8>);
+        MGB_LAUNCH_CHECK();
+        return MGB_SUCCESS;
+      }
+    }
+    run(spmv_dia_rows<T, 1, HDC, 3, 8>);
   } else {
     if (rpt == 1) run(spmv_dia_rows<T, 1, HDC, 1, 0>);
     else run(spmv_dia_rows<T, V, HDC, 1, 0>);

@@ -195,7 +195,6 @@ int launch_ell(const mgb_ell* A, const T* x, T* y, int init, cudaStream_t s) {
       if (vec4) return launch_ell_rows<T, 4, 0>(A, x, y, init, s);
       if (vec2) return launch_ell_rows<T, 2, 0>(A, x, y, init, s);
     }
-    if (ctas > 0x7fffffffLL) return launch_ell_rows<T, 1, 0>(A, x, y, init, s);
     spmv_ell_pairs<T, 2><<<(unsigned)ctas, ELL_PAIR_THREADS, 0, s>>>(A->nrows, A->ncols, A->width, A->pitch,
                                                                      A->column_indices,
                                                                      static_cast<const T*>(A->values), x, y, init);
