@@ -40,10 +40,39 @@ __device__ __forceinline__ int64_t warp_lower_bound(const int32_t* __restrict__ 
 // Shared-memory staging of one warp (RO: row offsets staged per chunk).
 template <typename T, int SEG, int RO = CSR_RO_STAGE>
 struct WarpStage {
+  static constexpr bool PIPE = false;
   T val[32 * (SEG + 1)];
   int32_t col[32 * (SEG + 1)];
   int32_t ro[RO];
 };
+
+// Double-buffered staging: step s + 1 is copied (cp.async) while step s's x
+// reads are in flight.  Two buffers per warp leave room for fewer warps, but
+// each of them always has loads in flight.  What matters as much is the L1
+// beside the buffers (the x misses in flight live in its lines): PIPE_CARVEOUT.
+template <typename T, int SEG, int RO>
+struct PipeStage {
+  static constexpr bool PIPE = true;
+  T val[2][32 * (SEG + 1)];
+  int32_t col[2][32 * (SEG + 1)];
+  int32_t ro[RO];
+};
+
+constexpr int PIPE_WARPS = 4;  // warps per CTA
+constexpr int PIPE_CTAS = 5;   // the register budget of 5 CTAs per SM
+constexpr int PIPE_RO = 256;   // row offsets staged per warp
+// Shared memory carve-out in percent (power-law matrix, 2e6 rows, FP64 / FP32):
+// 100: 369 / 318 us, 75: 217 / 187, 60: 193 / 167, 45: 191 / 161 (12 / 16 warps
+// per SM), 35: 198 / 167, 25: 239 / 207.
+constexpr int PIPE_CARVEOUT = 45;
+
+// dst = in ? *src : 0 in shared memory, asynchronously
+template <typename V>
+__device__ __forceinline__ void copy_or_zero(V* dst, const V* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src), "n"(sizeof(V)), "r"(in ? (int)sizeof(V) : 0)
+               : "memory");
+}
 
 // Rows [begin, end) of one warp chunk.
 struct RowRange {
@@ -97,15 +126,15 @@ __device__ __forceinline__ RowRange planned_rows(int64_t wc, int64_t nrows, cons
 // offsets, as the reference's kernels do.
 // IDX: the type of entry and row indices inside the routine (int32_t is
 // exact when nnz < 2^31 - 4096, as the launchers require, and nrows < 2^31 -
-// 32); RO: row offsets staged per chunk.
-template <typename T, int SEG, typename XL, bool BOUNDED = true, typename IDX = int64_t, int RO = CSR_RO_STAGE>
+// 32); RO: row offsets staged per chunk; STAGE: WarpStage (entries loaded and
+// stored a step at a time) or PipeStage (the next step's copied meanwhile).
+template <typename T, int SEG, typename XL, bool BOUNDED = true, typename IDX = int64_t, int RO = CSR_RO_STAGE,
+          typename STAGE = WarpStage<T, SEG, RO>>
 __device__ __forceinline__ RowRange csr_rows_x(RowRange rows, int64_t nrows, int64_t ncols,
                                                const int32_t* __restrict__ ro, const int32_t* __restrict__ ci,
                                                const T* __restrict__ va, XL xl, T* __restrict__ y, int init,
-                                               WarpStage<T, SEG, RO>& stg, int lane) {
+                                               STAGE& stg, int lane) {
   constexpr int CSR_PAD = SEG + 1;
-  T* sv = stg.val;
-  int32_t* sc = stg.col;
   int32_t* sro = stg.ro;
   const IDX r_begin = (IDX)rows.begin, r_end = (IDX)rows.end;
   if (r_begin >= r_end) return RowRange{r_begin, r_begin};
@@ -154,16 +183,43 @@ __device__ __forceinline__ RowRange csr_rows_x(RowRange rows, int64_t nrows, int
   IDX hrow = -1;
   T hval = T(0);
 
-  for (IDX s = 0; s < KW; s += SEG) {
-    __syncwarp();
+  // entries s..s + SEG of every lane range
+  auto stage = [&](IDX s, T* sv, int32_t* sc) {
 #pragma unroll
     for (int q = 0; q < SEG; q++) {
       const int f = q * 32 + lane;
       const int L = f / SEG, j = f % SEG;
       const IDX e = A0 + L * KW + s + j;
       const bool in = e >= E0 && e < E1;
-      sv[L * CSR_PAD + j] = in ? ldg_stream(va + e) : T(0);
-      sc[L * CSR_PAD + j] = in ? ldg_stream(ci + e) : 0;
+      if constexpr (STAGE::PIPE) {
+        copy_or_zero(sv + L * CSR_PAD + j, va + (in ? e : E0), in);
+        copy_or_zero(sc + L * CSR_PAD + j, ci + (in ? e : E0), in);
+      } else {
+        sv[L * CSR_PAD + j] = in ? ldg_stream(va + e) : T(0);
+        sc[L * CSR_PAD + j] = in ? ldg_stream(ci + e) : 0;
+      }
+    }
+  };
+  // nothing is copied past the end: no copy is under way when the buffers are next used
+  auto copy_ahead = [&](IDX s, int b) {
+    if constexpr (STAGE::PIPE) {
+      if (s < KW) stage(s, stg.val[b], stg.col[b]);
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+  };
+  copy_ahead(0, 0);
+  int buf = 0;
+  for (IDX s = 0; s < KW; s += SEG, buf ^= 1) {
+    __syncwarp();  // the reads of the buffer filled next are done
+    const T* sv;
+    const int32_t* sc;
+    if constexpr (STAGE::PIPE) {
+      copy_ahead(s + SEG, buf ^ 1);
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+      sv = stg.val[buf], sc = stg.col[buf];
+    } else {
+      stage(s, stg.val, stg.col);
+      sv = stg.val, sc = stg.col;
     }
     __syncwarp();
     T v[SEG], xv[SEG];
@@ -173,166 +229,6 @@ __device__ __forceinline__ RowRange csr_rows_x(RowRange rows, int64_t nrows, int
       const bool valid = e >= e_lo && e < lb;
       const int32_t c = sc[lane * CSR_PAD + k];
       v[k] = valid ? sv[lane * CSR_PAD + k] : T(0);
-      xv[k] = (valid && (uint64_t)(int64_t)c < (uint64_t)ncols) ? xl(c) : T(0);
-    }
-#pragma unroll
-    for (int k = 0; k < SEG; k++) {
-      const IDX e = la + s + k;
-      const bool valid = e >= e_lo && e < lb;
-      while (valid && e >= re && (!BOUNDED || r + 1 < r_end)) {
-        if (rs >= e_lo) { y[r] = acc; } else { hrow = r; hval = acc; }
-        r++;
-        rs = re;
-        re = ro_at(r + 1);
-        acc = init ? T(0) : y[r];
-      }
-      acc = fmadd(v[k], xv[k], acc);
-    }
-  }
-  // rows ending exactly at the lane end (and empty rows sitting there)
-  if (active) {
-    while (r < r_end && re <= lb) {
-      if (rs >= e_lo) { y[r] = acc; } else { hrow = r; hval = acc; }
-      r++;
-      if (r < r_end) {
-        rs = re;
-        re = ro_at(r + 1);
-        acc = init ? T(0) : y[r];  // empty rows at lb are flushed here
-      }
-    }
-  }
-  // tail partial (a row that started in this lane's range and continues into
-  // the next lane; a row starting exactly at lb belongs to the next lane)
-  // and segmented scan
-  const bool has_tail = active && r < r_end && rs < lb;
-  const IDX key = has_tail ? r : -1 - (IDX)lane;
-  T cv = has_tail ? acc : T(0);
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const T u = __shfl_up_sync(0xffffffffu, cv, d);
-    const IDX k2 = __shfl_up_sync(0xffffffffu, key, d);
-    if (lane >= d && k2 == key) cv += u;
-  }
-  const T vprev = __shfl_up_sync(0xffffffffu, cv, 1);
-  const IDX kprev = __shfl_up_sync(0xffffffffu, key, 1);
-  if (hrow >= 0) y[hrow] = (lane > 0 && kprev == hrow) ? hval + vprev : hval;
-  return RowRange{r_begin, r_end};
-}
-
-// Double-buffered staging: step s + 1 is copied (cp.async) while step s's x
-// reads are in flight.  Two buffers per warp leave room for fewer warps, but
-// each of them always has loads in flight.  What matters as much is the L1
-// beside the buffers (the x misses in flight live in its lines): PIPE_CARVEOUT.
-template <typename T, int SEG, int RO>
-struct PipeStage {
-  T val[2][32 * (SEG + 1)];
-  int32_t col[2][32 * (SEG + 1)];
-  int32_t ro[RO];
-};
-
-constexpr int PIPE_WARPS = 4;  // warps per CTA
-constexpr int PIPE_CTAS = 5;   // the register budget of 5 CTAs per SM
-constexpr int PIPE_RO = 256;   // row offsets staged per warp
-// Shared memory carve-out in percent (power-law matrix, 2e6 rows, FP64 / FP32):
-// 100: 369 / 318 us, 75: 217 / 187, 60: 193 / 167, 45: 191 / 161 (12 / 16 warps
-// per SM), 35: 198 / 167, 25: 239 / 207.
-constexpr int PIPE_CARVEOUT = 45;
-
-// dst = in ? *src : 0 in shared memory, asynchronously
-template <typename V>
-__device__ __forceinline__ void copy_or_zero(V* dst, const V* src, bool in) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-               "l"(src), "n"(sizeof(V)), "r"(in ? (int)sizeof(V) : 0)
-               : "memory");
-}
-
-// csr_rows_x with that staging.
-template <typename T, int SEG, typename XL, bool BOUNDED = true, typename IDX = int64_t, int RO = CSR_RO_STAGE>
-__device__ __forceinline__ RowRange csr_rows_pipe(RowRange rows, int64_t nrows, int64_t ncols,
-                                               const int32_t* __restrict__ ro, const int32_t* __restrict__ ci,
-                                               const T* __restrict__ va, XL xl, T* __restrict__ y, int init,
-                                               PipeStage<T, SEG, RO>& stg, int lane) {
-  int32_t* sro = stg.ro;
-  constexpr int CSR_PAD = SEG + 1;
-  const IDX r_begin = (IDX)rows.begin, r_end = (IDX)rows.end;
-  if (r_begin >= r_end) return RowRange{r_begin, r_begin};
-  const IDX nr = r_end - r_begin;
-  const bool staged = nr < RO;  // offsets r_begin..r_end in smem
-  __syncwarp();
-  if (staged)
-    for (IDX i = lane; i <= nr; i += 32) sro[i] = __ldg(ro + r_begin + i);
-  __syncwarp();
-  auto ro_at = [&](IDX i) -> IDX {
-    return staged ? (IDX)sro[i - r_begin] : (IDX)__ldg(ro + i);
-  };
-  const IDX E0 = ro_at(r_begin), E1 = ro_at(r_end);
-  if (E0 >= E1) {  // only empty rows
-    if (init)
-      for (IDX r = r_begin + lane; r < r_end; r += 32) y[r] = T(0);
-    return RowRange{r_begin, r_end};
-  }
-  const IDX A0 = E0 & ~(IDX)7;  // 32-byte aligned column segments
-  IDX KW = (E1 - A0 + 31) / 32;
-  KW = (KW + SEG - 1) / SEG * SEG;
-  const IDX la = A0 + lane * KW;
-  const IDX lb = min(la + KW, E1);
-  const IDX e_lo = max(la, E0);
-  const bool active = e_lo < lb;
-
-  // lane's first row: lane 0 starts at r_begin (so leading empty rows are
-  // flushed); others at the row containing e_lo (empty rows sitting at a
-  // lane boundary are flushed by the previous lane's tail loop).
-  IDX r = r_end;
-  if (active) {
-    if (lane == 0) {
-      r = r_begin;
-    } else {
-      IDX lo = r_begin, hi = r_end;  // first i in [lo, hi] with ro[i] > e_lo
-      while (lo < hi) {
-        const IDX mid = lo + ((hi - lo) >> 1);  // lo + hi may pass 2^31
-        if (ro_at(mid) <= e_lo) lo = mid + 1; else hi = mid;
-      }
-      r = lo - 1;
-    }
-  }
-  IDX rs = active ? ro_at(r) : 0;
-  IDX re = active ? ro_at(r + 1) : 0;
-  T acc = (active && rs >= e_lo && !init) ? y[r] : T(0);
-  IDX hrow = -1;
-  T hval = T(0);
-
-  auto stage = [&](IDX s, int buf) {
-    if (s < KW) {  // nothing is copied past the end: no copy is under way when the buffers are next used
-      T* sv = stg.val[buf];
-      int32_t* sc = stg.col[buf];
-#pragma unroll
-      for (int q = 0; q < SEG; q++) {
-        const int f = q * 32 + lane;
-        const int L = f / SEG, j = f % SEG;
-        const IDX e = A0 + L * KW + s + j;
-        const bool in = e >= E0 && e < E1;
-        copy_or_zero(sv + L * CSR_PAD + j, va + (in ? e : E0), in);
-        copy_or_zero(sc + L * CSR_PAD + j, ci + (in ? e : E0), in);
-      }
-    }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-  };
-  stage(0, 0);
-  int buf = 0;
-  for (IDX s = 0; s < KW; s += SEG, buf ^= 1) {
-    __syncwarp();  // the reads of the buffer filled next are done
-    stage(s + SEG, buf ^ 1);
-    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-    __syncwarp();
-    const T* sv = stg.val[buf] + lane * CSR_PAD;
-    const int32_t* sc = stg.col[buf] + lane * CSR_PAD;
-    T v[SEG], xv[SEG];
-#pragma unroll
-    for (int k = 0; k < SEG; k++) {
-      const IDX e = la + s + k;
-      const bool valid = e >= e_lo && e < lb;
-      const int32_t c = sc[k];
-      v[k] = valid ? sv[k] : T(0);
       xv[k] = (valid && (uint64_t)(int64_t)c < (uint64_t)ncols) ? xl(c) : T(0);
     }
 #pragma unroll
@@ -419,9 +315,8 @@ __device__ __forceinline__ RowRange csr_chunk(int64_t wc, int64_t nrows, int64_t
                                               const T* __restrict__ va, const T* __restrict__ x,
                                               T* __restrict__ y, int init, PipeStage<T, SEG, PIPE_RO>& stg,
                                               int lane) {
-  return csr_rows_pipe<T, SEG, XGlobal<T>, false, int32_t, PIPE_RO>(chunk_rows(wc, CHUNK, nrows, ro, lane), nrows,
-                                                                    ncols, ro, ci, va, XGlobal<T>{x}, y, init, stg,
-                                                                    lane);
+  return csr_rows_x<T, SEG, XGlobal<T>, false, int32_t, PIPE_RO>(chunk_rows(wc, CHUNK, nrows, ro, lane), nrows, ncols,
+                                                                 ro, ci, va, XGlobal<T>{x}, y, init, stg, lane);
 }
 
 }  // namespace csr

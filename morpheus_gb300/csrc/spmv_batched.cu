@@ -17,7 +17,7 @@
 // Tunables (CHUNK nonzeros per warp = 32 x lane range, SEG = entries staged
 // per lane per step, the "vector width" of the staging loads) form six
 // chunk-queue configurations, two of them (2 and 3) with double-buffered staging
-// (csr_rows_pipe).  Two more configurations give each CTA a whole
+// (PipeStage).  Two more configurations give each CTA a whole
 // matrix at a time (largest first): the CTA copies the matrix's x into
 // shared memory (up to 64 KB) with cp.async and its warps split the matrix
 // into nnz-balanced chunks, so the random x reads become shared-memory reads

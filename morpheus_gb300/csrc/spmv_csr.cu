@@ -29,7 +29,7 @@
 //    (4 x 64-byte pieces per instruction) into padded shared memory, so
 //    HBM reads stay sector-complete and shared-memory reads conflict-free.
 //    The multiply copies the next step's entries with cp.async while the lanes
-//    work on this one's (two buffers, csr_rows_pipe); the multiply with a fused
+//    work on this one's (two buffers, PipeStage); the multiply with a fused
 //    dot, and matrices of 2^31 - 256 rows and more, load and store them in turn
 //    (csr_chunk).  Row offsets of the chunk are staged too, so row-end tests
 //    never wait on global memory.
@@ -93,8 +93,8 @@ spmv_csr_segments(int64_t nrows, int64_t ncols, int64_t nnz, int64_t nchunks, in
 }
 
 // The same with double-buffered staging (no fused dot): 4 warps per CTA, 3 CTAs
-// per SM in FP64 and 4 in FP32 by shared memory.  Power-law matrix (2e6 rows):
-// FP64 206 -> 191 us, FP32 174 -> 161 us; y is bit-identical.
+// per SM in FP64 and 4 in FP32 by shared memory.  Power-law matrix (2e6 rows),
+// the multiply back to back: FP64 218 -> 190 us, FP32 175 -> 161; y is bit-identical.
 template <typename T>
 __global__ void __launch_bounds__(csr::PIPE_WARPS * 32, csr::PIPE_CTAS)
 spmv_csr_pipe(int64_t nrows, int64_t ncols, int64_t nchunks, int64_t chunk, const int32_t* __restrict__ ro,
@@ -106,7 +106,7 @@ spmv_csr_pipe(int64_t nrows, int64_t ncols, int64_t nchunks, int64_t chunk, cons
   for (int64_t wc = (int64_t)blockIdx.x * csr::PIPE_WARPS + w; wc < nchunks;
        wc += (int64_t)gridDim.x * csr::PIPE_WARPS) {
     const csr::RowRange rows = plan ? csr::planned_rows(wc, nrows, plan) : csr::chunk_rows(wc, chunk, nrows, ro, lane);
-    csr::csr_rows_pipe<T, csr::CSR_SEG, csr::XGlobal<T>, true, int32_t, csr::PIPE_RO>(
+    csr::csr_rows_x<T, csr::CSR_SEG, csr::XGlobal<T>, true, int32_t, csr::PIPE_RO>(
         rows, nrows, ncols, ro, ci, va, csr::XGlobal<T>{x}, y, init, stage[w], lane);
   }
 }
@@ -224,7 +224,11 @@ int launch_csr(const mgb_csr* A, const T* x, T* y, int init, void* stream, int v
 // 256) while the matrix would give fewer chunks than the GPU holds resident
 // warps and a chunk still spans at least 8 mean rows, so that small matrices
 // spread over every SM (chunks hold whole rows, so splitting matrices of long
-// rows finer only adds empty chunks).  The kernel runs nnz / chunk + 1
+// rows finer only adds empty chunks).  "Resident" is 24 warps per SM, the single
+// staging's; the pipelined kernel holds 12 (FP64) or 16, so it gets chunks for two
+// waves: power-law 120,000 / 500,000 / 1.4 M rows, single -> pipelined, FP64 37.8 ->
+// 29.7 / 73.9 -> 59.7 / 143.7 -> 139.3 us, FP32 27.6 -> 23.6 / 61.2 -> 51.3 / 125.5 ->
+// 117.7.  The kernel runs nnz / chunk + 1
 // chunks, so rows whose first entry is at nnz (trailing empty rows) always
 // belong to some chunk.
 int64_t segments_chunk(const mgb_csr* A) {
