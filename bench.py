@@ -21,6 +21,8 @@ Default (`--workload suite`): one run measures every benchmark configuration.
              this run by the library's peak kernels) and CPU baselines (the
              reference's Serial algorithm on one core and its OpenMP
              algorithm on every host core, both restated in oracle/).
+             The printed line keeps the microseconds; the whole goes to
+             standard error.
 
 One step = one y = A*x over the whole matrix; inputs are larger than L2
 except C1, which is timed with a 256 MB write between steps.
@@ -524,6 +526,41 @@ def spmv_entry(key, M, x_np, xt, steps, warmup, stream, unit_peaks, x_access, cp
     return out
 
 
+def _rounded(v):
+    """Floats to five significant digits, all the way down."""
+    if isinstance(v, dict):
+        return {k: _rounded(x) for k, x in v.items()}
+    return float(f"{v:.5g}") if isinstance(v, float) else v
+
+
+def short_line(line: dict) -> dict:
+    """The suite's line without the parts that make it longer than a caller's log keeps (3,000 characters): of the
+    rooflines and baselines the figures, of the per-config entries the microseconds."""
+    out = dict(line)
+    r = line["roofline"]
+    out["roofline"] = {k: r[k] for k in ("bound", "achieved", "peak", "unit", "frac", "traffic", "binding_unit",
+                                         "frac_of_binding_unit")}
+    c = line["csr_default"]
+    out["csr_default"] = {k: c[k] for k in ("us_per_spmv", "GB/s", "kernel")}
+    out["e2e"] = {k: v for k, v in line["e2e"].items() if k != "api"}
+    for k in ("unit_peaks", "selected_format_matches_reference_arm", "selector_switch_first_call_ms"):
+        out.pop(k, None)
+    if "cpu_baseline" in line:
+        out["cpu_baseline"] = {k: line["cpu_baseline"][k] for k in ("value", "unit", "cores")}
+    per = {}
+    for e in line.get("per_config", []):
+        for x in e.get("pairs", [e]):
+            for k, scale in (("us_per_spmv", 1), ("us", 1), ("us_per_batch", 1), ("ms_per_batch", 1e3), ("ms", 1e3)):
+                if k in x:
+                    per[x["config"].replace("stencil27_160", "st").replace("power_law_2e6", "pl")] = round(x[k] * scale, 1)
+                    break
+            if "learned" in x:
+                per[x["config"] + "_regret"] = round(x["learned"]["mean_regret"], 4)
+    out["per_config_us"] = per
+    out.pop("per_config", None)
+    return _rounded(out)
+
+
 def run_suite(args, rank: int, world: int, local_rank: int):
     import torch
 
@@ -724,7 +761,8 @@ def run_suite(args, rank: int, world: int, local_rank: int):
         per.extend(vector_entry(dev, stream, unit_peaks, ck))
     line["per_config"] = per
     line["suite_seconds"] = time.time() - t_start
-    print(json.dumps(line), flush=True)
+    print(json.dumps(line), file=sys.stderr, flush=True)
+    print(json.dumps(short_line(line)), flush=True)
     if world > 1:
         import torch.distributed as dist
         dist.barrier()

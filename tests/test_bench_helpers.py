@@ -67,3 +67,39 @@ def test_profile_traffic_reads_the_committed_summaries():
         t = bench.profile_traffic(key)
         assert t is not None and t[0] > 0, key
     assert np.isfinite(bench.profile_traffic("c5_batched_4096_csr_f64")[0])
+
+
+def test_the_printed_line_is_short_and_complete():
+    """A log that keeps 3,000 characters keeps the suite's line; its figures are those of the full one."""
+    import json
+    roof = bench.roofline({"format": 2, "nrows": 4_096_000, "ncols": 4_096_000, "ndiags": 27, "nnz": 109_215_352}, 8,
+                          192.123456789, {"hbm_gbs": 6679.8123456, "fp64_fma_per_s": 5.2512345e11}, "banded",
+                          (965300000.0, "profiles/spmv_dia_stencil27_f64.md " + "x" * 100))
+    cpu = {"value": 91.012345678, "unit": "GB/s", "cores": 72, "kind": "port", "sample": "y" * 200}
+    names = [f"c{k}_stencil27_160_offband_{k}_hdc_f64" for k in range(30)]
+    line = {"metric": bench.METRIC, "value": 4951.123456789, "unit": "GB/s", "n_gpus": 1, "steps": 50, "warmup": 5,
+            "ms_per_step": 0.192123456789, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
+            "dtype": "f64", "data": "synthetic " + "z" * 100, "selected_format": "DIA", "pct_hbm_peak": 72.123456789,
+            "config": bench.headline_config({"nrows": 4_096_000, "ncols": 4_096_000, "nnz": 109_215_352}, "dia", 1),
+            "selected_format_matches_reference_arm": True, "rel_err_vs_oracle": 1.23456789e-16, "roofline": roof,
+            "csr_default": {"us_per_spmv": 312.123456789, "GB/s": 4451.123456, "kernel": "row tiles",
+                            "rel_err_vs_oracle": 1e-16, "roofline": roof},
+            "speedup_vs_csr_default": 1.623456789, "selector_switch_ms": 1.5123456, "unit_peaks": roof,
+            "selector_switch_first_call_ms": 6.812345, "cpu_baseline": cpu, "suite_seconds": 100.123456,
+            "e2e": {"value": 200.123456789, "unit": "GB/s", "h2d_bytes_per_step": 917504108,
+                    "d2h_bytes_per_step": 32768000, "ms_per_step": 4.7123456, "api": "w" * 90},
+            "gpu_launches": 50, "clocks": {"sm_mhz": 2070.0, "sm_max_mhz": 2070.0, "reasons": ["sw_power_cap"],
+                                           "samples": 40},
+            "per_config": [{"config": n, "us_per_spmv": 100.123456 + i, "roofline": roof} for i, n in enumerate(names)]
+            + [{"config": "convert", "pairs": [{"config": "convert_x_coo_to_dia", "ms": 1.0123456}]},
+               {"config": "c4_selector_heldout", "learned": {"mean_regret": 0.0531234}}]}
+    short = bench.short_line(line)
+    assert len(json.dumps(short)) < 2900
+    for key in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+                "vs_baseline", "dtype", "data", "config", "e2e", "gpu_launches", "clocks", "roofline"):
+        assert key in short, key
+    assert short["value"] == pytest.approx(line["value"], rel=1e-4)
+    assert short["config"] == line["config"] and short["e2e"]["h2d_bytes_per_step"] == 917504108
+    assert short["per_config_us"]["convert_x_coo_to_dia"] == pytest.approx(1012.3, rel=1e-3)
+    assert short["per_config_us"]["c4_selector_heldout_regret"] == pytest.approx(0.0531, abs=1e-4)
+    assert len(short["per_config_us"]) == 32
