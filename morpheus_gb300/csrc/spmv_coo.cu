@@ -181,7 +181,7 @@ spmv_coo_segments(int64_t nrows, int64_t ncols, int64_t nnz, int64_t chunk, cons
     if (hrow >= 0) finalize(hrow, (lane > 0 && kprev == hrow) ? hval + vprev : hval);
     // rows after the last entry of the matrix (init): whole warp fills
     if (init && k == nchunks - 1)
-      for (IDX g = max(last_row + 1, (IDX)0) + lane; g < nrows; g += 32) y[g] = T(0);
+      for (int64_t g = max((int64_t)last_row + 1, (int64_t)0) + lane; g < nrows; g += 32) y[g] = T(0);
   }
 }
 

@@ -97,3 +97,18 @@ def test_csr_beyond_2_30_rows(cuda, planned, dtype):
         _lib.call(name, C.byref(desc), x.data_ptr(), y.data_ptr(), 1, None)
     torch.cuda.synchronize()
     assert torch.equal(y, want)
+
+
+def test_coo_of_2_31_rows(cuda):
+    """The largest number of rows (2^31 - 1), an entry in every 65,536: rows are zero-filled up to the last one."""
+    if torch.cuda.get_device_properties(0).total_memory < 80 * 2**30:
+        pytest.skip("needs a GPU with >= 80 GB")
+    dev, rows = torch.device("cuda"), (1 << 31) - 1
+    ri = torch.arange(0, rows, 65536, device=dev, dtype=torch.int64)
+    A = mgb.CooMatrix(rows, 3, ri.numel(), ri.int(), torch.ones_like(ri).int(),
+                      torch.full((ri.numel(),), 2.0, dtype=torch.float32, device=dev), dtype=torch.float32)
+    x = torch.tensor([0.0, 3.0, 0.0], device=dev)
+    y = torch.full((rows,), 7.0, dtype=torch.float32, device=dev)
+    mgb.multiply(A, x, y)
+    torch.cuda.synchronize()
+    assert torch.all(y[ri] == 6.0) and int(torch.count_nonzero(y)) == ri.numel()
