@@ -8,7 +8,7 @@
 // Serial multiply (impl/Coo/Serial/Morpheus_Multiply_Impl.hpp:38-59):
 // y = 0 if init, then y[I[n]] += V[n] * x[J[n]].
 //
-// Design: fixed chunks of up to COO_CHUNK consecutive entries, one warp each, cut
+// Design: fixed chunks of 256 or 512 consecutive entries, one warp each, cut
 // into 32 contiguous lane ranges (the lane-segment scheme of spmv_csr.cu, so
 // every FP64 FMA is issued by all 32 lanes).  Row indices, columns and values
 // are copied into padded shared memory a step ahead (cp.async, two buffers); a lane
@@ -26,27 +26,22 @@ namespace {
 
 constexpr int COO_WARPS = 4;
 constexpr int COO_CTAS = 5;                 // register budget per SM (shared memory allows 2 to 4)
-constexpr int64_t COO_CHUNK = 2048;         // entries per warp chunk at most
+constexpr int64_t COO_CHUNK = 2048;         // entries per warp chunk at most (allocation-free calls)
 
-// Entries per chunk.  FP64: 256 below COO_SHORT (steps of four entries, 16 warps
-// per SM), 512 from there on.  Larger chunks leave the last wave nearly empty at
-// some sizes; smaller ones pay carries.  Power-law COO of 350,000 / 700,000 / 1.0 M
-// / 1.6 M rows (5.3 to 24 M entries), us at 256: 43.1 / 77.8 / 101.5 / 153.5, 512: 45.1
-// / 80.2 / 107.1 / 160.2, 1024: 50.9 / 88.7, 2048: 51.8 / 90.0.  From COO_SHORT on (steps
-// of eight), 2.0 M rows and 27-point stencils on 100^3 and 160^3: 256: 231 / 189 / 758,
-// 512: 209 / 145 / 554, 1024: 220 / 160, 2048: 214 / 166 / 607.
-// FP32: 2048, halved (down to 256) while there are fewer than three chunks per
-// resident warp (16 per SM).  350,000 / 700,000 rows, us at two -> three: 43.1 -> 39.1 /
-// 76.8 -> 77.3; COO part of the HYB of 1.5 / 2.0 M rows with its ELL part: 159.1 ->
-// 157.9 / 212.5 -> 205.1; five: 160 / 205.
+// Entries per chunk: 512, and 256 where FP64 takes steps of four entries (below
+// COO_SHORT).  Larger chunks leave the last wave nearly empty at some sizes;
+// smaller ones pay carries.  us:
+//   FP64, power-law COO of 5.3 M entries, 10.6 M, 15 M, 24 M:
+//     256: 43.1, 77.8, 101.5, 153.5   512: 45.1, 80.2, 107.1, 160.2   1024: 50.9, 88.7   2048: 51.8, 90.0
+//   from COO_SHORT on (steps of eight), power-law of 30 M, 27-point stencils of 26 M and 109 M:
+//     256: 231, 189, 758   512: 209, 145, 554   1024: 220, 160   2048: 214, 166, 607
+//   FP32, power-law of 3 M, 10.6 M, 21 M, 30 M, 27-point stencils of 26 M and 109 M:
+//     256: 29.5, 72.5, 131.2, 181.7, 126.8, 489.8   512: 26.6, 70.8, 127.9, 176.2, 106.5, 389.2
+//     1024 or 2048: 29.6, 77.4, 139.6, 186.6, 134.7, 472.0   (single staging 28.9, 81.0, 136.0, 199.1, 131.5, 552.5)
 constexpr int64_t COO_SHORT = 24 << 20;
 template <typename T>
 inline int64_t coo_chunk_size(int64_t nnz) {
-  if (sizeof(T) == 8) return nnz < COO_SHORT ? 256 : 512;
-  int64_t chunk = COO_CHUNK;
-  const int64_t enough = (int64_t)num_sms() * 48;
-  while (chunk > 256 && nnz / chunk < enough) chunk >>= 1;
-  return chunk;
+  return sizeof(T) == 8 && nnz < COO_SHORT ? 256 : 512;
 }
 
 template <typename T>

@@ -174,7 +174,12 @@ int launch_ell_rows(const mgb_ell* A, const T* x, T* y, int init, cudaStream_t s
 // FP32: one row per thread everywhere (8 CTAs per SM).  FP64: pairs, except
 // mostly-padding slabs of more rows than threads fit the GPU, where four rows
 // per thread (two where the pitch is not a multiple of 4) read the padding's
-// indices in the fewest instructions.
+// indices in the fewest instructions.  At that line (311,296 rows on 152 SMs) and
+// above, four / pairs: 5-point 324,900 rows 24.6 / 25.5, 518,400 25.9 / 36.4, 722,500
+// 28.7 / 47.1; 9-point 518,400 28.6 / 36.9; HYB part 320,000 82 / 76, 500,000 94 / 91,
+// 600,000 98 / 110, 850,000 165 / 142, 1,200,000 184 / 191.  Between 0.3 and 0.5 M rows the
+// two are within what the arrays' place in memory makes of it (21 to 25 us for the
+// same slab of 324,900 rows).
 template <typename T>
 int launch_ell(const mgb_ell* A, const T* x, T* y, int init, cudaStream_t s) {
   MGB_REQUIRE(A != nullptr, MGB_ERR_BAD_ARGUMENT);

@@ -192,7 +192,10 @@ __global__ void __launch_bounds__(1024) sum_partials(int n, const T* __restrict_
 // Short vectors: one cluster of SMALL_CTAS CTAs reduces them and writes the
 // result, in one launch and without scratch (two kernels and an allocation
 // otherwise; latency is all there is).  The CTAs' sums meet in the first one's
-// shared memory, in a fixed order.
+// shared memory, in a fixed order.  The line is where eight SMs stop being enough
+// (dot, waxpby and reduce in turn, us, one cluster / the whole GPU, n = 65,536, 131,072,
+// 262,144, 1,048,576: FP64 68 / 81, 73 / 81, 82 / 80, 135 / 88; FP32 62 / 77, 62 / 77, 64 / 76,
+// 70 / 77).
 constexpr int SMALL_CTAS = 8;
 constexpr int SMALL_THREADS = 512;
 constexpr int64_t SMALL_N = 1 << 17;
