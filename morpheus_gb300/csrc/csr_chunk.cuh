@@ -153,7 +153,9 @@ __device__ __forceinline__ RowRange csr_rows_x(RowRange rows, int64_t nrows, int
       for (IDX r = r_begin + lane; r < r_end; r += 32) y[r] = T(0);
     return RowRange{r_begin, r_end};
   }
-  const IDX A0 = E0 & ~(IDX)7;  // 32-byte aligned column segments
+  // column segments aligned to a step, 32 bytes at most: lane 0's range reaches past E0 (it flushes the leading
+  // empty rows), however few entries the chunk has
+  const IDX A0 = E0 & ~(IDX)((SEG < 8 ? SEG : 8) - 1);
   IDX KW = (E1 - A0 + 31) / 32;
   KW = (KW + SEG - 1) / SEG * SEG;
   const IDX la = A0 + lane * KW;

@@ -145,3 +145,20 @@ def test_float32(cuda):
             np.abs(x.cpu().numpy().astype(np.float64)))
         err = np.linalg.norm(y.cpu().numpy() - ref) / max(np.linalg.norm(scale), 1e-300)
         assert err <= 1e-5
+
+
+# a last chunk of few entries that starts with empty rows, at an entry that is no multiple of eight
+@pytest.mark.parametrize("init", [True, False])
+@pytest.mark.parametrize("config", range(11))
+def test_short_last_chunk(cuda, config, init):
+    mats = [gen.random_lengths_csr(18, 6000, np.array([first] + [0] * 5 + [3] * 10 + [0] * 2), seed=first)
+            for first in (516, 1028, 1031, 2052, 4100)]
+    dev = [mgb.matrix_from_host(m) for m in mats]
+    xs = [torch.from_numpy(gen.x_vector(6000, seed=i)).cuda() for i in range(len(mats))]
+    ys = [torch.full((18,), 7.0, dtype=torch.float64, device="cuda") for _ in mats]
+    y0s = [y.cpu().numpy() for y in ys]
+    b = batched.CsrBatch(dev, xs, ys)
+    b.plan(config)
+    b.multiply(init=init)
+    torch.cuda.synchronize()
+    check(mats, xs, ys, y0s, init, 1e-12)
