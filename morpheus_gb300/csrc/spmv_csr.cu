@@ -52,11 +52,12 @@ constexpr int CSR_WARPS = 8;  // warps per CTA
 // partials[blockIdx.x] (the fused step of an iterative solver; the matrix is
 // square there; the launcher caps the grid at the resident CTAs).  With a
 // chunk plan the warps read their rows from it instead of searching the row
-// offsets.  Only these fused multiplies and matrices too tall for the pipelined
-// kernel come here.  SMALL: 32-bit indices in the chunk routine, 256 staged row
-// offsets and 4 CTAs per SM (64 registers) -- faster for FP32 (power-law
-// 183 -> 164 us) and slower for FP64 (195 -> 206 us), so FP32 only.
-template <typename T, bool DOT, bool SMALL = false>
+// offsets.  These fused multiplies, FP32 multiplies of short rows without a plan and
+// matrices too tall for the pipelined kernel come here.  SMALL: 32-bit indices in the
+// chunk routine, 256 staged row offsets and 4 CTAs per SM (64 registers) -- faster for
+// FP32 (power-law 183 -> 164 us) and slower for FP64 (195 -> 206 us), so FP32 only.
+// SEG: one for a matrix with and without a plan or a dot, so that y is bit-identical.
+template <typename T, bool DOT, bool SMALL, int SEG>
 __global__ void __launch_bounds__(CSR_WARPS * 32, SMALL ? 4 : 3)
 spmv_csr_segments(int64_t nrows, int64_t ncols, int64_t nnz, int64_t nchunks, int64_t chunk,
                   const int32_t* __restrict__ ro, const int32_t* __restrict__ ci,
@@ -64,14 +65,14 @@ spmv_csr_segments(int64_t nrows, int64_t ncols, int64_t nnz, int64_t nchunks, in
                   T* __restrict__ y, int init, T* __restrict__ partials, const int32_t* __restrict__ plan) {
   constexpr int RO = SMALL ? 256 : csr::CSR_RO_STAGE;
   using IDX = typename std::conditional<SMALL, int32_t, int64_t>::type;
-  __shared__ csr::WarpStage<T, csr::CSR_SEG, RO> stage[CSR_WARPS];
+  __shared__ csr::WarpStage<T, SEG, RO> stage[CSR_WARPS];
   const int lane = threadIdx.x & 31;
   const int w = threadIdx.x >> 5;
   T part = T(0);
   for (int64_t wc = (int64_t)blockIdx.x * CSR_WARPS + w; wc < nchunks;
        wc += (int64_t)gridDim.x * CSR_WARPS) {
     const csr::RowRange rows = plan ? csr::planned_rows(wc, nrows, plan) : csr::chunk_rows(wc, chunk, nrows, ro, lane);
-    const csr::RowRange rr = csr::csr_rows_x<T, csr::CSR_SEG, csr::XGlobal<T>, true, IDX>(
+    const csr::RowRange rr = csr::csr_rows_x<T, SEG, csr::XGlobal<T>, true, IDX, RO>(
         rows, nrows, ncols, ro, ci, va, csr::XGlobal<T>{x}, y, init, stage[w], lane);
     if (DOT) {
       __syncwarp();  // the chunk's y entries, written by any lane, are visible to the warp
@@ -94,19 +95,20 @@ spmv_csr_segments(int64_t nrows, int64_t ncols, int64_t nnz, int64_t nchunks, in
 
 // The same with double-buffered staging (no fused dot): 4 warps per CTA, 3 CTAs
 // per SM in FP64 and 4 in FP32 by shared memory.  Power-law matrix (2e6 rows),
-// the multiply back to back: FP64 218 -> 190 us, FP32 175 -> 161; y is bit-identical.
-template <typename T>
+// the multiply back to back: FP64 218 -> 190 us, FP32 175 -> 161.
+// SEG: entries staged per lane and step; the rule is at segments_short.
+template <typename T, int SEG>
 __global__ void __launch_bounds__(csr::PIPE_WARPS * 32, csr::PIPE_CTAS)
 spmv_csr_pipe(int64_t nrows, int64_t ncols, int64_t nchunks, int64_t chunk, const int32_t* __restrict__ ro,
               const int32_t* __restrict__ ci, const T* __restrict__ va, const T* __restrict__ x, T* __restrict__ y,
               int init, const int32_t* __restrict__ plan) {
-  __shared__ csr::PipeStage<T, csr::CSR_SEG, csr::PIPE_RO> stage[csr::PIPE_WARPS];
+  __shared__ csr::PipeStage<T, SEG, csr::PIPE_RO> stage[csr::PIPE_WARPS];
   const int lane = threadIdx.x & 31;
   const int w = threadIdx.x >> 5;
   for (int64_t wc = (int64_t)blockIdx.x * csr::PIPE_WARPS + w; wc < nchunks;
        wc += (int64_t)gridDim.x * csr::PIPE_WARPS) {
     const csr::RowRange rows = plan ? csr::planned_rows(wc, nrows, plan) : csr::chunk_rows(wc, chunk, nrows, ro, lane);
-    csr::csr_rows_x<T, csr::CSR_SEG, csr::XGlobal<T>, true, int32_t, csr::PIPE_RO>(
+    csr::csr_rows_x<T, SEG, csr::XGlobal<T>, true, int32_t, csr::PIPE_RO>(
         rows, nrows, ncols, ro, ci, va, csr::XGlobal<T>{x}, y, init, stage[w], lane);
   }
 }
@@ -220,7 +222,37 @@ int launch_csr(const mgb_csr* A, const T* x, T* y, int init, void* stream, int v
 
 }  // namespace
 
-// Chunk size of the lane-segment kernel: 2048 nonzeros, halved (down to
+// Rows of up to 8.5 entries on average: row ends, not x reads, are what the lanes
+// wait for, and more warps with smaller buffers (steps of four entries, 16 warps per
+// SM in FP64) and chunks of 512 beat steps of eight and chunks of 2048.  us, single
+// staging / steps of eight / steps of four with chunks of 512 (3 to 4 million rows):
+//                         FP64                    FP32
+//   band of 5        129 / 148 / 107        107 / 119 /  74
+//   band of 7        162 / 180 / 140        124 / 139 / 103
+//   band of 9        186 / 175 / 169        121 / 119 / 129
+//   random, 5        128 / 145 / 118        117 / 129 /  87
+//   random, 0 to 8   126 / 135 / 102        117 /  97 /  79
+//   random, 0 to 16  172 / 189 / 171        159 / 158 / 131
+//   power law (mean 15, 1.4 and 2 million rows)
+//                    144 / 139 / 147        125 / 118 / 117
+//                    206 / 187 / 204        175 / 161 / 160
+// With the dot (single staging, eight and 2048 / four and 512): band of 5 158 / 164
+// and 125 / 102, random 5 161 / 153 and 130 / 113, random 0 to 16 210 / 230 and
+// 175 / 171; it takes what the multiply takes, whose y is bit-identical.
+bool segments_short(const mgb_csr* A) { return 2 * A->nnz < 17 * A->nrows; }
+
+// A FP32 multiply without a plan searches every chunk's rows, which the 32 warps per
+// SM of the single staging hide better than the 16 of the double buffer up to this
+// mean row.  us, double / single: band of 5 96 / 91, of 8 59 / 52, of 10 60 / 55,
+// of 13 82 / 74, random 5 105 / 103, 9 66 / 58, 0 to 18 95 / 90; power law (mean 15)
+// and random 15 as fast by either.  FP64 (24 warps against 16): the double buffer,
+// band of 5 130 / 149, random 0 to 16 190 / 203, 5 132 / 131.
+template <typename T>
+bool plain_single(const mgb_csr* A) {
+  return sizeof(T) == 4 && A->nnz < 14 * A->nrows;
+}
+
+// Chunk size of the lane-segment kernel: 2048 nonzeros (512 for short rows), halved (down to
 // 256) while the matrix would give fewer chunks than the GPU holds resident
 // warps and a chunk still spans at least 8 mean rows, so that small matrices
 // spread over every SM (chunks hold whole rows, so splitting matrices of long
@@ -232,7 +264,7 @@ int launch_csr(const mgb_csr* A, const T* x, T* y, int init, void* stream, int v
 // chunks, so rows whose first entry is at nnz (trailing empty rows) always
 // belong to some chunk.
 int64_t segments_chunk(const mgb_csr* A) {
-  int64_t chunk = csr::CSR_CHUNK;
+  int64_t chunk = segments_short(A) ? 512 : csr::CSR_CHUNK;
   const int64_t resident = (int64_t)num_sms() * CSR_WARPS * 3;
   const int64_t mean_row = A->nnz / (A->nrows > 0 ? A->nrows : 1);
   while (chunk > 256 && A->nnz / chunk < resident && chunk / 2 >= 8 * mean_row) chunk >>= 1;
@@ -249,6 +281,20 @@ int make_plan(const mgb_csr* A, int32_t* plan, int64_t entries, cudaStream_t s) 
   MGB_REQUIRE(entries == nchunks + 1, MGB_ERR_BAD_ARGUMENT);
   csr_chunk_plan<<<prim::blocks_for(A->nrows + 1, 256), 256, 0, s>>>(A->nrows, nchunks, chunk, A->row_offsets,
                                                                       plan);
+  MGB_LAUNCH_CHECK();
+  return MGB_SUCCESS;
+}
+
+template <typename T, int SEG>
+int launch_pipe(const mgb_csr* A, int64_t nchunks, int64_t chunk, const T* x, T* y, int init, const int32_t* plan,
+                cudaStream_t s) {
+  static std::atomic<bool> carved[64];
+  if (int st = csr::set_carveout_once(spmv_csr_pipe<T, SEG>, carved, csr::PIPE_CARVEOUT)) return st;
+  int64_t blocks = (nchunks + csr::PIPE_WARPS - 1) / csr::PIPE_WARPS;
+  if (blocks > 0x7fffffffLL) blocks = 0x7fffffffLL;
+  spmv_csr_pipe<T, SEG><<<(unsigned)blocks, csr::PIPE_WARPS * 32, 0, s>>>(
+      A->nrows, A->ncols, nchunks, chunk, A->row_offsets, A->column_indices, static_cast<const T*>(A->values), x, y,
+      init, plan);
   MGB_LAUNCH_CHECK();
   return MGB_SUCCESS;
 }
@@ -282,29 +328,30 @@ int launch_csr_dot(const mgb_csr* A, const T* x, T* y, int init, void* stream, i
   if (npartials && !partials) return take_device_query_error();
   const T* va = static_cast<const T*>(A->values);
   const cudaStream_t s = as_stream(stream);
-  if (!partials && A->nrows < 0x7fffff00LL) {
-    static std::atomic<bool> carved[64];
-    if (int st = csr::set_carveout_once(spmv_csr_pipe<T>, carved, csr::PIPE_CARVEOUT)) return st;
-    blocks = (nchunks + csr::PIPE_WARPS - 1) / csr::PIPE_WARPS;
-    if (blocks > 0x7fffffffLL) blocks = 0x7fffffffLL;
-    spmv_csr_pipe<T><<<(unsigned)blocks, csr::PIPE_WARPS * 32, 0, s>>>(A->nrows, A->ncols, nchunks, chunk,
-                                                                       A->row_offsets, A->column_indices, va, x, y,
-                                                                       init, plan);
-    MGB_LAUNCH_CHECK();
-    return MGB_SUCCESS;
+  const bool short_rows = segments_short(A);
+  const bool single = partials || A->nrows >= 0x7fffff00LL || (plan == nullptr && plain_single<T>(A));
+  if (!single) {
+    return short_rows ? launch_pipe<T, 4>(A, nchunks, chunk, x, y, init, plan, s)
+                      : launch_pipe<T, csr::CSR_SEG>(A, nchunks, chunk, x, y, init, plan, s);
   }
-  if (small && partials)
-    spmv_csr_segments<T, true, true><<<(unsigned)blocks, CSR_WARPS * 32, 0, s>>>(
-        A->nrows, A->ncols, A->nnz, nchunks, chunk, A->row_offsets, A->column_indices, va, x, y, init, partials,
-        plan);
-  else if (partials)
-    spmv_csr_segments<T, true><<<(unsigned)blocks, CSR_WARPS * 32, 0, s>>>(
-        A->nrows, A->ncols, A->nnz, nchunks, chunk, A->row_offsets, A->column_indices, va, x, y, init, partials,
-        plan);
-  else
-    spmv_csr_segments<T, false><<<(unsigned)blocks, CSR_WARPS * 32, 0, s>>>(
-        A->nrows, A->ncols, A->nnz, nchunks, chunk, A->row_offsets, A->column_indices, va, x, y, init, nullptr,
-        plan);
+  const auto run = [&](auto kernel) {
+    kernel<<<(unsigned)blocks, CSR_WARPS * 32, 0, s>>>(A->nrows, A->ncols, A->nnz, nchunks, chunk, A->row_offsets,
+                                                       A->column_indices, va, x, y, init, partials, plan);
+  };
+  constexpr bool F32 = sizeof(T) == 4;
+  if (partials && small) {
+    if (short_rows) run(spmv_csr_segments<T, true, F32, 4>);
+    else run(spmv_csr_segments<T, true, F32, csr::CSR_SEG>);
+  } else if (partials) {
+    if (short_rows) run(spmv_csr_segments<T, true, false, 4>);
+    else run(spmv_csr_segments<T, true, false, csr::CSR_SEG>);
+  } else if (small) {
+    if (short_rows) run(spmv_csr_segments<T, false, F32, 4>);
+    else run(spmv_csr_segments<T, false, F32, csr::CSR_SEG>);
+  } else {
+    if (short_rows) run(spmv_csr_segments<T, false, false, 4>);
+    else run(spmv_csr_segments<T, false, false, csr::CSR_SEG>);
+  }
   MGB_LAUNCH_CHECK();
   return MGB_SUCCESS;
 }

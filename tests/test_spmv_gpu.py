@@ -573,3 +573,27 @@ def test_coo_chunk_limits(cuda, nnz):
         _lib.call(name, C.byref(desc), x.data_ptr(), y.data_ptr(), 1, None)
         torch.cuda.synchronize()
         assert torch.equal(y, want), name
+
+
+# rows short on average: chunks that start with empty rows at an entry that is no multiple of eight, with few entries
+# behind; around the mean lengths (8.5, and 14 in FP32 without a plan) at
+# which the kernel or its steps change; with and without a plan
+@pytest.mark.parametrize("init", [True, False])
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("lens", [[260] + [0] * 60 + [3] * 10, [263] + [0] * 90 + [1] * 5 + [0] * 3, [516] + [0] * 100 + [2] * 7,
+                                  [9, 8, 7, 8] * 500, [9, 9, 8, 10] * 500, [13, 14, 14, 14] * 500, [14] * 1501, [5] * 4001, [0, 1, 2, 13] * 700, [40] + [0] * 9])
+def test_segments_of_short_rows(cuda, lens, dtype, init):
+    A = gen.random_lengths_csr(len(lens), 700, np.asarray(lens), seed=len(lens), dtype=dtype)
+    M = mgb.matrix_from_host(A)
+    M._variant = mgb.CSR_SEGMENTS
+    x, y0 = gen.x_vector(700, seed=3, dtype=dtype), gen.x_vector(len(lens), seed=4, dtype=dtype)
+    y = torch.from_numpy(y0.copy()).cuda()
+    mgb.multiply(M, torch.from_numpy(x).cuda(), y, init=init)
+    y2 = torch.from_numpy(y0.copy()).cuda()
+    _unplanned_segments(M, torch.from_numpy(x).cuda(), y2, init)
+    assert torch.equal(y, y2)
+    rows = np.repeat(np.arange(len(lens)), lens)
+    prod = A["values"].astype(np.float64) * x.astype(np.float64)[A["column_indices"]]
+    want = np.bincount(rows, weights=prod, minlength=len(lens)) + (0.0 if init else y0.astype(np.float64))
+    size = np.bincount(rows, weights=np.abs(prod), minlength=len(lens)) + np.abs(y0)
+    assert np.all(np.abs(y.cpu().numpy() - want) <= (max(lens) + 32) * np.finfo(dtype).eps * size)
